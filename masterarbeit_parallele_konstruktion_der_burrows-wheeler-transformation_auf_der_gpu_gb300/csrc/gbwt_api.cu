@@ -86,7 +86,7 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
         if ((int64_t)z > so->capacity) return GBWT_BAD_PARAMETER;
         std::vector<uint32_t> h(z);
         check_cuda(cudaMemcpyAsync(h.data(), D, (size_t)z * 4, cudaMemcpyDeviceToHost, st->stream));
-        check_cuda(cudaStreamSynchronize(st->stream));
+        sync_stream(st);
         for (uint32_t i = 0; i < z; i++) so->D[i] = h[i];
         st->stats.kernel_launches = st->launches;
         return z;
@@ -121,7 +121,7 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
             h2.resize(z);
             check_cuda(cudaMemcpyAsync(h2.data(), pord.sa, (size_t)z * 4, cudaMemcpyDeviceToHost, st->stream));
         }
-        check_cuda(cudaStreamSynchronize(st->stream));
+        sync_stream(st);
         for (uint32_t i = 0; i < z; i++) so->ranks[i] = (int32_t)h[i];
         if (so->parse_sa)
             for (uint32_t i = 0; i < z; i++) so->parse_sa[i] = (int32_t)h2[i];
@@ -134,7 +134,7 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
     if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     uint32_t hflags[4];
     memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
     if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
@@ -155,18 +155,23 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
     return n;
 }
 
+// Runs f and turns what it throws into a return code.  A call that failed
+// half-way leaves no work queued: the next one may use another stream.
 template <typename F>
-static int64_t guarded(F f)
+static int64_t guarded(Storage *st, F f)
 {
+    int64_t rc;
     try {
         return f();
     } catch (const Error &e) {
-        return e.code;
+        rc = e.code;
     } catch (const std::bad_alloc &) {
-        return GBWT_NOT_ENOUGH_MEMORY;
+        rc = GBWT_NOT_ENOUGH_MEMORY;
     } catch (...) {
-        return GBWT_INTERNAL_ERROR;
+        rc = GBWT_INTERNAL_ERROR;
     }
+    if (st->stream) cudaStreamSynchronize(st->stream);
+    return rc;
 }
 
 }  // namespace gbwt
@@ -179,7 +184,7 @@ extern "C" int64_t gbwt_allocate_device_storage(void **storage, int64_t max_leng
     *storage = nullptr;
     Storage *st = new (std::nothrow) Storage();
     if (!st) return GBWT_NOT_ENOUGH_MEMORY;
-    int64_t rc = guarded([&]() -> int64_t {
+    int64_t rc = guarded(st, [&]() -> int64_t {
         check_cuda(cudaGetDevice(&st->device));
         int major = 0, minor = 0;
         check_cuda(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, st->device));
@@ -191,6 +196,9 @@ extern "C" int64_t gbwt_allocate_device_storage(void **storage, int64_t max_leng
         check_cuda(cudaMalloc(&st->d_flags, 64 * sizeof(uint32_t)));
         check_cuda(cudaMalloc(&st->d_scalars, 64 * sizeof(uint64_t)));
         check_cuda(cudaHostAlloc(&st->h_scalars, 256 * sizeof(uint64_t), cudaHostAllocDefault));
+        st->h_err = (uint32_t *)(st->h_scalars + 255);
+        *st->h_err = 0;
+        check_cuda(cudaMemsetAsync(st->d_scalars, 0, 64 * sizeof(uint64_t), st->stream));   // look-back ticket
         for (int i = 0; i < 10; i++) check_cuda(cudaEventCreate(&st->ev[i]));
         st->max_length = max_length;
         if (max_length > 0) {
@@ -244,7 +252,7 @@ extern "C" int64_t gbwt_pfp_bwt(void *storage, const uint8_t *T, uint8_t *L, int
 {
     Storage *st = (Storage *)storage;
     if (!st) return GBWT_BAD_PARAMETER;
-    return guarded([&]() { return pipeline(st, T, L, n, W, P, flags, UPTO_BWT, nullptr); });
+    return guarded(st, [&]() { return pipeline(st, T, L, n, W, P, flags, UPTO_BWT, nullptr); });
 }
 
 // Inverse BWT: the PFP output convention (primary = gbwt_stats.primary_index)
@@ -281,7 +289,7 @@ static int64_t unbwt_common(Storage *st, const uint8_t *L, uint8_t *T, int64_t n
     run_unbwt(st, dLc, un, pfp ? (uint32_t)primary + 1u : (uint32_t)primary, dT);
     if (!devptr) check_cuda(cudaMemcpyAsync(T, dT, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     if ((uint32_t)st->h_scalars[8] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
     st->stats.kernel_launches = st->launches;
     return n;
@@ -291,7 +299,7 @@ extern "C" int64_t gbwt_unbwt(void *storage, const uint8_t *L, uint8_t *T, int64
 {
     Storage *st = (Storage *)storage;
     if (!st) return GBWT_BAD_PARAMETER;
-    return guarded([&]() {
+    return guarded(st, [&]() {
         return unbwt_common(st, L, T, n, primary, true, (flags & GBWT_FLAG_DEVICE_POINTERS) != 0);
     });
 }
@@ -302,7 +310,7 @@ extern "C" int64_t gbwt_libcubwt_unbwt(void *storage, const uint8_t *T, uint8_t 
     (void)freq;       // recomputed on the device
     Storage *st = (Storage *)storage;
     if (!st) return GBWT_BAD_PARAMETER;
-    return guarded([&]() -> int64_t {
+    return guarded(st, [&]() -> int64_t {
         const int64_t rc = unbwt_common(st, T, U, n, i, false, false);
         return rc < 0 ? rc : GBWT_NO_ERROR;
     });
@@ -313,7 +321,7 @@ extern "C" int64_t gbwt_pfp_bwt_batch(void *storage, const uint8_t *T_concat, co
 {
     Storage *st = (Storage *)storage;
     if (!st) return GBWT_BAD_PARAMETER;
-    return guarded([&]() { return run_batch(st, T_concat, offsets, k, L_concat, W, P, flags, MAX_N); });
+    return guarded(st, [&]() { return run_batch(st, T_concat, offsets, k, L_concat, W, P, flags, MAX_N); });
 }
 
 extern "C" int64_t gbwt_pfp_trigger_scan(void *storage, const uint8_t *T, int64_t n, int32_t W, int32_t P,
@@ -325,7 +333,7 @@ extern "C" int64_t gbwt_pfp_trigger_scan(void *storage, const uint8_t *T, int64_
     so.D = D;
     so.capacity = capacity;
     if (n == 0) return 0;
-    return guarded([&]() { return pipeline(st, T, nullptr, n, W, P, flags & ~GBWT_FLAG_STAGE_TIMES, UPTO_SCAN, &so); });
+    return guarded(st, [&]() { return pipeline(st, T, nullptr, n, W, P, flags & ~GBWT_FLAG_STAGE_TIMES, UPTO_SCAN, &so); });
 }
 
 extern "C" int64_t gbwt_pfp_parse(void *storage, const uint8_t *T, int64_t n, int32_t W, int32_t P, uint32_t flags,
@@ -338,14 +346,14 @@ extern "C" int64_t gbwt_pfp_parse(void *storage, const uint8_t *T, int64_t n, in
     so.parse_sa = parse_sa;
     so.capacity = capacity;
     if (n == 0) return 0;
-    return guarded([&]() { return pipeline(st, T, nullptr, n, W, P, flags & ~GBWT_FLAG_STAGE_TIMES, UPTO_PARSE, &so); });
+    return guarded(st, [&]() { return pipeline(st, T, nullptr, n, W, P, flags & ~GBWT_FLAG_STAGE_TIMES, UPTO_PARSE, &so); });
 }
 
 extern "C" int64_t gbwt_set_kernel_probe(void *storage, int32_t kernel)
 {
     Storage *st = (Storage *)storage;
     if (!st || kernel < -1 || kernel > GBWT_PROBE_SEG_SORT) return GBWT_BAD_PARAMETER;
-    return guarded([&]() -> int64_t {
+    return guarded(st, [&]() -> int64_t {
         if (kernel >= 0 && !st->probe_ev) {
             const int cap = 1024;
             st->probe_ev = (cudaEvent_t *)calloc(2 * cap, sizeof(cudaEvent_t));
@@ -353,7 +361,7 @@ extern "C" int64_t gbwt_set_kernel_probe(void *storage, int32_t kernel)
             for (int i = 0; i < 2 * cap; i++) check_cuda(cudaEventCreate(&st->probe_ev[i]));
             st->probe_cap = cap;
         }
-        check_cuda(cudaStreamSynchronize(st->stream));
+        sync_stream(st);
         st->probe_kernel = kernel;
         st->probe_used = 0;
         st->probe_launches = 0;
@@ -420,7 +428,7 @@ static int64_t libcubwt_bwt(Storage *st, const uint8_t *T, uint8_t *L, int64_t n
     uint32_t present[8];
     check_cuda(cudaMemcpyAsync(st->h_scalars + 4, st->d_flags + 8, sizeof(present), cudaMemcpyDeviceToHost,
                                st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     memcpy(present, st->h_scalars + 4, sizeof(present));
     uint8_t *hmap = (uint8_t *)(st->h_scalars + 16);           // 256 pinned bytes each
     uint8_t *hunmap = (uint8_t *)(st->h_scalars + 48);
@@ -467,14 +475,14 @@ static int64_t libcubwt_bwt(Storage *st, const uint8_t *T, uint8_t *L, int64_t n
         int64_t rc = run_batch(st, dT, offs, 1, dO, 5, 16, GBWT_FLAG_DEVICE_POINTERS, MAX_N, &aux);
         if (rc < 0) return rc;
         check_cuda(cudaMemcpyAsync(I, dI, ni * 4, cudaMemcpyDeviceToHost, st->stream));
-        check_cuda(cudaStreamSynchronize(st->stream));
+        sync_stream(st);
         pidx = I[0] - 1u;                       // I[0] is the row of suffix 0, plus one
     }
     uint8_t *dL = slot<uint8_t>(st, S_LCB, (size_t)n + 16);
     k_libcubwt_layout<<<grid, 256, 0, st->stream>>>(dO, dL, un, pidx, dmaps + 256, T[n - 1]);
     after_launch(st);
     check_cuda(cudaMemcpyAsync(L, dL, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     return (int64_t)pidx + 1;
 }
 
@@ -484,7 +492,7 @@ extern "C" int64_t gbwt_libcubwt_bwt(void *storage, const uint8_t *T, uint8_t *L
 {
     Storage *st = (Storage *)storage;
     if (!st || !T || !L || n < 1 || n > MAX_N) return GBWT_BAD_PARAMETER;
-    return guarded([&]() { return libcubwt_bwt(st, T, L, n); });
+    return guarded(st, [&]() { return libcubwt_bwt(st, T, L, n); });
 }
 
 extern "C" int64_t gbwt_libcubwt_bwt_aux(void *storage, const uint8_t *T, uint8_t *L, int64_t n, int64_t r,
@@ -494,7 +502,7 @@ extern "C" int64_t gbwt_libcubwt_bwt_aux(void *storage, const uint8_t *T, uint8_
     if (!st || !T || !L || !I || n < 1 || n > MAX_N || r < 2 || (r & (r - 1)) != 0) return GBWT_BAD_PARAMETER;
     int r_log2 = 0;
     while ((1ll << r_log2) < r) r_log2++;
-    return guarded([&]() -> int64_t {
+    return guarded(st, [&]() -> int64_t {
         const int64_t rc = libcubwt_bwt(st, T, L, n, r_log2, I);
         return rc < 0 ? rc : GBWT_NO_ERROR;
     });
@@ -544,8 +552,8 @@ extern "C" int64_t gbwt_trim_device_storage(void *storage)
 {
     Storage *st = (Storage *)storage;
     if (!st) return GBWT_BAD_PARAMETER;
-    return guarded([&]() -> int64_t {
-        check_cuda(cudaStreamSynchronize(st->stream));
+    return guarded(st, [&]() -> int64_t {
+        sync_stream(st);
         for (int i = 0; i < S_NUM; i++)
             if (st->slots[i].p) {
                 check_cuda(cudaFree(st->slots[i].p));

@@ -30,7 +30,7 @@ enum Slot : int {
     S_LEXRANK, S_PARSE, S_PISA, S_PSA,
     S_GCOUNT, S_GCHAR, S_GMIX, S_GOFF, S_GRP, S_MOFF, S_MB, S_MC, S_MIXIDX, S_DELTA,
     S_ELEM0, S_ELEM1,
-    S_SCAN0, S_SCAN1, S_SCAN2, S_SCAN3, S_RSHIST,
+    S_LOOKBACK, S_RSHIST,
     S_TMP0, S_TMP1, S_TMP2, S_PIDPC, S_TILEG, S_ACTX2, S_ACTG2, S_LCB, S_LCBMAP,
     S_BX, S_BMETA, S_BTID, S_BZEND, S_BLAST, S_BCODE, S_SSTART,
     S_BIGL, S_BIGM,
@@ -50,6 +50,8 @@ struct Storage {
     uint64_t *d_scalars = nullptr;      // device scalars (64 entries)
     uint32_t *h_meta = nullptr;         // pinned batch layout (grows on demand)
     size_t h_meta_cap = 0;
+    uint32_t lb_seq = 0;                // number of the last look-back pass (status tags)
+    uint32_t *h_err = nullptr;          // pinned: set by a kernel whose bounded wait gave up
     gbwt_tuning tuning = {};            // 0 = default for every knob
     gbwt_stats stats;
     int64_t launches = 0;
@@ -93,12 +95,22 @@ T *slot(Storage *st, int s, size_t count)
     return (T *)b.p;
 }
 
+// Waits for the stream; results of a pass whose bounded wait gave up are refused.
+inline void sync_stream(Storage *st)
+{
+    check_cuda(cudaStreamSynchronize(st->stream));
+    if (*(volatile uint32_t *)st->h_err) {
+        *(volatile uint32_t *)st->h_err = 0;
+        throw Error{GBWT_TIMEOUT};
+    }
+}
+
 // Reads `k` device scalars (d_scalars[0..k)) into host memory synchronously.
 inline void fetch_scalars(Storage *st, int k)
 {
     check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, (size_t)k * sizeof(uint64_t),
                                cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
 }
 
 inline void after_launch(Storage *st)

@@ -610,7 +610,7 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)total, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     uint32_t hflags[4];
     memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
     if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;

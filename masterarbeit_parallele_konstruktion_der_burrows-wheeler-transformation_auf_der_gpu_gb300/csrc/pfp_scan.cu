@@ -325,7 +325,7 @@ static void launch_pair(Storage *st, const ScanArgs &a, unsigned blocks, uint32_
     device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, tot);
     check_cuda(cudaMemcpyAsync(st->h_scalars + 1, a.flags, 4, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, 8, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     uint32_t flags = (uint32_t)st->h_scalars[1];
     if (flags & ERR_BAD_BYTE) throw Error{GBWT_BAD_PARAMETER};
     if (flags & ERR_SMALL_RANGE) throw Error{GBWT_UNSUPPORTED_INPUT};
@@ -601,7 +601,7 @@ static uint32_t launch_pair_batch(Storage *st, const ScanArgs &a, const BatchSca
     device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, tot);
     check_cuda(cudaMemcpyAsync(st->h_scalars + 1, a.flags, 4, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, 8, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     const uint32_t flags = (uint32_t)st->h_scalars[1];
     if (flags & ERR_BAD_BYTE) throw Error{GBWT_BAD_PARAMETER};
     if (flags & ERR_SMALL_RANGE) throw Error{GBWT_UNSUPPORTED_INPUT};
@@ -647,7 +647,7 @@ uint32_t run_trigger_scan_batch(Storage *st, const uint8_t *dX, uint32_t N, int 
 // that must not be re-entered from a callback, or a process that pins all
 // device memory up front.  For them the trigger scan also runs without a
 // storage object and without any cudaMalloc: its scratch (per-CTA trigger
-// counts, the scan's tile partials, the error/total words) lives in the
+// counts, the scan's tile statuses, the error/total words) lives in the
 // file-scope array below, which every GPU that loads this library holds
 // until the process exits (NOALLOC_SCRATCH_WORDS * 4 bytes, about 1 MiB).
 // Texts are limited to NOALLOC_MAX_N bytes by that size.  All calls share
@@ -656,8 +656,11 @@ uint32_t run_trigger_scan_batch(Storage *st, const uint8_t *dX, uint32_t N, int 
 // ---------------------------------------------------------------------
 constexpr int64_t NOALLOC_MAX_N = (int64_t)1 << 30;
 constexpr uint32_t NOALLOC_MAX_BLOCKS = (uint32_t)(NOALLOC_MAX_N / TS_TILE);
-constexpr uint32_t NOALLOC_PARTIALS = (NOALLOC_MAX_BLOCKS + SC_TILE - 1) / SC_TILE;
+constexpr int NOALLOC_IT = 16;                                       // scan items per thread
+constexpr uint32_t NOALLOC_STILE = SC_THREADS * NOALLOC_IT;
+constexpr uint32_t NOALLOC_STILES = (NOALLOC_MAX_BLOCKS + NOALLOC_STILE - 1) / NOALLOC_STILE;
 constexpr uint32_t NOALLOC_SCRATCH_WORDS = NOALLOC_MAX_BLOCKS + 256 + 64;
+static_assert(NOALLOC_STILES * 2 <= 256, "the scan's tile statuses take 256 words");
 
 static __device__ __align__(256) uint32_t g_trigger_scratch[NOALLOC_SCRATCH_WORDS];
 
@@ -691,32 +694,24 @@ static int64_t noalloc_launch(const ScanArgs &a, unsigned blocks, uint32_t *scra
                               cudaStream_t stream)
 {
     uint32_t *counts = scratch;                         // [NOALLOC_MAX_BLOCKS]
-    uint32_t *partials = scratch + NOALLOC_MAX_BLOCKS;  // [256]
-    uint32_t *words = partials + 256;                   // [0] errors, [1] trigger count
-    check_cuda(cudaMemsetAsync(words, 0, 64 * sizeof(uint32_t), stream));
+    uint32_t *status = scratch + NOALLOC_MAX_BLOCKS;    // [256] tile statuses of the scan
+    uint32_t *words = status + 256;                     // [0] errors, [1] trigger count, [2] ticket, [3] wait gave up
+    check_cuda(cudaMemsetAsync(status, 0, (256 + 64) * sizeof(uint32_t), stream));
     ScanArgs b = a;
     b.flags = words;
     k_trigger<WT, PT, false, 1><<<blocks, TS_THREADS, 0, stream>>>(b, counts, nullptr, nullptr);
     check_cuda(cudaGetLastError());
-    const unsigned tiles = (blocks + SC_TILE - 1) / SC_TILE;
-    if (tiles == 1) {
-        k_scan_down<uint32_t, OpAdd><<<1, SC_THREADS, 0, stream>>>(LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts},
-                                                                    blocks, (const uint32_t *)nullptr, false, words + 1);
-    } else {
-        k_scan_reduce<uint32_t, OpAdd><<<tiles, SC_THREADS, 0, stream>>>(LoadArr<uint32_t>{counts}, blocks, partials);
-        k_scan_down<uint32_t, OpAdd><<<1, SC_THREADS, 0, stream>>>(LoadArr<uint32_t>{partials},
-                                                                    StoreArr<uint32_t>{partials}, tiles,
-                                                                    (const uint32_t *)nullptr, false, (uint32_t *)nullptr);
-        k_scan_down<uint32_t, OpAdd><<<tiles, SC_THREADS, 0, stream>>>(LoadArr<uint32_t>{counts},
-                                                                        StoreArr<uint32_t>{counts}, blocks, partials,
-                                                                        false, words + 1);
-    }
+    const unsigned tiles = (blocks + NOALLOC_STILE - 1) / NOALLOC_STILE;
+    const LookBack lb{(uint64_t *)status, tiles, 1u, words + 2, words + 3};
+    k_scan<uint32_t, OpAdd, NOALLOC_IT><<<tiles, SC_THREADS, 0, stream>>>(
+        LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, blocks, lb, false, words + 1);
     check_cuda(cudaGetLastError());
-    uint32_t host_words[2] = {0, 0};
+    uint32_t host_words[4] = {0, 0, 0, 0};
     check_cuda(cudaMemcpyAsync(host_words, words, sizeof(host_words), cudaMemcpyDeviceToHost, stream));
     check_cuda(cudaStreamSynchronize(stream));
     if (host_words[0] & ERR_BAD_BYTE) return GBWT_BAD_PARAMETER;
     if (host_words[0] & ERR_SMALL_RANGE) return GBWT_UNSUPPORTED_INPUT;
+    if (host_words[3]) return GBWT_TIMEOUT;
     const uint32_t c = host_words[1];
     if ((int64_t)c + 1 > capacity) return GBWT_BAD_PARAMETER;
     k_trigger<WT, PT, true, 1><<<blocks, TS_THREADS, 0, stream>>>(b, nullptr, counts, D);

@@ -763,7 +763,7 @@ static void big_groups(Storage *st, uint32_t N, uint32_t nbig, const uint32_t *d
     std::vector<uint32_t> hb(nbig), he(nbig), hoff(nbig + 1);
     check_cuda(cudaMemcpyAsync(hb.data(), dbigs, (size_t)nbig * 4, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(he.data(), dbigs + big_cap, (size_t)nbig * 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     std::sort(hb.begin(), hb.end());
     std::sort(he.begin(), he.end());
     hoff[0] = 0;
@@ -842,7 +842,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         if (h >= N) {
             // only legal when every suffix is finished already
             check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, 8, cudaMemcpyDeviceToHost, st->stream));
-            check_cuda(cudaStreamSynchronize(st->stream));
+            sync_stream(st);
             if (hw[(r + 1) & 1] != 0) throw Error{GBWT_INTERNAL_ERROR};
             break;
         }
@@ -865,7 +865,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         uint32_t nbig = 0;
         if (check_big) {
             check_cuda(cudaMemcpyAsync(st->h_scalars + 2, st->d_flags + 3, 8, cudaMemcpyDeviceToHost, st->stream));
-            check_cuda(cudaStreamSynchronize(st->stream));
+            sync_stream(st);
             const uint32_t *cnt = (const uint32_t *)(st->h_scalars + 2);
             nbig = cnt[0];
             if (nbig > big_cap || cnt[1] != nbig) throw Error{GBWT_INTERNAL_ERROR};
@@ -894,7 +894,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         r++;
         if (check_big || nbig || debug || A_ub >= DR_SYNC_MIN || r % DR_SYNC == 0) {
             check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, 8, cudaMemcpyDeviceToHost, st->stream));
-            check_cuda(cudaStreamSynchronize(st->stream));
+            sync_stream(st);
             A_ub = hw[(r + 1) & 1];        // the count this round produced (r already advanced)
             exact = true;
             if (debug) {
@@ -911,7 +911,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
     }
     // rounds that had work, and the probe's algorithmic bytes per round
     check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, (8 + DR_MAXR) * 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     int rounds = 0;
     for (int i = 0; i < r; i++) {
         const uint32_t a = hw[8 + i];
@@ -1042,7 +1042,7 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     uint32_t present[8];
     check_cuda(cudaMemcpyAsync(st->h_scalars + 4, st->d_flags + 8, sizeof(present), cudaMemcpyDeviceToHost,
                                st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     memcpy(present, st->h_scalars + 4, sizeof(present));
     uint8_t *hcode = (uint8_t *)(st->h_scalars + 16);          // 256 pinned bytes
     uint32_t sigma = 0;

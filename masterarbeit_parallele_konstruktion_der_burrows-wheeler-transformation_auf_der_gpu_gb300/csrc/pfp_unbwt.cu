@@ -258,7 +258,8 @@ void run_unbwt(Storage *st, const uint8_t *dLc, uint32_t n, uint32_t i, uint8_t 
     uint32_t *hist = slot<uint32_t>(st, S_RSHIST, (size_t)256 * num_tiles);
     k_rs_upsweep<uint8_t, 8><<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, 0, 0xFFu, hist, num_tiles, nullptr);
     after_launch(st);
-    scan_array_excl<uint32_t, OpAdd>(st, hist, (size_t)256 * num_tiles, 0);
+    device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
+                                 (uint32_t *)nullptr);
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
     k_lf_rank<8><<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, i, hist, num_tiles, rate_mask, rul, m, LF);
     after_launch(st);
@@ -283,7 +284,7 @@ void run_unbwt(Storage *st, const uint8_t *dLc, uint32_t n, uint32_t i, uint8_t 
     check_cuda(cudaMemcpyAsync(st->h_scalars + 1, st->d_flags + 4, 4, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 2, wt, 8, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 3, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaStreamSynchronize(st->stream));
+    sync_stream(st);
     if ((uint32_t)st->h_scalars[3] & ERR_INTERNAL) throw Error{GBWT_INTERNAL_ERROR};
     if ((uint32_t)st->h_scalars[1] != 0) throw Error{GBWT_BAD_PARAMETER};
     // from ruler 0 the whole cycle must come back to row 0 after n+1 steps

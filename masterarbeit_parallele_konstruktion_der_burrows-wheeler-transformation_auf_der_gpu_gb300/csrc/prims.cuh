@@ -1,6 +1,6 @@
 // prims.cuh -- device-wide scan and stable LSD radix sort (sm_103a).
 //
-// Scan: reduce-then-scan over tiles of 4096 items, with functor loads and
+// Scan: one pass over the input (decoupled look-back), with functor loads and
 // stores so that flags, compaction and segmented heads are computed on the
 // fly instead of being materialised.
 //
@@ -17,8 +17,6 @@
 namespace gbwt {
 
 constexpr int SC_THREADS = 256;
-constexpr int SC_ITEMS = 16;
-constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
 
 // Scan operators.  diff(inc, ex) returns a value v with op(ex, v) == inc:
 // the item itself for sums, the inclusive prefix for maxima (the scan hands
@@ -53,6 +51,20 @@ struct OpMaxAdd {
     }
 };
 
+// Warp shuffles of values wider than 8 bytes go member by member.
+template <typename T>
+__device__ __forceinline__ T shfl_xor_any(T v, int o)
+{
+    if constexpr (sizeof(T) <= 8) return __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    else return v.shfl_xor(o);
+}
+template <typename T>
+__device__ __forceinline__ T shfl_up_any(T v, int o)
+{
+    if constexpr (sizeof(T) <= 8) return __shfl_up_sync(0xFFFFFFFFu, v, o);
+    else return v.shfl_up(o);
+}
+
 // Block-wide exclusive scan (identity 0); `total` receives the block total.
 template <typename T, typename Op>
 __device__ __forceinline__ T block_excl_scan(T v, T &total, Op op, T *s_warp /*[32]*/)
@@ -62,7 +74,7 @@ __device__ __forceinline__ T block_excl_scan(T v, T &total, Op op, T *s_warp /*[
     T x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        T y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        T y = shfl_up_any(x, o);
         if (lane >= (unsigned)o) x = op(y, x);
     }
     if (lane == 31) s_warp[warp] = x;
@@ -71,7 +83,7 @@ __device__ __forceinline__ T block_excl_scan(T v, T &total, Op op, T *s_warp /*[
         T w = lane < nw ? s_warp[lane] : T(0);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            T y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+            T y = shfl_up_any(w, o);
             if (lane >= (unsigned)o) w = op(y, w);
         }
         s_warp[lane] = w;
@@ -79,75 +91,214 @@ __device__ __forceinline__ T block_excl_scan(T v, T &total, Op op, T *s_warp /*[
     __syncthreads();
     T wp = warp ? s_warp[warp - 1] : T(0);
     total = s_warp[nw - 1];
-    T xe = __shfl_up_sync(0xFFFFFFFFu, x, 1);
+    T xe = shfl_up_any(x, 1);
     if (lane == 0) xe = T(0);
     __syncthreads();
     return op(wp, xe);
 }
 
-// ---- scan kernels ---------------------------------------------------
-template <typename T, typename Op, typename Load>
-__global__ void __launch_bounds__(SC_THREADS) k_scan_reduce(Load load, size_t n, T *partial)
+// ---- single-pass scan -------------------------------------------------
+// One kernel per scan: every tile publishes its total, looks back over the
+// published totals of the tiles before it (a warp reads 32 at a time) and
+// publishes its inclusive prefix (Merrill & Garland 2016, "Single-pass
+// parallel prefix scan with decoupled look-back").  Against a reduce pass, a
+// scan of the tile totals and a second pass over the input (three to five
+// launches, every input loaded twice), the load functors -- often chains of
+// random reads -- run once and small inputs pay for one launch: the 8 MiB DNA
+// text takes 59 launches fewer and 1.15 instead of 1.30 ms, a batch of 24
+// texts 1.09 instead of 1.24 ms; at 512 MiB the two forms are level.
+//
+// Tiles are numbered by a ticket in the order their CTAs start, so a tile
+// only waits for tiles whose CTAs are already running and every wait ends.
+// A status is one 64-bit word per 32 bits of the value, each word carrying
+// the same tag (scan number << 2 | state) in its high half: words are read
+// and written whole, and a reader takes a value only when all its tags agree,
+// so no fence is needed.  The scan number differs from call to call, so old
+// statuses need no clearing; the CTA holding the last ticket resets the
+// ticket counter.
+constexpr uint32_t LB_TOTAL = 1u, LB_PREFIX = 2u;      // states
+constexpr uint32_t LB_MAX_POLLS = 1u << 22;            // seconds; a wait ends after microseconds
+
+struct LookBack {
+    uint64_t *status;       // word w of tile t at status[w * stride + t]
+    uint32_t stride;
+    uint32_t seq;           // number of this scan, 1 .. 2^30 - 1
+    uint32_t *ticket;       // 0 between scans
+    uint32_t *err;          // set to 1 when a wait gave up
+};
+
+// Status words for a pass of `tiles` tiles on the storage's stream.
+inline LookBack look_back(Storage *st, size_t tiles, size_t words)
 {
-    __shared__ T s_warp[32];
-    Op op;
-    size_t base = (size_t)blockIdx.x * SC_TILE;
-    T acc = T(0);
-#pragma unroll 4
-    for (int j = 0; j < SC_ITEMS; j++) {
-        size_t i = base + (size_t)j * SC_THREADS + threadIdx.x;
-        if (i < n) acc = op(acc, load(i));
+    const size_t bytes = tiles * words * sizeof(uint64_t);
+    const bool fresh = st->slots[S_LOOKBACK].cap < (bytes < 256 ? 256 : bytes);
+    uint64_t *status = slot<uint64_t>(st, S_LOOKBACK, tiles * words);
+    if (fresh || st->lb_seq >= (1u << 30) - 1u) {
+        check_cuda(cudaMemsetAsync(status, 0, st->slots[S_LOOKBACK].cap, st->stream));
+        st->lb_seq = 0;
     }
-    T total;
-    block_excl_scan<T, Op>(acc, total, op, s_warp);
-    if (threadIdx.x == 0) partial[blockIdx.x] = total;
+    st->lb_seq++;
+    return LookBack{status, (uint32_t)tiles, st->lb_seq, (uint32_t *)(st->d_scalars + 60), st->h_err};
 }
 
-// Stores run in striped order (consecutive threads on consecutive items, so
-// a store functor's writes at i coalesce): the blocked prefixes go back
-// through shared memory.  store(i, prefix, v) gets the exclusive (or
-// inclusive) prefix and v = op.diff(inclusive, exclusive) -- the item's
-// value for sums.
+__device__ __forceinline__ void lb_store(uint64_t *p, uint64_t v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint64_t lb_load(const uint64_t *p)
+{
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ void lb_publish(const LookBack &lb, uint32_t tile, T v, uint32_t state)
+{
+    constexpr int NW = sizeof(T) / 4;
+    uint32_t w[NW];
+    memcpy(w, &v, sizeof(T));
+    const uint64_t tag = (uint64_t)((lb.seq << 2) | state) << 32;
+#pragma unroll
+    for (int k = 0; k < NW; k++) lb_store(lb.status + (size_t)k * lb.stride + tile, tag | w[k]);
+}
+// State of a tile (0 = nothing usable yet) and its value.
+template <typename T>
+__device__ __forceinline__ uint32_t lb_read(const LookBack &lb, uint32_t tile, T &v)
+{
+    constexpr int NW = sizeof(T) / 4;
+    uint64_t q[NW];
+#pragma unroll
+    for (int k = 0; k < NW; k++) q[k] = lb_load(lb.status + (size_t)k * lb.stride + tile);
+    uint32_t w[NW];
+    const uint32_t tag = (uint32_t)(q[0] >> 32);
+    bool same = (tag >> 2) == lb.seq;
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+        same = same && (uint32_t)(q[k] >> 32) == tag;
+        w[k] = (uint32_t)q[k];
+    }
+    memcpy(&v, w, sizeof(T));
+    return same ? tag & 3u : 0u;
+}
+
+// Prefix of all tiles before `tile` (> 0), by one warp; every Op used here
+// commutes, so the lanes' values combine in any order.  A round reads
+// LB_WIDE x 32 statuses.  Measured on GB300 (32-bit sums in place): 34 M
+// items in 106 us with 1, 122 us with 4 and 156 us with 8; 3 M items in
+// 16.7, 20.1 and 24.9 us: the polls of waiting tiles compete with the
+// statuses being published, so fewer reads per round win.
+constexpr int LB_WIDE = 1;
+template <typename T, typename Op>
+__device__ __forceinline__ T lb_prefix(const LookBack &lb, uint32_t tile)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    Op op;
+    T acc = T(0);                              // per lane, combined at the end
+    int64_t top = (int64_t)tile - 1;           // nearest tile not yet included
+    uint32_t polls = 0;
+    bool found = false;
+    while (top >= 0 && !found) {
+        T v[LB_WIDE];
+        uint32_t state[LB_WIDE];
+#pragma unroll
+        for (int k = 0; k < LB_WIDE; k++) {
+            const int64_t i = top - (int64_t)(k * 32) - (int64_t)lane;
+            v[k] = T(0);
+            state[k] = LB_PREFIX;              // before the first tile: identity
+            if (i >= 0) state[k] = lb_read<T>(lb, (uint32_t)i, v[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < LB_WIDE; k++) {
+            const unsigned rm = __ballot_sync(0xFFFFFFFFu, state[k] != 0u);
+            const unsigned pm = __ballot_sync(0xFFFFFFFFu, state[k] == LB_PREFIX);
+            // lanes up to the nearest inclusive prefix, or all 32
+            const unsigned need = pm ? (0xFFFFFFFFu >> (32 - __ffs(pm))) : 0xFFFFFFFFu;
+            if ((rm & need) != need) {
+                // never runs out: see above.  The host refuses the result if it does.
+                if (++polls >= LB_MAX_POLLS) {
+                    if (lane == 0) *(volatile uint32_t *)lb.err = 1u;
+                    found = true;
+                }
+                break;
+            }
+            if ((need >> lane) & 1u) acc = op(acc, v[k]);
+            if (pm) { found = true; break; }
+            top -= 32;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = op(acc, shfl_xor_any(acc, o));
+    return acc;
+}
+
 // Shared-memory slot of tile item i: one padding slot per 32 items, so the
-// blocked accesses (thread t, items 16t..16t+15) hit distinct banks.
+// blocked accesses (thread t, items IT*t ..) hit distinct banks.
 __device__ __forceinline__ uint32_t sc_pad(uint32_t i) { return i + (i >> 5); }
 
-template <typename T, typename Op, typename Load, typename Store>
-__global__ void __launch_bounds__(SC_THREADS) k_scan_down(Load load, Store store, size_t n,
-                                                          const T *partial, bool inclusive,
-                                                          T *total_out)
+// Loads and stores run in striped order (consecutive threads on consecutive
+// items, so both coalesce); the blocked prefixes go through shared memory.
+// store(i, prefix, v) gets the exclusive (or inclusive) prefix and
+// v = op.diff(inclusive, exclusive) -- the item's value for sums.
+template <typename T, typename Op, int IT, typename Load, typename Store>
+__global__ void __launch_bounds__(SC_THREADS) k_scan(Load load, Store store, size_t n, LookBack lb, bool inclusive,
+                                                     T *total_out)
 {
-    __shared__ T s_tile[SC_TILE + SC_TILE / 32 + 1];
+    constexpr int TILE = SC_THREADS * IT;
+    __shared__ T s_tile[TILE + TILE / 32 + 1];
     __shared__ T s_warp[32];
+    __shared__ uint32_t s_id;
     Op op;
-    size_t base = (size_t)blockIdx.x * SC_TILE;
-    // striped (coalesced) loads into shared memory, then blocked reads
-#pragma unroll 4
-    for (int j = 0; j < SC_ITEMS; j++) {
-        size_t i = base + (size_t)j * SC_THREADS + threadIdx.x;
+    uint32_t tile = 0;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) {
+            s_id = atomicAdd(lb.ticket, 1u);
+            if (s_id == gridDim.x - 1) *lb.ticket = 0;
+        }
+        __syncthreads();
+        tile = s_id;
+    }
+    const size_t base = (size_t)tile * TILE;
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+        const size_t i = base + (size_t)j * SC_THREADS + threadIdx.x;
         s_tile[sc_pad(j * SC_THREADS + threadIdx.x)] = i < n ? load(i) : T(0);
     }
     __syncthreads();
-    T v[SC_ITEMS];
+    T v[IT];
     T sum = T(0);
 #pragma unroll
-    for (int j = 0; j < SC_ITEMS; j++) {
-        v[j] = s_tile[sc_pad(threadIdx.x * SC_ITEMS + j)];
+    for (int j = 0; j < IT; j++) {
+        v[j] = s_tile[sc_pad(threadIdx.x * IT + j)];
         sum = op(sum, v[j]);
     }
     T total;
-    T ex = block_excl_scan<T, Op>(sum, total, op, s_warp);   // ends with a barrier: s_tile is free
-    T run = partial ? op(partial[blockIdx.x], ex) : ex;
+    T run = block_excl_scan<T, Op>(sum, total, op, s_warp);   // ends with a barrier: s_tile and s_warp are free
+    if (gridDim.x > 1) {
+        if (threadIdx.x < 32) {
+            if (threadIdx.x == 0) lb_publish(lb, tile, total, tile ? LB_TOTAL : LB_PREFIX);
+            if (tile) {
+                const T pre = lb_prefix<T, Op>(lb, tile);
+                if (threadIdx.x == 0) {
+                    lb_publish(lb, tile, op(pre, total), LB_PREFIX);
+                    s_warp[0] = pre;
+                }
+            } else if (threadIdx.x == 0) {
+                s_warp[0] = T(0);
+            }
+        }
+        __syncthreads();
+        run = op(s_warp[0], run);
+    }
     // exclusive prefixes of the tile's items (items past n add the identity)
 #pragma unroll
-    for (int j = 0; j < SC_ITEMS; j++) {
-        s_tile[sc_pad(threadIdx.x * SC_ITEMS + j)] = run;
+    for (int j = 0; j < IT; j++) {
+        s_tile[sc_pad(threadIdx.x * IT + j)] = run;
         run = op(run, v[j]);
     }
-    if (threadIdx.x == SC_THREADS - 1) s_tile[sc_pad(SC_TILE)] = run;
+    if (threadIdx.x == SC_THREADS - 1) s_tile[sc_pad(TILE)] = run;
     __syncthreads();
 #pragma unroll 4
-    for (int j = 0; j < SC_ITEMS; j++) {
+    for (int j = 0; j < IT; j++) {
         const uint32_t li = (uint32_t)j * SC_THREADS + threadIdx.x;
         const size_t i = base + li;
         if (i < n) {
@@ -169,45 +320,25 @@ struct StoreArr {
     __device__ __forceinline__ void operator()(size_t i, T pre, T) const { a[i] = pre; }
 };
 
-// In-place exclusive scan of a plain array (used for partials and histograms).
-template <typename T, typename Op>
-void scan_array_excl(Storage *st, T *a, size_t m, int depth)
-{
-    if (m == 0) return;
-    size_t tiles = (m + SC_TILE - 1) / SC_TILE;
-    if (tiles == 1) {
-        k_scan_down<T, Op><<<1, SC_THREADS, 0, st->stream>>>(LoadArr<T>{a}, StoreArr<T>{a}, m,
-                                                              (const T *)nullptr, false, (T *)nullptr);
-        after_launch(st);
-        return;
-    }
-    if (depth >= 3) throw Error{GBWT_INTERNAL_ERROR};
-    T *part = slot<T>(st, S_SCAN1 + depth, tiles);
-    k_scan_reduce<T, Op><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(LoadArr<T>{a}, m, part);
-    after_launch(st);
-    scan_array_excl<T, Op>(st, part, tiles, depth + 1);
-    k_scan_down<T, Op><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(LoadArr<T>{a}, StoreArr<T>{a}, m,
-                                                                        part, false, (T *)nullptr);
-    after_launch(st);
-}
-
 // Scan of load(i), i in [0,n): store(i, prefix, value) is called with the
 // exclusive (or inclusive) prefix.  The total is written to *total_dev when
-// given (device pointer; left untouched for n == 0).
+// given (device pointer; left untouched for n == 0).  In-place scans are
+// fine: a tile reads its items before it writes them and no other tile's.
+// Inputs that give every SM fewer than eight such tiles take tiles of four
+// items per thread, so that they spread over the SMs instead of running as
+// one long chain of dependent loads; larger ones take 16, which quarters the
+// number of tiles that a prefix has to travel over.
 template <typename T, typename Op, typename Load, typename Store>
 void device_scan(Storage *st, size_t n, Load load, Store store, bool inclusive, T *total_dev)
 {
     if (n == 0) return;
-    size_t tiles = (n + SC_TILE - 1) / SC_TILE;
-    T *part = nullptr;
-    if (tiles > 1) {
-        part = slot<T>(st, S_SCAN0, tiles);
-        k_scan_reduce<T, Op><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, n, part);
-        after_launch(st);
-        scan_array_excl<T, Op>(st, part, tiles, 0);
-    }
-    k_scan_down<T, Op><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, store, n, part, inclusive,
-                                                                        total_dev);
+    constexpr int BIG = sizeof(T) <= 8 ? 16 : 8, SMALL = 4;
+    const bool small = n <= (size_t)st->num_sms * 8 * SC_THREADS * SMALL;
+    const size_t per = (size_t)SC_THREADS * (small ? SMALL : BIG);
+    const size_t tiles = (n + per - 1) / per;
+    const LookBack lb = look_back(st, tiles, sizeof(T) / 4);
+    if (small) k_scan<T, Op, SMALL><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, store, n, lb, inclusive, total_dev);
+    else k_scan<T, Op, BIG><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, store, n, lb, inclusive, total_dev);
     after_launch(st);
 }
 
@@ -439,7 +570,8 @@ void radix_sort(Storage *st, K *&keys, K *&keys_alt, uint32_t *&vals, uint32_t *
         uint32_t mask = (1u << bits) - 1u;
         k_rs_upsweep<K, BITS><<<num_tiles, RS_THREADS, 0, st->stream>>>(keys, n, shift, mask, hist, num_tiles, tseg);
         after_launch(st);
-        scan_array_excl<uint32_t, OpAdd>(st, hist, D * num_tiles, 0);
+        device_scan<uint32_t, OpAdd>(st, D * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
+                                     (uint32_t *)nullptr);
         probe_begin(st, GBWT_PROBE_RADIX_SCATTER);
         k_rs_downsweep<K, HAS_VAL, BITS, BALLOT><<<num_tiles, RS_THREADS, smem, st->stream>>>(keys, keys_alt, vals, vals_alt,
                                                                                       n, shift, mask, hist, num_tiles,
