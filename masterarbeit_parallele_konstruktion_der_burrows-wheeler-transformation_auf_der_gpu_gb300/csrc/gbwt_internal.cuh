@@ -28,7 +28,7 @@ enum Slot : int {
     S_DLEN, S_DSTART, S_DOFF, S_OCC, S_PCMIN, S_PCMAX, S_DICT, S_DPHR,
     S_KEY0, S_KEY1, S_VAL0, S_VAL1, S_ISA, S_SA, S_ACTX, S_ACTG, S_HEAD,
     S_LEXRANK, S_PARSE, S_PISA, S_PSA,
-    S_GCOUNT, S_GCHAR, S_GMIX, S_GOFF, S_GRP, S_MOFF, S_MB, S_MC, S_MIXIDX, S_DELTA,
+    S_GCOUNT, S_GCHAR, S_GRP, S_MOFF, S_MB, S_MC, S_DELTA,
     S_ELEM0, S_ELEM1,
     S_LOOKBACK, S_RSHIST,
     S_TMP0, S_TMP1, S_TMP2, S_PIDPC, S_TILEG, S_ACTX2, S_ACTG2, S_LCB, S_LCBMAP,

@@ -9,9 +9,9 @@
 // K:2509-3369, bitonic block sorts K:3556-4248).
 //
 // Here S comes out of the dictionary suffix order directly: equal suffixes
-// are one group of the prefix-doubling result.  For every group we add the
-// occurrence counts of its phrases (block length) and check whether all
-// preceding bytes agree (run).  Runs are written one group per thread with
+// are one group of the prefix-doubling result, named by the sorted position
+// of its first member.  For every group we add the occurrence counts of its
+// phrases (block length) and check whether all preceding bytes agree (run).  Runs are written one group per thread with
 // 16-byte stores (long blocks one CTA each).  For mixed groups, every phrase
 // occurrence -- visited in parse
 // suffix-array order, which is exactly the "rank of the next parse suffix"
@@ -42,11 +42,105 @@ __device__ __forceinline__ uint32_t pc_code(const uint8_t *dict, const uint32_t 
     return pcmin[q] == pcmax[q] ? pcmin[q] : PC_VAR;
 }
 
-// S groups (equal phrase suffixes longer than W) in dictionary order.  The
-// passes run over dictionary positions x in storage order, so the phrase
-// tables are read almost sequentially: (1) mark the sorted position isa[x]
-// of every long suffix's group head, (2) scan the marks into group numbers,
-// (3) read each position's group back through isa[x].
+// ---- single text: groups by the sorted position of their head ----------
+// stat[t] of the group whose head is sorted position t: x = block length, y =
+// the preceding bytes seen, byte c as c | (~c << 16).  OR-ing members keeps a
+// bit position clear in one half exactly when all bytes agree in it, so y's
+// halves are disjoint in their low bytes iff the block is one run.
+//
+// One pass over dictionary positions in storage order (phrase tables read
+// almost sequentially) with two reductions per long suffix into the 8-byte
+// word of its group.  Random sectors bound it: one read and one write-back per
+// suffix.  Numbering the groups first cost a byte scattered per suffix, a
+// random read of the number, a sum, a stored byte and a second pass comparing
+// the bytes (four random sectors per suffix).  All S-group kernels together:
+// 512 MiB DNA, W=35 (N = 130 M) 13.9 -> 4.3 ms, of it 3.5 here; W=5 1.28 -> 0.73
+// ms; 102 MB of versions 4.9 -> 1.7 ms.
+constexpr uint32_t GS_ANY = 0x00FF00FFu;       // a byte that varies
+__device__ __forceinline__ bool gs_mixed(uint32_t y) { return (y & (y >> 16) & 0xFFu) != 0; }
+
+__global__ void k_group_stats(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *isa, const uint8_t *dict,
+                              const uint32_t *occ, const uint32_t *pcmin, const uint32_t *pcmax, uint2 *stat)
+{
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= N) return;
+    uint32_t q, off, rem;
+    pi.get(x, q, off, rem);
+    if (rem <= W) return;
+    const uint32_t t = isa[x];
+    const uint32_t c = pc_code(dict, pcmin, pcmax, x, q, off);
+    atomicAdd(&stat[t].x, occ[q]);
+    atomicOr(&stat[t].y, c == PC_VAR ? GS_ANY : c | ((c ^ 0xFFu) << 16));
+}
+
+// One scan of the block lengths turns the statistics into places: stat[t]
+// becomes x = the output offset of t's block (for a position that heads no
+// group: of the next block; stat[N].x = n), y = tag: the run's byte, GS_MIX, or
+// GS_NONE.  Heads and mixed heads also go into bit vectors over sorted
+// positions, so that the few mixed blocks are numbered by a scan over words
+// (N / 32 items) instead of carrying three more sums through this one
+// (512 MiB DNA, W=35, N = 130 M: 1.51 ms for a scan of four sums).
+constexpr uint32_t GS_MIX = 0x80000000u, GS_NONE = 0x100u;
+struct LoadGCount {
+    const uint2 *stat;
+    __device__ __forceinline__ uint32_t operator()(size_t t) const { return stat[t].x; }
+};
+struct StoreGroup {
+    uint2 *stat;
+    uint32_t N;
+    uint32_t *heads, *mixed;
+    // called for consecutive t by consecutive lanes, warps starting at multiples of 32
+    __device__ __forceinline__ void operator()(size_t t, uint32_t pre, uint32_t v) const
+    {
+        const uint32_t y = stat[t].y;
+        const bool head = v != 0, mix = gs_mixed(y);
+        const uint32_t left = N - ((uint32_t)t & ~31u);          // lanes of this warp inside [0, N)
+        const unsigned lanes = left >= 32u ? 0xFFFFFFFFu : (1u << left) - 1u;
+        const unsigned hm = __ballot_sync(lanes, head), mm = __ballot_sync(lanes, mix);
+        if (((uint32_t)t & 31u) == 0) {
+            heads[t >> 5] = hm;
+            mixed[t >> 5] = mm;
+        }
+        stat[t] = make_uint2(pre, mix ? GS_MIX : head ? (y & 0xFFu) : GS_NONE);
+        if (t + 1 == N) stat[N] = make_uint2(pre + v, GS_NONE);
+    }
+};
+// Per word of the bit vectors: bytes in mixed blocks, mixed blocks, groups.
+struct LoadMixWord {
+    const uint2 *stat;
+    const uint32_t *heads, *mixed;
+    __device__ __forceinline__ Sum4 operator()(size_t w) const
+    {
+        uint32_t m = mixed[w], bytes = 0;
+        const uint32_t cnt = (uint32_t)__popc(m);
+        for (; m; m &= m - 1u) {
+            const size_t t = w * 32 + (size_t)(__ffs(m) - 1);
+            bytes += stat[t + 1].x - stat[t].x;
+        }
+        return Sum4(bytes, cnt, (uint32_t)__popc(heads[w]), 0u);
+    }
+};
+struct StoreMixWord {
+    uint2 *stat;
+    const uint32_t *mixed;
+    uint32_t *delta;            // per mixed block: output offset minus its place among the mixed bytes
+    __device__ __forceinline__ void operator()(size_t w, const Sum4 &pre, const Sum4 &) const
+    {
+        uint32_t place = pre.a, b = pre.b;
+        for (uint32_t m = mixed[w]; m; m &= m - 1u, b++) {
+            const size_t t = w * 32 + (size_t)(__ffs(m) - 1);
+            const uint32_t o = stat[t].x;
+            delta[b] = o - place;
+            place += stat[t + 1].x - o;
+            stat[t].y = GS_MIX | b;
+        }
+    }
+};
+
+// ---- batch: dense group numbers ------------------------------------------
+// The batch sorts its output by group, so the numbers have to be dense: mark
+// the sorted position isa[x] of every long suffix's group head, scan the
+// marks, read each position's number back through isa[x].
 __global__ void k_mark_sheads(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *isa, uint8_t *mark)
 {
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -60,122 +154,68 @@ struct LoadMark {
     __device__ __forceinline__ uint32_t operator()(size_t t) const { return m[t]; }
 };
 struct StoreGid {
-    const uint8_t *m;
     uint32_t *gid;
     __device__ __forceinline__ void operator()(size_t t, uint32_t inc, uint32_t v) const
     {
         if (v) gid[t] = inc - 1u;
     }
 };
-
-// Group of every long suffix; with `gcount` also the block lengths (sum of
-// the phrases' occurrence counts) and one preceding-byte code per group
-// (any member's: the mixed test compares every member with it).
 __global__ void k_group_of(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *isa, const uint32_t *gid,
-                           uint32_t *grp_of, const uint8_t *dict, const uint32_t *occ, const uint32_t *pcmin,
-                           const uint32_t *pcmax, uint32_t *gcount, uint16_t *gchar)
+                           uint32_t *grp_of)
 {
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= N) return;
     uint32_t q, off, rem;
     pi.get(x, q, off, rem);
-    if (rem <= W) return;
-    const uint32_t g = gid[isa[x]];
-    grp_of[x] = g;
-    if (gcount) {
-        atomicAdd(gcount + g, occ[q]);
-        gchar[g] = (uint16_t)pc_code(dict, pcmin, pcmax, x, q, off);
-    }
+    if (rem > W) grp_of[x] = gid[isa[x]];
 }
 
-// Passes (1)-(2); returns the number of groups, gid in slot S_TMP0.
-static uint32_t group_numbers(Storage *st, Phrases &ph, DictOrder &dord, int W, uint32_t *&gid)
+// Per-phrase lists of mixed suffixes, in dictionary (phrase, offset) order:
+// one bit per dictionary position (looked up in the mixed-head vector, N / 8
+// bytes that stay in L2), a scan of the words' counts, and a pass over the set
+// bits.  One position per thread keeps many lookups in flight; as the load of
+// a scan each thread ran a chain of them (512 MiB DNA, W=35: 2.9 ms for the
+// scan, 1.5 ms for these passes).
+__global__ void k_mix_flags(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *isa, const uint32_t *mixed,
+                            uint32_t *words)
 {
-    const uint32_t N = (uint32_t)ph.dict_bytes;
-    PosInfo pi{ph.dphr, ph.doff, ph.dlen};
-    uint8_t *mark = slot<uint8_t>(st, S_MB, N);
-    gid = slot<uint32_t>(st, S_TMP0, N);
-    check_cuda(cudaMemsetAsync(mark, 0, N, st->stream));
-    k_mark_sheads<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, mark);
-    after_launch(st);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    device_scan<uint32_t, OpAdd>(st, N, LoadMark{mark}, StoreGid{mark, gid}, true, (uint32_t *)st->d_scalars);
-    fetch_scalars(st, 1);
-    return (uint32_t)st->h_scalars[0];
-}
-
-// Pass 2 over dictionary positions: mark groups with differing bytes.
-__global__ void k_mark_mixed(uint32_t N, PosInfo pi, uint32_t W, const uint8_t *dict, const uint32_t *pcmin,
-                             const uint32_t *pcmax, const uint32_t *grp_of, const uint16_t *gchar, uint8_t *gmix)
-{
-    uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= N) return;
-    uint32_t q, off, rem;
-    pi.get(x, q, off, rem);
-    if (rem <= W) return;
-    const uint32_t g = grp_of[x];
-    const uint32_t c = pc_code(dict, pcmin, pcmax, x, q, off);
-    if (c == PC_VAR || c != gchar[g]) gmix[g] = 1;
-}
-
-struct LoadGCount {
-    const uint32_t *gcount;
-    __device__ __forceinline__ uint32_t operator()(size_t g) const { return gcount[g]; }
-};
-// Mixed groups: packed (count of mixed groups, bytes in mixed groups).
-struct LoadMixPair {
-    const uint32_t *gcount;
-    const uint8_t *gmix;
-    __device__ __forceinline__ uint64_t operator()(size_t g) const
-    {
-        return gmix[g] ? ((1ull << 32) | gcount[g]) : 0ull;
-    }
-};
-struct StoreMix {
-    const uint8_t *gmix;
-    const uint32_t *goff;
-    uint32_t *mixidx;
-    uint32_t *delta;
-    __device__ __forceinline__ void operator()(size_t g, uint64_t pre, uint64_t) const
-    {
-        if (!gmix[g]) return;
-        const uint32_t b = (uint32_t)(pre >> 32), mstart = (uint32_t)pre;
-        mixidx[g] = b;
-        delta[b] = goff[g] - mstart;
-    }
-};
-
-// Per-phrase lists of mixed suffixes, in dictionary (phrase, offset) order.
-struct LoadMixEntry {
-    PosInfo pi;
-    uint32_t W;
-    const uint32_t *grp_of;
-    const uint8_t *gmix;
-    __device__ __forceinline__ uint32_t operator()(size_t x) const
-    {
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    bool set = false;
+    if (x < N) {
         uint32_t q, off, rem;
-        pi.get((uint32_t)x, q, off, rem);
-        return (rem > W && gmix[grp_of[x]]) ? 1u : 0u;
-    }
-};
-struct StoreMixEntry {
-    PosInfo pi;
-    const uint8_t *dict;
-    const uint32_t *grp_of, *mixidx;
-    uint32_t *moff;
-    uint32_t *mb;
-    uint16_t *mc;
-    __device__ __forceinline__ void operator()(size_t x, uint32_t pre, uint32_t v) const
-    {
-        uint32_t q, off, rem;
-        pi.get((uint32_t)x, q, off, rem);
-        if (off == 0) moff[q] = pre;
-        if (v) {
-            mb[pre] = mixidx[grp_of[x]];
-            mc[pre] = (uint16_t)(off ? dict[x - 1] : PC_VAR);
+        pi.get(x, q, off, rem);
+        if (rem > W) {
+            const uint32_t t = isa[x];
+            set = (mixed[t >> 5] >> (t & 31u)) & 1u;
         }
     }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, set);
+    if ((threadIdx.x & 31u) == 0 && x < N) words[x >> 5] = m;
+}
+struct LoadPopc {
+    const uint32_t *w;
+    __device__ __forceinline__ uint32_t operator()(size_t i) const { return (uint32_t)__popc(w[i]); }
 };
+__device__ __forceinline__ uint32_t bits_before(const uint32_t *words, const uint32_t *pre, uint32_t x)
+{
+    return pre[x >> 5] + (uint32_t)__popc(words[x >> 5] & ((1u << (x & 31u)) - 1u));
+}
+__global__ void k_mix_offsets(uint32_t d, const uint32_t *doff, const uint32_t *words, const uint32_t *pre,
+                              uint32_t *moff)
+{
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < d) moff[q] = bits_before(words, pre, doff[q]);
+}
+__global__ void k_mix_entries(uint32_t N, const uint32_t *dphr, const uint32_t *doff, const uint8_t *dict,
+                              const uint32_t *isa, const uint2 *stat, const uint32_t *words, const uint32_t *pre,
+                              uint32_t *mb, uint16_t *mc)
+{
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= N || !((words[x >> 5] >> (x & 31u)) & 1u)) return;
+    const uint32_t e = bits_before(words, pre, x);
+    mb[e] = stat[isa[x]].y & ~GS_MIX;
+    mc[e] = (uint16_t)(x != doff[dphr[x]] ? dict[x - 1] : PC_VAR);
+}
 
 // Emission order: the last phrase first (its next-suffix rank is -1,
 // K:787-807), then the phrase before each parse suffix in suffix-array order.
@@ -307,50 +347,62 @@ __global__ void k_mixed_scatter(const E *elem, uint32_t M, const uint32_t *delta
     }
 }
 
-// Run fill, one thread per group: the block [goff[g], goff[g+1]) of a run
-// group is one byte repeated; the thread writes the bytes up to the first
-// 16-byte boundary one by one, the middle with 16-byte stores and the tail
-// one by one (neighbouring threads' edge bytes meet in L2).  Mixed groups are
-// skipped: the mixed scatter writes every byte of theirs.  Blocks longer than
-// RF_LONG bytes are listed and filled by one CTA each, so no thread carries a
-// long block.
+// Run fill, one thread per sorted position: the block of a run group is one
+// byte repeated, written in pieces of 1, 2, 4 and 8 bytes up to a 16-byte
+// boundary, 16-byte stores, and pieces again (neighbouring threads' edges meet
+// in L2).  Runs average tens of bytes, so their edges are most of the stores:
+// pieces take at most eight where bytes took up to thirty (512 MiB DNA: 342 ->
+// 187 us, 256 MiB of versions: 377 -> 134 us).  Mixed groups are skipped: the
+// mixed scatter writes every byte of theirs.  Blocks longer than RF_LONG bytes
+// are listed and filled by one CTA each, so no thread carries a long block.
 constexpr uint32_t RF_LONG = 512;
 
 __device__ __forceinline__ void fill_run(uint8_t *out, uint32_t b0, uint32_t b1, uint8_t c)
 {
-    uint32_t p = b0;
-    while (p < b1 && (((uintptr_t)(out + p)) & 15u)) out[p++] = c;
     const uint32_t w = (uint32_t)c * 0x01010101u;
-    const uint4 v = make_uint4(w, w, w, w);
-    for (; p + 16u <= b1; p += 16u) *(uint4 *)(out + p) = v;
-    for (; p < b1; p++) out[p] = c;
+    const uint64_t w2 = ((uint64_t)w << 32) | w;
+    uint8_t *p = out + b0;
+    uint32_t r = b1 - b0;
+    // a piece is skipped only when fewer bytes are left, so p stays aligned
+    // to every smaller piece
+    if (((uintptr_t)p & 1u) && r >= 1u) { *p = c; p += 1; r -= 1; }
+    if (((uintptr_t)p & 2u) && r >= 2u) { *(uint16_t *)p = (uint16_t)w; p += 2; r -= 2; }
+    if (((uintptr_t)p & 4u) && r >= 4u) { *(uint32_t *)p = w; p += 4; r -= 4; }
+    if (((uintptr_t)p & 8u) && r >= 8u) { *(uint64_t *)p = w2; p += 8; r -= 8; }
+    for (; r >= 16u; p += 16, r -= 16) *(uint4 *)p = make_uint4(w, w, w, w);
+    if (r & 8u) { *(uint64_t *)p = w2; p += 8; }
+    if (r & 4u) { *(uint32_t *)p = w; p += 4; }
+    if (r & 2u) { *(uint16_t *)p = (uint16_t)w; p += 2; }
+    if (r & 1u) *p = c;
 }
 
-__global__ void k_run_fill_groups(uint8_t *out, uint32_t n, const uint32_t *goff, uint32_t G, const uint16_t *gchar,
-                                  const uint8_t *gmix, uint32_t *longs, uint32_t long_cap, uint32_t *flags)
+__global__ void k_run_fill_groups(uint8_t *out, uint32_t n, const uint2 *stat, uint32_t N, uint32_t *longs,
+                                  uint32_t long_cap, uint32_t *flags)
 {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G || gmix[g]) return;
-    const uint32_t b0 = goff[g], b1 = goff[g + 1];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= N) return;
+    const uint2 s = stat[t];
+    if (s.y > 0xFFu) return;                  // mixed, or no group's head
+    const uint32_t b0 = s.x, b1 = t + 1u < N ? stat[t + 1u].x : n;
     if (b1 < b0 || b1 > n) { atomicOr(flags, ERR_INTERNAL); return; }
     if (b1 - b0 > RF_LONG) {
         const uint32_t i = atomicAdd(flags + 5, 1u);
-        if (i < long_cap) longs[i] = g;
+        if (i < long_cap) longs[i] = t;
         else atomicOr(flags, ERR_INTERNAL);
         return;
     }
-    fill_run(out, b0, b1, (uint8_t)gchar[g]);
+    fill_run(out, b0, b1, (uint8_t)s.y);
 }
 
 // One CTA per listed long run (the count is read on the device: no host sync).
-__global__ void k_run_fill_long(uint8_t *out, const uint32_t *goff, const uint16_t *gchar, const uint32_t *longs,
+__global__ void k_run_fill_long(uint8_t *out, uint32_t n, const uint2 *stat, uint32_t N, const uint32_t *longs,
                                 const uint32_t *nlong, uint32_t long_cap)
 {
     const uint32_t cnt = min(*nlong, long_cap);
     for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-        const uint32_t g = longs[i];
-        const uint32_t b0 = goff[g], b1 = goff[g + 1];
-        const uint8_t c = (uint8_t)gchar[g];
+        const uint32_t t = longs[i];
+        const uint32_t b0 = stat[t].x, b1 = t + 1u < N ? stat[t + 1u].x : n;
+        const uint8_t c = (uint8_t)stat[t].y;
         // head bytes to the first 16-byte boundary, then striped 16-byte stores
         uint32_t a0 = b0;
         while (a0 < b1 && (((uintptr_t)(out + a0)) & 15u)) a0++;
@@ -368,7 +420,8 @@ __global__ void k_run_fill_long(uint8_t *out, const uint32_t *goff, const uint16
 // its block is the group g0 of phrase 0 taken whole; inside a block the rows
 // follow the rank of the next parse suffix (last phrase: -1, K:787-807).
 struct PrimaryArgs {
-    const uint32_t *pid, *pisa, *doff, *dlen, *grp_of, *goff;
+    const uint32_t *pid, *pisa, *doff, *dlen, *isa;
+    const uint2 *stat;
     uint32_t z;
     uint32_t *counter;
 };
@@ -376,11 +429,11 @@ __global__ void k_primary_index(PrimaryArgs a)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t q0 = a.pid[0], len0 = a.dlen[q0];
-    const uint32_t g0 = a.grp_of[a.doff[q0]];
+    const uint32_t g0 = a.isa[a.doff[q0]];
     bool before = false;
     if (k < a.z && k != 0) {
         const uint32_t q = a.pid[k], lq = a.dlen[q];
-        if (lq >= len0 && a.grp_of[a.doff[q] + lq - len0] == g0) {
+        if (lq >= len0 && a.isa[a.doff[q] + lq - len0] == g0) {
             const int64_t nr0 = a.z > 1 ? (int64_t)a.pisa[1] : -1;
             const int64_t nrk = k + 1 < a.z ? (int64_t)a.pisa[k + 1] : -1;
             before = nrk < nr0;
@@ -388,7 +441,7 @@ __global__ void k_primary_index(PrimaryArgs a)
     }
     const unsigned m = __ballot_sync(0xFFFFFFFFu, before);
     if ((threadIdx.x & 31u) == 0 && m) atomicAdd(a.counter, (uint32_t)__popc(m));
-    if (k == 0) atomicAdd(a.counter, a.goff[g0]);
+    if (k == 0) atomicAdd(a.counter, a.stat[g0].x);
 }
 
 template <typename E>
@@ -424,11 +477,17 @@ uint32_t run_group_index(Storage *st, Phrases &ph, DictOrder &dord, int W, uint3
 {
     const uint32_t N = (uint32_t)ph.dict_bytes;
     PosInfo pi{ph.dphr, ph.doff, ph.dlen};
-    uint32_t *gid = nullptr;
-    const uint32_t G = group_numbers(st, ph, dord, W, gid);
+    uint8_t *mark = slot<uint8_t>(st, S_MB, N);
+    uint32_t *gid = slot<uint32_t>(st, S_TMP0, N);
+    check_cuda(cudaMemsetAsync(mark, 0, N, st->stream));
+    k_mark_sheads<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, mark);
+    after_launch(st);
+    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
+    device_scan<uint32_t, OpAdd>(st, N, LoadMark{mark}, StoreGid{gid}, true, (uint32_t *)st->d_scalars);
+    fetch_scalars(st, 1);
+    const uint32_t G = (uint32_t)st->h_scalars[0];
     grp_of = slot<uint32_t>(st, S_GRP, N);
-    k_group_of<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, gid, grp_of, nullptr,
-                                                         nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_group_of<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, gid, grp_of);
     after_launch(st);
     return G;
 }
@@ -438,52 +497,40 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
 {
     const uint32_t N = (uint32_t)ph.dict_bytes;
     PosInfo pi{ph.dphr, ph.doff, ph.dlen};
-    // groups: at most one per dictionary position
-    uint32_t *gcount = slot<uint32_t>(st, S_GCOUNT, N);
-    uint16_t *gchar = slot<uint16_t>(st, S_GCHAR, N);
-    uint32_t *grp_of = slot<uint32_t>(st, S_GRP, N);
-    uint32_t *gid = nullptr;
-    const uint32_t G = group_numbers(st, ph, dord, W, gid);
-    if (G == 0) throw Error{GBWT_INTERNAL_ERROR};
-    check_cuda(cudaMemsetAsync(gcount, 0, (size_t)G * 4, st->stream));
-    k_group_of<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, gid, grp_of, ph.dict, ph.occ,
-                                                         ph.pcmin, ph.pcmax, gcount, gchar);
+    uint2 *stat = slot<uint2>(st, S_GCOUNT, (size_t)N + 1);
+    check_cuda(cudaMemsetAsync(stat, 0, (size_t)N * sizeof(uint2), st->stream));
+    k_group_stats<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, ph.dict, ph.occ, ph.pcmin,
+                                                            ph.pcmax, stat);
     after_launch(st);
-    uint8_t *gmix = slot<uint8_t>(st, S_GMIX, G);
-    check_cuda(cudaMemsetAsync(gmix, 0, G, st->stream));
-    k_mark_mixed<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, ph.dict, ph.pcmin, ph.pcmax, grp_of,
-                                                           gchar, gmix);
-    after_launch(st);
-    uint32_t *goff = slot<uint32_t>(st, S_GOFF, (size_t)G + 1);
-    device_scan<uint32_t, OpAdd>(st, G, LoadGCount{gcount}, StoreArr<uint32_t>{goff}, false, goff + G);
-    uint32_t *mixidx = slot<uint32_t>(st, S_MIXIDX, G);
-    uint32_t *delta = slot<uint32_t>(st, S_DELTA, G);
-    check_cuda(cudaMemsetAsync(st->d_scalars + 1, 0, 8, st->stream));
-    device_scan<uint64_t, OpAdd>(st, G, LoadMixPair{gcount, gmix}, StoreMix{gmix, goff, mixidx, delta}, false,
-                                 (uint64_t *)(st->d_scalars + 1));
-    check_cuda(cudaMemcpyAsync(st->d_scalars + 2, goff + G, 4, cudaMemcpyDeviceToDevice, st->stream));
+    const size_t nw = ((size_t)N + 31) / 32;
+    uint32_t *heads = slot<uint32_t>(st, S_TMP0, nw), *mixed = slot<uint32_t>(st, S_TMP1, nw);
+    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 32, st->stream));
+    device_scan<uint32_t, OpAdd>(st, N, LoadGCount{stat}, StoreGroup{stat, N, heads, mixed}, false,
+                                 (uint32_t *)st->d_scalars);
+    // a mixed block has at least two bytes
+    uint32_t *delta = slot<uint32_t>(st, S_DELTA, (size_t)(N < n / 2 ? N : n / 2) + 1);
+    device_scan<Sum4, OpAdd>(st, nw, LoadMixWord{stat, heads, mixed}, StoreMixWord{stat, mixed, delta}, false,
+                             (Sum4 *)(st->d_scalars + 1));
     fetch_scalars(st, 3);
-    const uint32_t B = (uint32_t)(st->h_scalars[1] >> 32);
-    const uint32_t M = (uint32_t)st->h_scalars[1];
-    const uint32_t total = (uint32_t)st->h_scalars[2];
-    if (total != n) throw Error{GBWT_INTERNAL_ERROR};
+    const uint32_t total = (uint32_t)st->h_scalars[0], M = (uint32_t)st->h_scalars[1];
+    const uint32_t B = (uint32_t)(st->h_scalars[1] >> 32), G = (uint32_t)st->h_scalars[2];
+    if (total != n || G == 0) throw Error{GBWT_INTERNAL_ERROR};
     st->stats.s = G;
     st->stats.mixed_blocks = B;
     st->stats.mixed_elems = M;
     stage_mark(st, 4);
 
     k_primary_index<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(
-        PrimaryArgs{ph.pid, pord.isa, ph.doff, ph.dlen, grp_of, goff, ph.z, st->d_flags + 2});
+        PrimaryArgs{ph.pid, pord.isa, ph.doff, ph.dlen, dord.isa, stat, ph.z, st->d_flags + 2});
     after_launch(st);
     const uint32_t long_cap = n / RF_LONG + 1u;
     uint32_t *longs = slot<uint32_t>(st, S_TILEG, long_cap);
     check_cuda(cudaMemsetAsync(st->d_flags + 5, 0, 4, st->stream));
     probe_begin(st, GBWT_PROBE_RUN_FILL);
-    k_run_fill_groups<<<grid_for(G, 256), 256, 0, st->stream>>>(dOut, n, goff, G, gchar, gmix, longs, long_cap,
-                                                                st->d_flags);
-    probe_end(st, GBWT_PROBE_RUN_FILL, (uint64_t)(n - M) + 7ull * G);
+    k_run_fill_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(dOut, n, stat, N, longs, long_cap, st->d_flags);
+    probe_end(st, GBWT_PROBE_RUN_FILL, (uint64_t)(n - M) + 8ull * N);
     after_launch(st);
-    k_run_fill_long<<<st->num_sms * 4, 256, 0, st->stream>>>(dOut, goff, gchar, longs, st->d_flags + 5, long_cap);
+    k_run_fill_long<<<st->num_sms * 4, 256, 0, st->stream>>>(dOut, n, stat, N, longs, st->d_flags + 5, long_cap);
     after_launch(st);
     stage_mark(st, 5);
     if (B == 0) return;
@@ -492,8 +539,15 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     uint32_t *moff = slot<uint32_t>(st, S_MOFF, (size_t)ph.d + 1);
     uint32_t *mb = slot<uint32_t>(st, S_MB, N);
     uint16_t *mc = slot<uint16_t>(st, S_MC, N);
-    device_scan<uint32_t, OpAdd>(st, N, LoadMixEntry{pi, (uint32_t)W, grp_of, gmix},
-                                 StoreMixEntry{pi, ph.dict, grp_of, mixidx, moff, mb, mc}, false, moff + ph.d);
+    uint32_t *words = slot<uint32_t>(st, S_TMP2, nw), *pre = heads;      // heads are counted
+    k_mix_flags<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, mixed, words);
+    after_launch(st);
+    device_scan<uint32_t, OpAdd>(st, nw, LoadPopc{words}, StoreArr<uint32_t>{pre}, false, moff + ph.d);
+    k_mix_offsets<<<grid_for(ph.d, 256), 256, 0, st->stream>>>(ph.d, ph.doff, words, pre, moff);
+    after_launch(st);
+    k_mix_entries<<<grid_for(N, 256), 256, 0, st->stream>>>(N, ph.dphr, ph.doff, ph.dict, dord.isa, stat, words, pre,
+                                                            mb, mc);
+    after_launch(st);
     if (B < (1u << 24)) mixed_blocks<uint32_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut);
     else mixed_blocks<uint64_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut);
 }
