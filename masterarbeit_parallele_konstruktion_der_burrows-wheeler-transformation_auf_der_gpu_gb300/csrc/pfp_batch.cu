@@ -155,7 +155,8 @@ struct BatchLayout {
     uint32_t tiles = 0;             // padded element tiles
     uint32_t max_local = 1;         // most texts in one segment
     // word offsets into h_meta / the device copy
-    size_t o_xstart = 0, o_ioff = 0, o_pshift = 0, o_tloc = 0, o_tseg = 0, o_tout = 0, words = 0;
+    size_t o_xstart = 0, o_ioff = 0, o_pshift = 0, o_tloc = 0, o_tseg = 0, o_tout = 0, o_sid = 0, words = 0;
+    uint32_t segs = 0;
 };
 
 // Text-major order of the parse suffix array: stable partition by text.
@@ -376,7 +377,8 @@ static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, 
     bl.o_tloc = bl.o_pshift + kk;
     bl.o_tseg = (bl.o_tloc + kk + 1) & ~(size_t)1;      // 8-byte aligned uint2 arrays
     bl.o_tout = bl.o_tseg + 2 * (size_t)bl.tiles;
-    bl.words = bl.o_tout + 2 * (size_t)bl.tiles;
+    bl.o_sid = bl.o_tout + 2 * (size_t)bl.tiles;
+    bl.words = bl.o_sid + (size_t)bl.tiles;
     if (st->h_meta_cap < bl.words) {
         if (st->h_meta) check_cuda(cudaFreeHost(st->h_meta));
         st->h_meta = nullptr;
@@ -387,7 +389,7 @@ static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, 
     }
     uint32_t *h = st->h_meta;
     uint32_t *xs = h + bl.o_xstart, *io = h + bl.o_ioff, *ps = h + bl.o_pshift, *tl = h + bl.o_tloc;
-    uint32_t *tseg = h + bl.o_tseg, *tout = h + bl.o_tout;
+    uint32_t *tseg = h + bl.o_tseg, *tout = h + bl.o_tout, *sid = h + bl.o_sid;
     uint32_t i = 0, seg_first_text = 0, tile = 0;
     uint64_t x = 0, seg_obase = 0;
     seg_real = 0;
@@ -398,7 +400,9 @@ static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, 
             tseg[2 * (tile + b) + 1] = nt;
             tout[2 * (tile + b)] = (uint32_t)seg_obase;
             tout[2 * (tile + b) + 1] = (uint32_t)seg_real;
+            sid[tile + b] = bl.segs;
         }
+        bl.segs++;
         const uint32_t ntext = last_text - seg_first_text;
         if (ntext > bl.max_local) bl.max_local = ntext;
         // element position = output position + padding of earlier segments
@@ -445,6 +449,7 @@ static void batch_output(Storage *st, const BatchLayout &bl, const uint32_t *dme
                                                            M, st->d_flags, emx, pos);
     after_launch(st);
     const uint2 *tseg = (const uint2 *)(dmeta + bl.o_tseg);
+    const RsSegs sg{tseg, dmeta + bl.o_sid, bl.segs};
     // sort by (text, group) only: the byte rides along, and elements of one
     // group keep their parse-suffix order.  9-bit digits when they save a
     // pass (e.g. 25 group bits: 3 passes instead of 4); wider digits make the
@@ -456,15 +461,15 @@ static void batch_output(Storage *st, const BatchLayout &bl, const uint32_t *dme
     // keys-only passes rank every k-th item with ballots (uniform group
     // digits make the match-only ranking pipe-bound; tuning knob)
     const int bal = st->tuning.batch_ballot ? st->tuning.batch_ballot : 3;
-    if (aux) radix_sort<E, true, 8>(st, elem, elem_alt, pos, pos_alt, M, bb, bb + sb, tseg);
+    if (aux) radix_sort<E, true, 8>(st, elem, elem_alt, pos, pos_alt, M, bb, bb + sb, sg);
     else if (nine) {
-        if (bal == 2) radix_sort<E, false, 9, 2>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
-        else if (bal == 3) radix_sort<E, false, 9, 3>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
-        else radix_sort<E, false, 9, 0>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
+        if (bal == 2) radix_sort<E, false, 9, 2>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
+        else if (bal == 3) radix_sort<E, false, 9, 3>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
+        else radix_sort<E, false, 9, 0>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
     } else {
-        if (bal == 2) radix_sort<E, false, 8, 2>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
-        else if (bal == 3) radix_sort<E, false, 8, 3>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
-        else radix_sort<E, false, 8, 0>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, tseg);
+        if (bal == 2) radix_sort<E, false, 8, 2>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
+        else if (bal == 3) radix_sort<E, false, 8, 3>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
+        else radix_sort<E, false, 8, 0>(st, elem, elem_alt, nv, nv2, M, bb, bb + sb, sg);
     }
     stage_mark(st, 5);
     k_bextract<E><<<bl.tiles, 256, 0, st->stream>>>(elem, tseg, (const uint2 *)(dmeta + bl.o_tout), codes + 256,

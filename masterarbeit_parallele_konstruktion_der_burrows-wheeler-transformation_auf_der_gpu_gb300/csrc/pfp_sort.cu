@@ -100,12 +100,6 @@ __global__ void k_text_endmap(const uint32_t *zend, uint32_t k, uint32_t *endmap
     atomicOr(endmap + (e >> 11), 1u << ((e >> 6) & 31u));
 }
 
-__global__ void k_iota(uint32_t *v, uint32_t n)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = i;
-}
-
 // Active test after a round whose prefix length is now `h`.
 template <typename Rem>
 struct ActiveTest {
@@ -959,9 +953,7 @@ static int prefix_doubling(Storage *st, uint32_t N, int key0_bits, uint32_t h0, 
     uint32_t *act_x2 = slot<uint32_t>(st, S_ACTX2, N);   // next active list
     uint32_t *act_g2 = slot<uint32_t>(st, S_ACTG2, N);
 
-    k_iota<<<grid_for(N, 256), 256, 0, st->stream>>>(vals, N);
-    after_launch(st);
-    radix_sort<uint64_t, true>(st, keys, keys_alt, vals, vals_alt, N, 0, key0_bits);
+    radix_sort<uint64_t, true>(st, keys, keys_alt, vals, vals_alt, N, 0, key0_bits, RsSegs(), true);
     ActiveTest<Rem> at{keys, vals, N, h0, rem};
     check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     // the words take 16 bytes per 32 elements of the alternate key buffer,

@@ -61,6 +61,46 @@ __device__ __forceinline__ uint32_t ub_ruler_index(const uint32_t *rul, uint32_t
     return lo;
 }
 
+// Symbol counts of every tile, digit-major over the tiles.
+__global__ void __launch_bounds__(RS_THREADS) k_byte_hist(const uint8_t *__restrict__ keys, uint32_t n,
+                                                          uint32_t *__restrict__ tile_hist, uint32_t num_tiles)
+{
+    constexpr int D = 256;
+    __shared__ uint32_t h[RS_WARPS * D];       // one histogram per warp
+    for (int d = threadIdx.x; d < RS_WARPS * D; d += RS_THREADS) h[d] = 0;
+    __syncthreads();
+    uint32_t *wh = h + (threadIdx.x >> 5) * D;
+    const size_t base = (size_t)blockIdx.x * RS_TILE;
+    constexpr int KPV = 16;                          // symbols per 16-byte load
+    constexpr int NV = RS_ITEMS / KPV;
+    if (base + RS_TILE <= n && (((uintptr_t)keys) & 15u) == 0) {
+        // full tile: every load issued before any count (counting needs no order)
+        uint4 v[NV];
+#pragma unroll
+        for (int j = 0; j < NV; j++) v[j] = __ldg((const uint4 *)(keys + base) + (size_t)j * RS_THREADS + threadIdx.x);
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+            uint8_t kk[KPV];
+            memcpy(kk, &v[j], 16);
+#pragma unroll
+            for (int q = 0; q < KPV; q++) atomicAdd(&wh[kk[q]], 1u);
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < RS_ITEMS; j++) {
+            size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
+            if (i < n) atomicAdd(&wh[keys[i]], 1u);
+        }
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < D; d += RS_THREADS) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; w++) sum += h[w * D + d];
+        tile_hist[(size_t)d * num_tiles + blockIdx.x] = sum;
+    }
+}
+
 // LF of every row.  Element e of Lc is row e (e < i) or e+1 (e >= i).  An
 // entry whose target row is a ruler holds UB_RULER | the ruler's index.
 template <int BITS>
@@ -256,7 +296,7 @@ void run_unbwt(Storage *st, const uint8_t *dLc, uint32_t n, uint32_t i, uint8_t 
     // LF
     const uint32_t num_tiles = (uint32_t)(((size_t)n + RS_TILE - 1) / RS_TILE);
     uint32_t *hist = slot<uint32_t>(st, S_RSHIST, (size_t)256 * num_tiles);
-    k_rs_upsweep<uint8_t, 8><<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, 0, 0xFFu, hist, num_tiles, nullptr);
+    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, hist, num_tiles);
     after_launch(st);
     device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
                                  (uint32_t *)nullptr);

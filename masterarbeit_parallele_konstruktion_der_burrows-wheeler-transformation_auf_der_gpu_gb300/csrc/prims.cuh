@@ -4,12 +4,9 @@
 // stores so that flags, compaction and segmented heads are computed on the
 // fly instead of being materialised.
 //
-// Radix sort: stable LSD passes over 8-bit digits.  Each pass runs a tile
-// histogram (per-warp shared atomics), a digit-major exclusive scan of the
-// tile histograms, and a scatter kernel that ranks keys inside each warp with
-// __match_any_sync multisplit, reorders the tile in shared memory and writes
-// each digit's run with consecutive addresses.  (Measured on GB300: atomics
-// beat match-aggregation for counting; for the stable ranking, match beats a
+// Radix sort: stable LSD passes over 8-bit digits.  A pass ranks keys inside each warp with __match_any_sync multisplit, reorders the
+// tile in shared memory and writes each digit's run with consecutive
+// addresses.  (Measured on GB300: for the stable ranking, match beats a
 // ballot-per-bit multisplit, whose ALU cost exceeds the match pipe's.)
 #pragma once
 #include "gbwt_internal.cuh"
@@ -364,7 +361,23 @@ void device_scan(Storage *st, size_t n, Load load, Store store, bool inclusive, 
 }
 
 // ---------------------------------------------------------------------
-// Stable LSD radix sort
+// Stable LSD radix sort, in two forms.
+//
+// Up to two tiles per SM (one wave): one kernel counts the digits of every
+// pass in one read of the keys, and each pass is one kernel in which a tile
+// counts its digits, publishes the counts and looks back over the tiles before
+// it, digit by digit (onesweep: Adinets & Merrill 2022, "Onesweep: a faster
+// least significant digit radix sort for GPUs").  A single tile needs no
+// counts either: one launch per pass.
+//
+// Above that: a tile histogram, a scan of all tile histograms and a scatter
+// per pass.  The look-back then costs more than the launches: tiles of 4096
+// keys leave at 40 to 80 a microsecond, and with an L2 read of about 0.7 us
+// between the dies every digit walks back over tens of tiles.
+//
+// Measured, 40-bit keys with values in 5 passes, look-back / histograms: 1 M
+// keys (20 to 100 tiles) 89..102 / 124 us, 168 tiles 135 / 163 us, 300 tiles 162
+// / 165 us, 1500 tiles 569 / 557 us; per pass of 243 M 32-bit keys 1541 / 890 us.
 // ---------------------------------------------------------------------
 constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 16;
@@ -403,22 +416,30 @@ __device__ __forceinline__ unsigned rs_peers_ballot(uint32_t d)
 }
 
 
+// A segmented sort: the tiles are grouped into segments of whole tiles that
+// are sorted on their own.
+struct RsSegs {
+    const uint2 *tseg = nullptr;      // per tile: {first tile, tiles} of its segment (null: one segment)
+    const uint32_t *sid = nullptr;    // per tile: number of its segment
+    uint32_t nseg = 1;
+};
+
 // Histogram slot of digit d for tile b.  Unsegmented: digit-major over all
 // tiles.  Segmented (tseg[b] = {first tile, tiles} of b's segment, every
 // segment a whole number of tiles): segment-major, then digit-major inside
 // the segment, so one exclusive scan gives every tile its offsets inside its
 // own segment and each pass sorts the segments independently.
-__device__ __forceinline__ size_t rs_hist_index(const uint2 *tseg, uint32_t b, uint32_t d, uint32_t num_tiles, int D)
+__device__ __forceinline__ size_t rs_hist_index(const RsSegs &sg, uint32_t b, uint32_t d, uint32_t num_tiles, int D)
 {
-    if (!tseg) return (size_t)d * num_tiles + b;
-    const uint2 q = tseg[b];
+    if (!sg.tseg) return (size_t)d * num_tiles + b;
+    const uint2 q = sg.tseg[b];
     return (size_t)q.x * D + (size_t)d * q.y + (b - q.x);
 }
 
 template <typename K, int BITS>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *__restrict__ keys, uint32_t n, int shift,
                                                            uint32_t mask, uint32_t *__restrict__ tile_hist,
-                                                           uint32_t num_tiles, const uint2 *__restrict__ tseg)
+                                                           uint32_t num_tiles, RsSegs sg)
 {
     constexpr int D = 1 << BITS;
     __shared__ uint32_t h[RS_WARPS * D];       // one histogram per warp
@@ -452,23 +473,100 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *__restrict__
         uint32_t sum = 0;
 #pragma unroll
         for (int w = 0; w < RS_WARPS; w++) sum += h[w * D + d];
-        tile_hist[rs_hist_index(tseg, blockIdx.x, d, num_tiles, D)] = sum;
+        tile_hist[rs_hist_index(sg, blockIdx.x, d, num_tiles, D)] = sum;
     }
+}
+
+// Digit counts of all `np` passes: hist[(p * nseg + segment) * D + digit].  A
+// CTA counts RH_TILES consecutive tiles at a time in shared memory (several
+// copies: the digits of a small alphabet repeat) and adds to the global counts
+// when the segment changes and at its end.
+constexpr int RH_TILES = 8;
+template <typename K, int BITS>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K *__restrict__ keys, uint32_t n, int begin_bit,
+                                                        int end_bit, RsSegs sg, uint32_t num_tiles,
+                                                        uint32_t *__restrict__ hist)
+{
+    constexpr int D = 1 << BITS;
+    constexpr int PMAX = ((int)sizeof(K) * 8 + BITS - 1) / BITS;
+    constexpr int FIT = 32768 / (PMAX * D * 4);
+    constexpr int COPIES = FIT >= 4 ? 4 : FIT >= 2 ? 2 : 1;
+    __shared__ uint32_t h[COPIES * PMAX * D];
+    const int np = (end_bit - begin_bit + BITS - 1) / BITS;
+    for (int i = threadIdx.x; i < COPIES * PMAX * D; i += RS_THREADS) h[i] = 0;
+    __syncthreads();
+    uint32_t *mine = h + ((threadIdx.x >> 5) % COPIES) * (PMAX * D);
+    const uint32_t chunks = (num_tiles + RH_TILES - 1) / RH_TILES;
+    uint32_t cur = 0xFFFFFFFFu;               // segment whose counts are in shared memory
+    auto flush = [&]() {
+        __syncthreads();
+        for (int i = threadIdx.x; i < np * D; i += RS_THREADS) {
+            uint32_t c = 0;
+#pragma unroll
+            for (int k = 0; k < COPIES; k++) {
+                c += h[k * (PMAX * D) + i];
+                h[k * (PMAX * D) + i] = 0;
+            }
+            const uint32_t pass = (uint32_t)i / D, d = (uint32_t)i % D;
+            if (c) atomicAdd(hist + ((size_t)pass * sg.nseg + cur) * D + d, c);
+        }
+        __syncthreads();
+    };
+    auto count = [&](K k) {
+        for (int p = 0; p < np; p++) {
+            const int shift = begin_bit + p * BITS;
+            const int bits = end_bit - shift < BITS ? end_bit - shift : BITS;
+            atomicAdd(&mine[p * D + rs_digit(k, shift, (1u << bits) - 1u)], 1u);
+        }
+    };
+    constexpr int KPV = 16 / (int)sizeof(K);          // keys per 16-byte load
+    constexpr int NV = RS_ITEMS / KPV;
+    const bool aligned = (((uintptr_t)keys) & 15u) == 0;
+    for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        for (uint32_t b = c * RH_TILES; b < num_tiles && b < (c + 1) * RH_TILES; b++) {
+            const uint32_t s = sg.sid ? sg.sid[b] : 0u;
+            if (s != cur) {
+                if (cur != 0xFFFFFFFFu) flush();
+                cur = s;
+            }
+            const size_t base = (size_t)b * RS_TILE;
+            if (aligned && base + RS_TILE <= n) {
+                uint4 v[NV];
+#pragma unroll
+                for (int j = 0; j < NV; j++)
+                    v[j] = __ldg((const uint4 *)(keys + base) + (size_t)j * RS_THREADS + threadIdx.x);
+#pragma unroll
+                for (int j = 0; j < NV; j++) {
+                    K kk[KPV];
+                    memcpy(kk, &v[j], 16);
+#pragma unroll
+                    for (int q = 0; q < KPV; q++) count(kk[q]);
+                }
+            } else {
+                for (int j = 0; j < RS_ITEMS; j++) {
+                    const size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
+                    if (i < n) count(keys[i]);
+                }
+            }
+        }
+    }
+    if (cur != 0xFFFFFFFFu) flush();
 }
 
 template <typename K, bool HAS_VAL, int BITS>
 constexpr size_t rs_smem_bytes()
 {
     return (size_t)RS_TILE * sizeof(K) + (HAS_VAL ? (size_t)RS_TILE * 4 : 0) + (size_t)RS_WARPS * (1 << BITS) * 4 +
-           (size_t)(1 << BITS) * 4 * 2 + 32 * 4;
+           (size_t)(1 << BITS) * 4 * 2 + 32 * 8;
 }
 
+// Scatter of one pass, places from the scanned tile histograms.
 template <typename K, bool HAS_VAL, int BITS, int BALLOT>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict__ kin, K *__restrict__ kout,
                                                              const uint32_t *__restrict__ vin,
                                                              uint32_t *__restrict__ vout, uint32_t n, int shift,
                                                              uint32_t mask, const uint32_t *__restrict__ tile_off,
-                                                             uint32_t num_tiles, const uint2 *__restrict__ tseg)
+                                                             uint32_t num_tiles, RsSegs sg)
 {
     constexpr int D = 1 << BITS;
     constexpr int DPT = D / RS_THREADS;       // digits per thread in the per-digit phase
@@ -495,7 +593,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
         size_t idx = wbase + (size_t)i * 32 + lane;
         bool valid = idx < n;
         k[i] = valid ? kin[idx] : K(0);
-        if (HAS_VAL) v[i] = valid ? vin[idx] : 0u;
+        if (HAS_VAL) v[i] = !vin ? (uint32_t)idx : valid ? vin[idx] : 0u;
         dg[i] = valid ? rs_digit(k[i], shift, mask) : 0xFFFFFFFFu;
     }
     uint32_t *wh = s_wh + warp * D;
@@ -542,7 +640,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
             const uint32_t d = threadIdx.x * DPT + e;
             s_dstart[d] = ex;
             ex += cnt[e];
-            s_goff[d] = tile_off[rs_hist_index(tseg, blockIdx.x, d, num_tiles, D)];
+            s_goff[d] = tile_off[rs_hist_index(sg, blockIdx.x, d, num_tiles, D)];
         }
     }
     __syncthreads();
@@ -565,38 +663,222 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
     }
 }
 
+// One pass by look-back.  status[tile * D + digit] is a look-back word: the
+// tile's own count (LB_TOTAL) or the count up to and including the tile
+// (LB_PREFIX).  Counts are published before the tile is reordered in shared
+// memory, so most predecessors have theirs in place when the look-back
+// starts.  A single tile needs neither counts nor look-back.
+template <typename K, bool HAS_VAL, int BITS, int BALLOT>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ kin, K *__restrict__ kout,
+                                                        const uint32_t *__restrict__ vin,
+                                                        uint32_t *__restrict__ vout, uint32_t n, int shift,
+                                                        uint32_t mask, const uint32_t *__restrict__ hist, RsSegs sg,
+                                                        LookBack lb)
+{
+    constexpr int D = 1 << BITS;
+    constexpr int DPT = D / RS_THREADS;       // digits per thread in the per-digit phases
+    extern __shared__ __align__(16) unsigned char rs_smem[];
+    K *s_k = (K *)rs_smem;
+    uint32_t *s_v = (uint32_t *)(s_k + RS_TILE);
+    uint32_t *s_wh = HAS_VAL ? s_v + RS_TILE : s_v;
+    uint32_t *s_dstart = s_wh + RS_WARPS * D;
+    uint32_t *s_goff = s_dstart + D;
+    uint64_t *s_scan = (uint64_t *)(s_goff + D);
+
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t tile = 0;
+    if (gridDim.x > 1 && threadIdx.x == 0) {
+        tile = atomicAdd(lb.ticket, 1u);
+        if (tile == gridDim.x - 1) *lb.ticket = 0;
+        s_dstart[0] = tile;
+    }
+    for (int i = threadIdx.x; i < RS_WARPS * D; i += RS_THREADS) s_wh[i] = 0;
+    __syncthreads();
+    if (gridDim.x > 1) tile = s_dstart[0];
+
+    const size_t tile_base = (size_t)tile * RS_TILE;
+    const size_t wbase = tile_base + (size_t)warp * (RS_ITEMS * 32);
+    K k[RS_ITEMS];
+    uint32_t v[RS_ITEMS];
+    uint32_t rk[RS_ITEMS];
+    uint32_t dg[RS_ITEMS];
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; i++) {
+        size_t idx = wbase + (size_t)i * 32 + lane;
+        bool valid = idx < n;
+        k[i] = valid ? kin[idx] : K(0);
+        if (HAS_VAL) v[i] = !vin ? (uint32_t)idx : valid ? vin[idx] : 0u;
+        dg[i] = valid ? rs_digit(k[i], shift, mask) : 0xFFFFFFFFu;
+    }
+    uint32_t *wh = s_wh + warp * D;
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; i++) {
+        // the lowest lane of each digit class reads and advances the warp's
+        // counter; the others take the old value from it
+        const uint32_t d = dg[i];
+        const unsigned peers = (BALLOT > 0 && i % (BALLOT > 0 ? BALLOT : 1) == (BALLOT > 0 ? BALLOT - 1 : 0))
+                                   ? rs_peers_ballot<BITS>(d)
+                                   : __match_any_sync(0xFFFFFFFFu, d);
+        const unsigned leader = (unsigned)(__ffs(peers) - 1);
+        uint32_t prior = 0;
+        if (lane == leader && d != 0xFFFFFFFFu) {
+            prior = wh[d];
+            wh[d] = prior + (uint32_t)__popc(peers);
+        }
+        prior = __shfl_sync(0xFFFFFFFFu, prior, leader);
+        rk[i] = prior + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread t owns digits [t*DPT, t*DPT + DPT): the tile's counts (low words)
+    // and the segment's (high words) scanned together
+    uint2 q = make_uint2(0u, gridDim.x);
+    uint32_t seg = 0;
+    if (sg.tseg) { q = sg.tseg[tile]; seg = sg.sid[tile]; }
+    uint32_t cnt[DPT], gbase[DPT];
+    {
+        uint64_t both[DPT], sum = 0;
+#pragma unroll
+        for (int e = 0; e < DPT; e++) {
+            const uint32_t d = threadIdx.x * DPT + e;
+            uint32_t run = 0;
+#pragma unroll
+            for (int w = 0; w < RS_WARPS; w++) {
+                uint32_t c = s_wh[w * D + d];
+                s_wh[w * D + d] = run;
+                run += c;
+            }
+            cnt[e] = run;
+            if (q.y > 1) {
+                lb_store(lb.status + (size_t)tile * D + d,
+                         ((uint64_t)((lb.seq << 2) | (tile == q.x ? LB_PREFIX : LB_TOTAL)) << 32) | run);
+                both[e] = ((uint64_t)hist[(size_t)seg * D + d] << 32) | run;
+            } else {
+                both[e] = ((uint64_t)run << 32) | run;       // alone in its segment
+            }
+            sum += both[e];
+        }
+        uint64_t total;
+        uint64_t ex = block_excl_scan<uint64_t, OpAdd>(sum, total, OpAdd(), s_scan);
+#pragma unroll
+        for (int e = 0; e < DPT; e++) {
+            s_dstart[threadIdx.x * DPT + e] = (uint32_t)ex;
+            gbase[e] = q.x * (uint32_t)RS_TILE + (uint32_t)(ex >> 32);
+            ex += both[e];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RS_ITEMS; i++) {
+        if (dg[i] != 0xFFFFFFFFu) {
+            uint32_t lp = s_dstart[dg[i]] + s_wh[warp * D + dg[i]] + rk[i];
+            s_k[lp] = k[i];
+            if (HAS_VAL) s_v[lp] = v[i];
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < DPT; e++) {
+        const uint32_t d = threadIdx.x * DPT + e;
+        uint32_t pre = 0;
+        if (tile != q.x) {
+            uint32_t p = tile, polls = 0;
+            for (;;) {
+                const uint64_t w = lb_load(lb.status + (size_t)(p - 1u) * D + d);
+                const uint32_t tag = (uint32_t)(w >> 32);
+                if ((tag >> 2) != lb.seq) {
+                    // never runs out (tickets, see above); places only shrink, the host refuses the result
+                    if (++polls >= LB_MAX_POLLS) { *(volatile uint32_t *)lb.err = 1u; break; }
+                    continue;
+                }
+                pre += (uint32_t)w;
+                p--;
+                if ((tag & 3u) == LB_PREFIX) break;
+            }
+            lb_store(lb.status + (size_t)tile * D + d,
+                     ((uint64_t)((lb.seq << 2) | LB_PREFIX) << 32) | (pre + cnt[e]));
+        }
+        s_goff[d] = gbase[e] + pre - s_dstart[d];
+    }
+    __syncthreads();
+    const uint32_t tile_n = (uint32_t)(((size_t)n - tile_base) < (size_t)RS_TILE ? ((size_t)n - tile_base) : RS_TILE);
+    for (uint32_t j = threadIdx.x; j < tile_n; j += RS_THREADS) {
+        K kk = s_k[j];
+        const uint32_t g = s_goff[rs_digit(kk, shift, mask)] + j;
+        kout[g] = kk;
+        if (HAS_VAL) vout[g] = s_v[j];
+    }
+}
+
+static __global__ void k_iota(uint32_t *v, uint32_t n)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) v[i] = i;
+}
+
 // Sorts (keys, vals) stably by bits [begin_bit, end_bit) with BITS-bit digits
 // (8: 256 buckets; 10: 1024 buckets, fewer passes for 17..20-bit keys).  On
 // return `keys` and `vals` point at the sorted data (the *_alt buffers hold
-// garbage).  With `tseg` (see rs_hist_index; n a multiple of RS_TILE) every
-// segment is sorted on its own.
+// garbage).  With `iota` the values are the positions 0..n-1 (vals need not be
+// filled).  With segments (n a multiple of RS_TILE) every segment is sorted on
+// its own.
 template <typename K, bool HAS_VAL, int BITS = 8, int BALLOT = 0>
 void radix_sort(Storage *st, K *&keys, K *&keys_alt, uint32_t *&vals, uint32_t *&vals_alt, uint32_t n,
-                int begin_bit, int end_bit, const uint2 *tseg = nullptr)
+                int begin_bit, int end_bit, RsSegs sg = RsSegs(), bool iota = false)
 {
     static_assert((1 << BITS) % RS_THREADS == 0, "digit count must be a multiple of the CTA size");
-    if (n <= 1 || end_bit <= begin_bit) return;
+    if (n <= 1 || end_bit <= begin_bit) {
+        if (iota && n) {
+            k_iota<<<grid_for(n, 256), 256, 0, st->stream>>>(vals, n);
+            after_launch(st);
+        }
+        return;
+    }
     static bool attr_set = false;
     constexpr size_t smem = rs_smem_bytes<K, HAS_VAL, BITS>();
     if (!attr_set) {
+        check_cuda(cudaFuncSetAttribute(k_rs_pass<K, HAS_VAL, BITS, BALLOT>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         check_cuda(cudaFuncSetAttribute(k_rs_downsweep<K, HAS_VAL, BITS, BALLOT>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
     const uint32_t num_tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
     const size_t D = (size_t)1 << BITS;
-    uint32_t *hist = slot<uint32_t>(st, S_RSHIST, D * num_tiles);
-    for (int shift = begin_bit; shift < end_bit; shift += BITS) {
+    const int np = (end_bit - begin_bit + BITS - 1) / BITS;
+    uint32_t *hist = nullptr;
+    const bool small = num_tiles <= 2u * (uint32_t)st->num_sms;
+    if (!small) {
+        hist = slot<uint32_t>(st, S_RSHIST, D * num_tiles);
+    } else if (num_tiles > 1) {
+        const size_t words = (size_t)np * sg.nseg * D;
+        hist = slot<uint32_t>(st, S_RSHIST, words);
+        check_cuda(cudaMemsetAsync(hist, 0, words * sizeof(uint32_t), st->stream));
+        unsigned grid = grid_for(num_tiles, RH_TILES);
+        if (grid > (unsigned)st->num_sms * 6) grid = (unsigned)st->num_sms * 6;
+        k_rs_hist<K, BITS><<<grid, RS_THREADS, 0, st->stream>>>(keys, n, begin_bit, end_bit, sg, num_tiles, hist);
+        after_launch(st);
+    }
+    for (int p = 0; p < np; p++) {
+        const int shift = begin_bit + p * BITS;
         int bits = end_bit - shift < BITS ? end_bit - shift : BITS;
         uint32_t mask = (1u << bits) - 1u;
-        k_rs_upsweep<K, BITS><<<num_tiles, RS_THREADS, 0, st->stream>>>(keys, n, shift, mask, hist, num_tiles, tseg);
-        after_launch(st);
-        device_scan<uint32_t, OpAdd>(st, D * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
-                                     (uint32_t *)nullptr);
+        LookBack lb{};
+        if (!small) {
+            k_rs_upsweep<K, BITS><<<num_tiles, RS_THREADS, 0, st->stream>>>(keys, n, shift, mask, hist, num_tiles, sg);
+            after_launch(st);
+            device_scan<uint32_t, OpAdd>(st, D * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
+                                         (uint32_t *)nullptr);
+        } else if (num_tiles > 1) {
+            lb = look_back(st, (size_t)num_tiles * D, 1);
+        }
         probe_begin(st, GBWT_PROBE_RADIX_SCATTER);
-        k_rs_downsweep<K, HAS_VAL, BITS, BALLOT><<<num_tiles, RS_THREADS, smem, st->stream>>>(keys, keys_alt, vals, vals_alt,
-                                                                                      n, shift, mask, hist, num_tiles,
-                                                                                      tseg);
+        const uint32_t *vi = iota && p == 0 ? nullptr : vals;
+        if (small)
+            k_rs_pass<K, HAS_VAL, BITS, BALLOT><<<num_tiles, RS_THREADS, smem, st->stream>>>(
+                keys, keys_alt, vi, vals_alt, n, shift, mask, hist ? hist + (size_t)p * sg.nseg * D : nullptr, sg, lb);
+        else
+            k_rs_downsweep<K, HAS_VAL, BITS, BALLOT><<<num_tiles, RS_THREADS, smem, st->stream>>>(
+                keys, keys_alt, vi, vals_alt, n, shift, mask, hist, num_tiles, sg);
         probe_end(st, GBWT_PROBE_RADIX_SCATTER, (uint64_t)n * 2 * (sizeof(K) + (HAS_VAL ? 4 : 0)));
         after_launch(st);
         K *t = keys; keys = keys_alt; keys_alt = t;
