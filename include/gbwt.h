@@ -65,7 +65,8 @@ typedef struct gbwt_stats {
     int64_t mixed_blocks;   /* S entries whose BWT block is not one run      */
     int64_t mixed_elems;    /* BWT bytes inside mixed blocks                 */
     int64_t dict_rounds;    /* prefix-doubling rounds, dictionary sort       */
-    int64_t parse_rounds;   /* prefix-doubling rounds, parse suffix array    */
+    int64_t parse_rounds;   /* prefix-doubling rounds, parse suffix array
+                               (of both levels when the parse was parsed)    */
     int64_t hash_retries;   /* fingerprint retries (collision or table full)  */
     int64_t kernel_launches;/* kernels launched by the last call             */
     int64_t primary_index;  /* output row of the suffix starting at T[0]
@@ -226,9 +227,10 @@ typedef struct gbwt_tuning {
     int32_t dict_key_bits;      /* dictionary sort, first key: at most this many bits of recoded
                                    symbols (8..64; default 64: as many symbols as fit)             */
     int32_t parse_key_phrases;  /* parse suffix array, first round: 1 or 2 phrase ranks sorted by
-                                   radix; 0 (default): one text's first round comes straight from
-                                   the phrase buckets of the dictionary order, no sort (batches
-                                   then sort 2 ranks)                                              */
+                                   radix; 0 (default): a large repetitive text's parse is parsed
+                                   again and sorted at that level; else the first round comes
+                                   straight from the phrase buckets of the dictionary order, no
+                                   sort (batches then sort 2 ranks)                                */
     int32_t mixed_radix_bits;   /* mixed-block element sort digit width: 8 or 10 (default 8)       */
     int32_t batch_ballot;       /* batch output sort ranking: every k-th item by ballots (2 or 3),
                                    1 = match only (default 3)                                       */

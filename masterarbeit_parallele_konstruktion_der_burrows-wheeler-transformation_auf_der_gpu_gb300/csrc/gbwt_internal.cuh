@@ -34,6 +34,9 @@ enum Slot : int {
     S_TMP0, S_TMP1, S_TMP2, S_PIDPC, S_TILEG, S_ACTX2, S_ACTG2, S_LCB, S_LCBMAP,
     S_BX, S_BMETA, S_BTID, S_BZEND, S_BLAST, S_BCODE, S_SSTART,
     S_BIGL, S_BIGM,
+    // second-level parse
+    S_2SYM, S_2TRIG, S_2START, S_2SLOT, S_2PID, S_2DLEN, S_2DOFF, S_2DSTART, S_2OCC, S_2DICT, S_2DPHR, S_2ISA, S_2SA,
+    S_2RANK, S_2PISA, S_2PSA,
     S_NUM
 };
 
@@ -156,9 +159,10 @@ inline int tune_seg_tiles(const Storage *st) { return st->tuning.batch_seg_tiles
 inline int tune_pad_eighths(const Storage *st) { return st->tuning.batch_pad_eighths ? st->tuning.batch_pad_eighths : 1; }
 inline int tune_unbwt_rate_log2(const Storage *st) { return st->tuning.unbwt_rate_log2 ? st->tuning.unbwt_rate_log2 : 7; }
 inline int tune_dict_key_bits(const Storage *st) { return st->tuning.dict_key_bits ? st->tuning.dict_key_bits : 64; }
-// 0 (default): single-text parse round 0 from the phrase buckets, no sort
-// (the batch parse then sorts two phrase ranks); 1 or 2: a radix sort of
-// the first one or two phrase ranks.
+// 0 (default): single-text parses are parsed again when large and repetitive,
+// else round 0 comes from the phrase buckets, no sort (the batch parse then
+// sorts two phrase ranks); 1 or 2: a radix sort of the first one or two phrase
+// ranks.
 inline int tune_parse_key_phrases(const Storage *st) { return st->tuning.parse_key_phrases; }
 
 inline int bits_for(uint64_t v)   // bits needed to represent values in [0, v]
@@ -229,9 +233,18 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
 
 struct ParseOrder {
     uint32_t *sa = nullptr;      // [z] suffix array of the parse
-    uint32_t *isa = nullptr;     // [z] inverse
+    uint32_t *isa = nullptr;     // [z] inverse; null after the second-level parse
+    const uint32_t *first = nullptr;   // [2] ranks of suffixes 0 and 1 (1 only when z > 1)
     int rounds = 0;
 };
+// Pieces of the two sorts that the second-level parse uses on its own strings.
+int sort_phrase_suffixes(Storage *st, uint32_t N, int key_bits, uint32_t h0, const uint32_t *dphr, const uint32_t *doff,
+                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa);
+void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, const uint32_t *doff, uint32_t *lexrank);
+int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
+                     const uint32_t *occ, uint32_t *isa, uint32_t *sa);
+// Parse suffix array by parsing the parse; false (nothing done) when that does not pay.
+bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord);
 void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord);
 void run_parse_sa_batch(Storage *st, Phrases &ph, DictOrder &dord, const BatchText &bt, ParseOrder &pord);
 // Group index of every dictionary position that starts a suffix longer than

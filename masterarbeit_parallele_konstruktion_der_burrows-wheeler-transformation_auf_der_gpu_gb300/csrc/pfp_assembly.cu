@@ -220,12 +220,12 @@ __global__ void k_mix_entries(uint32_t N, const uint32_t *dphr, const uint32_t *
 // Emission order: the last phrase first (its next-suffix rank is -1,
 // K:787-807), then the phrase before each parse suffix in suffix-array order.
 struct Emit {
-    const uint32_t *psa, *pisa, *pid, *moff, *D;
+    const uint32_t *psa, *first, *pid, *moff, *D;     // first[0]: rank of parse suffix 0
     uint32_t z;
     __device__ __forceinline__ uint32_t occ_at(size_t t) const
     {
         if (t == 0) return z - 1u;
-        const uint32_t pos0 = pisa[0];
+        const uint32_t pos0 = first[0];
         const uint32_t r = (uint32_t)t - 1u < pos0 ? (uint32_t)t - 1u : (uint32_t)t;
         return psa[r] - 1u;
     }
@@ -419,29 +419,46 @@ __global__ void k_run_fill_long(uint8_t *out, uint32_t n, const uint2 *stat, uin
 // Output row of the suffix starting at text position 0 (the "primary index"):
 // its block is the group g0 of phrase 0 taken whole; inside a block the rows
 // follow the rank of the next parse suffix (last phrase: -1, K:787-807).
+// counter = goff[g0] + the occurrences of g0's string ranked before text
+// position 0's.  Pass 1 (text order, tables read in sequence) marks, in a bit
+// vector over parse positions, the suffixes that follow the other occurrences;
+// pass 2 (suffix-array order) counts the marked ones before suffix 1.  An
+// occurrence that ends the parse comes first.  The inverse of the parse
+// suffix array is not needed.
 struct PrimaryArgs {
-    const uint32_t *pid, *pisa, *doff, *dlen, *isa;
+    const uint32_t *pid, *doff, *dlen, *isa;
     const uint2 *stat;
     uint32_t z;
+    uint32_t *marks;
     uint32_t *counter;
 };
-__global__ void k_primary_index(PrimaryArgs a)
+__global__ void k_primary_marks(PrimaryArgs a)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t q0 = a.pid[0], len0 = a.dlen[q0];
     const uint32_t g0 = a.isa[a.doff[q0]];
-    bool before = false;
+    bool same = false;
     if (k < a.z && k != 0) {
         const uint32_t q = a.pid[k], lq = a.dlen[q];
-        if (lq >= len0 && a.isa[a.doff[q] + lq - len0] == g0) {
-            const int64_t nr0 = a.z > 1 ? (int64_t)a.pisa[1] : -1;
-            const int64_t nrk = k + 1 < a.z ? (int64_t)a.pisa[k + 1] : -1;
-            before = nrk < nr0;
-        }
+        same = lq >= len0 && a.isa[a.doff[q] + lq - len0] == g0;
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, same);
+    if ((threadIdx.x & 31u) == 0 && k < a.z) a.marks[k >> 5] = m;
+    if (k == 0) atomicAdd(a.counter, a.stat[g0].x);
+    if (same && k + 1u == a.z) atomicAdd(a.counter, 1u);
+}
+__global__ void k_primary_count(const uint32_t *sa, const uint32_t *first, uint32_t z, const uint32_t *marks,
+                                uint32_t *counter)
+{
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (z < 2u || blockIdx.x * blockDim.x >= first[1]) return;
+    bool before = false;
+    if (r < first[1]) {
+        const uint32_t x = sa[r];            // the suffix after occurrence x - 1
+        before = x > 1u && ((marks[(x - 1u) >> 5] >> ((x - 1u) & 31u)) & 1u);
     }
     const unsigned m = __ballot_sync(0xFFFFFFFFu, before);
-    if ((threadIdx.x & 31u) == 0 && m) atomicAdd(a.counter, (uint32_t)__popc(m));
-    if (k == 0) atomicAdd(a.counter, a.stat[g0].x);
+    if ((threadIdx.x & 31u) == 0 && m) atomicAdd(counter, (uint32_t)__popc(m));
 }
 
 template <typename E>
@@ -452,7 +469,7 @@ static void mixed_blocks(Storage *st, const uint8_t *dT, uint32_t n, int W, Phra
     E *elem = slot<E>(st, S_ELEM0, M);
     E *elem_alt = slot<E>(st, S_ELEM1, M);
     const uint32_t z = ph.z;
-    Emit e{pord.sa, pord.isa, ph.pid, moff, ph.D, z};
+    Emit e{pord.sa, pord.first, ph.pid, moff, ph.D, z};
     uint32_t *emq = slot<uint32_t>(st, S_TMP0, z);
     uint32_t *ecnt = slot<uint32_t>(st, S_TMP1, (size_t)z + 1);
     uint8_t *emp = (uint8_t *)slot<uint32_t>(st, S_TMP2, z / 4 + 1);
@@ -520,8 +537,11 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     st->stats.mixed_elems = M;
     stage_mark(st, 4);
 
-    k_primary_index<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(
-        PrimaryArgs{ph.pid, pord.isa, ph.doff, ph.dlen, dord.isa, stat, ph.z, st->d_flags + 2});
+    uint32_t *marks = slot<uint32_t>(st, S_TMP2, ((size_t)ph.z + 31) / 32);
+    k_primary_marks<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(
+        PrimaryArgs{ph.pid, ph.doff, ph.dlen, dord.isa, stat, ph.z, marks, st->d_flags + 2});
+    after_launch(st);
+    k_primary_count<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(pord.sa, pord.first, ph.z, marks, st->d_flags + 2);
     after_launch(st);
     const uint32_t long_cap = n / RF_LONG + 1u;
     uint32_t *longs = slot<uint32_t>(st, S_TILEG, long_cap);

@@ -1045,6 +1045,25 @@ __global__ void k_phrase_lexrank(const uint32_t *isa, const uint32_t *doff, uint
     lexrank[q] = pre[w] + (uint32_t)__popc(bits[w] & ((1u << (p & 31)) - 1u));
 }
 
+void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, const uint32_t *doff, uint32_t *lexrank)
+{
+    const size_t words = ((size_t)N + 31) / 32;
+    uint32_t *bits = slot<uint32_t>(st, S_TMP0, words);
+    uint32_t *pre = slot<uint32_t>(st, S_TMP2, words);
+    check_cuda(cudaMemsetAsync(bits, 0, words * sizeof(uint32_t), st->stream));
+    k_mark_phrase_heads<<<grid_for(d, 256), 256, 0, st->stream>>>(isa, doff, d, bits);
+    after_launch(st);
+    device_scan<uint32_t, OpAdd>(st, words, LoadPopc{bits}, StoreWordPre{pre}, false, (uint32_t *)nullptr);
+    k_phrase_lexrank<<<grid_for(d, 256), 256, 0, st->stream>>>(isa, doff, d, bits, pre, lexrank);
+    after_launch(st);
+}
+
+int sort_phrase_suffixes(Storage *st, uint32_t N, int key_bits, uint32_t h0, const uint32_t *dphr, const uint32_t *doff,
+                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa)
+{
+    return prefix_doubling(st, N, key_bits, h0, DictRem{dphr, doff, dlen, rem8}, isa, sa, true);
+}
+
 void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
 {
     (void)W;
@@ -1079,21 +1098,12 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     uint8_t *rem8 = slot<uint8_t>(st, S_TMP0, N);
     k_dict_keys<<<grid_for(N, 256), 256, 0, st->stream>>>(ph.dict, N, rem, dcode, bps, h0, keys, rem8);
     after_launch(st);
-    rem.rem8 = rem8;
     dord.isa = slot<uint32_t>(st, S_ISA, N);
     dord.sa = slot<uint32_t>(st, S_SA, N);
-    dord.rounds = prefix_doubling(st, N, h0 * bps + 1, (uint32_t)h0, rem, dord.isa, dord.sa, true);
+    dord.rounds = sort_phrase_suffixes(st, N, h0 * bps + 1, (uint32_t)h0, ph.dphr, ph.doff, ph.dlen, rem8, dord.isa,
+                                       dord.sa);
     dord.lexrank = slot<uint32_t>(st, S_LEXRANK, ph.d);
-    const size_t words = ((size_t)N + 31) / 32;
-    uint32_t *bits = slot<uint32_t>(st, S_TMP0, words);
-    uint32_t *pre = slot<uint32_t>(st, S_TMP2, words);
-    check_cuda(cudaMemsetAsync(bits, 0, words * sizeof(uint32_t), st->stream));
-    k_mark_phrase_heads<<<grid_for(ph.d, 256), 256, 0, st->stream>>>(dord.isa, ph.doff, ph.d, bits);
-    after_launch(st);
-    device_scan<uint32_t, OpAdd>(st, words, LoadPopc{bits}, StoreWordPre{pre}, false, (uint32_t *)nullptr);
-    k_phrase_lexrank<<<grid_for(ph.d, 256), 256, 0, st->stream>>>(dord.isa, ph.doff, ph.d, bits, pre,
-                                                                   dord.lexrank);
-    after_launch(st);
+    phrase_ranks(st, N, ph.d, dord.isa, ph.doff, dord.lexrank);
 }
 
 // First parse key: one phrase rank (two == false), or two (the second 0
@@ -1170,12 +1180,41 @@ __global__ void k_bucket_scatter(const uint32_t *pid, const uint2 *info, uint32_
     }
 }
 
+// Parse suffix array from the phrase buckets (the last phrase occurs once: its
+// suffix, the only one ending within one phrase, is finished in round 0).
+int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
+                     const uint32_t *occ, uint32_t *isa, uint32_t *sa)
+{
+    uint32_t *cnt_r = slot<uint32_t>(st, S_TMP0, d);
+    uint64_t *bst = slot<uint64_t>(st, S_KEY1, d);
+    uint32_t *cur = slot<uint32_t>(st, S_TMP1, d);
+    uint32_t *act_x = slot<uint32_t>(st, S_ACTX, z);
+    uint32_t *act_g = slot<uint32_t>(st, S_ACTG, z);
+    uint32_t *act_x2 = slot<uint32_t>(st, S_ACTX2, z);
+    uint32_t *act_g2 = slot<uint32_t>(st, S_ACTG2, z);
+    k_bucket_counts<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, occ, d, cnt_r);
+    after_launch(st);
+    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
+    device_scan<uint64_t, OpAdd>(st, d, LoadBucket{cnt_r}, StoreBucket{bst}, false, (uint64_t *)st->d_scalars);
+    check_cuda(cudaMemsetAsync(cur, 0, (size_t)d * 4, st->stream));
+    uint2 *info = slot<uint2>(st, S_KEY0, d);
+    k_bucket_info<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, bst, occ, d, info);
+    after_launch(st);
+    k_bucket_scatter<<<grid_for(z, 256), 256, 0, st->stream>>>(pid, info, z, cur, isa, sa, act_x, act_g, st->d_flags);
+    after_launch(st);
+    fetch_scalars(st, 1);
+    const uint64_t tot = st->h_scalars[0];
+    if ((uint32_t)(tot >> 32) != z) throw Error{GBWT_INTERNAL_ERROR};
+    return 1 + doubling_rounds(st, z, 1, (uint32_t)tot, ParseRem{z}, isa, sa, act_x, act_g, act_x2, act_g2, true);
+}
+
 void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord)
 {
     const uint32_t z = ph.z;
+    const int kp = tune_parse_key_phrases(st);
+    if (kp == 0 && run_parse_sa_level2(st, ph, dord, pord)) return;
     pord.isa = slot<uint32_t>(st, S_PISA, z);
     pord.sa = slot<uint32_t>(st, S_PSA, z);
-    const int kp = tune_parse_key_phrases(st);
     if (kp == 1 || kp == 2) {
         // round 0 by a radix sort of the first one or two phrase ranks
         uint64_t *keys = slot<uint64_t>(st, S_KEY0, z);
@@ -1184,34 +1223,10 @@ void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord)
         after_launch(st);
         pord.rounds = prefix_doubling(st, z, kp == 2 ? lb + bits_for(ph.d - 1) : bits_for(ph.d - 1), (uint32_t)kp,
                                       ParseRem{z}, pord.isa, pord.sa);
-        return;
+    } else {
+        pord.rounds = parse_sa_buckets(st, z, ph.d, ph.pid, dord.lexrank, ph.occ, pord.isa, pord.sa);
     }
-    // round 0 from the phrase buckets (the last phrase occurs once: its
-    // suffix, the only one ending within one phrase, is finished here)
-    const uint32_t d = ph.d;
-    uint32_t *cnt_r = slot<uint32_t>(st, S_TMP0, d);
-    uint64_t *bst = slot<uint64_t>(st, S_KEY1, d);
-    uint32_t *cur = slot<uint32_t>(st, S_TMP1, d);
-    uint32_t *act_x = slot<uint32_t>(st, S_ACTX, z);
-    uint32_t *act_g = slot<uint32_t>(st, S_ACTG, z);
-    uint32_t *act_x2 = slot<uint32_t>(st, S_ACTX2, z);
-    uint32_t *act_g2 = slot<uint32_t>(st, S_ACTG2, z);
-    k_bucket_counts<<<grid_for(d, 256), 256, 0, st->stream>>>(dord.lexrank, ph.occ, d, cnt_r);
-    after_launch(st);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    device_scan<uint64_t, OpAdd>(st, d, LoadBucket{cnt_r}, StoreBucket{bst}, false, (uint64_t *)st->d_scalars);
-    check_cuda(cudaMemsetAsync(cur, 0, (size_t)d * 4, st->stream));
-    uint2 *info = slot<uint2>(st, S_KEY0, d);
-    k_bucket_info<<<grid_for(d, 256), 256, 0, st->stream>>>(dord.lexrank, bst, ph.occ, d, info);
-    after_launch(st);
-    k_bucket_scatter<<<grid_for(z, 256), 256, 0, st->stream>>>(ph.pid, info, z, cur, pord.isa, pord.sa, act_x, act_g,
-                                                               st->d_flags);
-    after_launch(st);
-    fetch_scalars(st, 1);
-    const uint64_t tot = st->h_scalars[0];
-    if ((uint32_t)(tot >> 32) != z) throw Error{GBWT_INTERNAL_ERROR};
-    pord.rounds = 1 + doubling_rounds(st, z, 1, (uint32_t)tot, ParseRem{z}, pord.isa, pord.sa, act_x, act_g, act_x2,
-                                      act_g2, true);
+    pord.first = pord.isa;
 }
 
 // Batch: the second symbol of a key is 0 when phrase i ends its text.
