@@ -10,13 +10,18 @@
 // GB300 layout: a tile is 4096 window starts; the 4096+W-1 bytes it needs
 // are staged in shared memory with 16-byte loads (a CTA loads several tiles
 // before it uses any); every thread pulls its 16 windows (+ W-1 halo) into
-// registers with 16-byte shared loads and rolls the hash mod P
-// (h(s+1) = 2h(s) - T[s]*2^W + T[s+W]); for W=5, P=16 it hashes four
-// windows at once with packed byte arithmetic instead.  The first-word test
-// rolls an exact packed register for W <= 8 and a 64-bit polynomial
-// fingerprint (verified byte by byte on a hit) for longer windows.  Trigger
-// positions are compacted with popc + a CTA scan; the count pass also
-// validates the input bytes (K:130-132) without trapping.
+// registers with 16-byte shared loads.  W=5 windows are hashed without
+// rolling: P=16 four windows at once in packed byte arithmetic, other P with
+// two byte dot products per window.  Other W roll the hash mod P (h(s+1) =
+// 2h(s) - T[s]*2^W + T[s+W]).  The first-word test compares up to eight bytes at
+// once and the rest byte by byte on a hit.  The text is read once: this pass
+// keeps a 16-bit trigger mask per thread (n / 8 bytes), and the pass that
+// writes the positions reads the masks.  The first pass also validates the
+// input bytes (K:130-132) without trapping.
+//
+// Both passes, before / after on GB300: 512 MiB, W=5 P=16 0.50 / 0.36 ms, W=35 P=81
+// 3.10 / 0.81 ms; 256 MiB, W=5 P=23 0.71 / 0.17 ms; a 4096-text batch 1.34 / 0.61
+// ms.  The counting pass is bound by instructions (2.0 TB/s of text at W=5).
 #include "prims.cuh"
 #include <mutex>
 
@@ -26,7 +31,6 @@ constexpr int TS_THREADS = 256;
 constexpr int TS_PER_THREAD = 16;
 constexpr int TS_TILE = TS_THREADS * TS_PER_THREAD;
 constexpr int TS_MAXW = 64;
-constexpr uint64_t FP_BASE = 0x100000001B3ull;
 
 struct ScanArgs {
     const uint8_t *T;
@@ -39,6 +43,72 @@ struct ScanArgs {
 };
 
 __device__ __forceinline__ uint32_t bget(const uint32_t *w, int i) { return (w[i >> 2] >> (8 * (i & 3))) & 0xFFu; }
+// The 8 bytes from byte i on (little-endian), words w[i/4 .. i/4+2].
+__device__ __forceinline__ uint64_t bget8(const uint32_t *w, int i)
+{
+    const uint32_t sh = 8u * (i & 3);
+    return ((uint64_t)__funnelshift_r(w[(i >> 2) + 1], w[(i >> 2) + 2], sh) << 32) |
+           __funnelshift_r(w[i >> 2], w[(i >> 2) + 1], sh);
+}
+// First min(W, 8) bytes at p, little-endian, and the mask of those bytes.
+__device__ __forceinline__ uint64_t first8(const uint8_t *p, int W)
+{
+    uint64_t v = 0;
+    for (int i = 0; i < W && i < 8; i++) v |= (uint64_t)p[i] << (8 * i);
+    return v;
+}
+__device__ __forceinline__ uint64_t mask8(int W) { return W >= 8 ? ~0ull : (1ull << (8 * W)) - 1ull; }
+
+// Trigger bits of 16 windows of width 5 (w: their 20 bytes) against the first
+// window f (5 bytes, little-endian); no range checks.
+template <int PT>
+__device__ __forceinline__ uint32_t windows5(const uint32_t *w, uint64_t f)
+{
+    uint32_t m = 0;
+    if constexpr (PT == 16) {
+        // Packed byte arithmetic, four windows per 32-bit word.  Window s
+        // hashes 8 T[s+1] + 4 T[s+2] + 2 T[s+3] + T[s+4] (mod 16): the weight
+        // of T[s] is 2^4 = 0 mod 16.  Each term reduced mod 16 before its
+        // shift keeps every byte lane below 64, so one 32-bit add serves four
+        // windows.  The first-word test is an OR of byte-wise XORs with the
+        // broadcast first five bytes.  A lane is zero exactly when
+        // ~(((v & 0x7F..) + 0x7F..) | v | 0x7F..) has its top bit set.
+        uint32_t fb[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) fb[k] = ((uint32_t)(f >> (8 * k)) & 0xFFu) * 0x01010101u;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t x0 = w[q], x4 = w[q + 1];
+            const uint32_t x1 = __funnelshift_r(x0, x4, 8);
+            const uint32_t x2 = __funnelshift_r(x0, x4, 16);
+            const uint32_t x3 = __funnelshift_r(x0, x4, 24);
+            const uint32_t hsum = (((x1 & 0x01010101u) << 3) + ((x2 & 0x03030303u) << 2) +
+                                   ((x3 & 0x07070707u) << 1) + (x4 & 0x0F0F0F0Fu)) & 0x0F0F0F0Fu;
+            const uint32_t e = (x0 ^ fb[0]) | (x1 ^ fb[1]) | (x2 ^ fb[2]) | (x3 ^ fb[3]) | (x4 ^ fb[4]);
+            const uint32_t zh = ~(((hsum & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | hsum | 0x7F7F7F7Fu);
+            const uint32_t ze = ~(((e & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | e | 0x7F7F7F7Fu);
+            // lane top bits (bits 7, 15, 23, 31) -> four mask bits
+            const uint32_t lanes = ((zh | ze) >> 7) & 0x01010101u;
+            m |= ((lanes * 0x00204081u) >> 21 & 0xFu) << (4 * q);
+        }
+    } else {
+        // x_s = bytes s..s+3: the hash is a dot product of x_s with the
+        // weights 2^4, 2^3, 2^2, 2 (mod P) plus T[s+4], the top byte of
+        // x_(s+1); at most 255 * 5 * (P - 1), so one reduction suffices
+        constexpr uint32_t w4 = (16u % PT) | ((8u % PT) << 8) | ((4u % PT) << 16) | ((2u % PT) << 24);
+        const uint32_t f0 = (uint32_t)f, f1 = (uint32_t)(f >> 8);
+        uint32_t x = w[0];
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const int n = j + 1;
+            const uint32_t xn = (n & 3) ? __funnelshift_r(w[n >> 2], w[(n >> 2) + 1], 8 * (n & 3)) : w[n >> 2];
+            const uint32_t h = __dp4a(x, w4, xn >> 24);
+            if (h % (uint32_t)PT == 0 || (x == f0 && xn == f1)) m |= 1u << j;
+            x = xn;
+        }
+    }
+    return m;
+}
 
 // 2^W mod P: a compile-time constant in the specialised kernels (0 for
 // W=5, P=16, where the outgoing byte drops out of the rolling hash).
@@ -88,13 +158,13 @@ __device__ __forceinline__ void stage_tile(const ScanArgs &a, uint8_t *s, size_t
 }
 
 // One tile: returns this thread's 16-bit trigger mask and checks bytes.
+// fw8: the first min(W, 8) bytes of the text; s_fw: all W of them.
 template <int WT, int PT>
 __device__ __forceinline__ uint32_t tile_triggers(const ScanArgs &a, const uint8_t *s, const uint8_t *s_fw,
-                                                  uint64_t fw_packed, uint64_t fp0, uint64_t fp_pow,
-                                                  size_t base, bool check_bytes)
+                                                  uint64_t fw8, size_t base, bool check_bytes)
 {
     constexpr int NB = TS_PER_THREAD + (WT > 0 ? WT : TS_MAXW) - 1;   // bytes needed
-    constexpr int NV = (NB + 15) / 16;                                 // uint4 loads
+    constexpr int NV = (NB + 7 + 15) / 16;                             // uint4 loads (bget8 reads up to 7 more)
     const int W = WT > 0 ? WT : a.W;
     const uint32_t P = PT > 0 ? (uint32_t)PT : (uint32_t)a.P;
     const size_t s0 = base + (size_t)threadIdx.x * TS_PER_THREAD;
@@ -133,86 +203,36 @@ __device__ __forceinline__ uint32_t tile_triggers(const ScanArgs &a, const uint8
                                                                     : (1u << (uint32_t)(last_valid - s0 + 1)) - 1u;
     if (s0 == 0) range &= ~1u;
 
-    if constexpr (WT == 5 && PT == 16) {
-        // Packed byte arithmetic, four windows per 32-bit word.  Window s
-        // hashes 8 T[s+1] + 4 T[s+2] + 2 T[s+3] + T[s+4] (mod 16): the weight
-        // of T[s] is 2^4 = 0 mod 16.  Each term reduced mod 16 before its
-        // shift keeps every byte lane below 64, so one 32-bit add serves four
-        // windows.  The first-word test is an OR of byte-wise XORs with the
-        // broadcast first five bytes.  A lane is zero exactly when
-        // ~(((v & 0x7F..) + 0x7F..) | v | 0x7F..) has its top bit set.
-        uint32_t f[5];
-#pragma unroll
-        for (int k = 0; k < 5; k++) f[k] = (uint32_t)s_fw[k] * 0x01010101u;
-        uint32_t m = 0;
-#pragma unroll
-        for (int q = 0; q < TS_PER_THREAD / 4; q++) {
-            const uint32_t x0 = w[q], x4 = w[q + 1];
-            const uint32_t x1 = __funnelshift_r(x0, x4, 8);
-            const uint32_t x2 = __funnelshift_r(x0, x4, 16);
-            const uint32_t x3 = __funnelshift_r(x0, x4, 24);
-            const uint32_t hsum = (((x1 & 0x01010101u) << 3) + ((x2 & 0x03030303u) << 2) +
-                                   ((x3 & 0x07070707u) << 1) + (x4 & 0x0F0F0F0Fu)) & 0x0F0F0F0Fu;
-            const uint32_t e = (x0 ^ f[0]) | (x1 ^ f[1]) | (x2 ^ f[2]) | (x3 ^ f[3]) | (x4 ^ f[4]);
-            const uint32_t zh = ~(((hsum & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | hsum | 0x7F7F7F7Fu);
-            const uint32_t ze = ~(((e & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | e | 0x7F7F7F7Fu);
-            // lane top bits (bits 7, 15, 23, 31) -> four mask bits
-            const uint32_t lanes = ((zh | ze) >> 7) & 0x01010101u;
-            m |= ((lanes * 0x00204081u) >> 21 & 0xFu) << (4 * q);
-        }
-        return m & range;
-    }
+    if constexpr (WT == 5 && PT > 0) return windows5<PT>(w, fw8) & range;
 
-    // hash of the first window: sum b[i] * 2^(W-1-i) mod P
+    // hash of the first window: sum b[i] * 2^(W-1-i) mod P, at most
+    // 64 * 255 * 65534 < 2^32 before the reduction
     uint32_t h = 0;
     {
         uint32_t pw = 1;
-        uint32_t acc = 0;
 #pragma unroll
         for (int i = (WT > 0 ? WT : TS_MAXW) - 1; i >= 0; i--) {
             if (WT == 0 && i >= W) continue;
-            acc += bget(w, i) * pw;
+            h += bget(w, i) * pw;
             pw = (pw * 2u) % P;
-            if (WT == 0 || WT > 16) acc %= P;
         }
-        h = acc % P;
+        h %= P;
     }
-    // first-word test state
-    uint64_t reg = 0, fp = 0;
-    if (WT > 0 && WT <= 8) {
-#pragma unroll
-        for (int i = 0; i < (WT > 0 ? WT : 1); i++) reg = (reg << 8) | bget(w, i);
-    } else {
-#pragma unroll
-        for (int i = 0; i < (WT > 0 ? WT : TS_MAXW); i++) {
-            if (WT == 0 && i >= W) break;
-            fp = fp * FP_BASE + bget(w, i);
-        }
-    }
-    const uint64_t regmask = (WT > 0 && WT < 8) ? ((1ull << (8 * (WT > 0 ? WT : 1))) - 1ull) : ~0ull;
-
+    const uint64_t m8 = mask8(W);
     const uint32_t wW = (WT > 0 && PT > 0) ? pow2_mod(WT > 0 ? WT : 1, PT > 0 ? PT : 1) : a.wW;
     uint32_t mask = 0;
 #pragma unroll
     for (int j = 0; j < TS_PER_THREAD; j++) {
-        const size_t sj = s0 + j;
-        bool eq;
-        if (WT > 0 && WT <= 8) {
-            eq = reg == fw_packed;
-        } else {
-            eq = false;
-            if (fp == fp0) {
-                eq = true;
-                for (int i = 0; i < W; i++)
-                    if (s[sj - base + i] != s_fw[i]) { eq = false; break; }
-            }
+        bool eq = ((bget8(w, j) ^ fw8) & m8) == 0;
+        if (eq && W > 8) {
+            const uint8_t *win = src + j;
+            for (int i = 8; i < W; i++)
+                if (win[i] != s_fw[i]) { eq = false; break; }
         }
         if (h == 0 || eq) mask |= 1u << j;
         if (j + 1 < TS_PER_THREAD) {
             const uint32_t out = bget(w, j), in = bget(w, j + W);
             h = (2u * h + in + 256u * P - out * wW) % P;
-            if (WT > 0 && WT <= 8) reg = ((reg << 8) | in) & regmask;
-            else fp = fp * FP_BASE - (uint64_t)out * fp_pow + in;
         }
     }
     return mask & range;
@@ -220,12 +240,14 @@ __device__ __forceinline__ uint32_t tile_triggers(const ScanArgs &a, const uint8
 
 // SUB consecutive 4096-window tiles per CTA: all of their bytes are loaded
 // before any is used, so more bytes are in flight per SM than with one tile
-// (the scan is otherwise latency-bound on its load).  Trigger order is tile
-// by tile, thread by thread: the write pass scans the SUB per-thread counts as
-// 16-bit lanes of one 64-bit value.
+// (the scan is otherwise latency-bound on its load).  The counting pass stores
+// every thread's mask (masks[window / 16]) for k_trigger_write.  WRITE (the
+// allocation-free scan, which has no room for masks) hashes the text again:
+// trigger order is tile by tile, thread by thread, and the SUB per-thread counts
+// are scanned as 16-bit lanes of one 64-bit value.
 template <int WT, int PT, bool WRITE, int SUB>
 __global__ void __launch_bounds__(TS_THREADS) k_trigger(ScanArgs a, uint32_t *counts, const uint32_t *offsets,
-                                                        uint32_t *D)
+                                                        uint32_t *D, uint16_t *masks)
 {
     static_assert(SUB >= 1 && SUB <= 4, "the write pass packs SUB counts into 16-bit lanes");
     __shared__ __align__(16) uint8_t s[SUB * TS_TILE + TS_MAXW + 64];
@@ -270,19 +292,14 @@ __global__ void __launch_bounds__(TS_THREADS) k_trigger(ScanArgs a, uint32_t *co
     if (threadIdx.x < (unsigned)W) s_fw[threadIdx.x] = threadIdx.x < a.n ? __ldg(a.T + threadIdx.x) : 1;
     __syncthreads();
 
-    uint64_t fw_packed = 0, fp0 = 0, fp_pow = 1;
-    for (int i = 0; i < W; i++) {
-        fw_packed = (fw_packed << 8) | s_fw[i];
-        fp0 = fp0 * FP_BASE + s_fw[i];
-        fp_pow *= FP_BASE;
-    }
+    const uint64_t fw8 = first8(s_fw, W);
     uint32_t mask[SUB];
     uint64_t packed = 0;
 #pragma unroll
     for (int k = 0; k < SUB; k++) {
-        mask[k] = tile_triggers<WT, PT>(a, s + (size_t)k * TS_TILE, s_fw, fw_packed, fp0, fp_pow,
-                                         base + (size_t)k * TS_TILE, !WRITE);
+        mask[k] = tile_triggers<WT, PT>(a, s + (size_t)k * TS_TILE, s_fw, fw8, base + (size_t)k * TS_TILE, !WRITE);
         packed |= (uint64_t)__popc(mask[k]) << (16 * k);
+        if (!WRITE && masks) masks[((size_t)blockIdx.x * SUB + k) * TS_THREADS + threadIdx.x] = (uint16_t)mask[k];
     }
     uint64_t total;
     const uint64_t ex = block_excl_scan<uint64_t, OpAdd>(packed, total, OpAdd(), s_warp);
@@ -310,13 +327,33 @@ __global__ void __launch_bounds__(TS_THREADS) k_trigger(ScanArgs a, uint32_t *co
     }
 }
 
+// Positions from the masks of a counting pass: a CTA covers WINDOWS of it
+// (4096 or 16384), each thread one mask or four.
+template <int WINDOWS>
+__global__ void __launch_bounds__(TS_THREADS) k_trigger_write(const uint16_t *masks, const uint32_t *offsets,
+                                                              uint32_t W, uint32_t *D)
+{
+    constexpr int PER = WINDOWS / TS_THREADS / 16;       // masks per thread
+    static_assert(PER == 1 || PER == 4, "one or four masks per thread");
+    __shared__ uint32_t s_warp[32];
+    const size_t m0 = (size_t)blockIdx.x * (WINDOWS / 16) + (size_t)threadIdx.x * PER;
+    uint64_t m;
+    if constexpr (PER == 4) m = *(const uint64_t *)(masks + m0);
+    else m = masks[m0];
+    uint32_t total;
+    uint32_t o = offsets[blockIdx.x] + block_excl_scan<uint32_t, OpAdd>((uint32_t)__popcll(m), total, OpAdd(), s_warp);
+    const uint32_t p0 = (uint32_t)m0 * 16u + W - 1u;
+    for (; m; m &= m - 1ull) D[o++] = p0 + (uint32_t)__ffsll((long long)m) - 1u;
+}
+
 constexpr int TS_SUB = 4;      // tiles per CTA in the pipeline's scan
 
 template <int WT, int PT>
 static void launch_pair(Storage *st, const ScanArgs &a, unsigned blocks, uint32_t *counts, uint32_t *&D)
 {
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger<WT, PT, false, TS_SUB><<<blocks, TS_THREADS, 0, st->stream>>>(a, counts, nullptr, nullptr);
+    uint16_t *masks = slot<uint16_t>(st, S_TMP1, (size_t)blocks * TS_SUB * TS_THREADS);
+    k_trigger<WT, PT, false, TS_SUB><<<blocks, TS_THREADS, 0, st->stream>>>(a, counts, nullptr, nullptr, masks);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, a.n);
     after_launch(st);
     // exclusive scan of block counts; total -> d_scalars[0]
@@ -332,8 +369,8 @@ static void launch_pair(Storage *st, const ScanArgs &a, unsigned blocks, uint32_
     uint32_t c = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
     D = slot<uint32_t>(st, S_D, (size_t)c + 1);
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger<WT, PT, true, TS_SUB><<<blocks, TS_THREADS, 0, st->stream>>>(a, nullptr, counts, D);
-    probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n + 4ull * c);
+    k_trigger_write<TS_SUB * TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D);
+    probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n / 8 + 4ull * c);
     after_launch(st);
     k_set_u32<<<1, 1, 0, st->stream>>>(D + c, a.n + (uint32_t)a.W - 1u);
     after_launch(st);
@@ -373,24 +410,16 @@ uint32_t run_trigger_scan(Storage *st, const uint8_t *dT, uint32_t n, int W, int
 // ---------------------------------------------------------------------
 struct BatchScanArgs {
     const uint32_t *tile_text;   // [tiles] text starts before each tile
-    const uint64_t *fw;          // [k] first window of each text (packed, or fingerprint)
+    const uint64_t *fw;          // [k] first min(W, 8) bytes of each text, little-endian
     const uint32_t *xstart;      // [k] text starts in X
 };
 
-// First windows: packed big-endian bytes for W <= 8, else the fingerprint
-// used by the scan (both as computed by tile_triggers).
+// First words of the texts (a text shorter than eight bytes goes on with its
+// sentinels; X has room past its end).
 __global__ void k_first_words(const uint8_t *X, const uint32_t *xstart, uint32_t k, int W, uint64_t *fw)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= k) return;
-    const uint8_t *p = X + xstart[t];
-    uint64_t v = 0;
-    if (W <= 8) {
-        for (int i = 0; i < W; i++) v = (v << 8) | p[i];
-    } else {
-        for (int i = 0; i < W; i++) v = v * FP_BASE + p[i];
-    }
-    fw[t] = v;
+    if (t < k) fw[t] = first8(X + xstart[t], W);
 }
 
 // tile_text[b] = number of text starts below b * TS_TILE.
@@ -409,15 +438,14 @@ __global__ void k_tile_text(const uint32_t *xstart, uint32_t k, uint32_t tiles, 
 
 template <int WT, int PT>
 __device__ __forceinline__ uint32_t tile_triggers_batch(const ScanArgs &a, const BatchScanArgs &b, const uint8_t *s,
-                                                        uint32_t prevb, size_t base, uint32_t tcur, uint64_t fp_pow)
+                                                        uint32_t prevb, size_t base, uint32_t tcur)
 {
     constexpr int NB = TS_PER_THREAD + (WT > 0 ? WT : TS_MAXW) - 1;
-    constexpr int NV = (NB + 15) / 16;
+    constexpr int NV = (NB + 7 + 15) / 16;
     const int W = WT > 0 ? WT : a.W;
     const uint32_t P = PT > 0 ? (uint32_t)PT : (uint32_t)a.P;
     const size_t s0 = base + (size_t)threadIdx.x * TS_PER_THREAD;
     if (s0 >= a.n) return 0;
-
     uint32_t w[NV * 4];
     const uint8_t *src = s + (size_t)threadIdx.x * TS_PER_THREAD;
 #pragma unroll
@@ -425,33 +453,6 @@ __device__ __forceinline__ uint32_t tile_triggers_batch(const ScanArgs &a, const
         uint4 q = *(const uint4 *)(src + v * 16);
         w[v * 4 + 0] = q.x; w[v * 4 + 1] = q.y; w[v * 4 + 2] = q.z; w[v * 4 + 3] = q.w;
     }
-    uint32_t h = 0, c1 = prevb == 1u;
-    {
-        uint32_t pw = 1, acc = 0;
-#pragma unroll
-        for (int i = (WT > 0 ? WT : TS_MAXW) - 1; i >= 0; i--) {
-            if (WT == 0 && i >= W) continue;
-            const uint32_t c = bget(w, i);
-            acc += c * pw;
-            c1 += c == 1u;
-            pw = (pw * 2u) % P;
-            if (WT == 0 || WT > 16) acc %= P;
-        }
-        h = acc % P;
-    }
-    uint64_t reg = 0, fp = 0;
-    if (WT > 0 && WT <= 8) {
-#pragma unroll
-        for (int i = 0; i < (WT > 0 ? WT : 1); i++) reg = (reg << 8) | bget(w, i);
-    } else {
-#pragma unroll
-        for (int i = 0; i < (WT > 0 ? WT : TS_MAXW); i++) {
-            if (WT == 0 && i >= W) break;
-            fp = fp * FP_BASE + bget(w, i);
-        }
-    }
-    const uint64_t regmask = (WT > 0 && WT < 8) ? ((1ull << (8 * (WT > 0 ? WT : 1))) - 1ull) : ~0ull;
-    const uint32_t wW = (WT > 0 && PT > 0) ? pow2_mod(WT > 0 ? WT : 1, PT > 0 ? PT : 1) : a.wW;
     uint64_t cur = tcur ? __ldg(b.fw + tcur - 1) : 0ull;
 
     // Almost every thread sees no sentinel byte, neither just before its
@@ -470,55 +471,43 @@ __device__ __forceinline__ uint32_t tile_triggers_batch(const ScanArgs &a, const
         }
         clean = ones == 0;
     }
-    uint32_t mask = 0;
-    if (clean) {
-#pragma unroll
-        for (int j = 0; j < TS_PER_THREAD; j++) {
-            bool eq;
-            if (WT > 0 && WT <= 8) {
-                eq = reg == cur;
-            } else {
-                eq = false;
-                if (fp == cur) {
-                    const uint8_t *f = a.T + __ldg(b.xstart + tcur - 1);
-                    eq = true;
-                    for (int i = 0; i < W; i++)
-                        if (s[s0 + j - base + i] != __ldg(f + i)) { eq = false; break; }
-                }
-            }
-            if (h == 0 || eq) mask |= 1u << j;
-            if (j + 1 < TS_PER_THREAD) {
-                const uint32_t out = bget(w, j), in = bget(w, j + W);
-                h = (2u * h + in + 256u * P - out * wW) % P;
-                if (WT > 0 && WT <= 8) reg = ((reg << 8) | in) & regmask;
-                else fp = fp * FP_BASE - (uint64_t)out * fp_pow + in;
-            }
-        }
-        return mask;
+    if constexpr (WT == 5 && PT > 0) {
+        if (clean) return windows5<PT>(w, cur);
     }
+
+    uint32_t h = 0, c1 = prevb == 1u;
+    {
+        uint32_t pw = 1;
+#pragma unroll
+        for (int i = (WT > 0 ? WT : TS_MAXW) - 1; i >= 0; i--) {
+            if (WT == 0 && i >= W) continue;
+            const uint32_t c = bget(w, i);
+            h += c * pw;
+            c1 += c == 1u;
+            pw = (pw * 2u) % P;
+        }
+        h %= P;
+    }
+    const uint64_t m8 = mask8(W);
+    const uint32_t wW = (WT > 0 && PT > 0) ? pow2_mod(WT > 0 ? WT : 1, PT > 0 ? PT : 1) : a.wW;
+    uint32_t mask = 0;
 #pragma unroll
     for (int j = 0; j < TS_PER_THREAD; j++) {
         const size_t sj = s0 + j;
         const uint32_t pb = j ? bget(w, j - 1) : prevb, c = bget(w, j);
         const bool inside = sj < a.n;
-        if (inside && pb == 1u && c != 1u) {          // a text starts at sj
+        if (!clean && inside && pb == 1u && c != 1u) {          // a text starts at sj
             tcur++;
             cur = __ldg(b.fw + tcur - 1);
         }
         if (inside) {
             bool hit = false;
-            if (c1 == 0) {
-                bool eq;
-                if (WT > 0 && WT <= 8) {
-                    eq = reg == cur;
-                } else {
-                    eq = false;
-                    if (fp == cur) {
-                        const uint8_t *f = a.T + __ldg(b.xstart + tcur - 1);
-                        eq = true;
-                        for (int i = 0; i < W; i++)
-                            if (s[sj - base + i] != __ldg(f + i)) { eq = false; break; }
-                    }
+            if (clean || c1 == 0) {
+                bool eq = ((bget8(w, j) ^ cur) & m8) == 0;
+                if (eq && W > 8) {
+                    const uint8_t *f = a.T + __ldg(b.xstart + tcur - 1), *win = src + j;
+                    for (int i = 8; i < W; i++)
+                        if (win[i] != __ldg(f + i)) { eq = false; break; }
                 }
                 hit = h == 0 || eq;
             } else {
@@ -530,16 +519,14 @@ __device__ __forceinline__ uint32_t tile_triggers_batch(const ScanArgs &a, const
             const uint32_t in = bget(w, j + W);
             h = (2u * h + in + 256u * P - c * wW) % P;
             c1 += (in == 1u) - (pb == 1u);
-            if (WT > 0 && WT <= 8) reg = ((reg << 8) | in) & regmask;
-            else fp = fp * FP_BASE - (uint64_t)c * fp_pow + in;
         }
     }
     return mask;
 }
 
-template <int WT, int PT, bool WRITE>
+template <int WT, int PT>
 __global__ void __launch_bounds__(TS_THREADS) k_trigger_batch(ScanArgs a, BatchScanArgs b, uint32_t *counts,
-                                                              const uint32_t *offsets, uint32_t *D)
+                                                              uint16_t *masks)
 {
     __shared__ __align__(16) uint8_t s[TS_TILE + TS_MAXW + 64];
     __shared__ uint32_t s_warp[32];
@@ -570,22 +557,11 @@ __global__ void __launch_bounds__(TS_THREADS) k_trigger_batch(ScanArgs a, BatchS
     const uint32_t ex_st = block_excl_scan<uint32_t, OpAdd>(nst, tot, OpAdd(), s_warp);
     const uint32_t tcur = __ldg(b.tile_text + blockIdx.x) + ex_st;
     __syncthreads();
-    uint64_t fp_pow = 1;
-    for (int i = 0; i < W; i++) fp_pow *= FP_BASE;
-    uint32_t mask = tile_triggers_batch<WT, PT>(a, b, s, prevb, base, tcur, fp_pow);
-    uint32_t cnt = __popc(mask), total;
-    uint32_t ex = block_excl_scan<uint32_t, OpAdd>(cnt, total, OpAdd(), s_warp);
-    if (!WRITE) {
-        if (threadIdx.x == 0) counts[blockIdx.x] = total;
-        return;
-    }
-    uint32_t out = offsets[blockIdx.x] + ex;
-    const uint32_t s0 = (uint32_t)(base + o);
-    while (mask) {
-        int j = __ffs(mask) - 1;
-        mask &= mask - 1;
-        D[out++] = s0 + (uint32_t)j + (uint32_t)W - 1u;
-    }
+    const uint32_t mask = tile_triggers_batch<WT, PT>(a, b, s, prevb, base, tcur);
+    masks[(size_t)blockIdx.x * TS_THREADS + threadIdx.x] = (uint16_t)mask;
+    uint32_t total;
+    block_excl_scan<uint32_t, OpAdd>((uint32_t)__popc(mask), total, OpAdd(), s_warp);
+    if (threadIdx.x == 0) counts[blockIdx.x] = total;
 }
 
 template <int WT, int PT>
@@ -593,7 +569,8 @@ static uint32_t launch_pair_batch(Storage *st, const ScanArgs &a, const BatchSca
                                   uint32_t *counts, uint32_t *&D)
 {
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger_batch<WT, PT, false><<<blocks, TS_THREADS, 0, st->stream>>>(a, b, counts, nullptr, nullptr);
+    uint16_t *masks = slot<uint16_t>(st, S_BIGL, (size_t)blocks * TS_THREADS);
+    k_trigger_batch<WT, PT><<<blocks, TS_THREADS, 0, st->stream>>>(a, b, counts, masks);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, a.n);
     after_launch(st);
     uint32_t *tot = (uint32_t *)st->d_scalars;
@@ -608,8 +585,8 @@ static uint32_t launch_pair_batch(Storage *st, const ScanArgs &a, const BatchSca
     const uint32_t c = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
     D = slot<uint32_t>(st, S_D, (size_t)c + 1);
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger_batch<WT, PT, true><<<blocks, TS_THREADS, 0, st->stream>>>(a, b, nullptr, counts, D);
-    probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n + 4ull * c);
+    k_trigger_write<TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D);
+    probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n / 8 + 4ull * c);
     after_launch(st);
     return c;
 }
@@ -699,7 +676,7 @@ static int64_t noalloc_launch(const ScanArgs &a, unsigned blocks, uint32_t *scra
     check_cuda(cudaMemsetAsync(status, 0, (256 + 64) * sizeof(uint32_t), stream));
     ScanArgs b = a;
     b.flags = words;
-    k_trigger<WT, PT, false, 1><<<blocks, TS_THREADS, 0, stream>>>(b, counts, nullptr, nullptr);
+    k_trigger<WT, PT, false, 1><<<blocks, TS_THREADS, 0, stream>>>(b, counts, nullptr, nullptr, nullptr);
     check_cuda(cudaGetLastError());
     const unsigned tiles = (blocks + NOALLOC_STILE - 1) / NOALLOC_STILE;
     const LookBack lb{(uint64_t *)status, tiles, 1u, words + 2, words + 3};
@@ -714,7 +691,7 @@ static int64_t noalloc_launch(const ScanArgs &a, unsigned blocks, uint32_t *scra
     if (host_words[3]) return GBWT_TIMEOUT;
     const uint32_t c = host_words[1];
     if ((int64_t)c + 1 > capacity) return GBWT_BAD_PARAMETER;
-    k_trigger<WT, PT, true, 1><<<blocks, TS_THREADS, 0, stream>>>(b, nullptr, counts, D);
+    k_trigger<WT, PT, true, 1><<<blocks, TS_THREADS, 0, stream>>>(b, nullptr, counts, D, nullptr);
     k_set_u32<<<1, 1, 0, stream>>>(D + c, a.n + (uint32_t)a.W - 1u);
     check_cuda(cudaGetLastError());
     check_cuda(cudaStreamSynchronize(stream));
