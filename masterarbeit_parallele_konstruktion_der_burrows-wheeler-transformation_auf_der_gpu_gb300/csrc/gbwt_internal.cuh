@@ -36,7 +36,7 @@ enum Slot : int {
     S_BIGL, S_BIGM,
     // second-level parse
     S_2SYM, S_2TRIG, S_2START, S_2SLOT, S_2PID, S_2DLEN, S_2DOFF, S_2DSTART, S_2OCC, S_2DICT, S_2DPHR, S_2ISA, S_2SA,
-    S_2RANK, S_2PISA, S_2PSA,
+    S_2RANK, S_2PISA, S_2PSA, S_2TSTART, S_2TID, S_2ZEND,
     S_NUM
 };
 
@@ -244,7 +244,10 @@ void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, cons
 int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
                      const uint32_t *occ, uint32_t *isa, uint32_t *sa);
 // Parse suffix array by parsing the parse; false (nothing done) when that does not pay.
-bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord);
+bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord, const BatchText *bt);
+// Suffix array over all texts' parses (text of phrase i: ptid[i]; one past text t's last: zend[t]).
+int parse_sa_batch(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
+                   const uint32_t *ptid, const uint32_t *zend, uint32_t k, bool two, uint32_t *isa, uint32_t *sa);
 void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord);
 void run_parse_sa_batch(Storage *st, Phrases &ph, DictOrder &dord, const BatchText &bt, ParseOrder &pord);
 // Group index of every dictionary position that starts a suffix longer than

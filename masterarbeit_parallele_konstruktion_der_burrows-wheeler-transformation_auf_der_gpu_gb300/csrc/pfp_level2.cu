@@ -12,7 +12,10 @@
 //   symbols   V[i] = lexicographic rank of phrase i, plus 1; V[z] = 0 ends it
 //   triggers  positions 1..z-1 whose symbol hashes below a threshold (one in
 //             L2_RATE), and the end; phrase j of the second level spans
-//             V[s_j .. s_{j+1}], both triggers included
+//             V[s_j .. s_{j+1}], both triggers included.  In a batch every text
+//             starts a phrase, and the phrase before it ends with the symbol 0
+//             instead: no phrase crosses a text, and suffixes of different
+//             texts may tie, as in the plain batch parse
 //   phrases   exact deduplication (hash table, then symbol by symbol), one
 //             dictionary, sorted by the engine that sorts the first one
 //   parse     suffix array of the second-level parse, L2_RATE times shorter
@@ -55,18 +58,24 @@ __device__ __forceinline__ bool l2_trigger(uint32_t v)
     return x < 0xFFFFFFFFu / L2_RATE;
 }
 
-// Symbols and trigger bits.
-__global__ void k_l2_symbols(const uint32_t *pid, const uint32_t *lexrank, uint32_t z, uint32_t *V, uint32_t *bits)
+// Symbols, start bits (triggers and text starts) and, with ptid (the text of
+// every phrase), text-start bits.  Position 0 starts a phrase without a bit.
+__global__ void k_l2_symbols(const uint32_t *pid, const uint32_t *lexrank, const uint32_t *ptid, uint32_t z, uint32_t *V,
+                             uint32_t *bits, uint32_t *tstart)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool t = false;
+    bool t = false, ts = false;
     if (i < z) {
         const uint32_t v = lexrank[pid[i]] + 1u;
         V[i] = v;
-        t = i > 0 && l2_trigger(v);
+        ts = ptid && i > 0 && ptid[i] != ptid[i - 1];
+        t = ts || (i > 0 && l2_trigger(v));
     }
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, t);
-    if ((threadIdx.x & 31u) == 0 && i < z) bits[i >> 5] = m;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, t), tm = __ballot_sync(0xFFFFFFFFu, ts);
+    if ((threadIdx.x & 31u) == 0 && i < z) {
+        bits[i >> 5] = m;
+        if (tstart) tstart[i >> 5] = tm;
+    }
 }
 struct LoadTrigWord {
     const uint32_t *w;
@@ -89,7 +98,18 @@ __global__ void k_l2_ends(uint32_t *s, uint32_t z2, uint32_t z)
     s[z2] = z;
 }
 
-__device__ __forceinline__ uint32_t l2_symbol(const uint32_t *V, uint32_t z, uint32_t i) { return i < z ? __ldg(V + i) : 0u; }
+// The symbols: V, and at a phrase's end e the trigger there or 0 at the end of
+// a text.
+struct L2Text {
+    const uint32_t *V, *tstart;      // tstart: text-start bits of a batch, else null
+    uint32_t z;
+    __device__ __forceinline__ uint32_t inside(uint32_t i) const { return __ldg(V + i); }
+    __device__ __forceinline__ uint32_t end(uint32_t e) const
+    {
+        if (e >= z || (tstart && ((tstart[e >> 5] >> (e & 31u)) & 1u))) return 0u;
+        return __ldg(V + e);
+    }
+};
 
 __device__ __forceinline__ uint64_t l2_mulmod(uint64_t a, uint64_t b)
 {
@@ -102,7 +122,7 @@ __device__ __forceinline__ uint64_t l2_mulmod(uint64_t a, uint64_t b)
 // Fingerprint (polynomial mod 2^61 - 1) and table slot of every phrase.
 // give_up: [0] phrase too long or table full, [1] distinct phrases so far,
 // [2] two phrases share a fingerprint.
-__global__ void k_l2_hash(const uint32_t *V, uint32_t z, const uint32_t *s, uint32_t z2, uint64_t base,
+__global__ void k_l2_hash(L2Text V, const uint32_t *s, uint32_t z2, uint64_t base,
                           unsigned long long *tkeys, uint32_t *tvals, int logc, uint32_t limit, uint32_t *slot_of,
                           uint32_t *give_up)
 {
@@ -116,7 +136,7 @@ __global__ void k_l2_hash(const uint32_t *V, uint32_t z, const uint32_t *s, uint
     }
     uint64_t h = len;
     for (uint32_t i = a; i <= e; i++) {
-        h = l2_mulmod(h, base) + l2_symbol(V, z, i) + 1u;
+        h = l2_mulmod(h, base) + (i < e ? V.inside(i) : V.end(e)) + 1u;
         if (h >= L2_M61) h -= L2_M61;
     }
     const unsigned long long key = h + 1u;                       // 0 marks an empty slot
@@ -143,7 +163,7 @@ __global__ void k_l2_hash(const uint32_t *V, uint32_t z, const uint32_t *s, uint
 }
 
 // Every phrase against its representative, symbol by symbol.
-__global__ void k_l2_verify(const uint32_t *V, uint32_t z, const uint32_t *s, uint32_t z2, const uint32_t *tvals,
+__global__ void k_l2_verify(L2Text V, const uint32_t *s, uint32_t z2, const uint32_t *tvals,
                             const uint32_t *slot_of, uint32_t *isrep, uint32_t *give_up)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -158,8 +178,9 @@ __global__ void k_l2_verify(const uint32_t *V, uint32_t z, const uint32_t *s, ui
     if (r >= z2) { give_up[2] = 1; return; }
     const uint32_t a = s[j], b = s[r], len = s[j + 1] - a;
     if (s[r + 1] - b != len) { give_up[2] = 1; return; }
-    for (uint32_t i = 0; i <= len; i++)
-        if (l2_symbol(V, z, a + i) != l2_symbol(V, z, b + i)) { give_up[2] = 1; return; }
+    for (uint32_t i = 0; i < len; i++)
+        if (V.inside(a + i) != V.inside(b + i)) { give_up[2] = 1; return; }
+    if (V.end(a + len) != V.end(b + len)) give_up[2] = 1;
 }
 
 // Dense ids and dictionary offsets of the representatives in one scan:
@@ -194,14 +215,14 @@ __global__ void k_l2_ids(const uint32_t *slot_of, const uint32_t *dense, uint32_
     atomicAdd(occ + id, 1u);
 }
 // Eight lanes per distinct phrase (they average about ten symbols).
-__global__ void k_l2_dict(const uint32_t *V, uint32_t z, uint32_t d, const uint32_t *doff, const uint32_t *dlen,
+__global__ void k_l2_dict(L2Text V, uint32_t d, const uint32_t *doff, const uint32_t *dlen,
                           const uint32_t *dstart, uint32_t *dict, uint32_t *dphr)
 {
     const uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     if (id >= d) return;
     const uint32_t off = doff[id], len = dlen[id], st = dstart[id];
     for (uint32_t i = threadIdx.x & 7u; i < len; i += 8u) {
-        dict[off + i] = l2_symbol(V, z, st + i);
+        dict[off + i] = i + 1u < len ? V.inside(st + i) : V.end(st + i);
         dphr[off + i] = id;
     }
 }
@@ -247,6 +268,40 @@ __global__ void k_l2_slots(const uint32_t *psa, const uint32_t *pisa, const uint
     if (t >= z2) return;
     uint32_t j = z2 - 1u;
     if (t) j = psa[t - 1u < pisa[0] ? t - 1u : t] - 1u;
+    from[t] = doff[pid[j]];
+    to[t] = s[j];
+    cnt[t] = s[j + 1] - s[j];
+}
+// Batch: the text of every second-level phrase, and one past each text's last.
+__global__ void k_l2_texts(const uint32_t *s, uint32_t z2, const uint32_t *ptid, uint32_t *tid2, uint32_t *zend2)
+{
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= z2) return;
+    const uint32_t t = ptid[s[j]];
+    tid2[j] = t;
+    if (j + 1u == z2 || ptid[s[j + 1]] != t) zend2[t] = j + 1u;
+}
+// Batch slots: every text's last phrase, then the phrase before each suffix in
+// suffix-array order (an empty slot for a text's first).
+__global__ void k_l2_slots_batch(const uint32_t *psa, const uint32_t *pid, const uint32_t *s, const uint32_t *doff,
+                                 const uint32_t *tid2, const uint32_t *zend2, uint32_t k, uint32_t z2, uint32_t *from,
+                                 uint32_t *to, uint32_t *cnt)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= k + z2) return;
+    uint32_t j;
+    if (t < k) {
+        j = zend2[t] - 1u;
+    } else {
+        const uint32_t x = psa[t - k];
+        if (x == 0 || tid2[x] != tid2[x - 1u]) {
+            from[t] = 0;
+            to[t] = 0;
+            cnt[t] = 0;
+            return;
+        }
+        j = x - 1u;
+    }
     from[t] = doff[pid[j]];
     to[t] = s[j];
     cnt[t] = s[j + 1] - s[j];
@@ -310,18 +365,21 @@ __global__ void k_l2_first(const uint32_t *sa, uint32_t z, uint32_t *first)
     if (r < z && sa[r] < 2u) first[sa[r]] = r;
 }
 
-bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord)
+bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord, const BatchText *bt)
 {
     const uint32_t z = ph.z;
     if (z < L2_MIN_Z || ph.d > z / L2_DISTINCT) return false;
     // symbols, triggers, phrase starts
-    uint32_t *V = slot<uint32_t>(st, S_2SYM, z);
+    uint32_t *sym = slot<uint32_t>(st, S_2SYM, z);
     const size_t zw = ((size_t)z + 31) / 32;
     uint32_t *trig = slot<uint32_t>(st, S_2TRIG, zw);
-    k_l2_symbols<<<grid_for(z, 256), 256, 0, st->stream>>>(ph.pid, dord.lexrank, z, V, trig);
+    uint32_t *tstart = bt ? slot<uint32_t>(st, S_2TSTART, zw) : nullptr;
+    k_l2_symbols<<<grid_for(z, 256), 256, 0, st->stream>>>(ph.pid, dord.lexrank, bt ? bt->ptid : nullptr, z, sym, trig,
+                                                           tstart);
     after_launch(st);
+    const L2Text V{sym, tstart, z};
     // starts are stored by the scan that counts them: room for one in three
-    // positions triggering, more means symbols that hash alike and no gain
+    // positions, more means symbols that hash alike (or tiny texts) and no gain
     const uint32_t cap = z / 3u;
     uint32_t *s = slot<uint32_t>(st, S_2START, (size_t)cap + 2);
     check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
@@ -346,10 +404,10 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     check_cuda(cudaMemsetAsync(tkeys, 0, (size_t)c * 8, st->stream));
     check_cuda(cudaMemsetAsync(give_up, 0, 3 * 4, st->stream));
     check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    k_l2_hash<<<grid_for(z2, 256), 256, 0, st->stream>>>(V, z, s, z2, 0x0A5C3D1F2B4E6987ull, tkeys, tvals, logc, limit,
+    k_l2_hash<<<grid_for(z2, 256), 256, 0, st->stream>>>(V, s, z2, 0x0A5C3D1F2B4E6987ull, tkeys, tvals, logc, limit,
                                                          slot_of, give_up);
     after_launch(st);
-    k_l2_verify<<<grid_for(z2, 256), 256, 0, st->stream>>>(V, z, s, z2, tvals, slot_of, pid, give_up);
+    k_l2_verify<<<grid_for(z2, 256), 256, 0, st->stream>>>(V, s, z2, tvals, slot_of, pid, give_up);
     after_launch(st);
     check_cuda(cudaMemcpyAsync(st->h_scalars + 4, give_up, 3 * 4, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
@@ -366,7 +424,7 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     after_launch(st);
     // dictionary and its order
     uint32_t *dict = slot<uint32_t>(st, S_2DICT, N), *dphr = slot<uint32_t>(st, S_2DPHR, N);
-    k_l2_dict<<<grid_for((size_t)d * 8, 256), 256, 0, st->stream>>>(V, z, d, doff, dlen, dstart, dict, dphr);
+    k_l2_dict<<<grid_for((size_t)d * 8, 256), 256, 0, st->stream>>>(V, d, doff, dlen, dstart, dict, dphr);
     after_launch(st);
     const int bps = bits_for((uint64_t)ph.d + 1u);
     const int h0 = 2;      // 1, 2 or 3 symbols in the first key: 4.45, 4.19, 4.26 ms (512 MiB DNA); 2 * bps < 64
@@ -380,7 +438,16 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     phrase_ranks(st, N, d, isa, doff, rank);
     // suffix array of the second-level parse
     uint32_t *pisa = slot<uint32_t>(st, S_2PISA, z2), *psa = slot<uint32_t>(st, S_2PSA, z2);
-    pord.rounds += parse_sa_buckets(st, z2, d, pid, rank, occ, pisa, psa);
+    uint32_t *tid2 = nullptr, *zend2 = nullptr;
+    if (bt) {
+        tid2 = slot<uint32_t>(st, S_2TID, z2);
+        zend2 = slot<uint32_t>(st, S_2ZEND, bt->k);
+        k_l2_texts<<<grid_for(z2, 256), 256, 0, st->stream>>>(s, z2, bt->ptid, tid2, zend2);
+        after_launch(st);
+        pord.rounds += parse_sa_batch(st, z2, d, pid, rank, tid2, zend2, bt->k, true, pisa, psa);
+    } else {
+        pord.rounds += parse_sa_buckets(st, z2, d, pid, rank, occ, pisa, psa);
+    }
     // group numbers per dictionary position (sa is dead: it takes them)
     const size_t nw = ((size_t)N + 31) / 32;
     uint32_t *bits = slot<uint32_t>(st, S_TMP0, nw), *pre = slot<uint32_t>(st, S_TMP1, nw);
@@ -393,22 +460,28 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     k_l2_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(N, rem8, isa, bits, pre, grp);
     after_launch(st);
     // emission and the sort by group
-    uint32_t *from = slot<uint32_t>(st, S_ACTX, z2), *to = slot<uint32_t>(st, S_ACTG, z2);
-    uint32_t *cnt = slot<uint32_t>(st, S_ACTX2, (size_t)z2 + 1);
-    k_l2_slots<<<grid_for(z2, 256), 256, 0, st->stream>>>(psa, pisa, pid, s, doff, z2, from, to, cnt);
+    const uint32_t S = bt ? bt->k + z2 : z2;
+    uint32_t *from = slot<uint32_t>(st, S_ACTX, S), *to = slot<uint32_t>(st, S_ACTG, S);
+    uint32_t *cnt = slot<uint32_t>(st, S_ACTX2, (size_t)S + 1);
+    if (bt)
+        k_l2_slots_batch<<<grid_for(S, 256), 256, 0, st->stream>>>(psa, pid, s, doff, tid2, zend2, bt->k, z2, from, to,
+                                                                   cnt);
+    else
+        k_l2_slots<<<grid_for(S, 256), 256, 0, st->stream>>>(psa, pisa, pid, s, doff, z2, from, to, cnt);
     after_launch(st);
-    device_scan<uint32_t, OpAdd>(st, z2, LoadArr<uint32_t>{cnt}, StoreArr<uint32_t>{cnt}, false, cnt + z2);
-    check_cuda(cudaMemcpyAsync(st->d_scalars + 1, cnt + z2, 4, cudaMemcpyDeviceToDevice, st->stream));
+    device_scan<uint32_t, OpAdd>(st, S, LoadArr<uint32_t>{cnt}, StoreArr<uint32_t>{cnt}, false, cnt + S);
+    check_cuda(cudaMemcpyAsync(st->d_scalars + 1, cnt + S, 4, cudaMemcpyDeviceToDevice, st->stream));
     fetch_scalars(st, 2);
     const uint32_t G = (uint32_t)st->h_scalars[0];
     if (G == 0 || (uint32_t)st->h_scalars[1] != z) throw Error{GBWT_INTERNAL_ERROR};
     uint32_t *k = slot<uint32_t>(st, S_KEY0, z), *k_alt = slot<uint32_t>(st, S_KEY1, z);
     uint32_t *v = slot<uint32_t>(st, S_PSA, z), *v_alt = slot<uint32_t>(st, S_PISA, z);
-    k_l2_emit<<<grid_for(z2, EL_T), EL_T, 0, st->stream>>>(z2, cnt, from, to, grp, z, k, v, st->d_flags);
+    k_l2_emit<<<grid_for(S, EL_T), EL_T, 0, st->stream>>>(S, cnt, from, to, grp, z, k, v, st->d_flags);
     after_launch(st);
     radix_sort<uint32_t, true>(st, k, k_alt, v, v_alt, z, 0, bits_for(G - 1u));
     pord.sa = v;
     pord.isa = nullptr;
+    if (bt) return true;
     uint32_t *first = st->d_flags + 32;
     k_l2_first<<<grid_for(z, 256), 256, 0, st->stream>>>(v, z, first);
     after_launch(st);

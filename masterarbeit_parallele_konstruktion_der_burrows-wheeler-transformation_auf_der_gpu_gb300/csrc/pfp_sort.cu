@@ -1212,7 +1212,7 @@ void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord)
 {
     const uint32_t z = ph.z;
     const int kp = tune_parse_key_phrases(st);
-    if (kp == 0 && run_parse_sa_level2(st, ph, dord, pord)) return;
+    if (kp == 0 && run_parse_sa_level2(st, ph, dord, pord, nullptr)) return;
     pord.isa = slot<uint32_t>(st, S_PISA, z);
     pord.sa = slot<uint32_t>(st, S_PSA, z);
     if (kp == 1 || kp == 2) {
@@ -1244,27 +1244,34 @@ __global__ void k_parse_keys_batch(const uint32_t *pid, const uint32_t *lexrank,
 // Suffix array over all texts' parses at once.  Suffixes of different texts
 // may be equal strings and then share a rank; the order restricted to one
 // text is that text's own parse suffix array.
-void run_parse_sa_batch(Storage *st, Phrases &ph, DictOrder &dord, const BatchText &bt, ParseOrder &pord)
+int parse_sa_batch(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
+                   const uint32_t *ptid, const uint32_t *zend, uint32_t k, bool two, uint32_t *isa, uint32_t *sa)
 {
-    const uint32_t z = ph.z;
     uint64_t *keys = slot<uint64_t>(st, S_KEY0, z);
-    const int lb = bits_for(ph.d);
-    const bool two = tune_parse_key_phrases(st) != 1;
-    k_parse_keys_batch<<<grid_for(z, 256), 256, 0, st->stream>>>(ph.pid, dord.lexrank, bt.ptid, z, lb, two, keys);
+    const int lb = bits_for(d);
+    k_parse_keys_batch<<<grid_for(z, 256), 256, 0, st->stream>>>(pid, lexrank, ptid, z, lb, two, keys);
     after_launch(st);
     uint32_t *remv = slot<uint32_t>(st, S_TMP0, z);
-    k_batch_rem<<<grid_for(z, 256), 256, 0, st->stream>>>(bt.ptid, bt.zend, z, remv);
+    k_batch_rem<<<grid_for(z, 256), 256, 0, st->stream>>>(ptid, zend, z, remv);
     after_launch(st);
     // bitmap words for positions up to z + BR_MAPH (ranges reach past z)
     const size_t map_words = ((size_t)z + BR_MAPH + 64u * 32u) / (64u * 32u) + 1u;
     uint32_t *endmap = slot<uint32_t>(st, S_TMP1, map_words);
     check_cuda(cudaMemsetAsync(endmap, 0, map_words * 4, st->stream));
-    k_text_endmap<<<grid_for(bt.k, 256), 256, 0, st->stream>>>(bt.zend, bt.k, endmap);
+    k_text_endmap<<<grid_for(k, 256), 256, 0, st->stream>>>(zend, k, endmap);
     after_launch(st);
-    pord.isa = slot<uint32_t>(st, S_PISA, z);
-    pord.sa = slot<uint32_t>(st, S_PSA, z);
-    pord.rounds = prefix_doubling(st, z, two ? lb + bits_for(ph.d - 1) : bits_for(ph.d - 1), two ? 2u : 1u,
-                                  BatchParseRem{remv, endmap}, pord.isa, pord.sa);
+    return prefix_doubling(st, z, two ? lb + bits_for(d - 1) : bits_for(d - 1), two ? 2u : 1u,
+                           BatchParseRem{remv, endmap}, isa, sa);
+}
+
+void run_parse_sa_batch(Storage *st, Phrases &ph, DictOrder &dord, const BatchText &bt, ParseOrder &pord)
+{
+    const int kp = tune_parse_key_phrases(st);
+    if (kp == 0 && run_parse_sa_level2(st, ph, dord, pord, &bt)) return;
+    pord.isa = slot<uint32_t>(st, S_PISA, ph.z);
+    pord.sa = slot<uint32_t>(st, S_PSA, ph.z);
+    pord.rounds = parse_sa_batch(st, ph.z, ph.d, ph.pid, dord.lexrank, bt.ptid, bt.zend, bt.k, kp != 1, pord.isa,
+                                 pord.sa);
 }
 
 }  // namespace gbwt

@@ -69,3 +69,30 @@ def test_parse_suffix_array(storage, orc):
     a, b = sa[:-1], sa[1:]
     lt = (ranks[a] < ranks[b]) | ((ranks[a] == ranks[b]) & (inv[a + 1] < inv[b + 1]))
     assert np.array_equal(np.sort(sa), np.arange(n)) and bool(lt.all())
+
+
+@pytest.mark.parametrize("kind", ["even", "uneven", "shared", "tiny among large", "constant"])
+def test_batch(storage, orc, kind):
+    # W = 1, P = 1: as many phrases as bytes; texts that share content or end inside a repeat
+    rng = np.random.default_rng(len(kind))
+    if kind == "even":
+        texts = [_copies(i, 4000, 150_000, 4, 1e-3) for i in range(30)]
+    elif kind == "uneven":
+        texts = [_copies(i, 900 + 37 * i, int(n), 5, 1e-3) for i, n in enumerate(rng.integers(1, 900_000, size=14))]
+        texts.append(_copies(99, 5000, MIN_Z // 2, 5, 1e-3))
+    elif kind == "shared":
+        whole = _copies(5, 20_000, 700_000, 4, 1e-3)
+        texts = [whole[a:] for a in rng.integers(0, 100_000, size=8)] + [whole[:300_001], whole.copy(), whole.copy()]
+    elif kind == "tiny among large":
+        texts = [_copies(1, 30_000, MIN_Z + 5, 4, 1e-3)] + [np.full(1 + i % 3, 2 + i % 4, np.uint8) for i in range(50)]
+    else:
+        texts = [np.full(400_000, 2 + i % 2, np.uint8) for i in range(12)]
+    assert sum(len(t) for t in texts) >= MIN_Z
+    for L, t in zip(storage.pfp_bwt_batch(texts, 1, 1), texts):
+        assert np.array_equal(L, orc.sa_bwt(t)), len(t)
+
+
+def test_batch_wider_windows(storage, orc):
+    texts = [_copies(50 + i, 20_000 + 991 * i, 1_400_000 + 7 * i, 4, 1e-3) for i in range(12)]
+    for L, t in zip(storage.pfp_bwt_batch(texts, 2, 3), texts):
+        assert np.array_equal(L, orc.sa_bwt(t))
