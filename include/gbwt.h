@@ -58,7 +58,10 @@ extern "C" {
 typedef struct gbwt_stats {
     int64_t n;              /* text length                                   */
     int64_t z;              /* phrase occurrences (K: size_D)                */
-    int64_t d;              /* distinct phrases                              */
+    int64_t d;              /* distinct phrases; in a batch whose dictionary
+                               keeps its texts apart, equal phrases of
+                               different texts count each (dict_bytes and s
+                               likewise)                                     */
     int64_t dict_bytes;     /* sum of distinct phrase lengths                */
     int64_t s;              /* |S|: distinct phrase suffixes longer than W   */
     int64_t s_elems;        /* (phrase, offset) pairs behind S               */

@@ -129,7 +129,7 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
         return z;
     }
 
-    run_assembly(st, dT, un, W, ph, dord, pord, dOut);
+    run_assembly(st, dT, un, W, ph, dord, pord, dOut, un);
     stage_mark(st, 6);
     if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,

@@ -32,7 +32,7 @@ enum Slot : int {
     S_ELEM0, S_ELEM1,
     S_LOOKBACK, S_RSHIST,
     S_TMP0, S_TMP1, S_TMP2, S_PIDPC, S_TILEG, S_ACTX2, S_ACTG2, S_LCB, S_LCBMAP,
-    S_BX, S_BMETA, S_BTID, S_BZEND, S_BLAST, S_BCODE, S_SSTART,
+    S_BX, S_BMETA, S_BTID, S_BZEND, S_BLAST, S_BCODE, S_SSTART, S_DTID, S_PKEYS, S_PVALS, S_PSLOT,
     S_BIGL, S_BIGM,
     // second-level parse
     S_2SYM, S_2TRIG, S_2START, S_2SLOT, S_2PID, S_2DLEN, S_2DOFF, S_2DSTART, S_2OCC, S_2DICT, S_2DPHR, S_2ISA, S_2SA,
@@ -210,6 +210,8 @@ struct Phrases {
     uint32_t *pcmin = nullptr, *pcmax = nullptr;  // [d] min/max preceding byte
     uint8_t *dict = nullptr;           // [dict_bytes] concatenated phrases
     uint32_t *dphr = nullptr;          // [dict_bytes] phrase id per position
+    uint32_t *dtid = nullptr;          // [d] text of the distinct phrase (a batch kept apart by text), else null
+    uint32_t texts = 1;                // texts that the dictionary keeps apart
 };
 // A batch of texts laid out in one padded buffer X: text t at xstart[t],
 // followed by W sentinel bytes (value 1) that no text byte can take.  A
@@ -221,7 +223,10 @@ struct BatchText {
     const uint32_t *zend = nullptr;    // [k] one past the last phrase of each text
     const uint8_t *lastb = nullptr;    // [k] last byte of each text
 };
-void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, const BatchText *bt = nullptr);
+// With may_part, equal phrases of different texts of a batch stay distinct
+// where that costs little (then ph.dtid is set).
+void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, const BatchText *bt = nullptr,
+                 bool may_part = false);
 
 struct DictOrder {
     uint32_t *isa = nullptr;     // [dict_bytes] final group head per position
@@ -254,8 +259,10 @@ void run_parse_sa_batch(Storage *st, Phrases &ph, DictOrder &dord, const BatchTe
 // W (equal suffixes share one group; groups numbered in dictionary order).
 uint32_t run_group_index(Storage *st, Phrases &ph, DictOrder &dord, int W, uint32_t *&grp_of);
 
-void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
-                  DictOrder &dord, ParseOrder &pord, uint8_t *dOut);
+// bt: a batch kept apart by text (dT is the padded buffer of n bytes, the output
+// n_out bytes, text after text); null: one text, n_out = n.
+void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, DictOrder &dord, ParseOrder &pord,
+                  uint8_t *dOut, uint32_t n_out, const BatchText *bt = nullptr);
 
 void stage_mark(Storage *st, int idx);
 

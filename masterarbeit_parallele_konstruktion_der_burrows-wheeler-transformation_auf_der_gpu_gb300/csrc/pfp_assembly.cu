@@ -233,8 +233,8 @@ struct Emit {
 
 // Per emission slot t: phrase id, number of mixed elements and the byte
 // preceding the occurrence (the random gathers happen once, here).
-__global__ void k_emit_prep(Emit e, const uint32_t *pidpc, const uint8_t *T, uint32_t n, int W, uint32_t *emq,
-                            uint8_t *emp, uint32_t *ecnt)
+__global__ void k_emit_prep(Emit e, const uint32_t *pidpc, const uint8_t *T, uint32_t n, int W, const uint32_t *ptid,
+                            const uint8_t *lastb, uint32_t *emq, uint8_t *emp, uint32_t *ecnt)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= e.z) return;
@@ -246,8 +246,12 @@ __global__ void k_emit_prep(Emit e, const uint32_t *pidpc, const uint8_t *T, uin
         prev = v & 0xFFu;
     } else {
         q = e.pid[k];
-        const uint32_t start = k ? e.D[k - 1] - (uint32_t)W + 1u : 0u;
-        prev = preceding_byte(T, n, start);
+        if (ptid && (k == 0 || T[e.D[k - 1]] == 1)) {
+            prev = lastb[ptid[k]];            // a text's first phrase follows the text's last byte
+        } else {
+            const uint32_t start = k ? e.D[k - 1] - (uint32_t)W + 1u : 0u;
+            prev = preceding_byte(T, n, start);
+        }
     }
     emq[t] = q;
     emp[t] = (uint8_t)prev;
@@ -464,7 +468,7 @@ __global__ void k_primary_count(const uint32_t *sa, const uint32_t *first, uint3
 template <typename E>
 static void mixed_blocks(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, ParseOrder &pord,
                          const uint32_t *moff, const uint32_t *mb, const uint16_t *mc, const uint32_t *delta,
-                         uint32_t B, uint32_t M, uint8_t *dOut)
+                         uint32_t B, uint32_t M, uint8_t *dOut, uint32_t n_out, const BatchText *bt)
 {
     E *elem = slot<E>(st, S_ELEM0, M);
     E *elem_alt = slot<E>(st, S_ELEM1, M);
@@ -473,7 +477,8 @@ static void mixed_blocks(Storage *st, const uint8_t *dT, uint32_t n, int W, Phra
     uint32_t *emq = slot<uint32_t>(st, S_TMP0, z);
     uint32_t *ecnt = slot<uint32_t>(st, S_TMP1, (size_t)z + 1);
     uint8_t *emp = (uint8_t *)slot<uint32_t>(st, S_TMP2, z / 4 + 1);
-    k_emit_prep<<<grid_for(z, 256), 256, 0, st->stream>>>(e, ph.pidpc, dT, n, W, emq, emp, ecnt);
+    k_emit_prep<<<grid_for(z, 256), 256, 0, st->stream>>>(e, ph.pidpc, dT, n, W, bt ? bt->ptid : nullptr,
+                                                            bt ? bt->lastb : nullptr, emq, emp, ecnt);
     after_launch(st);
     // in-place exclusive scan of the counts; ecnt[z] = total
     device_scan<uint32_t, OpAdd>(st, z, LoadArr<uint32_t>{ecnt}, StoreArr<uint32_t>{ecnt}, false, ecnt + z);
@@ -485,7 +490,7 @@ static void mixed_blocks(Storage *st, const uint8_t *dT, uint32_t n, int W, Phra
     if (st->tuning.mixed_radix_bits == 10) radix_sort<E, false, 10>(st, elem, elem_alt, nv, nv2, M, 8, 8 + bits_for(B - 1));
     else radix_sort<E, false, 8>(st, elem, elem_alt, nv, nv2, M, 8, 8 + bits_for(B - 1));
     probe_begin(st, GBWT_PROBE_MIXED_SCATTER);
-    k_mixed_scatter<E><<<grid_for((M + 3) / 4, 256), 256, 0, st->stream>>>(elem, M, delta, B, dOut, n, st->d_flags);
+    k_mixed_scatter<E><<<grid_for((M + 3) / 4, 256), 256, 0, st->stream>>>(elem, M, delta, B, dOut, n_out, st->d_flags);
     probe_end(st, GBWT_PROBE_MIXED_SCATTER, (uint64_t)M * (sizeof(E) + 1));
     after_launch(st);
 }
@@ -509,8 +514,8 @@ uint32_t run_group_index(Storage *st, Phrases &ph, DictOrder &dord, int W, uint3
     return G;
 }
 
-void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, DictOrder &dord,
-                  ParseOrder &pord, uint8_t *dOut)
+void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, DictOrder &dord, ParseOrder &pord,
+                  uint8_t *dOut, uint32_t n_out, const BatchText *bt)
 {
     const uint32_t N = (uint32_t)ph.dict_bytes;
     PosInfo pi{ph.dphr, ph.doff, ph.dlen};
@@ -525,32 +530,34 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     device_scan<uint32_t, OpAdd>(st, N, LoadGCount{stat}, StoreGroup{stat, N, heads, mixed}, false,
                                  (uint32_t *)st->d_scalars);
     // a mixed block has at least two bytes
-    uint32_t *delta = slot<uint32_t>(st, S_DELTA, (size_t)(N < n / 2 ? N : n / 2) + 1);
+    uint32_t *delta = slot<uint32_t>(st, S_DELTA, (size_t)(N < n_out / 2 ? N : n_out / 2) + 1);
     device_scan<Sum4, OpAdd>(st, nw, LoadMixWord{stat, heads, mixed}, StoreMixWord{stat, mixed, delta}, false,
                              (Sum4 *)(st->d_scalars + 1));
     fetch_scalars(st, 3);
     const uint32_t total = (uint32_t)st->h_scalars[0], M = (uint32_t)st->h_scalars[1];
     const uint32_t B = (uint32_t)(st->h_scalars[1] >> 32), G = (uint32_t)st->h_scalars[2];
-    if (total != n || G == 0) throw Error{GBWT_INTERNAL_ERROR};
+    if (total != n_out || G == 0) throw Error{GBWT_INTERNAL_ERROR};
     st->stats.s = G;
     st->stats.mixed_blocks = B;
     st->stats.mixed_elems = M;
     stage_mark(st, 4);
 
-    uint32_t *marks = slot<uint32_t>(st, S_TMP2, ((size_t)ph.z + 31) / 32);
-    k_primary_marks<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(
-        PrimaryArgs{ph.pid, ph.doff, ph.dlen, dord.isa, stat, ph.z, marks, st->d_flags + 2});
-    after_launch(st);
-    k_primary_count<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(pord.sa, pord.first, ph.z, marks, st->d_flags + 2);
-    after_launch(st);
-    const uint32_t long_cap = n / RF_LONG + 1u;
+    if (!bt) {
+        uint32_t *marks = slot<uint32_t>(st, S_TMP2, ((size_t)ph.z + 31) / 32);
+        k_primary_marks<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(
+            PrimaryArgs{ph.pid, ph.doff, ph.dlen, dord.isa, stat, ph.z, marks, st->d_flags + 2});
+        after_launch(st);
+        k_primary_count<<<grid_for(ph.z, 256), 256, 0, st->stream>>>(pord.sa, pord.first, ph.z, marks, st->d_flags + 2);
+        after_launch(st);
+    }
+    const uint32_t long_cap = n_out / RF_LONG + 1u;
     uint32_t *longs = slot<uint32_t>(st, S_TILEG, long_cap);
     check_cuda(cudaMemsetAsync(st->d_flags + 5, 0, 4, st->stream));
     probe_begin(st, GBWT_PROBE_RUN_FILL);
-    k_run_fill_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(dOut, n, stat, N, longs, long_cap, st->d_flags);
-    probe_end(st, GBWT_PROBE_RUN_FILL, (uint64_t)(n - M) + 8ull * N);
+    k_run_fill_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(dOut, n_out, stat, N, longs, long_cap, st->d_flags);
+    probe_end(st, GBWT_PROBE_RUN_FILL, (uint64_t)(n_out - M) + 8ull * N);
     after_launch(st);
-    k_run_fill_long<<<st->num_sms * 4, 256, 0, st->stream>>>(dOut, n, stat, N, longs, st->d_flags + 5, long_cap);
+    k_run_fill_long<<<st->num_sms * 4, 256, 0, st->stream>>>(dOut, n_out, stat, N, longs, st->d_flags + 5, long_cap);
     after_launch(st);
     stage_mark(st, 5);
     if (B == 0) return;
@@ -568,8 +575,8 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     k_mix_entries<<<grid_for(N, 256), 256, 0, st->stream>>>(N, ph.dphr, ph.doff, ph.dict, dord.isa, stat, words, pre,
                                                             mb, mc);
     after_launch(st);
-    if (B < (1u << 24)) mixed_blocks<uint32_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut);
-    else mixed_blocks<uint64_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut);
+    if (B < (1u << 24)) mixed_blocks<uint32_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut, n_out, bt);
+    else mixed_blocks<uint64_t>(st, dT, n, W, ph, pord, moff, mb, mc, delta, B, M, dOut, n_out, bt);
 }
 
 }  // namespace gbwt

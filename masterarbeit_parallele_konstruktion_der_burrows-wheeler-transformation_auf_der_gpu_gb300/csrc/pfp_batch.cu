@@ -9,6 +9,18 @@
 //          input bytes are checked while copying (K:130-132).
 //   scan   per-text trigger windows and forced final triggers, read from X
 //          alone (pfp_scan.cu); phrase i belongs to text ptid[i].
+//   dedup  the dictionary keeps the texts apart: equal phrases of different
+//          texts are distinct, and the suffix order has the text above the
+//          symbols, so everything after it is text by text -- one parse, whose
+//          suffixes never tie across texts (a text's last phrase, with its
+//          sentinels, occurs once), and the single text's assembly, whose
+//          blocks follow each other in the order of the output.
+//
+// Texts that share much of their content (versions of one document, one per
+// text) would repeat it in such a dictionary.  When keeping the texts apart
+// adds more than a quarter to the dictionary's bytes, the batch takes the other
+// path:
+//
 //   dedup  one dictionary for all texts.  Within one text phrases are
 //          prefix-free exactly as in its own run, so the dictionary order
 //          restricted to one text's suffixes is that run's order.
@@ -20,6 +32,11 @@
 //          phrase first, K:787-807); a stable radix sort by (text, group)
 //          leaves the elements of text t at its own output offsets, in its
 //          own BWT order.  The byte payload rides in the low 8 key bits.
+//
+// Sorting an element per text position was a third of a batch: 4096 texts with
+// bases of their own (512 MiB) take 26.9 ms on the second path and 18.0 ms on the
+// first.  The choice costs one pass over the phrases (k_pairs, 0.75 ms there, less
+// where it ends early: 64 texts that are copies of one, 256 MiB, 16.2 ms in all).
 #include "prims.cuh"
 
 namespace gbwt {
@@ -343,7 +360,8 @@ __global__ void k_bextract(const E *elem, const uint2 *tseg, const uint2 *tout, 
 // text per segment when the tile padding costs at most pad_eighths / 8 of
 // the elements (the key then needs no text bits); otherwise texts are
 // grouped until a segment holds seg_tiles tiles (tuning knobs).
-static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, int W)
+// Without `segments` only the texts (xstart, ioff) are laid out.
+static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, int W, bool segments)
 {
     BatchLayout bl;
     bl.total = (uint64_t)offsets[k];
@@ -368,6 +386,7 @@ static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, 
         }
     }
     tiles += (seg_real + RS_TILE - 1) / RS_TILE;
+    if (!segments) tiles = 0;
     if (tiles > 0xFFFFFFFFull / RS_TILE) throw Error{GBWT_UNSUPPORTED_INPUT};
     bl.k = kk;
     bl.tiles = (uint32_t)tiles;
@@ -418,13 +437,13 @@ static BatchLayout batch_layout(Storage *st, const int64_t *offsets, int32_t k, 
         if (!len) continue;
         xs[i] = (uint32_t)x;
         io[i] = (uint32_t)offsets[t];
-        tl[i] = i - seg_first_text;
+        if (segments) tl[i] = i - seg_first_text;
         x += len + (uint64_t)W;
         seg_real += len;
         i++;
-        if (seg_real >= seg_min) close_segment(i);
+        if (segments && seg_real >= seg_min) close_segment(i);
     }
-    if (seg_real) close_segment(i);
+    if (segments && seg_real) close_segment(i);
     xs[kk] = (uint32_t)x;
     bl.N = x;
     return bl;
@@ -478,6 +497,31 @@ static void batch_output(Storage *st, const BatchLayout &bl, const uint32_t *dme
     after_launch(st);
 }
 
+// Output to the host, error bits and stage times.
+static int64_t batch_end(Storage *st, uint8_t *L, const uint8_t *dOut, uint64_t total, bool devptr)
+{
+    stage_mark(st, 6);
+    if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)total, cudaMemcpyDeviceToHost, st->stream));
+    check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                               st->stream));
+    sync_stream(st);
+    uint32_t hflags[4];
+    memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
+    if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
+    if (hflags[0] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
+    if (st->stage_times) {
+        for (int i = 0; i < 7; i++) {
+            float ms = 0.f;
+            if (cudaEventElapsedTime(&ms, st->ev[i], st->ev[i + 1]) != cudaSuccess) ms = 0.f;
+            st->stats.stage_ms[i] = ms;
+        }
+        float tot = 0.f;
+        if (cudaEventElapsedTime(&tot, st->ev[0], st->ev[7]) == cudaSuccess) st->stats.stage_ms[7] = tot;
+    }
+    st->stats.kernel_launches = st->launches;
+    return (int64_t)total;
+}
+
 int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t k, uint8_t *L, int W, int P,
                   uint32_t flags, int64_t max_n, const BatchAux *aux)
 {
@@ -496,7 +540,7 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     if (!T || !L) return GBWT_BAD_PARAMETER;
     // 32-bit positions inside, with room for the sentinel runs
     if ((uint64_t)total_i + (uint64_t)W * (uint64_t)k > (uint64_t)max_n) return GBWT_UNSUPPORTED_INPUT;
-    const BatchLayout bl = batch_layout(st, offsets, k, W);
+    BatchLayout bl = batch_layout(st, offsets, k, W, false);
     const uint32_t kk = bl.k;
     const uint64_t total = bl.total, N = bl.N;
 
@@ -543,11 +587,32 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     Phrases ph;
     ph.z = z;
     ph.D = D;
-    run_phrases(st, X, un, W, ph, &bt);
+    // row samples need an element per text position: the second path
+    run_phrases(st, X, un, W, ph, &bt, !aux && kk > 1);
+    const bool apart = !aux && (kk == 1 || ph.dtid);
     st->stats.d = ph.d;
     st->stats.dict_bytes = (int64_t)ph.dict_bytes;
     stage_mark(st, 1);
 
+    if (apart) {
+        DictOrder dord;
+        run_dict_sort(st, ph, W, small, dord);
+        st->stats.dict_rounds = dord.rounds;
+        stage_mark(st, 2);
+        ParseOrder pord;
+        run_parse_sa(st, ph, dord, pord);
+        st->stats.parse_rounds = pord.rounds;
+        stage_mark(st, 3);
+        run_assembly(st, X, un, W, ph, dord, pord, dOut, (uint32_t)total, &bt);
+        return batch_end(st, L, dOut, total, devptr);
+    }
+
+    // segments of the output sort, laid out beside the texts
+    bl = batch_layout(st, offsets, k, W, true);
+    meta = slot<uint32_t>(st, S_BMETA, bl.words);
+    check_cuda(cudaMemcpyAsync(meta, st->h_meta, bl.words * 4, cudaMemcpyHostToDevice, st->stream));
+    xstart = meta + bl.o_xstart;
+    bt.xstart = xstart;
     DictOrder dord;
     run_dict_sort(st, ph, W, small, dord);
     st->stats.dict_rounds = dord.rounds;
@@ -611,26 +676,8 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     else
         batch_output<uint64_t>(st, bl, meta, S, ecnt, emq, emt, emp, grp_of, ph.dict, codes, gb, bb, tlb, dOut, emx,
                                aux);
-    stage_mark(st, 6);
-    if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)total, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                               st->stream));
-    sync_stream(st);
-    uint32_t hflags[4];
-    memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
-    if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
-    if (hflags[0] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
-    if (st->stage_times) {
-        for (int i = 0; i < 7; i++) {
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, st->ev[i], st->ev[i + 1]) != cudaSuccess) ms = 0.f;
-            st->stats.stage_ms[i] = ms;
-        }
-        float tot = 0.f;
-        if (cudaEventElapsedTime(&tot, st->ev[0], st->ev[7]) == cudaSuccess) st->stats.stage_ms[7] = tot;
-    }
-    st->stats.kernel_launches = st->launches;
-    return total_i;
+    return batch_end(st, L, dOut, total, devptr);
 }
+
 
 }  // namespace gbwt

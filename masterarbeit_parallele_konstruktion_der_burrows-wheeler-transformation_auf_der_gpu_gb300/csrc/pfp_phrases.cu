@@ -21,6 +21,7 @@ namespace gbwt {
 constexpr int PH_THREADS = 256;
 constexpr int PH_SPAN = 24576;
 constexpr uint64_t M61 = (1ull << 61) - 1ull;
+constexpr uint32_t PH_PROBES = 2048;      // a longer run means a table too full to go on
 
 // Phrase k spans [start, end]: end = D[k]; start = D[k-1]-W+1 (consecutive
 // phrases overlap by W, K:578-592).  In a batch of texts (xsep = the padded
@@ -43,6 +44,30 @@ __device__ __forceinline__ uint64_t mulmod61(uint64_t a, uint64_t b)
     return r >= M61 ? r - M61 : r;
 }
 
+// What keeping a batch's texts apart would cost: bytes of the distinct phrases
+// and of the distinct (text, phrase) pairs, and whether the count of pairs was
+// given up.  The texts are kept apart when that adds at most a quarter to the
+// dictionary.
+struct Parting {
+    unsigned long long bytes, pair_bytes;
+    uint32_t full, pad;
+};
+__host__ __device__ __forceinline__ bool part_texts(const Parting &p)
+{
+    return !p.full && p.pair_bytes * 4ull <= p.bytes * 5ull;
+}
+// Sum of v over the CTA, to one thread (the others 0); all threads take part.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v)
+{
+    __shared__ uint32_t s_sum;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    const uint32_t w = __reduce_add_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31u) == 0 && w) atomicAdd(&s_sum, w);
+    __syncthreads();
+    return threadIdx.x == 0 ? s_sum : 0u;
+}
+
 struct HashArgs {
     const uint8_t *T;
     uint32_t n;
@@ -58,38 +83,14 @@ struct HashArgs {
     uint32_t *slot_of;
     uint32_t *flags;
     const uint8_t *xsep;    // batch: padded text buffer, else null
+    uint32_t *full;         // set with ERR_TABLE_FULL: away from the counters that every insert updates
+    unsigned long long *bytes;      // PART: sum of the distinct phrases' lengths
 };
 
-__global__ void __launch_bounds__(PH_THREADS) k_phrase_hash(HashArgs a)
+// Fingerprint of phrase k and its table slot.
+__device__ __forceinline__ void phrase_insert(const HashArgs &a, uint32_t k, const uint8_t *s_txt, uint32_t a_al,
+                                              bool staged, uint32_t &fresh)
 {
-    __shared__ __align__(16) uint8_t s_txt[PH_SPAN];
-    const uint32_t k0 = blockIdx.x * PH_THREADS;
-    const uint32_t klast = min(k0 + PH_THREADS - 1u, a.z - 1u);
-    const uint32_t sa = k0 ? a.D[k0 - 1] - (uint32_t)a.W + 1u : 0u;
-    const uint32_t sb = a.D[klast];
-    const uint32_t a_al = sa & ~15u;
-    // +32: the word reads of the last chunk may touch 12 bytes past the span
-    const bool staged = (size_t)(sb - a_al) + 32 <= PH_SPAN;
-    if (staged) {
-        const bool aligned = (((uintptr_t)a.T) & 15u) == 0;
-        const uint32_t nvec = (sb - a_al) / 16 + 1;
-        for (uint32_t v = threadIdx.x; v < nvec; v += PH_THREADS) {
-            uint32_t p = a_al + v * 16;
-            uint4 val;
-            if (aligned && (size_t)p + 16 <= a.n) {
-                val = __ldg((const uint4 *)(a.T + p));
-            } else {
-                uint8_t b[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++) b[j] = text_at(a.T, a.n, p + j);
-                memcpy(&val, b, 16);
-            }
-            *(uint4 *)(s_txt + v * 16) = val;
-        }
-    }
-    __syncthreads();
-    const uint32_t k = k0 + threadIdx.x;
-    if (k >= a.z) return;
     uint32_t start, end;
     phrase_span(a.D, k, a.W, a.xsep, start, end);
     const uint32_t len = end - start + 1u;
@@ -128,21 +129,110 @@ __global__ void __launch_bounds__(PH_THREADS) k_phrase_hash(HashArgs a)
         if (cur == 0ull) {
             // the inserting occurrence is the slot's representative
             a.tvals[pos] = k;
-            uint32_t c = atomicAdd(a.flags + 1, 1u);
-            if (c >= a.limit) atomicOr(a.flags, ERR_TABLE_FULL);
+            fresh = len;
             ok = true;
             break;
         }
         if (cur == key) { ok = true; break; }
         pos = (pos + 1u) & a.cmask;
-        if ((probe & 7u) == 7u && (*(volatile uint32_t *)a.flags & ERR_TABLE_FULL)) break;
+        if (probe >= PH_PROBES || ((probe & 7u) == 7u && *(volatile uint32_t *)a.full)) break;
     }
     if (!ok) {
         atomicOr(a.flags, ERR_TABLE_FULL);
+        *a.full = 1u;
         a.slot_of[k] = 0;
         return;
     }
     a.slot_of[k] = pos;
+}
+
+// PART: a batch that may be kept apart by text; its distinct bytes are summed.
+template <bool PART>
+__global__ void __launch_bounds__(PH_THREADS) k_phrase_hash(HashArgs a)
+{
+    __shared__ __align__(16) uint8_t s_txt[PH_SPAN];
+    __shared__ bool s_full;         // the table is full: the stage is run again with a larger one
+    uint32_t flag0 = 0;             // loaded beside the text, kept for the barrier
+    if (threadIdx.x == 0) flag0 = *(volatile uint32_t *)a.full;
+    const uint32_t k0 = blockIdx.x * PH_THREADS;
+    const uint32_t klast = min(k0 + PH_THREADS - 1u, a.z - 1u);
+    const uint32_t sa = k0 ? a.D[k0 - 1] - (uint32_t)a.W + 1u : 0u;
+    const uint32_t sb = a.D[klast];
+    const uint32_t a_al = sa & ~15u;
+    // +32: the word reads of the last chunk may touch 12 bytes past the span
+    const bool staged = (size_t)(sb - a_al) + 32 <= PH_SPAN;
+    if (staged) {
+        const bool aligned = (((uintptr_t)a.T) & 15u) == 0;
+        const uint32_t nvec = (sb - a_al) / 16 + 1;
+        for (uint32_t v = threadIdx.x; v < nvec; v += PH_THREADS) {
+            uint32_t p = a_al + v * 16;
+            uint4 val;
+            if (aligned && (size_t)p + 16 <= a.n) {
+                val = __ldg((const uint4 *)(a.T + p));
+            } else {
+                uint8_t b[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) b[j] = text_at(a.T, a.n, p + j);
+                memcpy(&val, b, 16);
+            }
+            *(uint4 *)(s_txt + v * 16) = val;
+        }
+    }
+    if (threadIdx.x == 0) s_full = flag0 != 0;
+    __syncthreads();
+    const uint32_t k = k0 + threadIdx.x;
+    uint32_t fresh = 0;             // length of a phrase first seen here
+    if (k < a.z && !s_full) phrase_insert(a, k, s_txt, a_al, staged, fresh);
+    // the inserts of a CTA are counted together: one atomic on the counter
+    const uint32_t count = (uint32_t)__syncthreads_count(fresh != 0u);
+    if (threadIdx.x == 0 && count && atomicAdd(a.flags + 1, count) + count > a.limit) {
+        atomicOr(a.flags, ERR_TABLE_FULL);
+        *a.full = 1u;
+    }
+    if constexpr (PART) {
+        const uint32_t sum = block_sum(fresh);
+        if (sum) atomicAdd(a.bytes, (unsigned long long)sum);
+    }
+}
+// The distinct (text, content slot) pairs, exact keys: a pair's slot per phrase.
+// A kernel of its own: inside the fingerprint kernel, which lives on shared
+// memory, the second chain of random reads took 3.0 ms of a 4096-text batch,
+// here 0.75 ms.  Sums go through one atomic per CTA (one per insert: 1.6 ms more).
+constexpr uint32_t PAIR_PROBES = 128;      // a longer run means a table too full to go on
+__global__ void k_pairs(const uint32_t *D, uint32_t z, int W, const uint8_t *xsep, const uint32_t *ptid,
+                        const uint32_t *slot_of, const uint32_t *flags,
+                        unsigned long long *pkeys, uint32_t *pvals, uint32_t pmask, uint32_t *pslot, Parting *part)
+{
+    __shared__ bool s_stop;
+    if (threadIdx.x == 0) s_stop = (*flags & ERR_TABLE_FULL) || *(volatile uint32_t *)&part->full;
+    __syncthreads();
+    if (s_stop) return;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t fresh = 0;
+    if (k < z) {
+        const unsigned long long pair = ((unsigned long long)(ptid[k] + 1u) << 32) | slot_of[k];
+        uint32_t q = (uint32_t)((pair * 0x9E3779B97F4A7C15ull) >> 32) & pmask;
+        for (uint32_t probe = 0;; probe++, q = (q + 1u) & pmask) {
+            unsigned long long cur = __ldcg(pkeys + q);
+            if (cur == 0ull) cur = atomicCAS(pkeys + q, 0ull, pair);
+            if (cur == 0ull) {
+                pvals[q] = k;
+                uint32_t s, e;
+                phrase_span(D, k, W, xsep, s, e);
+                fresh = e - s + 1u;
+                break;
+            }
+            if (cur == pair) break;
+            if (probe >= PAIR_PROBES) {
+                part->full = 1u;
+                break;
+            }
+        }
+        pslot[k] = q;
+    }
+    const uint32_t sum = block_sum(fresh);
+    // past the line the answer is known, and the CTAs to come need not look
+    if (sum && (atomicAdd(&part->pair_bytes, (unsigned long long)sum) + sum) * 4ull > part->bytes * 5ull) part->full = 1u;
 }
 
 // 8 text bytes starting at T + p (any alignment): two aligned 8-byte loads
@@ -157,16 +247,28 @@ __device__ __forceinline__ uint64_t load8_any(const uint8_t *T, uint32_t p)
 }
 
 // Compares each occurrence with its representative; marks representatives.
+// Where a batch's texts are kept apart, the pairs take the contents' place:
+// their representatives and slots.
 // Inside the text 8 bytes at a time; the tail and the sentinel run after
 // the text byte by byte.
 __global__ void k_phrase_verify(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, int W,
-                                const uint32_t *tvals, const uint32_t *slot_of, uint32_t *isrep, uint32_t *flags,
-                                const uint8_t *xsep)
+                                const uint32_t *tvals, uint32_t *slot_of, uint32_t *isrep, uint32_t *flags,
+                                const uint8_t *xsep, const uint32_t *pvals, const uint32_t *pslot, const Parting *part)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= z) return;
+    if (*(volatile uint32_t *)flags & ERR_TABLE_FULL) {          // the stage is run again; slots may be missing
+        isrep[k] = 0;
+        return;
+    }
     const uint32_t rep = tvals[slot_of[k]];
-    isrep[k] = rep == k;
+    if (part && part_texts(*part)) {
+        const uint32_t q = pslot[k];
+        isrep[k] = pvals[q] == k;
+        slot_of[k] = q;
+    } else {
+        isrep[k] = rep == k;
+    }
     if (rep == k) return;
     if (rep >= z) { atomicOr(flags, ERR_COLLISION); return; }
     uint32_t s1, e1, s2, e2;
@@ -202,9 +304,12 @@ struct StoreDense {
     uint32_t *dstart;
     int W;
     const uint8_t *xsep;
+    const uint32_t *ptid;
+    uint32_t *dtid;
     __device__ __forceinline__ void operator()(size_t k, uint32_t pre, uint32_t v) const
     {
         if (!v) return;
+        if (dtid) dtid[pre] = ptid[k];
         uint32_t s, e;
         phrase_span(D, (uint32_t)k, W, xsep, s, e);
         tdense[slot_of[k]] = pre;
@@ -268,8 +373,12 @@ static uint32_t pow2_at_least(uint64_t v)
     return (uint32_t)c;
 }
 
-void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, const BatchText *bt)
+void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph, const BatchText *bt, bool may_part)
 {
+    const uint32_t *ptid = may_part ? bt->ptid : nullptr;
+    uint32_t *dtid = may_part ? slot<uint32_t>(st, S_DTID, ph.z) : nullptr;
+    Parting *part = (Parting *)(st->d_scalars + 8);
+    static_assert(sizeof(Parting) == 24, "three words of the device scalars");
     const uint8_t *xsep = bt ? dT : nullptr;
     const uint32_t z = ph.z;
     uint32_t *slot_of = slot<uint32_t>(st, S_SLOT, z);
@@ -285,13 +394,24 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         if (attempt > 6) throw Error{GBWT_INTERNAL_ERROR};
         unsigned long long *tkeys = slot<unsigned long long>(st, S_TKEYS, c);
         uint32_t *tvals = slot<uint32_t>(st, S_TVALS, c);
-        tdense = slot<uint32_t>(st, S_TDENSE, c);
+        // pairs: twice the slots, so that a dictionary that just fits parts too
+        const uint32_t c2 = may_part ? (full_c / 2 > c ? c * 2 : c) : 0u;
+        unsigned long long *pkeys = may_part ? slot<unsigned long long>(st, S_PKEYS, c2) : nullptr;
+        uint32_t *pvals = may_part ? slot<uint32_t>(st, S_PVALS, c2) : nullptr;
+        uint32_t *pslot = may_part ? slot<uint32_t>(st, S_PSLOT, z) : nullptr;
+        if (may_part) {
+            check_cuda(cudaMemsetAsync(pkeys, 0, (size_t)c2 * 8, st->stream));
+            check_cuda(cudaMemsetAsync(part, 0, sizeof(Parting), st->stream));
+        }
+        tdense = slot<uint32_t>(st, S_TDENSE, c2 > c ? c2 : c);
         dlen = slot<uint32_t>(st, S_DLEN, (size_t)z + 1);
         dstart = slot<uint32_t>(st, S_DSTART, (size_t)z + 1);
         check_cuda(cudaMemsetAsync(tkeys, 0, (size_t)c * 8, st->stream));
         check_cuda(cudaMemsetAsync(st->d_flags, 0, 8, st->stream));
+        check_cuda(cudaMemsetAsync(st->d_flags + 48, 0, 4, st->stream));
         check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
         HashArgs a;
+        a.full = st->d_flags + 48;
         a.T = dT; a.n = n; a.D = ph.D; a.z = z; a.W = W;
         a.base = (seed % (M61 - 1000)) + 257;
         a.tkeys = tkeys; a.tvals = tvals; a.cmask = c - 1;
@@ -300,17 +420,26 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         a.logc = logc;
         a.limit = (uint32_t)(((uint64_t)c * 3) / 4);
         a.slot_of = slot_of; a.flags = st->d_flags; a.xsep = xsep;
+        a.bytes = may_part ? &part->bytes : nullptr;
         probe_begin(st, GBWT_PROBE_PHRASE_HASH);
-        k_phrase_hash<<<grid_for(z, PH_THREADS), PH_THREADS, 0, st->stream>>>(a);
+        if (may_part) k_phrase_hash<true><<<grid_for(z, PH_THREADS), PH_THREADS, 0, st->stream>>>(a);
+        else k_phrase_hash<false><<<grid_for(z, PH_THREADS), PH_THREADS, 0, st->stream>>>(a);
         // text bytes of all phrases (n + (W-1)(z-1) overlap) + D read + slot write
         probe_end(st, GBWT_PROBE_PHRASE_HASH, (uint64_t)n + (uint64_t)(W - 1) * (z - 1) + 8ull * z);
         after_launch(st);
+        if (may_part) {
+            k_pairs<<<grid_for(z, 256), 256, 0, st->stream>>>(ph.D, z, W, xsep, bt->ptid, slot_of, st->d_flags, pkeys,
+                                                              pvals, c2 - 1u, pslot, part);
+            after_launch(st);
+        }
         k_phrase_verify<<<grid_for(z, 256), 256, 0, st->stream>>>(dT, n, ph.D, z, W, tvals, slot_of, isrep,
-                                                                  st->d_flags, xsep);
+                                                                  st->d_flags, xsep, pvals, pslot, may_part ? part : nullptr);
         after_launch(st);
-        device_scan<uint32_t, OpAdd>(st, z, LoadU32{isrep}, StoreDense{ph.D, slot_of, tdense, dlen, dstart, W, xsep},
+        device_scan<uint32_t, OpAdd>(st, z, LoadU32{isrep}, StoreDense{ph.D, slot_of, tdense, dlen, dstart, W, xsep, ptid, dtid},
                                      false, (uint32_t *)st->d_scalars);
         check_cuda(cudaMemcpyAsync(st->h_scalars + 1, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
+        if (may_part)
+            check_cuda(cudaMemcpyAsync(st->h_scalars + 4, part, sizeof(Parting), cudaMemcpyDeviceToHost, st->stream));
         fetch_scalars(st, 1);
         uint32_t flags = (uint32_t)(st->h_scalars[1] & 0xFFFFFFFFu);
         d = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
@@ -323,6 +452,11 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         break;
     }
     ph.d = d;
+    Parting hp{};
+    if (may_part) memcpy(&hp, st->h_scalars + 4, sizeof(hp));
+    const bool parted = may_part && part_texts(hp);
+    ph.dtid = parted ? dtid : nullptr;
+    ph.texts = parted ? bt->k : 1u;
     uint32_t *pid = isrep;   // isrep is dead after the scan
     uint32_t *occ = slot<uint32_t>(st, S_OCC, d);
     uint32_t *pcmin = slot<uint32_t>(st, S_PCMIN, d);

@@ -996,9 +996,10 @@ __global__ void k_alpha_present(const uint8_t *dict, uint32_t N, uint32_t *bits)
 // every group uniform in whether its strings end within h0 symbols: without
 // it a suffix of exactly h0 symbols would tie with longer suffixes sharing
 // those symbols.  The recoding is monotone, so the order is the byte order.
-// Also writes rem8[x] = min(rem(x), 255) (see DictRem).
+// A batch kept apart by text has the phrase's text above the symbols: the
+// order is text by text.  Also writes rem8[x] = min(rem(x), 255) (see DictRem).
 __global__ void k_dict_keys(const uint8_t *dict, uint32_t N, DictRem rem, const uint8_t *code, int bps, int h0,
-                            uint64_t *keys, uint8_t *rem8)
+                            const uint32_t *dtid, uint64_t *keys, uint8_t *rem8)
 {
     __shared__ uint8_t s_code[256];
     s_code[threadIdx.x] = code[threadIdx.x];     // blockDim == 256
@@ -1006,7 +1007,7 @@ __global__ void k_dict_keys(const uint8_t *dict, uint32_t N, DictRem rem, const 
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= N) return;
     const uint32_t r = rem(x);
-    uint64_t key = 0;
+    uint64_t key = dtid ? dtid[rem.dphr[x]] : 0u;
     for (int i = 0; i < h0; i++) key = (key << bps) | (uint64_t)((uint32_t)i < r ? s_code[dict[x + i]] : 0u);
     key = (key << 1) | (r > (uint32_t)h0 ? 1u : 0u);
     keys[x] = key;
@@ -1091,16 +1092,18 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     // as many symbols as fit the first key's bit budget (radix passes over
     // the dictionary vs later doubling rounds: a tuning knob)
     const int key_bits = tune_dict_key_bits(st);
-    const int h0 = (key_bits - 1) / bps > 0 ? (key_bits - 1) / bps : 1;
+    const int tb = ph.dtid ? bits_for(ph.texts - 1u) : 0;      // at most 31; a symbol takes at most 8 bits
+    int h0 = (key_bits - 1) / bps > 0 ? (key_bits - 1) / bps : 1;
+    if (h0 * bps + tb + 1 > 64) h0 = (63 - tb) / bps;
     uint8_t *dcode = slot<uint8_t>(st, S_TMP1, 256);
     check_cuda(cudaMemcpyAsync(dcode, hcode, 256, cudaMemcpyHostToDevice, st->stream));
     uint64_t *keys = slot<uint64_t>(st, S_KEY0, N);
     uint8_t *rem8 = slot<uint8_t>(st, S_TMP0, N);
-    k_dict_keys<<<grid_for(N, 256), 256, 0, st->stream>>>(ph.dict, N, rem, dcode, bps, h0, keys, rem8);
+    k_dict_keys<<<grid_for(N, 256), 256, 0, st->stream>>>(ph.dict, N, rem, dcode, bps, h0, ph.dtid, keys, rem8);
     after_launch(st);
     dord.isa = slot<uint32_t>(st, S_ISA, N);
     dord.sa = slot<uint32_t>(st, S_SA, N);
-    dord.rounds = sort_phrase_suffixes(st, N, h0 * bps + 1, (uint32_t)h0, ph.dphr, ph.doff, ph.dlen, rem8, dord.isa,
+    dord.rounds = sort_phrase_suffixes(st, N, tb + h0 * bps + 1, (uint32_t)h0, ph.dphr, ph.doff, ph.dlen, rem8, dord.isa,
                                        dord.sa);
     dord.lexrank = slot<uint32_t>(st, S_LEXRANK, ph.d);
     phrase_ranks(st, N, ph.d, dord.isa, ph.doff, dord.lexrank);
