@@ -351,18 +351,21 @@ struct StoreOff32 {
     __device__ __forceinline__ void operator()(size_t i, uint64_t pre, uint64_t) const { a[i] = (uint32_t)pre; }
 };
 
-// One warp per distinct phrase: copy its bytes and tag positions with the id.
+// LANES lanes per distinct phrase: copy its bytes and tag positions with the id.
+// A warp per phrase leaves most lanes idle on phrases of twenty bytes: eight
+// lanes take 102 MB of versions (18 bytes on average) from 447 to 193 us and the
+// 512 MiB DNA text (30) from 130 to 75 us.  Phrases of 64 bytes and more on average
+// fill two rows of a warp and keep it (W=35: 160 bytes, 130 MB in 270 us).
+template <int LANES>
 __global__ void k_dict_copy(const uint8_t *T, uint32_t n, uint32_t d, const uint32_t *doff, const uint32_t *dlen,
                             const uint32_t *dstart, uint8_t *dict, uint32_t *dphr)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; id < d; id += nw) {
-        const uint32_t off = doff[id], len = dlen[id], st = dstart[id];
-        for (uint32_t j = lane; j < len; j += 32) {
-            dict[off + j] = text_at(T, n, st + j);
-            dphr[off + j] = id;
-        }
+    const uint32_t id = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    if (id >= d) return;
+    const uint32_t off = doff[id], len = dlen[id], st = dstart[id];
+    for (uint32_t j = threadIdx.x % LANES; j < len; j += LANES) {
+        dict[off + j] = text_at(T, n, st + j);
+        dphr[off + j] = id;
     }
 }
 
@@ -482,9 +485,10 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
     after_launch(st);
     uint8_t *dict = slot<uint8_t>(st, S_DICT, dict_bytes + 16);
     uint32_t *dphr = slot<uint32_t>(st, S_DPHR, dict_bytes + 1);
-    unsigned blocks = grid_for((size_t)d * 32, 256);
-    if (blocks > 8192) blocks = 8192;
-    k_dict_copy<<<blocks, 256, 0, st->stream>>>(dT, n, d, doff, dlen, dstart, dict, dphr);
+    if (dict_bytes >= (uint64_t)d * 64u)
+        k_dict_copy<32><<<grid_for((size_t)d * 32, 256), 256, 0, st->stream>>>(dT, n, d, doff, dlen, dstart, dict, dphr);
+    else
+        k_dict_copy<8><<<grid_for((size_t)d * 8, 256), 256, 0, st->stream>>>(dT, n, d, doff, dlen, dstart, dict, dphr);
     after_launch(st);
     ph.pid = pid; ph.dlen = dlen; ph.doff = doff; ph.occ = occ; ph.pcmin = pcmin; ph.pcmax = pcmax;
     ph.dict = dict; ph.dphr = dphr; ph.dict_bytes = dict_bytes;
