@@ -280,13 +280,8 @@ static int64_t unbwt_common(Storage *st, const uint8_t *L, uint8_t *T, int64_t n
         dT = slot<uint8_t>(st, S_OUT, (size_t)n + 16);
     }
     check_cuda(cudaMemsetAsync(st->d_flags, 0, 64 * sizeof(uint32_t), st->stream));
-    const uint8_t *dLc = dL;
-    if (pfp) {
-        uint8_t *lc = slot<uint8_t>(st, S_LCB, (size_t)n + 16);
-        pfp_to_libcubwt(st, dL, un, (uint32_t)primary, lc);
-        dLc = lc;
-    }
-    run_unbwt(st, dLc, un, pfp ? (uint32_t)primary + 1u : (uint32_t)primary, dT);
+    if (pfp) run_unbwt(st, dL, un, 0u, (uint32_t)primary, dT);
+    else run_unbwt(st, dL, un, (uint32_t)primary, 0xFFFFFFFFu, dT);
     if (!devptr) check_cuda(cudaMemcpyAsync(T, dT, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
     check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);

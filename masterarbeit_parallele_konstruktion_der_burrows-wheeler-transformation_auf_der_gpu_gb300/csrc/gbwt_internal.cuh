@@ -157,7 +157,7 @@ inline unsigned grid_for(size_t n, unsigned per_block)
 inline int tune_hash_log2(const Storage *st) { return st->tuning.hash_log2_max ? st->tuning.hash_log2_max : 22; }
 inline int tune_seg_tiles(const Storage *st) { return st->tuning.batch_seg_tiles ? st->tuning.batch_seg_tiles : 8; }
 inline int tune_pad_eighths(const Storage *st) { return st->tuning.batch_pad_eighths ? st->tuning.batch_pad_eighths : 1; }
-inline int tune_unbwt_rate_log2(const Storage *st) { return st->tuning.unbwt_rate_log2 ? st->tuning.unbwt_rate_log2 : 7; }
+inline int tune_unbwt_rate_log2(const Storage *st) { return st->tuning.unbwt_rate_log2 ? st->tuning.unbwt_rate_log2 : 5; }
 inline int tune_dict_key_bits(const Storage *st) { return st->tuning.dict_key_bits ? st->tuning.dict_key_bits : 64; }
 // 0 (default): single-text parses are parsed again when large and repetitive,
 // else round 0 comes from the phrase buckets, no sort (the batch parse then
@@ -266,8 +266,9 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
 
 void stage_mark(Storage *st, int idx);
 
-void pfp_to_libcubwt(Storage *st, const uint8_t *dO, uint32_t n, uint32_t p, uint8_t *dLc);
-void run_unbwt(Storage *st, const uint8_t *dLc, uint32_t n, uint32_t i, uint8_t *dT);
+// Inverse of the PFP output with primary row p, or (p = 0xFFFFFFFF) of libcubwt's
+// L with primary index i.
+void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t p, uint8_t *dT);
 
 // Sampled suffix array of a one-text batch: aux[p >> r_log2] = row + 1 of
 // the suffix starting at p, for every p that is a multiple of 2^r_log2.

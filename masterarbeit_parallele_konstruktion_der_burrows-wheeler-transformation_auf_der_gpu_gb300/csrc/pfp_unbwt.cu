@@ -3,67 +3,108 @@
 // The reference declares libcubwt_unbwt but does not define it
 // (libcubwt.cuh:101; its LF kernels are at libcubwt.cu:2453-2925).  Here:
 //
-//   B      the full BWT of T$ (n+1 rows, '$' at row i = libcubwt's primary
-//          index); the n non-'$' rows are libcubwt's L.
+//   rows   0..n of the BWT of T$; row 0 is the suffix "$".  Element e of the
+//          input belongs to a row (UbIn): libcubwt's L lists the rows without
+//          the '$' row; the PFP output O lists rows 1..n, with row 0's symbol
+//          standing in the '$' row.  Both are read as they are.
 //   LF     LF(r) = 1 + (position of row r in the stable sort of the non-'$'
 //          rows by symbol), LF($ row) = 0.  One counting pass: tile
 //          histograms, a digit-major scan, and a ranking pass (warp match
 //          multisplit, as in the radix downsweep) that writes LF in row
 //          order, so nothing is scattered.
-//   walk   T[n-1-k] = B[LF^k(0)].  Rows whose hash falls in 1/rate are
-//          rulers (row 0 always); an LF entry whose target is a ruler holds
-//          bit 31 | the ruler's index.  One thread per ruler follows LF to
-//          the next ruler and records the distance; pointer jumping over
-//          the ruler chain gives every ruler its distance from row 0; a
-//          second walk writes every text byte.  The symbol of a row comes
-//          from the bucket its LF value falls in, so a step reads one word.
-// Walks end at the next ruler; the rulers split the single LF cycle, so the
-// steps of all walks sum to n+1.  A BWT whose LF has more than one cycle is
-// rejected (the ruler chain from row 0 is not one list through all rulers,
-// or does not come back to row 0 after n+1 steps).
+//   walk   T[n-1-k] = B[LF^k(0)].  Blocks of 32 rows whose hash falls in 1/rate
+//          are rulers (block 0 always); an LF entry whose target is a ruler
+//          row holds bit 31 | the row's ruler number.  A lane follows LF from a
+//          ruler row to the next one and records the distance; list ranking
+//          over the chain of ruler rows gives each its distance from row 0; a
+//          second walk writes every text byte.  The symbol of a row comes from
+//          the bucket its LF value falls in, so a step reads one word.
+//
+// Neighbouring rows with the same symbol have neighbouring LF rows, and in a
+// repetitive text they stay together for as long as the copies agree.  A warp
+// walks from the 32 rows of one block, so its lanes read the same few sectors
+// and mostly arrive together; rulers chosen row by row gave a warp 32 stretches
+// of different lengths, and a sector per lane and step.
+//
+// The hash is a permutation of [0, 2^kb), 2^kb the power of two at or above the
+// number of blocks, so a block's number is its hash over the rate and its place
+// the inverse hash of that: no list of rulers, no search in it.  The chain is
+// ranked through one ruler in 16: sequential hops between those, pointer
+// jumping over them, and the hops again.
+//
+// 128 MiB of DNA copies, before / after on GB300, one row in 64 a ruler: LF 1.37 / 0.31
+// ms, first walk 2.22 / 1.25, list ranking 1.11 / 0.18, second walk 3.46 / 1.75, in
+// all 9.1 / 3.6 ms; one in 16, 32, 64, 128: 3.0, 3.0, 3.5, 4.3 ms (512 MiB: 12.2,
+// 10.6, 10.7, 12.5; 64 MiB of random DNA: 3.0, 3.3, 3.7, 4.9, before 4.7 at best).
+//
+// LF is a permutation, so a walk ends at the latest at its own ruler; the input
+// is a BWT exactly when the cycle of row 0 has all n + 1 rows.
 #include "prims.cuh"
 
 namespace gbwt {
 
 constexpr uint32_t UB_RULER = 0x80000000u;
 constexpr uint32_t UB_NIL = 0xFFFFFFFFu;
+constexpr int UB_SUPER_LOG2 = 4;          // one ruler in 16 carries the list ranking
+constexpr int UB_LUT_LOG2 = 12;
 
-__device__ __forceinline__ uint32_t ub_mix(uint32_t x)
+// Permutation of [0, 2^kb): xor-shifts by at least half the bits undo
+// themselves, odd factors have inverses modulo 2^32.
+constexpr uint32_t UB_MUL1 = 0x2C1B3C6Du, UB_MUL2 = 0x297A2D39u;
+constexpr uint32_t ub_inverse(uint32_t a)
 {
-    x ^= x >> 16;
-    x *= 0x85EBCA6Bu;
-    x ^= x >> 13;
-    x *= 0xC2B2AE35u;
-    x ^= x >> 16;
+    uint32_t x = a;                        // correct to 3 bits; each step doubles them
+    for (int i = 0; i < 5; i++) x *= 2u - a * x;
     return x;
 }
-__device__ __forceinline__ bool ub_is_ruler(uint32_t r, uint32_t rate_mask)
-{
-    return r == 0 || (ub_mix(r) & rate_mask) == 0;
-}
-
-// libcubwt's L from the PFP output O and its primary row p: O[p], O[0..p), O[p+1..n).
-__global__ void k_pfp_to_libcubwt(const uint8_t *O, uint32_t n, uint32_t p, uint8_t *Lc)
-{
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    Lc[e] = e == 0 ? O[p] : (e <= p ? O[e - 1] : O[e]);
-}
-
-// Index of ruler row t in the sorted ruler list.
-__device__ __forceinline__ uint32_t ub_ruler_index(const uint32_t *rul, uint32_t m, uint32_t t)
-{
-    uint32_t lo = 0, hi = m - 1u;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (rul[mid] < t) lo = mid + 1u; else hi = mid;
+constexpr uint32_t UB_INV1 = ub_inverse(UB_MUL1), UB_INV2 = ub_inverse(UB_MUL2);
+static_assert(UB_MUL1 * UB_INV1 == 1u && UB_MUL2 * UB_INV2 == 1u, "inverses modulo 2^32");
+struct UbHash {
+    uint32_t mask;       // 2^kb - 1
+    int half;            // ceil(kb / 2)
+    int rate_log2;
+    uint32_t rows;
+    __device__ __forceinline__ uint32_t mix(uint32_t x) const
+    {
+        x ^= x >> half;
+        x = (x * UB_MUL1) & mask;
+        x ^= x >> half;
+        x = (x * UB_MUL2) & mask;
+        return x ^ (x >> half);
     }
-    return lo;
-}
+    __device__ __forceinline__ uint32_t unmix(uint32_t x) const
+    {
+        x ^= x >> half;
+        x = (x * UB_INV2) & mask;
+        x ^= x >> half;
+        x = (x * UB_INV1) & mask;
+        return x ^ (x >> half);
+    }
+    // LF entry for target row t: t, or its ruler number with bit 31
+    __device__ __forceinline__ uint32_t entry(uint32_t t) const
+    {
+        const uint32_t h = mix(t >> 5);
+        return (h & ((1u << rate_log2) - 1u)) ? t : (UB_RULER | ((h >> rate_log2) << 5) | (t & 31u));
+    }
+    __device__ __forceinline__ uint32_t row_of(uint32_t ruler) const
+    {
+        return (unmix((ruler >> 5) << rate_log2) << 5) | (ruler & 31u);
+    }
+};
 
-// Symbol counts of every tile, digit-major over the tiles.
-__global__ void __launch_bounds__(RS_THREADS) k_byte_hist(const uint8_t *__restrict__ keys, uint32_t n,
-                                                          uint32_t *__restrict__ tile_hist, uint32_t num_tiles)
+// Where the input's elements belong.  PFP: element e is row e + 1, except
+// element p, whose symbol is row 0's (its place is the '$' row).  libcubwt:
+// element e is row e before the '$' row, e + 1 from there on.
+struct UbIn {
+    const uint8_t *L;
+    uint32_t n;
+    uint32_t dollar;     // '$' row
+    uint32_t p;          // PFP: element of row 0; libcubwt: none (UB_NIL)
+    __device__ __forceinline__ uint32_t row(uint32_t e) const { return p != UB_NIL ? e + 1u : (e < dollar ? e : e + 1u); }
+};
+
+// Symbol counts of every tile (element p left out), digit-major over the tiles.
+__global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__restrict__ tile_hist, uint32_t num_tiles)
 {
     constexpr int D = 256;
     __shared__ uint32_t h[RS_WARPS * D];       // one histogram per warp
@@ -71,25 +112,17 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(const uint8_t *__restr
     __syncthreads();
     uint32_t *wh = h + (threadIdx.x >> 5) * D;
     const size_t base = (size_t)blockIdx.x * RS_TILE;
-    constexpr int KPV = 16;                          // symbols per 16-byte load
-    constexpr int NV = RS_ITEMS / KPV;
-    if (base + RS_TILE <= n && (((uintptr_t)keys) & 15u) == 0) {
-        // full tile: every load issued before any count (counting needs no order)
-        uint4 v[NV];
+    if (base + RS_TILE <= in.n && (((uintptr_t)in.L) & 15u) == 0) {
+        const uint4 v = __ldg((const uint4 *)(in.L + base) + threadIdx.x);       // 16 symbols per thread
+        uint8_t kk[16];
+        memcpy(kk, &v, 16);
 #pragma unroll
-        for (int j = 0; j < NV; j++) v[j] = __ldg((const uint4 *)(keys + base) + (size_t)j * RS_THREADS + threadIdx.x);
-#pragma unroll
-        for (int j = 0; j < NV; j++) {
-            uint8_t kk[KPV];
-            memcpy(kk, &v[j], 16);
-#pragma unroll
-            for (int q = 0; q < KPV; q++) atomicAdd(&wh[kk[q]], 1u);
-        }
+        for (int q = 0; q < 16; q++) atomicAdd(&wh[kk[q]], 1u);
     } else {
 #pragma unroll 4
         for (int j = 0; j < RS_ITEMS; j++) {
-            size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
-            if (i < n) atomicAdd(&wh[keys[i]], 1u);
+            const size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
+            if (i < in.n) atomicAdd(&wh[in.L[i]], 1u);
         }
     }
     __syncthreads();
@@ -97,25 +130,24 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(const uint8_t *__restr
         uint32_t sum = 0;
 #pragma unroll
         for (int w = 0; w < RS_WARPS; w++) sum += h[w * D + d];
+        if (in.p != UB_NIL && in.p >= base && in.p < base + RS_TILE && in.L[in.p] == d) sum--;
         tile_hist[(size_t)d * num_tiles + blockIdx.x] = sum;
     }
 }
 
-// LF of every row.  Element e of Lc is row e (e < i) or e+1 (e >= i).  An
-// entry whose target row is a ruler holds UB_RULER | the ruler's index.
-template <int BITS>
-__global__ void __launch_bounds__(RS_THREADS) k_lf_rank(const uint8_t *__restrict__ Lc, uint32_t n, uint32_t i,
-                                                        const uint32_t *__restrict__ tile_off, uint32_t num_tiles,
-                                                        uint32_t rate_mask, const uint32_t *__restrict__ rul,
-                                                        uint32_t m, uint32_t *__restrict__ LF)
+// LF of every row (entries as UbHash::entry).  Row 0 precedes all rows of its
+// symbol c0 in the sort: with PFP input its element is left out of the counts
+// and every other position at or above c0's bucket moves up by one.
+__global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t *__restrict__ tile_off,
+                                                        uint32_t num_tiles, UbHash hash, uint32_t *__restrict__ LF)
 {
-    constexpr int D = 1 << BITS;
-    constexpr int DPT = D / RS_THREADS;
+    constexpr int D = 256;
     __shared__ uint32_t s_wh[RS_WARPS * D];
     __shared__ uint32_t s_goff[D];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int q = threadIdx.x; q < RS_WARPS * D; q += RS_THREADS) s_wh[q] = 0;
     __syncthreads();
+    const uint32_t c0 = in.p != UB_NIL ? in.L[in.p] : 256u;
     const size_t tile_base = (size_t)blockIdx.x * RS_TILE;
     const size_t wbase = tile_base + (size_t)warp * (RS_ITEMS * 32);
     uint32_t dg[RS_ITEMS], rk[RS_ITEMS];
@@ -123,7 +155,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(const uint8_t *__restric
 #pragma unroll
     for (int q = 0; q < RS_ITEMS; q++) {
         const size_t idx = wbase + (size_t)q * 32 + lane;
-        dg[q] = idx < n ? (uint32_t)Lc[idx] : 0xFFFFFFFFu;
+        dg[q] = idx < in.n && idx != in.p ? (uint32_t)in.L[idx] : 0xFFFFFFFFu;
     }
 #pragma unroll
     for (int q = 0; q < RS_ITEMS; q++) {
@@ -143,9 +175,8 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(const uint8_t *__restric
     }
     __syncthreads();
     // per digit: exclusive prefix over the warps, and the tile's global offset
-#pragma unroll
-    for (int e = 0; e < DPT; e++) {
-        const uint32_t d = threadIdx.x * DPT + e;
+    {
+        const uint32_t d = threadIdx.x;
         uint32_t run = 0;
 #pragma unroll
         for (int w = 0; w < RS_WARPS; w++) {
@@ -153,186 +184,210 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(const uint8_t *__restric
             s_wh[w * D + d] = run;
             run += c;
         }
-        s_goff[d] = tile_off[(size_t)d * num_tiles + blockIdx.x];
+        const uint32_t off = tile_off[(size_t)d * num_tiles + blockIdx.x];
+        s_goff[d] = 1u + off + (c0 <= d ? 1u : 0u);
+        // row 0 (PFP) and the '$' row, by the first tile
+        if (blockIdx.x == 0 && d == c0) LF[0] = hash.entry(1u + off);
+        if (blockIdx.x == 0 && d == 0) LF[in.dollar] = UB_RULER;      // row 0 is ruler 0
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < RS_ITEMS; q++) {
         const uint32_t d = dg[q];
         if (d == 0xFFFFFFFFu) continue;
-        const size_t e = wbase + (size_t)q * 32 + lane;
-        // position among all non-'$' rows of this symbol's bucket
-        const uint32_t t = 1u + s_goff[d] + s_wh[warp * D + d] + rk[q];
-        const uint32_t row = (uint32_t)e < i ? (uint32_t)e : (uint32_t)e + 1u;
-        LF[row] = ub_is_ruler(t, rate_mask) ? (UB_RULER | ub_ruler_index(rul, m, t)) : t;
+        LF[in.row((uint32_t)(wbase + (size_t)q * 32 + lane))] = hash.entry(s_goff[d] + s_wh[warp * D + d] + rk[q]);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) LF[i] = UB_RULER | 0u;      // '$' row -> row 0 = ruler 0
 }
 
-struct LoadRuler {
-    uint32_t rate_mask;
-    __device__ __forceinline__ uint32_t operator()(size_t r) const
-    {
-        return ub_is_ruler((uint32_t)r, rate_mask) ? 1u : 0u;
-    }
-};
-struct StoreRuler {
-    uint32_t *rul;
-    __device__ __forceinline__ void operator()(size_t r, uint32_t pre, uint32_t v) const
-    {
-        if (v) rul[pre] = (uint32_t)r;
-    }
-};
-
-// Pass 1: next ruler and distance from each ruler along LF.  The ruler
-// whose successor is ruler 0 ends the chain (no successor; its weight is
-// the last hop back to row 0).
-__global__ void k_walk_count(const uint32_t *LF, const uint32_t *rul, uint32_t m, uint32_t rows, uint32_t *succ,
-                             uint64_t *wt, uint32_t *flags)
+// First walk: the next ruler and the distance to it.  A warp takes block after
+// block of 32 ruler rows.
+__global__ void k_walk_count(const uint32_t *__restrict__ LF, UbHash hash, uint32_t slots, uint32_t *succ, uint32_t *wt)
 {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    uint32_t r = rul[j], steps = 0, v;
-    for (;;) {
-        v = __ldg(LF + r);
-        steps++;
-        if ((v & UB_RULER) || steps > rows) break;
-        r = v;
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < slots; j += step) {
+        uint32_t r = hash.row_of(j), steps = 0, v = UB_NIL;
+        if (r < hash.rows) {               // else a hash value past the rows: no ruler
+            do {
+                v = __ldg(LF + r);
+                r = v;
+                steps++;
+            } while (!(v & UB_RULER) && steps <= hash.rows);
+            v &= ~UB_RULER;
+        }
+        succ[j] = v;
+        wt[j] = steps;
     }
-    if (steps > rows) atomicOr(flags, ERR_INTERNAL);
-    const uint32_t nx = v & ~UB_RULER;
-    succ[j] = nx == 0 ? UB_NIL : nx;
-    wt[j] = steps;
 }
 
-// Pointer jumping (list ranking): after r rounds wt[j] is the distance over
-// the next 2^r rulers (or to the chain's end).  Double-buffered; `open`
-// counts rulers that still have a successor.
-__global__ void k_jump(const uint32_t *succ, const uint64_t *wt, uint32_t m, uint32_t *succ2, uint64_t *wt2,
-                       uint32_t *open)
+// Hops between super-rulers (numbers that are multiples of 2^UB_SUPER_LOG2):
+// the next one and the distance.  The one whose next is ruler 0 ends the chain.
+__global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
+                             uint32_t *ssucc, uint32_t *swt)
 {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    const uint32_t s = succ[j];
-    if (s == UB_NIL) {
-        succ2[j] = UB_NIL;
-        wt2[j] = wt[j];
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= supers) return;
+    uint32_t j = s << UB_SUPER_LOG2, acc = 0, hops = 0;
+    if (hash.row_of(j) >= hash.rows) {
+        ssucc[s] = UB_NIL;
+        swt[s] = 0;
         return;
     }
-    wt2[j] = wt[j] + wt[s];
-    const uint32_t s2 = succ[s];
-    succ2[j] = s2;
-    if (s2 != UB_NIL) atomicAdd(open, 1u);
+    do {
+        acc += wt[j];
+        j = succ[j];
+    } while (j < slots && (j & ((1u << UB_SUPER_LOG2) - 1u)) && ++hops < slots);
+    ssucc[s] = j == 0 || j >= slots ? UB_NIL : j >> UB_SUPER_LOG2;
+    swt[s] = acc;
 }
 
-// Offsets from row 0: off[j] = total - (distance from ruler j to the end).
-__global__ void k_ruler_off(const uint64_t *wt, uint32_t m, uint32_t *off)
+// Pointer jumping: after r rounds wt[s] is the distance over the next 2^r
+// super-rulers (or to the chain's end).  Double-buffered.
+__global__ void k_jump(const uint32_t *succ, const uint32_t *wt, uint32_t m, uint32_t *succ2, uint32_t *wt2)
 {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    off[j] = (uint32_t)(wt[0] - wt[j]);
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= m) return;
+    const uint32_t t = succ[s];
+    succ2[s] = t == UB_NIL ? UB_NIL : succ[t];
+    wt2[s] = wt[s] + (t == UB_NIL ? 0u : wt[t]);
 }
 
-// Pass 2: every ruler writes the text bytes of its stretch.  sym(row) is
-// the bucket of LF(row)-1 among the cumulative symbol counts cum[0..256].
-__global__ void k_walk_emit(const uint32_t *LF, const uint32_t *rul, const uint32_t *off, uint32_t m,
-                            const uint32_t *cum, uint32_t n, uint8_t *T)
+// Distances from row 0 for every ruler: the hops again, from rows - (distance
+// of the super-ruler to the end).
+__global__ void k_ruler_off(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
+                            const uint32_t *sdist, uint32_t *off)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= supers) return;
+    uint32_t j = s << UB_SUPER_LOG2, hops = 0;
+    if (hash.row_of(j) >= hash.rows) return;
+    uint32_t o = hash.rows - sdist[s];
+    do {
+        off[j] = o;
+        o += wt[j];
+        j = succ[j];
+    } while (j < slots && (j & ((1u << UB_SUPER_LOG2) - 1u)) && ++hops < slots);
+}
+
+// Second walk: every ruler writes the text bytes of its stretch, from high to
+// low addresses, gathered into 8-byte words.  sym(row) is the bucket of
+// LF(row) - 1 among the cumulative counts cum[0..256]: a table over the value's
+// high bits gives the first candidate.
+__global__ void __launch_bounds__(256) k_walk_emit(const uint32_t *__restrict__ LF, UbHash hash, uint32_t slots,
+                                                   const uint32_t *off, const uint32_t *cum, int lut_shift, uint32_t n,
+                                                   uint8_t *T)
 {
     __shared__ uint32_t s_cum[257];
+    __shared__ uint8_t s_lut[1 << UB_LUT_LOG2];
     for (int c = threadIdx.x; c < 257; c += blockDim.x) s_cum[c] = cum[c];
     __syncthreads();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m) return;
-    uint32_t r = rul[j], k = off[j];
-    for (uint32_t s = 0; s <= n; s++, k++) {
-        const uint32_t v = __ldg(LF + r);
-        const bool last = (v & UB_RULER) != 0;
-        const uint32_t t = last ? rul[v & ~UB_RULER] : v;
-        if (k < n && t > 0) {
-            uint32_t lo = 0, hi = 255;           // last c with cum[c] <= t-1
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1u) >> 1;
-                if (s_cum[mid] <= t - 1u) lo = mid; else hi = mid - 1u;
-            }
-            T[n - 1u - k] = (uint8_t)lo;
+    for (uint32_t q = threadIdx.x; q < (1u << UB_LUT_LOG2); q += blockDim.x) {
+        const uint64_t first = (uint64_t)q << lut_shift;
+        uint32_t lo = 0, hi = 255;           // last c with cum[c] <= first
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1u) >> 1;
+            if (s_cum[mid] <= first) lo = mid; else hi = mid - 1u;
         }
-        if (last) break;
-        r = t;
+        s_lut[q] = (uint8_t)lo;
+    }
+    __syncthreads();
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < slots; j += step) {
+        uint32_t r = hash.row_of(j);
+        if (r >= hash.rows) continue;
+        uint32_t k = off[j], in_word = 0;    // bytes gathered in `word`
+        uint64_t word = 0;
+        for (bool last = false; !last; k++) {
+            const uint32_t v = __ldg(LF + r);
+            last = (v & UB_RULER) != 0;
+            r = last ? hash.row_of(v & ~UB_RULER) : v;
+            if (k >= n || r == 0) break;     // the '$' row: the stretch ends here
+            uint32_t c = s_lut[(r - 1u) >> lut_shift];
+            while (s_cum[c + 1] <= r - 1u) c++;
+            uint8_t *p = T + (n - 1u - k);
+            word = (word << 8) | c;          // bytes come from high to low addresses
+            in_word++;
+            if (last || ((uintptr_t)p & 7u) == 0) {
+                if (in_word == 8u) *(uint64_t *)p = word;
+                else for (uint32_t q = 0; q < in_word; q++) p[q] = (uint8_t)(word >> (8u * q));
+                in_word = 0;
+                word = 0;
+            }
+        }
+        // bytes before the '$' row: the lowest is T[0]
+        for (uint32_t q = 0; q < in_word; q++) T[q] = (uint8_t)(word >> (8u * q));
     }
 }
 
-// Cumulative symbol counts: the scanned tile histogram's first tile entries.
-__global__ void k_unbwt_cum(const uint32_t *tile_off, uint32_t num_tiles, uint32_t n, uint32_t *cum)
+// Cumulative symbol counts of all non-'$' rows from the scanned tile
+// histograms (row 0's symbol added back for PFP input).
+__global__ void k_unbwt_cum(UbIn in, const uint32_t *tile_off, uint32_t num_tiles, uint32_t *cum)
 {
     const uint32_t c = threadIdx.x;
-    cum[c] = tile_off[(size_t)c * num_tiles];
-    if (c == 0) cum[256] = n;
+    const uint32_t c0 = in.p != UB_NIL ? in.L[in.p] : 256u;
+    cum[c] = tile_off[(size_t)c * num_tiles] + (c0 < c ? 1u : 0u);
+    if (c == 0) cum[256] = in.n;
 }
 
-void pfp_to_libcubwt(Storage *st, const uint8_t *dO, uint32_t n, uint32_t p, uint8_t *dLc)
-{
-    k_pfp_to_libcubwt<<<grid_for(n, 256), 256, 0, st->stream>>>(dO, n, p, dLc);
-    after_launch(st);
-}
-
-// Inverse of libcubwt's convention: Lc (n bytes, device), primary index i in [1, n].
-void run_unbwt(Storage *st, const uint8_t *dLc, uint32_t n, uint32_t i, uint8_t *dT)
+// Inverse of the PFP output (p: its primary row, i unused) or of libcubwt's L
+// (p = 0xFFFFFFFF, i its primary index in [1, n]).
+void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t p, uint8_t *dT)
 {
     const uint32_t rows = n + 1u;
-    // ~1/128 of the rows are rulers (tuning knob): the longest walk (about
-    // rate * ln m steps of one dependent load each) sets the time of both
-    // walk passes; small inputs use denser rulers
+    UbIn in{dL, n, p != UB_NIL ? p + 1u : i, p};
+    // ~1/32 of the rows are rulers (tuning knob); small inputs use denser ones
     const uint32_t rate_max = 1u << tune_unbwt_rate_log2(st);
     uint32_t rate = 4;
     while (rate < rate_max && (uint64_t)rate * 65536u < rows) rate <<= 1;
-    const uint32_t rate_mask = rate - 1u;
-    // rulers in row order
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    uint32_t *rul = slot<uint32_t>(st, S_SA, rows / 2 + 1024);
-    device_scan<uint32_t, OpAdd>(st, rows, LoadRuler{rate_mask}, StoreRuler{rul}, false, (uint32_t *)st->d_scalars);
-    fetch_scalars(st, 1);
-    const uint32_t m = (uint32_t)st->h_scalars[0];
-    if (m == 0 || m > rows / 2 + 1024 || m >= UB_RULER) throw Error{GBWT_INTERNAL_ERROR};
+    const int kb = bits_for((rows - 1u) >> 5);
+    UbHash hash;
+    hash.mask = (uint32_t)((1ull << kb) - 1ull);
+    hash.half = (kb + 1) / 2;
+    hash.rate_log2 = 0;
+    while ((1u << hash.rate_log2) < rate && hash.rate_log2 < kb) hash.rate_log2++;
+    hash.rows = rows;
+    const uint32_t slots = (uint32_t)((1ull << kb) >> hash.rate_log2) << 5;
+    const uint32_t supers = (slots + (1u << UB_SUPER_LOG2) - 1u) >> UB_SUPER_LOG2;
     // LF
     const uint32_t num_tiles = (uint32_t)(((size_t)n + RS_TILE - 1) / RS_TILE);
     uint32_t *hist = slot<uint32_t>(st, S_RSHIST, (size_t)256 * num_tiles);
-    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, hist, num_tiles);
+    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles);
     after_launch(st);
     device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
                                  (uint32_t *)nullptr);
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
-    k_lf_rank<8><<<num_tiles, RS_THREADS, 0, st->stream>>>(dLc, n, i, hist, num_tiles, rate_mask, rul, m, LF);
+    k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF);
     after_launch(st);
     uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
-    k_unbwt_cum<<<1, 256, 0, st->stream>>>(hist, num_tiles, n, cum);
+    k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);
     after_launch(st);
     // walk 1 and list ranking of the ruler chain
-    uint32_t *succ = slot<uint32_t>(st, S_TMP0, m), *succ2 = slot<uint32_t>(st, S_TMP1, m);
-    uint64_t *wt = slot<uint64_t>(st, S_KEY0, m), *wt2 = slot<uint64_t>(st, S_KEY1, m);
-    k_walk_count<<<grid_for(m, 128), 128, 0, st->stream>>>(LF, rul, m, rows, succ, wt, st->d_flags);
+    uint32_t *succ = slot<uint32_t>(st, S_TMP0, slots), *wt = slot<uint32_t>(st, S_TMP1, slots);
+    unsigned grid = grid_for(slots, 256);
+    const unsigned full = (unsigned)st->num_sms * 8u;          // 2048 threads per SM
+    if (grid > full) grid = full;
+    k_walk_count<<<grid, 256, 0, st->stream>>>(LF, hash, slots, succ, wt);
     after_launch(st);
-    // one list of m rulers closes after ceil(log2 m) rounds; anything still
-    // open then lies on a cycle that does not pass row 0
-    const int rounds = bits_for(m) + 1;
+    uint32_t *ssucc = slot<uint32_t>(st, S_VAL0, supers), *ssucc2 = slot<uint32_t>(st, S_VAL1, supers);
+    uint32_t *swt = slot<uint32_t>(st, S_KEY0, supers), *swt2 = slot<uint32_t>(st, S_KEY1, supers);
+    k_super_hops<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, hash, supers, slots, ssucc, swt);
+    after_launch(st);
+    const int rounds = bits_for(supers);
     for (int r = 0; r < rounds; r++) {
-        if (r == rounds - 1) check_cuda(cudaMemsetAsync(st->d_flags + 4, 0, 4, st->stream));
-        k_jump<<<grid_for(m, 256), 256, 0, st->stream>>>(succ, wt, m, succ2, wt2, st->d_flags + 4);
+        k_jump<<<grid_for(supers, 256), 256, 0, st->stream>>>(ssucc, swt, supers, ssucc2, swt2);
         after_launch(st);
-        uint32_t *ts = succ; succ = succ2; succ2 = ts;
-        uint64_t *tw = wt; wt = wt2; wt2 = tw;
+        uint32_t *ts = ssucc; ssucc = ssucc2; ssucc2 = ts;
+        uint32_t *tw = swt; swt = swt2; swt2 = tw;
     }
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 1, st->d_flags + 4, 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 2, wt, 8, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 3, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
+    // from ruler 0 the cycle must come back to row 0 after n+1 steps, its list closed
+    check_cuda(cudaMemcpyAsync(st->h_scalars + 1, ssucc, 4, cudaMemcpyDeviceToHost, st->stream));
+    check_cuda(cudaMemcpyAsync(st->h_scalars + 2, swt, 4, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
-    if ((uint32_t)st->h_scalars[3] & ERR_INTERNAL) throw Error{GBWT_INTERNAL_ERROR};
-    if ((uint32_t)st->h_scalars[1] != 0) throw Error{GBWT_BAD_PARAMETER};
-    // from ruler 0 the whole cycle must come back to row 0 after n+1 steps
-    if (st->h_scalars[2] != (uint64_t)rows) throw Error{GBWT_BAD_PARAMETER};
-    uint32_t *off = slot<uint32_t>(st, S_VAL0, m);
-    k_ruler_off<<<grid_for(m, 256), 256, 0, st->stream>>>(wt, m, off);
+    if ((uint32_t)st->h_scalars[1] != UB_NIL || (uint32_t)st->h_scalars[2] != rows) throw Error{GBWT_BAD_PARAMETER};
+    uint32_t *off = slot<uint32_t>(st, S_SA, slots);
+    k_ruler_off<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, hash, supers, slots, swt, off);
     after_launch(st);
-    k_walk_emit<<<grid_for(m, 128), 128, 0, st->stream>>>(LF, rul, off, m, cum, n, dT);
+    const int lut_shift = kb + 5 > UB_LUT_LOG2 ? kb + 5 - UB_LUT_LOG2 : 0;
+    k_walk_emit<<<grid, 256, 0, st->stream>>>(LF, hash, slots, off, cum, lut_shift, n, dT);
     after_launch(st);
 }
 
