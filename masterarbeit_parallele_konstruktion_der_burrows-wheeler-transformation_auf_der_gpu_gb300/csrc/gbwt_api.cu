@@ -95,6 +95,10 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
     Phrases ph;
     ph.z = z;
     ph.D = D;
+    if (un <= SMALL_TEXT) {
+        alpha_present(st, dT, un, st->d_flags + 8);
+        ph.have_alpha = true;
+    }
     run_phrases(st, dT, un, W, ph);
     st->stats.d = ph.d;
     st->stats.dict_bytes = (int64_t)ph.dict_bytes;

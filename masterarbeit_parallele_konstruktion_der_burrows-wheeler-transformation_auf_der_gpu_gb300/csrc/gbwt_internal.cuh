@@ -25,7 +25,7 @@ enum : uint32_t {
 enum Slot : int {
     S_TEXT = 0, S_OUT,
     S_D, S_PID, S_SLOT, S_TKEYS, S_TVALS, S_TDENSE,
-    S_DLEN, S_DSTART, S_DOFF, S_OCC, S_PCMIN, S_PCMAX, S_DICT, S_DPHR,
+    S_DLEN, S_DSTART, S_DOFF, S_OCC, S_DICT, S_DPHR,
     S_KEY0, S_KEY1, S_VAL0, S_VAL1, S_ISA, S_SA, S_ACTX, S_ACTG, S_HEAD,
     S_LEXRANK, S_PARSE, S_PISA, S_PSA,
     S_GCOUNT, S_GCHAR, S_GRP, S_MOFF, S_MB, S_MC, S_DELTA,
@@ -192,9 +192,6 @@ __device__ __forceinline__ uint8_t preceding_byte(const uint8_t *T, uint32_t n, 
     return p ? __ldg(T + p - 1) : __ldg(T + n - 1);
 }
 
-// Writes one value (kept per translation unit).
-static __global__ void k_set_u32(uint32_t *p, uint32_t v) { *p = v; }
-
 // Host-side declarations of the pipeline stages (implemented in the .cu files).
 uint32_t run_trigger_scan(Storage *st, const uint8_t *dT, uint32_t n, int W, int P, bool small,
                           uint32_t *&D);
@@ -206,8 +203,9 @@ struct Phrases {
     uint32_t *pidpc = nullptr;         // [z] id << 8 | preceding byte (d < 2^24), else null
     uint32_t *dlen = nullptr;          // [d] length of distinct phrase
     uint32_t *doff = nullptr;          // [d+1] offset in dictionary buffer
-    uint32_t *occ = nullptr;           // [d] occurrences
-    uint32_t *pcmin = nullptr, *pcmax = nullptr;  // [d] min/max preceding byte
+    uint2 *occpc = nullptr;            // [d] occurrences; preceding bytes seen, byte c as c | (~c << 16)
+    bool have_alpha = false;           // alpha: set of the text's byte values, if collected already
+    uint32_t alpha[8] = {};
     uint8_t *dict = nullptr;           // [dict_bytes] concatenated phrases
     uint32_t *dphr = nullptr;          // [dict_bytes] phrase id per position
     uint32_t *dtid = nullptr;          // [d] text of the distinct phrase (a batch kept apart by text), else null
@@ -234,6 +232,11 @@ struct DictOrder {
     uint32_t *lexrank = nullptr; // [d] dense lexicographic rank of each phrase
     int rounds = 0;
 };
+// Set of the byte values of p[0..n), OR-ed into bits[0..8).
+void alpha_present(Storage *st, const uint8_t *p, uint32_t n, uint32_t *bits);
+// Texts up to this size give their alphabet, read back with the phrase counts:
+// a pass of a few microseconds for a host round trip of twelve.
+constexpr uint32_t SMALL_TEXT = 4u << 20;
 void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord);
 
 struct ParseOrder {
@@ -247,7 +250,7 @@ int sort_phrase_suffixes(Storage *st, uint32_t N, int key_bits, uint32_t h0, con
                          const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa);
 void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, const uint32_t *doff, uint32_t *lexrank);
 int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
-                     const uint32_t *occ, uint32_t *isa, uint32_t *sa);
+                     const uint32_t *occ, int stride, uint32_t *isa, uint32_t *sa);   // occ[q * stride]
 // Parse suffix array by parsing the parse; false (nothing done) when that does not pay.
 bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord, const BatchText *bt);
 // Suffix array over all texts' parses (text of phrase i: ptid[i]; one past text t's last: zend[t]).

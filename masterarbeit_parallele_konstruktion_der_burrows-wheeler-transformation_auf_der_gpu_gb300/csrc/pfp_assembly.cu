@@ -34,14 +34,6 @@ struct PosInfo {
     }
 };
 
-// Preceding-byte code of the phrase suffix starting at dictionary position x.
-__device__ __forceinline__ uint32_t pc_code(const uint8_t *dict, const uint32_t *pcmin, const uint32_t *pcmax,
-                                            uint32_t x, uint32_t q, uint32_t off)
-{
-    if (off) return dict[x - 1];
-    return pcmin[q] == pcmax[q] ? pcmin[q] : PC_VAR;
-}
-
 // ---- single text: groups by the sorted position of their head ----------
 // stat[t] of the group whose head is sorted position t: x = block length, y =
 // the preceding bytes seen, byte c as c | (~c << 16).  OR-ing members keeps a
@@ -56,11 +48,10 @@ __device__ __forceinline__ uint32_t pc_code(const uint8_t *dict, const uint32_t 
 // the bytes (four random sectors per suffix).  All S-group kernels together:
 // 512 MiB DNA, W=35 (N = 130 M) 13.9 -> 4.3 ms, of it 3.5 here; W=5 1.28 -> 0.73
 // ms; 102 MB of versions 4.9 -> 1.7 ms.
-constexpr uint32_t GS_ANY = 0x00FF00FFu;       // a byte that varies
 __device__ __forceinline__ bool gs_mixed(uint32_t y) { return (y & (y >> 16) & 0xFFu) != 0; }
 
 __global__ void k_group_stats(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *isa, const uint8_t *dict,
-                              const uint32_t *occ, const uint32_t *pcmin, const uint32_t *pcmax, uint2 *stat)
+                              const uint2 *occpc, uint2 *stat)
 {
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= N) return;
@@ -68,9 +59,10 @@ __global__ void k_group_stats(uint32_t N, PosInfo pi, uint32_t W, const uint32_t
     pi.get(x, q, off, rem);
     if (rem <= W) return;
     const uint32_t t = isa[x];
-    const uint32_t c = pc_code(dict, pcmin, pcmax, x, q, off);
-    atomicAdd(&stat[t].x, occ[q]);
-    atomicOr(&stat[t].y, c == PC_VAR ? GS_ANY : c | ((c ^ 0xFFu) << 16));
+    const uint2 oc = occpc[q];                  // a whole phrase: the bytes before its occurrences
+    const uint32_t c = off ? dict[x - 1] : 0u;
+    atomicAdd(&stat[t].x, oc.x);
+    atomicOr(&stat[t].y, off ? c | ((c ^ 0xFFu) << 16) : oc.y);
 }
 
 // One scan of the block lengths turns the statistics into places: stat[t]
@@ -504,7 +496,6 @@ uint32_t run_group_index(Storage *st, Phrases &ph, DictOrder &dord, int W, uint3
     check_cuda(cudaMemsetAsync(mark, 0, N, st->stream));
     k_mark_sheads<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, mark);
     after_launch(st);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     device_scan<uint32_t, OpAdd>(st, N, LoadMark{mark}, StoreGid{gid}, true, (uint32_t *)st->d_scalars);
     fetch_scalars(st, 1);
     const uint32_t G = (uint32_t)st->h_scalars[0];
@@ -521,12 +512,10 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     PosInfo pi{ph.dphr, ph.doff, ph.dlen};
     uint2 *stat = slot<uint2>(st, S_GCOUNT, (size_t)N + 1);
     check_cuda(cudaMemsetAsync(stat, 0, (size_t)N * sizeof(uint2), st->stream));
-    k_group_stats<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, ph.dict, ph.occ, ph.pcmin,
-                                                            ph.pcmax, stat);
+    k_group_stats<<<grid_for(N, 256), 256, 0, st->stream>>>(N, pi, (uint32_t)W, dord.isa, ph.dict, ph.occpc, stat);
     after_launch(st);
     const size_t nw = ((size_t)N + 31) / 32;
     uint32_t *heads = slot<uint32_t>(st, S_TMP0, nw), *mixed = slot<uint32_t>(st, S_TMP1, nw);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 32, st->stream));
     device_scan<uint32_t, OpAdd>(st, N, LoadGCount{stat}, StoreGroup{stat, N, heads, mixed}, false,
                                  (uint32_t *)st->d_scalars);
     // a mixed block has at least two bytes
@@ -552,7 +541,6 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
     }
     const uint32_t long_cap = n_out / RF_LONG + 1u;
     uint32_t *longs = slot<uint32_t>(st, S_TILEG, long_cap);
-    check_cuda(cudaMemsetAsync(st->d_flags + 5, 0, 4, st->stream));
     probe_begin(st, GBWT_PROBE_RUN_FILL);
     k_run_fill_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(dOut, n_out, stat, N, longs, long_cap, st->d_flags);
     probe_end(st, GBWT_PROBE_RUN_FILL, (uint64_t)(n_out - M) + 8ull * N);

@@ -576,7 +576,6 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     st->stats.z = z;
     uint32_t *ptid = slot<uint32_t>(st, S_BTID, z);
     uint32_t *zend = slot<uint32_t>(st, S_BZEND, kk);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     device_scan<uint32_t, OpAdd>(st, z, LoadFinal{X, D}, StoreTid{ptid, zend}, false, (uint32_t *)st->d_scalars);
     fetch_scalars(st, 1);
     if ((uint32_t)st->h_scalars[0] != kk) throw Error{GBWT_INTERNAL_ERROR};
@@ -587,6 +586,10 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     Phrases ph;
     ph.z = z;
     ph.D = D;
+    if (un <= SMALL_TEXT) {
+        alpha_present(st, X, un, st->d_flags + 8);
+        ph.have_alpha = true;
+    }
     // row samples need an element per text position: the second path
     run_phrases(st, X, un, W, ph, &bt, !aux && kk > 1);
     const bool apart = !aux && (kk == 1 || ph.dtid);

@@ -382,7 +382,6 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     // positions, more means symbols that hash alike (or tiny texts) and no gain
     const uint32_t cap = z / 3u;
     uint32_t *s = slot<uint32_t>(st, S_2START, (size_t)cap + 2);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     device_scan<uint32_t, OpAdd>(st, zw, LoadTrigWord{trig}, StoreStarts{trig, s, cap}, false, (uint32_t *)st->d_scalars);
     fetch_scalars(st, 1);
     const uint32_t z2 = (uint32_t)st->h_scalars[0] + 1u;
@@ -403,7 +402,6 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     uint32_t *give_up = st->d_flags + 28;
     check_cuda(cudaMemsetAsync(tkeys, 0, (size_t)c * 8, st->stream));
     check_cuda(cudaMemsetAsync(give_up, 0, 3 * 4, st->stream));
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     k_l2_hash<<<grid_for(z2, 256), 256, 0, st->stream>>>(V, s, z2, 0x0A5C3D1F2B4E6987ull, tkeys, tvals, logc, limit,
                                                          slot_of, give_up);
     after_launch(st);
@@ -446,7 +444,7 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
         after_launch(st);
         pord.rounds += parse_sa_batch(st, z2, d, pid, rank, tid2, zend2, bt->k, true, pisa, psa);
     } else {
-        pord.rounds += parse_sa_buckets(st, z2, d, pid, rank, occ, pisa, psa);
+        pord.rounds += parse_sa_buckets(st, z2, d, pid, rank, occ, 1, pisa, psa);
     }
     // group numbers per dictionary position (sa is dead: it takes them)
     const size_t nw = ((size_t)N + 31) / 32;
@@ -455,7 +453,6 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     check_cuda(cudaMemsetAsync(bits, 0, nw * 4, st->stream));
     k_l2_heads<<<grid_for(N, 256), 256, 0, st->stream>>>(N, rem8, isa, bits);
     after_launch(st);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 16, st->stream));
     device_scan<uint32_t, OpAdd>(st, nw, LoadTrigWord{bits}, StoreArr<uint32_t>{pre}, false, (uint32_t *)st->d_scalars);
     k_l2_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(N, rem8, isa, bits, pre, grp);
     after_launch(st);

@@ -322,7 +322,7 @@ struct StoreDense {
 // every distinct phrase.
 __global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, int W,
                                   const uint32_t *slot_of, const uint32_t *tdense, uint32_t *pid, uint32_t *pidpc,
-                                  uint32_t *occ, uint32_t *pcmin, uint32_t *pcmax, const uint8_t *xsep,
+                                  uint2 *occpc, const uint8_t *xsep,
                                   const uint32_t *ptid, const uint8_t *lastb)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -337,9 +337,8 @@ __global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *
     if (pidpc) pidpc[k] = (id << 8) | c;     // only when ids fit 24 bits
     // one atomic each per occurrence: neighbouring occurrences rarely share a
     // phrase, so warp aggregation (a match per warp) costs more than it saves
-    atomicAdd(occ + id, 1u);
-    atomicMin(pcmin + id, c);
-    atomicMax(pcmax + id, c);
+    atomicAdd(&occpc[id].x, 1u);
+    atomicOr(&occpc[id].y, c | ((c ^ 0xFFu) << 16));
 }
 
 struct LoadLen64 {
@@ -348,7 +347,12 @@ struct LoadLen64 {
 };
 struct StoreOff32 {
     uint32_t *a;
-    __device__ __forceinline__ void operator()(size_t i, uint64_t pre, uint64_t) const { a[i] = (uint32_t)pre; }
+    size_t n;                   // a[n] = the total
+    __device__ __forceinline__ void operator()(size_t i, uint64_t pre, uint64_t v) const
+    {
+        a[i] = (uint32_t)pre;
+        if (i + 1 == n) a[n] = (uint32_t)(pre + v);
+    }
 };
 
 // LANES lanes per distinct phrase: copy its bytes and tag positions with the id.
@@ -412,7 +416,6 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         check_cuda(cudaMemsetAsync(tkeys, 0, (size_t)c * 8, st->stream));
         check_cuda(cudaMemsetAsync(st->d_flags, 0, 8, st->stream));
         check_cuda(cudaMemsetAsync(st->d_flags + 48, 0, 4, st->stream));
-        check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
         HashArgs a;
         a.full = st->d_flags + 48;
         a.T = dT; a.n = n; a.D = ph.D; a.z = z; a.W = W;
@@ -439,13 +442,13 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
                                                                   st->d_flags, xsep, pvals, pslot, may_part ? part : nullptr);
         after_launch(st);
         device_scan<uint32_t, OpAdd>(st, z, LoadU32{isrep}, StoreDense{ph.D, slot_of, tdense, dlen, dstart, W, xsep, ptid, dtid},
-                                     false, (uint32_t *)st->d_scalars);
-        check_cuda(cudaMemcpyAsync(st->h_scalars + 1, st->d_flags, 4, cudaMemcpyDeviceToHost, st->stream));
+                                     false, st->d_flags + 6);
+        check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_flags, 32, cudaMemcpyDeviceToHost, st->stream));
         if (may_part)
             check_cuda(cudaMemcpyAsync(st->h_scalars + 4, part, sizeof(Parting), cudaMemcpyDeviceToHost, st->stream));
-        fetch_scalars(st, 1);
-        uint32_t flags = (uint32_t)(st->h_scalars[1] & 0xFFFFFFFFu);
-        d = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
+        sync_stream(st);
+        const uint32_t flags = (uint32_t)st->h_scalars[0];
+        d = (uint32_t)st->h_scalars[3];
         if (flags & ERR_TABLE_FULL) { c = full_c; st->stats.hash_retries++; continue; }
         if (flags & ERR_COLLISION) {
             seed = seed * 6364136223846793005ull + 1442695040888963407ull;
@@ -461,28 +464,24 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
     ph.dtid = parted ? dtid : nullptr;
     ph.texts = parted ? bt->k : 1u;
     uint32_t *pid = isrep;   // isrep is dead after the scan
-    uint32_t *occ = slot<uint32_t>(st, S_OCC, d);
-    uint32_t *pcmin = slot<uint32_t>(st, S_PCMIN, d);
-    uint32_t *pcmax = slot<uint32_t>(st, S_PCMAX, d);
-    check_cuda(cudaMemsetAsync(occ, 0, (size_t)d * 4, st->stream));
-    check_cuda(cudaMemsetAsync(pcmin, 0xFF, (size_t)d * 4, st->stream));
-    check_cuda(cudaMemsetAsync(pcmax, 0, (size_t)d * 4, st->stream));
+    uint2 *occpc = slot<uint2>(st, S_OCC, d);
+    check_cuda(cudaMemsetAsync(occpc, 0, (size_t)d * sizeof(uint2), st->stream));
     uint32_t *pidpc = d < (1u << 24) ? slot<uint32_t>(st, S_PIDPC, z) : nullptr;
     k_phrase_finalize<<<grid_for(z, 256), 256, 0, st->stream>>>(dT, n, ph.D, z, W, slot_of, tdense, pid, pidpc,
-                                                                occ, pcmin, pcmax, xsep,
+                                                                occpc, xsep,
                                                                 bt ? bt->ptid : nullptr,
                                                                 bt ? bt->lastb : nullptr);
     ph.pidpc = pidpc;
     after_launch(st);
     // dictionary offsets (64-bit scan, checked against 2^32)
     uint32_t *doff = slot<uint32_t>(st, S_DOFF, (size_t)d + 1);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    device_scan<uint64_t, OpAdd>(st, d, LoadLen64{dlen}, StoreOff32{doff}, false, (uint64_t *)st->d_scalars);
+    device_scan<uint64_t, OpAdd>(st, d, LoadLen64{dlen}, StoreOff32{doff, d}, false, (uint64_t *)st->d_scalars);
+    if (ph.have_alpha)
+        check_cuda(cudaMemcpyAsync(st->h_scalars + 4, st->d_flags + 8, sizeof(ph.alpha), cudaMemcpyDeviceToHost, st->stream));
     fetch_scalars(st, 1);
+    if (ph.have_alpha) memcpy(ph.alpha, st->h_scalars + 4, sizeof(ph.alpha));
     const uint64_t dict_bytes = st->h_scalars[0];
     if (dict_bytes >= 0xFFFFFF00ull) throw Error{GBWT_UNSUPPORTED_INPUT};
-    k_set_u32<<<1, 1, 0, st->stream>>>(doff + d, (uint32_t)dict_bytes);
-    after_launch(st);
     uint8_t *dict = slot<uint8_t>(st, S_DICT, dict_bytes + 16);
     uint32_t *dphr = slot<uint32_t>(st, S_DPHR, dict_bytes + 1);
     if (dict_bytes >= (uint64_t)d * 64u)
@@ -490,7 +489,7 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
     else
         k_dict_copy<8><<<grid_for((size_t)d * 8, 256), 256, 0, st->stream>>>(dT, n, d, doff, dlen, dstart, dict, dphr);
     after_launch(st);
-    ph.pid = pid; ph.dlen = dlen; ph.doff = doff; ph.occ = occ; ph.pcmin = pcmin; ph.pcmax = pcmax;
+    ph.pid = pid; ph.dlen = dlen; ph.doff = doff; ph.occpc = occpc;
     ph.dict = dict; ph.dphr = dphr; ph.dict_bytes = dict_bytes;
 }
 

@@ -328,11 +328,13 @@ __global__ void __launch_bounds__(TS_THREADS) k_trigger(ScanArgs a, uint32_t *co
 }
 
 // Positions from the masks of a counting pass: a CTA covers WINDOWS of it
-// (4096 or 16384), each thread one mask or four.
+// (4096 or 16384), each thread one mask or four.  A last position other than 0
+// goes after the `count` found ones (one text's forced final trigger).
 template <int WINDOWS>
 __global__ void __launch_bounds__(TS_THREADS) k_trigger_write(const uint16_t *masks, const uint32_t *offsets,
-                                                              uint32_t W, uint32_t *D)
+                                                              uint32_t W, uint32_t *D, uint32_t count, uint32_t last)
 {
+    if (last && blockIdx.x == 0 && threadIdx.x == 0) D[count] = last;
     constexpr int PER = WINDOWS / TS_THREADS / 16;       // masks per thread
     static_assert(PER == 1 || PER == 4, "one or four masks per thread");
     __shared__ uint32_t s_warp[32];
@@ -356,23 +358,19 @@ static void launch_pair(Storage *st, const ScanArgs &a, unsigned blocks, uint32_
     k_trigger<WT, PT, false, TS_SUB><<<blocks, TS_THREADS, 0, st->stream>>>(a, counts, nullptr, nullptr, masks);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, a.n);
     after_launch(st);
-    // exclusive scan of block counts; total -> d_scalars[0]
-    uint32_t *tot = (uint32_t *)st->d_scalars;
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, tot);
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 1, a.flags, 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, 8, cudaMemcpyDeviceToHost, st->stream));
+    // exclusive scan of block counts; total beside the error bits: one copy
+    device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, a.flags + 6);
+    check_cuda(cudaMemcpyAsync(st->h_scalars, a.flags, 32, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
-    uint32_t flags = (uint32_t)st->h_scalars[1];
+    const uint32_t flags = (uint32_t)st->h_scalars[0];
     if (flags & ERR_BAD_BYTE) throw Error{GBWT_BAD_PARAMETER};
     if (flags & ERR_SMALL_RANGE) throw Error{GBWT_UNSUPPORTED_INPUT};
-    uint32_t c = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
+    const uint32_t c = (uint32_t)st->h_scalars[3];
     D = slot<uint32_t>(st, S_D, (size_t)c + 1);
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger_write<TS_SUB * TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D);
+    k_trigger_write<TS_SUB * TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D, c,
+                                                                             a.n + (uint32_t)a.W - 1u);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n / 8 + 4ull * c);
-    after_launch(st);
-    k_set_u32<<<1, 1, 0, st->stream>>>(D + c, a.n + (uint32_t)a.W - 1u);
     after_launch(st);
     st->h_scalars[0] = c;
 }
@@ -573,19 +571,16 @@ static uint32_t launch_pair_batch(Storage *st, const ScanArgs &a, const BatchSca
     k_trigger_batch<WT, PT><<<blocks, TS_THREADS, 0, st->stream>>>(a, b, counts, masks);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, a.n);
     after_launch(st);
-    uint32_t *tot = (uint32_t *)st->d_scalars;
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
-    device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, tot);
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 1, a.flags, 4, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, 8, cudaMemcpyDeviceToHost, st->stream));
+    device_scan<uint32_t, OpAdd>(st, blocks, LoadArr<uint32_t>{counts}, StoreArr<uint32_t>{counts}, false, a.flags + 6);
+    check_cuda(cudaMemcpyAsync(st->h_scalars, a.flags, 32, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
-    const uint32_t flags = (uint32_t)st->h_scalars[1];
+    const uint32_t flags = (uint32_t)st->h_scalars[0];
     if (flags & ERR_BAD_BYTE) throw Error{GBWT_BAD_PARAMETER};
     if (flags & ERR_SMALL_RANGE) throw Error{GBWT_UNSUPPORTED_INPUT};
-    const uint32_t c = (uint32_t)(st->h_scalars[0] & 0xFFFFFFFFu);
+    const uint32_t c = (uint32_t)st->h_scalars[3];
     D = slot<uint32_t>(st, S_D, (size_t)c + 1);
     probe_begin(st, GBWT_PROBE_TRIGGER_SCAN);
-    k_trigger_write<TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D);
+    k_trigger_write<TS_TILE><<<blocks, TS_THREADS, 0, st->stream>>>(masks, counts, (uint32_t)a.W, D, 0u, 0u);
     probe_end(st, GBWT_PROBE_TRIGGER_SCAN, (uint64_t)a.n / 8 + 4ull * c);
     after_launch(st);
     return c;
@@ -615,6 +610,8 @@ uint32_t run_trigger_scan_batch(Storage *st, const uint8_t *dX, uint32_t N, int 
     if (W == 35 && P == 81) return launch_pair_batch<35, 81>(st, a, b, blocks, counts, D);
     return launch_pair_batch<0, 0>(st, a, b, blocks, counts, D);
 }
+
+__global__ void k_set_u32(uint32_t *p, uint32_t v) { *p = v; }
 
 // ---------------------------------------------------------------------
 // Allocation-free trigger scan.

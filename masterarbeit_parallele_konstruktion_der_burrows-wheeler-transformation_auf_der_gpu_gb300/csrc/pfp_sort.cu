@@ -442,23 +442,29 @@ __device__ __forceinline__ void warp_group(uint64_t *key, uint32_t s, uint32_t g
 
 // key2[a] = isa[x+h] + 1 for every active element (all reads of this round's
 // ranks happen before any update); tstart[b] = first group start in tile b
-// (SS_TILE active indices; 0xFFFFFFFF before, via memset).  With `bigs`,
+// (SS_TILE active indices; 0xFFFFFFFF before: the gather of one round sets
+// tnext, the starts of the next).  Zeroes the round's counter.  With `bigs`,
 // groups too large for the shared-memory path (more than SS_SEGMAX members)
-// are listed: flags[3] / flags[4] count their starts / ends, bigs[i] = the
+// are listed: nbig[0] / nbig[1] count their starts / ends from ~0, bigs[i] = the
 // i-th start, bigs[big_cap + i] = the i-th end (one past the last member;
 // both lists in no particular order), and tbig[b] = the start of the one that
 // starts in tile b (a tile holds at most one: such a group is longer than a
 // tile).
 __global__ void k_round_gather(const uint32_t *act_x, const uint32_t *act_g, const uint32_t *isa, uint32_t A_arg,
                                const uint32_t *Ap, uint32_t h, uint32_t *key2, uint32_t *flags, uint32_t *tstart,
-                               uint32_t *bigs, uint32_t big_cap, uint32_t *tbig, uint32_t *hist)
+                               uint32_t *tnext, uint32_t *nbig, uint32_t *bigs, uint32_t big_cap, uint32_t *tbig,
+                               uint32_t *hist, uint32_t *counter)
 {
     // the active count: a launch argument when the host knows it, else read
     // on the device (the grid then covers an upper bound)
     const uint32_t A = Ap ? *Ap : A_arg;
-    if (hist && blockIdx.x == 0 && threadIdx.x == 0) *hist = A;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *hist = A;
+        *counter = 0;
+    }
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x >= A) return;
+    if (a % SS_TILE == 0) tnext[a / SS_TILE] = 0xFFFFFFFFu;
     bool gnew = false;
     if (a < A) {
         key2[a] = isa[act_x[a] + h] + 1u;
@@ -466,14 +472,14 @@ __global__ void k_round_gather(const uint32_t *act_x, const uint32_t *act_g, con
         gnew = a == 0 || act_g[a - 1] != g;
         if (bigs) {
             if (gnew && a + SS_SEGMAX < A && act_g[a + SS_SEGMAX] == g) {
-                const uint32_t i = atomicAdd(flags + 3, 1u);
+                const uint32_t i = atomicAdd(nbig, 1u) + 1u;
                 if (i < big_cap) bigs[i] = a;
                 else atomicOr(flags, ERR_INTERNAL);
                 tbig[a / SS_TILE] = a;
             }
             const bool gend = a + 1u == A || act_g[a + 1u] != g;
             if (gend && a >= SS_SEGMAX && act_g[a - SS_SEGMAX] == g) {
-                const uint32_t i = atomicAdd(flags + 4, 1u);
+                const uint32_t i = atomicAdd(nbig + 1, 1u) + 1u;
                 if (i < big_cap) bigs[big_cap + i] = a + 1u;
                 else atomicOr(flags, ERR_INTERNAL);
             }
@@ -809,7 +815,6 @@ static void big_groups(Storage *st, uint32_t N, uint32_t nbig, const uint32_t *d
 }
 
 __global__ void k_add_u32(uint32_t *dst, const uint32_t *src) { *dst += *src; }
-__global__ void k_set_word(uint32_t *dst, uint32_t v) { *dst = v; }
 
 // Prefix-doubling rounds from prefix length h with A active elements listed
 // group by group in act_x (suffix) / act_g (group head); isa holds every
@@ -839,12 +844,20 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
     }
     const bool debug = getenv("GBWT_DEBUG") != nullptr;
     // device words: [0], [1] the two round counters, [2] the side path's
-    // count, [8 + r] the active count round r started with
+    // count, [8 + r] the active count round r started with; read back whole
     uint32_t *dw = (uint32_t *)(st->d_scalars + 16);
     const uint32_t *hw = (const uint32_t *)(st->h_scalars + 160);   // pinned words past the byte tables
-    check_cuda(cudaMemsetAsync(dw, 0, (8 + DR_MAXR) * 4, st->stream));
-    k_set_word<<<1, 1, 0, st->stream>>>(dw + 1, A);     // round 0's count, read by round 1's kernels
-    after_launch(st);
+    auto read_back = [&]() {
+        check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, (8 + DR_MAXR) * 4, cudaMemcpyDeviceToHost, st->stream));
+        sync_stream(st);
+    };
+    // tile words, all ones: big-group counters, tile starts of even and odd
+    // rounds, big-group starts; one memset for all rounds
+    const uint32_t max_tiles = grid_for(A, SS_TILE);
+    uint32_t *tw = slot<uint32_t>(st, S_SSTART, (size_t)max_tiles * 3 + 2);
+    uint32_t *nbig_dev = tw, *tbig = tw + 2 + 2 * (size_t)max_tiles;
+    if (A) check_cuda(cudaMemsetAsync(tw, 0xFF, ((size_t)max_tiles * 3 + 2) * 4, st->stream));
+    if (A <= SS_SEGMAX) check_big = false;       // no room for a big group
     uint32_t A_ub = A;
     bool exact = true;               // A_ub is the count itself, not a bound
     int r = 0;
@@ -853,8 +866,8 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         uint32_t *Aprev = dw + ((r + 1) & 1), *Acur = dw + (r & 1);
         if (h >= N) {
             // only legal when every suffix is finished already
-            check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, 8, cudaMemcpyDeviceToHost, st->stream));
-            sync_stream(st);
+            if (exact) throw Error{GBWT_INTERNAL_ERROR};
+            read_back();
             if (hw[(r + 1) & 1] != 0) throw Error{GBWT_INTERNAL_ERROR};
             break;
         }
@@ -862,29 +875,29 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         // gather this round's keys before any rank changes; list big groups
         uint32_t *key2 = slot<uint32_t>(st, S_TMP2, N);
         const uint32_t ss_tiles = grid_for(A_ub, SS_TILE);
-        uint32_t *tstart = slot<uint32_t>(st, S_SSTART, (size_t)ss_tiles * 2);
-        uint32_t *tbig = tstart + ss_tiles;
+        uint32_t *tstart = tw + 2 + (size_t)(r & 1) * max_tiles, *tnext = tw + 2 + (size_t)((r + 1) & 1) * max_tiles;
         const uint32_t big_cap = A_ub / SS_SEGMAX + 1u;
         uint32_t *bigs = check_big ? slot<uint32_t>(st, S_BIGL, (size_t)big_cap * 2) : nullptr;
-        if (check_big) check_cuda(cudaMemsetAsync(st->d_flags + 3, 0, 8, st->stream));
-        check_cuda(cudaMemsetAsync(tstart, 0xFF, (size_t)ss_tiles * 4 * (check_big ? 2 : 1), st->stream));
+        if (check_big && r > 0) {
+            check_cuda(cudaMemsetAsync(nbig_dev, 0xFF, 8, st->stream));
+            check_cuda(cudaMemsetAsync(tbig, 0xFF, (size_t)ss_tiles * 4, st->stream));
+        }
         static_assert(SS_TILE % 256 == 0, "gather blocks must not straddle tiles");
         const uint32_t *Adev = exact ? nullptr : Aprev;     // a known count goes in as an argument
-        k_round_gather<<<grid_for(A_ub, 256), 256, 0, st->stream>>>(act_x, act_g, isa, A_ub, Adev, (uint32_t)h,
-                                                                    key2, st->d_flags, tstart, bigs, big_cap, tbig,
-                                                                    dw + 8 + r);
+        k_round_gather<<<grid_for(A_ub, 256), 256, 0, st->stream>>>(act_x, act_g, isa, A_ub, Adev, (uint32_t)h, key2,
+                                                                    st->d_flags, tstart, tnext, nbig_dev, bigs, big_cap,
+                                                                    tbig, dw + 8 + r, Acur);
         after_launch(st);
         uint32_t nbig = 0;
         if (check_big) {
-            check_cuda(cudaMemcpyAsync(st->h_scalars + 2, st->d_flags + 3, 8, cudaMemcpyDeviceToHost, st->stream));
+            check_cuda(cudaMemcpyAsync(st->h_scalars + 2, nbig_dev, 8, cudaMemcpyDeviceToHost, st->stream));
             sync_stream(st);
             const uint32_t *cnt = (const uint32_t *)(st->h_scalars + 2);
-            nbig = cnt[0];
-            if (nbig > big_cap || cnt[1] != nbig) throw Error{GBWT_INTERNAL_ERROR};
+            nbig = cnt[0] + 1u;
+            if (nbig > big_cap || cnt[1] != cnt[0]) throw Error{GBWT_INTERNAL_ERROR};
         }
         check_big = nbig > 0;
         if (debug) fprintf(stderr, "gbwt: round h=%llu active<=%u big groups=%u\n", (unsigned long long)h, A_ub, nbig);
-        check_cuda(cudaMemsetAsync(Acur, 0, 4, st->stream));
         if (debug) check_cuda(cudaMemsetAsync(st->d_flags + 16, 0, 8 * sizeof(uint32_t), st->stream));
         probe_begin(st, GBWT_PROBE_SEG_SORT);
         k_seg_sort<Rem><<<ss_tiles, SS_THREADS, SS_SMEM, st->stream>>>(
@@ -905,8 +918,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         h *= 2;
         r++;
         if (check_big || nbig || debug || A_ub >= DR_SYNC_MIN || r % DR_SYNC == 0) {
-            check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, 8, cudaMemcpyDeviceToHost, st->stream));
-            sync_stream(st);
+            read_back();
             A_ub = hw[(r + 1) & 1];        // the count this round produced (r already advanced)
             exact = true;
             if (debug) {
@@ -921,9 +933,8 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
             exact = false;
         }
     }
-    // rounds that had work, and the probe's algorithmic bytes per round
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 160, dw, (8 + DR_MAXR) * 4, cudaMemcpyDeviceToHost, st->stream));
-    sync_stream(st);
+    // rounds that had work, and the probe's algorithmic bytes per round (the
+    // loop ends on a read-back)
     int rounds = 0;
     for (int i = 0; i < r; i++) {
         const uint32_t a = hw[8 + i];
@@ -955,7 +966,6 @@ static int prefix_doubling(Storage *st, uint32_t N, int key0_bits, uint32_t h0, 
 
     radix_sort<uint64_t, true>(st, keys, keys_alt, vals, vals_alt, N, 0, key0_bits, RsSegs(), true);
     ActiveTest<Rem> at{keys, vals, N, h0, rem};
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     // the words take 16 bytes per 32 elements of the alternate key buffer,
     // which is free now (8 bytes per element; a slot has at least 256 bytes)
     const size_t nw = ((size_t)N + 31) / 32;
@@ -981,7 +991,7 @@ __global__ void k_alpha_present(const uint8_t *dict, uint32_t N, uint32_t *bits)
     __shared__ uint8_t s_on[256];
     s_on[threadIdx.x] = 0;                   // blockDim == 256
     __syncthreads();
-    const uint32_t nv = N / 16u;             // dict is a slot of its own: 16-byte aligned
+    const uint32_t nv = (((uintptr_t)dict) & 15u) ? 0u : N / 16u;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         const uint4 q = __ldg((const uint4 *)dict + v);
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -993,10 +1003,19 @@ __global__ void k_alpha_present(const uint8_t *dict, uint32_t N, uint32_t *bits)
             s_on[w[k] >> 24] = 1;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x < N - nv * 16u) s_on[dict[nv * 16u + threadIdx.x]] = 1;
+    // the last bytes; all of them when the pointer is not aligned
+    for (uint32_t i = nv * 16u + blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) s_on[dict[i]] = 1;
     __syncthreads();
     const unsigned m = __ballot_sync(0xFFFFFFFFu, s_on[threadIdx.x] != 0);
     if ((threadIdx.x & 31u) == 0 && m) atomicOr(bits + (threadIdx.x >> 5), m);
+}
+
+void alpha_present(Storage *st, const uint8_t *p, uint32_t n, uint32_t *bits)
+{
+    unsigned grid = grid_for(n, 256 * 16);
+    if (grid > (unsigned)st->num_sms * 4) grid = (unsigned)st->num_sms * 4;
+    k_alpha_present<<<grid, 256, 0, st->stream>>>(p, n, bits);
+    after_launch(st);
 }
 
 // Initial dictionary keys: the next h0 symbols of the phrase suffix, each
@@ -1013,14 +1032,15 @@ __global__ void k_alpha_present(const uint8_t *dict, uint32_t N, uint32_t *bits)
 // shift in one each, and symbols past a phrase's end are masked out of the
 // finished key.  Reading h0 codes per position took 1.46 ms on 130 M positions
 // (512 MiB DNA, W=35, h0 = 21), now 0.71 ms; 260 us -> 149 us on 26 M (W=5).
+struct ByteTable { uint8_t b[256]; };
 constexpr int DK_T = 256;
 constexpr int DK_PER = 4;
-__global__ void __launch_bounds__(DK_T) k_dict_keys(const uint8_t *dict, uint32_t N, DictRem rem, const uint8_t *code,
-                                                    int bps, int h0, const uint32_t *dtid, uint64_t *keys, uint8_t *rem8)
+__global__ void __launch_bounds__(DK_T) k_dict_keys(const uint8_t *dict, uint32_t N, DictRem rem,
+                                                    const __grid_constant__ ByteTable code, int bps, int h0, const uint32_t *dtid, uint64_t *keys, uint8_t *rem8)
 {
     __shared__ uint8_t s_code[256];
     __shared__ uint8_t s_sym[DK_T * DK_PER + 64];
-    s_code[threadIdx.x] = code[threadIdx.x];     // blockDim == 256
+    s_code[threadIdx.x] = code.b[threadIdx.x];   // blockDim == 256
     __syncthreads();
     const uint32_t x0 = blockIdx.x * (DK_T * DK_PER);
     for (uint32_t i = threadIdx.x; i < DK_T * DK_PER + 64u; i += DK_T)
@@ -1103,17 +1123,20 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     (void)small;   // the alphabet recoding below covers the small-alphabet packing
     const uint32_t N = (uint32_t)ph.dict_bytes;
     DictRem rem{ph.dphr, ph.doff, ph.dlen, nullptr};
-    // alphabet of the dictionary -> dense codes 1..sigma
-    check_cuda(cudaMemsetAsync(st->d_flags + 8, 0, 8 * sizeof(uint32_t), st->stream));
-    unsigned ag = grid_for(N, 256);
-    if (ag > (unsigned)st->num_sms * 4) ag = (unsigned)st->num_sms * 4;
-    k_alpha_present<<<ag, 256, 0, st->stream>>>(ph.dict, N, st->d_flags + 8);
-    after_launch(st);
+    // alphabet of the dictionary -> dense codes 1..sigma (small texts: taken
+    // from the text with an earlier read-back)
     uint32_t present[8];
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 4, st->d_flags + 8, sizeof(present), cudaMemcpyDeviceToHost,
-                               st->stream));
-    sync_stream(st);
-    memcpy(present, st->h_scalars + 4, sizeof(present));
+    if (ph.have_alpha) {
+        memcpy(present, ph.alpha, sizeof(present));
+        present[0] |= 2u;                                      // the sentinel byte 1
+    } else {
+        check_cuda(cudaMemsetAsync(st->d_flags + 8, 0, 8 * sizeof(uint32_t), st->stream));
+        alpha_present(st, ph.dict, N, st->d_flags + 8);
+        check_cuda(cudaMemcpyAsync(st->h_scalars + 4, st->d_flags + 8, sizeof(present), cudaMemcpyDeviceToHost,
+                                   st->stream));
+        sync_stream(st);
+        memcpy(present, st->h_scalars + 4, sizeof(present));
+    }
     uint8_t *hcode = (uint8_t *)(st->h_scalars + 16);          // 256 pinned bytes
     uint32_t sigma = 0;
     for (int c = 0; c < 256; c++) {
@@ -1127,8 +1150,8 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     const int tb = ph.dtid ? bits_for(ph.texts - 1u) : 0;      // at most 31; a symbol takes at most 8 bits
     int h0 = (key_bits - 1) / bps > 0 ? (key_bits - 1) / bps : 1;
     if (h0 * bps + tb + 1 > 64) h0 = (63 - tb) / bps;
-    uint8_t *dcode = slot<uint8_t>(st, S_TMP1, 256);
-    check_cuda(cudaMemcpyAsync(dcode, hcode, 256, cudaMemcpyHostToDevice, st->stream));
+    ByteTable dcode;                                            // goes along as a kernel argument
+    memcpy(dcode.b, hcode, sizeof(dcode.b));
     uint64_t *keys = slot<uint64_t>(st, S_KEY0, N);
     uint8_t *rem8 = slot<uint8_t>(st, S_TMP0, N);
     k_dict_keys<<<grid_for(N, DK_T * DK_PER), DK_T, 0, st->stream>>>(ph.dict, N, rem, dcode, bps, h0, ph.dtid, keys, rem8);
@@ -1163,10 +1186,10 @@ __global__ void k_parse_keys(const uint32_t *pid, const uint32_t *lexrank, uint3
 // bucket, in no particular order inside a bucket: the rounds sort every
 // group by its next key and all parse suffixes differ, so no order among
 // equal keys survives to the result.
-__global__ void k_bucket_counts(const uint32_t *lexrank, const uint32_t *occ, uint32_t d, uint32_t *cnt_r)
+__global__ void k_bucket_counts(const uint32_t *lexrank, const uint32_t *occ, int stride, uint32_t d, uint32_t *cnt_r)
 {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < d) cnt_r[lexrank[q]] = occ[q];
+    if (q < d) cnt_r[lexrank[q]] = occ[(size_t)q * stride];
 }
 // packed per rank: (occurrences << 32) | (occurrences staying active)
 struct LoadBucket {
@@ -1184,13 +1207,13 @@ struct StoreBucket {
 // Per phrase: (bucket start, active-list start), the second 0xFFFFFFFF for a
 // phrase that occurs once.  One random lookup per occurrence instead of three
 // (rank, bucket, count) in the scatter below.
-__global__ void k_bucket_info(const uint32_t *lexrank, const uint64_t *bst, const uint32_t *occ, uint32_t d,
+__global__ void k_bucket_info(const uint32_t *lexrank, const uint64_t *bst, const uint32_t *occ, int stride, uint32_t d,
                               uint2 *info)
 {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= d) return;
     const uint64_t p = bst[lexrank[q]];
-    info[q] = make_uint2((uint32_t)(p >> 32), occ[q] > 1u ? (uint32_t)p : 0xFFFFFFFFu);
+    info[q] = make_uint2((uint32_t)(p >> 32), occ[(size_t)q * stride] > 1u ? (uint32_t)p : 0xFFFFFFFFu);
 }
 __global__ void k_bucket_scatter(const uint32_t *pid, const uint2 *info, uint32_t z, uint32_t *cur, uint32_t *isa,
                                  uint32_t *sa, uint32_t *act_x, uint32_t *act_g, uint32_t *flags)
@@ -1218,7 +1241,7 @@ __global__ void k_bucket_scatter(const uint32_t *pid, const uint2 *info, uint32_
 // Parse suffix array from the phrase buckets (the last phrase occurs once: its
 // suffix, the only one ending within one phrase, is finished in round 0).
 int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
-                     const uint32_t *occ, uint32_t *isa, uint32_t *sa)
+                     const uint32_t *occ, int stride, uint32_t *isa, uint32_t *sa)
 {
     uint32_t *cnt_r = slot<uint32_t>(st, S_TMP0, d);
     uint64_t *bst = slot<uint64_t>(st, S_KEY1, d);
@@ -1227,13 +1250,12 @@ int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, c
     uint32_t *act_g = slot<uint32_t>(st, S_ACTG, z);
     uint32_t *act_x2 = slot<uint32_t>(st, S_ACTX2, z);
     uint32_t *act_g2 = slot<uint32_t>(st, S_ACTG2, z);
-    k_bucket_counts<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, occ, d, cnt_r);
+    k_bucket_counts<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, occ, stride, d, cnt_r);
     after_launch(st);
-    check_cuda(cudaMemsetAsync(st->d_scalars, 0, 8, st->stream));
     device_scan<uint64_t, OpAdd>(st, d, LoadBucket{cnt_r}, StoreBucket{bst}, false, (uint64_t *)st->d_scalars);
     check_cuda(cudaMemsetAsync(cur, 0, (size_t)d * 4, st->stream));
     uint2 *info = slot<uint2>(st, S_KEY0, d);
-    k_bucket_info<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, bst, occ, d, info);
+    k_bucket_info<<<grid_for(d, 256), 256, 0, st->stream>>>(lexrank, bst, occ, stride, d, info);
     after_launch(st);
     k_bucket_scatter<<<grid_for(z, 256), 256, 0, st->stream>>>(pid, info, z, cur, isa, sa, act_x, act_g, st->d_flags);
     after_launch(st);
@@ -1259,7 +1281,8 @@ void run_parse_sa(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &pord)
         pord.rounds = prefix_doubling(st, z, kp == 2 ? lb + bits_for(ph.d - 1) : bits_for(ph.d - 1), (uint32_t)kp,
                                       ParseRem{z}, pord.isa, pord.sa);
     } else {
-        pord.rounds = parse_sa_buckets(st, z, ph.d, ph.pid, dord.lexrank, ph.occ, pord.isa, pord.sa);
+        pord.rounds = parse_sa_buckets(st, z, ph.d, ph.pid, dord.lexrank, (const uint32_t *)ph.occpc, 2,
+                                       pord.isa, pord.sa);
     }
     pord.first = pord.isa;
 }
