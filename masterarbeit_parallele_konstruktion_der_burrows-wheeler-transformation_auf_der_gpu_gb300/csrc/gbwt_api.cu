@@ -105,11 +105,13 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
     stage_mark(st, 1);
 
     DictOrder dord;
+    st->round_words = 40;
     run_dict_sort(st, ph, W, small, dord);
     st->stats.dict_rounds = dord.rounds;
     stage_mark(st, 2);
 
     ParseOrder pord;
+    st->round_words = 42;
     run_parse_sa(st, ph, dord, pord);
     st->stats.parse_rounds = pord.rounds;
     stage_mark(st, 3);
@@ -136,11 +138,7 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
     run_assembly(st, dT, un, W, ph, dord, pord, dOut, un);
     stage_mark(st, 6);
     if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)n, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                               st->stream));
-    sync_stream(st);
-    uint32_t hflags[4];
-    memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
+    const uint32_t *hflags = read_flags(st);
     if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
     if (hflags[0] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
     st->stats.primary_index = hflags[2];

@@ -53,6 +53,7 @@ struct Storage {
     uint64_t *d_scalars = nullptr;      // device scalars (64 entries)
     uint32_t *h_meta = nullptr;         // pinned batch layout (grows on demand)
     size_t h_meta_cap = 0;
+    int round_words = 40;               // d_flags words of k_seg_rounds: rounds and elements (40 dictionary, 42 parse)
     uint32_t lb_seq = 0;                // number of the last look-back pass (status tags)
     uint32_t *h_err = nullptr;          // pinned: set by a kernel whose bounded wait gave up
     gbwt_tuning tuning = {};            // 0 = default for every knob
@@ -114,6 +115,20 @@ inline void fetch_scalars(Storage *st, int k)
     check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_scalars, (size_t)k * sizeof(uint64_t),
                                cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
+}
+
+// Waits for the end of a call: error bits, counters and the rounds that ran
+// without a read-back.  Returns the d_flags words.
+inline const uint32_t *read_flags(Storage *st)
+{
+    check_cuda(cudaMemcpyAsync(st->h_scalars + 160, st->d_flags, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                               st->stream));
+    sync_stream(st);
+    const uint32_t *f = (const uint32_t *)(st->h_scalars + 160);
+    st->stats.dict_rounds += f[40];
+    st->stats.parse_rounds += f[42];
+    if (st->probe_kernel == GBWT_PROBE_SEG_SORT) st->probe_bytes += (int64_t)24 * ((int64_t)f[41] + f[43]);
+    return f;
 }
 
 inline void after_launch(Storage *st)

@@ -502,11 +502,7 @@ static int64_t batch_end(Storage *st, uint8_t *L, const uint8_t *dOut, uint64_t 
 {
     stage_mark(st, 6);
     if (!devptr) check_cuda(cudaMemcpyAsync(L, dOut, (size_t)total, cudaMemcpyDeviceToHost, st->stream));
-    check_cuda(cudaMemcpyAsync(st->h_scalars + 8, st->d_flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                               st->stream));
-    sync_stream(st);
-    uint32_t hflags[4];
-    memcpy(hflags, st->h_scalars + 8, sizeof(hflags));
+    const uint32_t *hflags = read_flags(st);
     if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
     if (hflags[0] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
     if (st->stage_times) {
@@ -599,10 +595,12 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
 
     if (apart) {
         DictOrder dord;
+        st->round_words = 40;
         run_dict_sort(st, ph, W, small, dord);
         st->stats.dict_rounds = dord.rounds;
         stage_mark(st, 2);
         ParseOrder pord;
+        st->round_words = 42;
         run_parse_sa(st, ph, dord, pord);
         st->stats.parse_rounds = pord.rounds;
         stage_mark(st, 3);
@@ -617,6 +615,7 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     xstart = meta + bl.o_xstart;
     bt.xstart = xstart;
     DictOrder dord;
+    st->round_words = 40;
     run_dict_sort(st, ph, W, small, dord);
     st->stats.dict_rounds = dord.rounds;
     // byte codes of the dictionary's alphabet (pinned, written by the sort):
@@ -639,6 +638,7 @@ int64_t run_batch(Storage *st, const uint8_t *T, const int64_t *offsets, int32_t
     stage_mark(st, 2);
 
     ParseOrder pord;
+    st->round_words = 42;
     run_parse_sa_batch(st, ph, dord, bt, pord);
     st->stats.parse_rounds = pord.rounds;
     // text-major order of the parse suffix array (stable: each text keeps its order)

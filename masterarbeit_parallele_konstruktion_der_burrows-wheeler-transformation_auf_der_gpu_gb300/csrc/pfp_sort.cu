@@ -496,68 +496,49 @@ __global__ void k_round_gather(const uint32_t *act_x, const uint32_t *act_g, con
     if (threadIdx.x == 0 && s_first != 0xFFFFFFFFu) atomicMin(tstart + s_first / SS_TILE, s_first);
 }
 
+// The CTA's shared memory.
+struct SegMem {
+    uint64_t *key;       // (isa[x+h]+1) << 32 | local index
+    uint32_t *x;         // local index -> x
+    uint32_t *sg;        // segment -> group head g
+    uint32_t *ss;        // segment -> local start index
+    uint32_t *nh;        // group ids while loading, then sorted slot -> new head | done bit
+    uint32_t *misc;      // [2] warp counter, [3] big, [4] base, [5] warp groups
+    uint64_t *scan;
+    uint32_t *big;
+    uint16_t *seg;       // local index -> segment
+    uint16_t *perm;      // sorted slot -> local index
+    uint16_t *mid;       // segments above SS_COUNTMAX
+    uint2 *act;          // sorted active slots (x, new head); takes the keys' place
+    __device__ __forceinline__ explicit SegMem(unsigned char *p)
+    {
+        key = (uint64_t *)p;
+        x = (uint32_t *)(key + SS_CAP);
+        sg = x + SS_CAP;
+        ss = sg + SS_CAP;
+        nh = ss + SS_CAP;
+        misc = nh + SS_CAP;
+        scan = (uint64_t *)(misc + 8);
+        big = misc + 8 + 64;
+        seg = (uint16_t *)(misc + SS_MISC_WORDS);
+        perm = seg + SS_CAP;
+        mid = perm + SS_CAP;
+        act = (uint2 *)p;
+    }
+};
+
+// Sorts the groups of cnt loaded elements (key, x, nh = group id), writes ranks
+// and finished suffixes, and leaves the elements that stay active in m.act, in
+// slot order; returns their number.  With `counter` the number is added to it
+// and m.misc[4] gets the old value (after the caller's next barrier).
 template <typename Rem>
-__global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__restrict__ act_x,
-                                                            const uint32_t *__restrict__ act_g,
-                                                            const uint32_t *__restrict__ key2,
-                                                            const uint32_t *__restrict__ tstart,
-                                                            const uint32_t *__restrict__ tbig, uint32_t A_arg,
-                                                            const uint32_t *__restrict__ Ap, uint32_t h2, Rem rem, uint32_t *isa, uint32_t *sa,
-                                                            uint32_t *out_x, uint32_t *out_g, uint32_t *counter,
-                                                            uint32_t *flags, bool collect_stats)
+__device__ __forceinline__ uint32_t seg_sort_tile(const SegMem &m, uint32_t cnt, uint32_t h2, const Rem &rem,
+                                                  uint32_t *isa, uint32_t *sa, uint32_t *counter, uint32_t *flags,
+                                                  bool collect_stats)
 {
-    extern __shared__ __align__(16) unsigned char ss_smem[];
-    uint64_t *s_key = (uint64_t *)ss_smem;           // (isa[x+h]+1) << 32 | local index
-    uint32_t *s_x = (uint32_t *)(s_key + SS_CAP);    // local index -> x
-    uint32_t *s_sg = s_x + SS_CAP;                   // segment -> group head g
-    uint32_t *s_ss = s_sg + SS_CAP;                  // segment -> local start index
-    uint32_t *s_nh = s_ss + SS_CAP;                  // sorted slot -> new head | done bit
-    uint32_t *s_misc = s_nh + SS_CAP;                // [2] warp counter, [3] big, [4] base, [5] warp groups
-    uint64_t *s_scan = (uint64_t *)(s_misc + 8);
-    uint32_t *s_big = s_misc + 8 + 64;
-    uint16_t *s_seg = (uint16_t *)(s_misc + SS_MISC_WORDS);   // local index -> segment
-    uint16_t *s_perm = s_seg + SS_CAP;                        // sorted slot -> local index
-    uint16_t *s_mid = s_perm + SS_CAP;                        // segments above SS_COUNTMAX
-
-    // the CTA's elements: from the first group start in its tile to the
-    // first group start in the next tile (or A)
-    const uint32_t A = Ap ? *Ap : A_arg;             // from the device: the grid covers an upper bound
-    const uint32_t tiles = (A + SS_TILE - 1) / SS_TILE;
-    if (blockIdx.x >= tiles) return;
-    const uint32_t s0 = tstart[blockIdx.x];
-    if (s0 == 0xFFFFFFFFu) return;                   // no group starts in this tile
-    uint32_t e1;
-    const uint32_t bstart = tbig ? tbig[blockIdx.x] : 0xFFFFFFFFu;
-    if (bstart != 0xFFFFFFFFu) {
-        // a group too large for this path starts in this tile (at or after
-        // s0) and runs past it: the range ends there, the big-group path
-        // sorts it
-        e1 = bstart;
-    } else {
-        e1 = blockIdx.x + 1 < tiles ? tstart[blockIdx.x + 1] : A;
-        if (e1 == 0xFFFFFFFFu) {
-            // only the last tile, partly filled, may lack a start
-            if (blockIdx.x + 2 < tiles) { if (threadIdx.x == 0) atomicOr(flags, ERR_INTERNAL); return; }
-            e1 = A;
-        }
-    }
-    const uint32_t cnt = e1 - s0;
-    if (cnt == 0) return;
-    if (cnt > (uint32_t)SS_CAP) { if (threadIdx.x == 0) atomicOr(flags, ERR_INTERNAL); return; }
-
-    // coalesced loads into shared memory (s_nh holds the group ids for now)
-#pragma unroll
-    for (int j = 0; j < SS_PER_THREAD; j++) {
-        const uint32_t i = (uint32_t)j * SS_THREADS + threadIdx.x;
-        if (i < cnt) {
-            const uint32_t a = s0 + i;
-            // unique key: (isa[x+h]+1, local index) -- stable, deterministic
-            s_key[i] = ((uint64_t)key2[a] << 32) | i;
-            s_x[i] = act_x[a];
-            s_nh[i] = act_g[a];
-        }
-    }
-    __syncthreads();
+    uint64_t *s_key = m.key, *s_scan = m.scan;
+    uint32_t *s_x = m.x, *s_sg = m.sg, *s_ss = m.ss, *s_nh = m.nh, *s_misc = m.misc, *s_big = m.big;
+    uint16_t *s_seg = m.seg, *s_perm = m.perm, *s_mid = m.mid;
     // segments in element order, warp-striped: warp w owns local indices
     // [w*256, w*256+256) as 8 rows of 32 lanes (ballots give the order
     // inside a row; consecutive lanes touch consecutive banks)
@@ -631,8 +612,8 @@ __global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__re
         const uint64_t kk = s_key[i];
         const uint32_t k2 = (uint32_t)(kk >> 32);
         uint32_t lt = 0, eq = 0, pos = 0;
-        for (uint32_t m = ss; m < se; m++) {
-            const uint64_t o = s_key[m];
+        for (uint32_t e = ss; e < se; e++) {
+            const uint64_t o = s_key[e];
             const uint32_t o2 = (uint32_t)(o >> 32);
             lt += o2 < k2;
             eq += o2 == k2;
@@ -647,11 +628,11 @@ __global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__re
     // ones up to SS_WARPMAX, and derive the new heads of all of them.
     const uint32_t nmid = s_misc[5];
     for (;;) {
-        uint32_t m = 0;
-        if (lane == 0) m = atomicAdd(&s_misc[2], 1u);
-        m = __shfl_sync(0xFFFFFFFFu, m, 0);
-        if (m >= nmid) break;
-        const uint32_t sg = s_mid[m];
+        uint32_t next = 0;
+        if (lane == 0) next = atomicAdd(&s_misc[2], 1u);
+        next = __shfl_sync(0xFFFFFFFFu, next, 0);
+        if (next >= nmid) break;
+        const uint32_t sg = s_mid[next];
         const uint32_t ss = s_ss[sg], se = s_ss[sg + 1], s = se - ss;
         const uint32_t g = s_sg[sg];
         // (groups above SS_WARPMAX were sorted by the CTA above; warp_group
@@ -676,18 +657,16 @@ __global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__re
     uint32_t apre = (uint32_t)block_excl_scan<uint64_t, OpAdd>(lane == 0 ? (uint64_t)wact : 0ull, atot, OpAdd(),
                                                               s_scan);
     apre = __shfl_sync(0xFFFFFFFFu, apre, 0);
-    if (threadIdx.x == 0) s_misc[4] = atot ? atomicAdd(counter, (uint32_t)atot) : 0u;
+    if (counter && threadIdx.x == 0) s_misc[4] = atot ? atomicAdd(counter, (uint32_t)atot) : 0u;
     // active slots (x, new head) staged in slot order; the keys are dead
-    uint2 *s_act = (uint2 *)s_key;
+    uint2 *s_act = m.act;
 #pragma unroll
     for (int j = 0; j < SS_PER_THREAD; j++) {
         const uint32_t p = wb + (uint32_t)j * 32u + lane;
         if ((actm[j] >> lane) & 1u) s_act[apre + (uint32_t)__popc(actm[j] & lt)] = make_uint2(s_x[s_perm[p]], s_nh[p]);
         apre += (uint32_t)__popc(actm[j]);
     }
-    __syncthreads();
-    const uint32_t base = s_misc[4];
-    // striped: ranks, finished suffixes, next active list
+    // striped: ranks, finished suffixes
     for (uint32_t p = threadIdx.x; p < cnt; p += SS_THREADS) {
         const uint32_t v = s_nh[p];
         const uint32_t nh = v & 0x7FFFFFFFu;
@@ -698,11 +677,125 @@ __global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__re
         if (nh != s_sg[sg]) isa[x] = nh;
         if (v >> 31) sa[s_sg[sg] + (p - s_ss[sg])] = x;
     }
-    for (uint32_t k = threadIdx.x; k < (uint32_t)atot; k += SS_THREADS) {
-        const uint2 e = s_act[k];
+    return (uint32_t)atot;
+}
+
+template <typename Rem>
+__global__ void __launch_bounds__(SS_THREADS, 2) k_seg_sort(const uint32_t *__restrict__ act_x,
+                                                            const uint32_t *__restrict__ act_g,
+                                                            const uint32_t *__restrict__ key2,
+                                                            const uint32_t *__restrict__ tstart,
+                                                            const uint32_t *__restrict__ tbig, uint32_t A_arg,
+                                                            const uint32_t *__restrict__ Ap, uint32_t h2, Rem rem, uint32_t *isa, uint32_t *sa,
+                                                            uint32_t *out_x, uint32_t *out_g, uint32_t *counter,
+                                                            uint32_t *flags, bool collect_stats)
+{
+    extern __shared__ __align__(16) unsigned char ss_smem[];
+    const SegMem m(ss_smem);
+
+    // the CTA's elements: from the first group start in its tile to the
+    // first group start in the next tile (or A)
+    const uint32_t A = Ap ? *Ap : A_arg;             // from the device: the grid covers an upper bound
+    const uint32_t tiles = (A + SS_TILE - 1) / SS_TILE;
+    if (blockIdx.x >= tiles) return;
+    const uint32_t s0 = tstart[blockIdx.x];
+    if (s0 == 0xFFFFFFFFu) return;                   // no group starts in this tile
+    uint32_t e1;
+    const uint32_t bstart = tbig ? tbig[blockIdx.x] : 0xFFFFFFFFu;
+    if (bstart != 0xFFFFFFFFu) {
+        // a group too large for this path starts in this tile (at or after
+        // s0) and runs past it: the range ends there, the big-group path
+        // sorts it
+        e1 = bstart;
+    } else {
+        e1 = blockIdx.x + 1 < tiles ? tstart[blockIdx.x + 1] : A;
+        if (e1 == 0xFFFFFFFFu) {
+            // only the last tile, partly filled, may lack a start
+            if (blockIdx.x + 2 < tiles) { if (threadIdx.x == 0) atomicOr(flags, ERR_INTERNAL); return; }
+            e1 = A;
+        }
+    }
+    const uint32_t cnt = e1 - s0;
+    if (cnt == 0) return;
+    if (cnt > (uint32_t)SS_CAP) { if (threadIdx.x == 0) atomicOr(flags, ERR_INTERNAL); return; }
+
+    // coalesced loads into shared memory (m.nh holds the group ids for now)
+#pragma unroll
+    for (int j = 0; j < SS_PER_THREAD; j++) {
+        const uint32_t i = (uint32_t)j * SS_THREADS + threadIdx.x;
+        if (i < cnt) {
+            const uint32_t a = s0 + i;
+            // unique key: (isa[x+h]+1, local index) -- stable, deterministic
+            m.key[i] = ((uint64_t)key2[a] << 32) | i;
+            m.x[i] = act_x[a];
+            m.nh[i] = act_g[a];
+        }
+    }
+    __syncthreads();
+    const uint32_t atot = seg_sort_tile<Rem>(m, cnt, h2, rem, isa, sa, counter, flags, collect_stats);
+    __syncthreads();
+    const uint32_t base = m.misc[4];
+    for (uint32_t k = threadIdx.x; k < atot; k += SS_THREADS) {
+        const uint2 e = m.act[k];
         out_x[base + k] = e.x;
         out_g[base + k] = e.y;
     }
+}
+
+// All remaining rounds of at most SS_CAP active elements in one CTA: their
+// keys are gathered, sorted and written between barriers, the active list
+// stays in shared memory.  A round of few elements is two launches of about
+// seven microseconds each plus the host's reads of the count (24 KiB DNA text:
+// twelve rounds of its two sorts, 506 -> 392 us for the call).
+template <typename Rem>
+__global__ void __launch_bounds__(SS_THREADS, 1) k_seg_rounds(const uint32_t *__restrict__ act_x,
+                                                              const uint32_t *__restrict__ act_g, uint32_t A, uint32_t N,
+                                                              uint64_t h, Rem rem, uint32_t *isa, uint32_t *sa,
+                                                              int max_rounds, uint32_t *counts, uint32_t *flags)
+{
+    extern __shared__ __align__(16) unsigned char ss_smem[];
+    const SegMem m(ss_smem);
+    uint2 e[SS_PER_THREAD];
+#pragma unroll
+    for (int j = 0; j < SS_PER_THREAD; j++) {
+        const uint32_t i = (uint32_t)j * SS_THREADS + threadIdx.x;
+        if (i < A) e[j] = make_uint2(act_x[i], act_g[i]);
+    }
+    uint32_t elems = 0;                   // active elements of all rounds
+    for (int r = 0; r < max_rounds; r++) {
+        if (A == 0) {
+            if (threadIdx.x == 0) {
+                counts[0] += (uint32_t)r;
+                counts[1] += elems;
+            }
+            return;
+        }
+        elems += A;
+        if (h >= N) break;                // only legal when every suffix is finished already
+        const uint32_t h2 = (uint32_t)(2 * h < 0xFFFFFFFFull ? 2 * h : 0xFFFFFFFFull);
+        // ranks are read before any of this round's writes (plain loads: the
+        // CTA sees its own earlier writes)
+#pragma unroll
+        for (int j = 0; j < SS_PER_THREAD; j++) {
+            const uint32_t i = (uint32_t)j * SS_THREADS + threadIdx.x;
+            if (i < A) {
+                m.key[i] = ((uint64_t)(*(volatile uint32_t *)(isa + e[j].x + h) + 1u) << 32) | i;
+                m.x[i] = e[j].x;
+                m.nh[i] = e[j].y;
+            }
+        }
+        __syncthreads();
+        A = seg_sort_tile<Rem>(m, A, h2, rem, isa, sa, nullptr, flags, false);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SS_PER_THREAD; j++) {
+            const uint32_t i = (uint32_t)j * SS_THREADS + threadIdx.x;
+            if (i < A) e[j] = m.act[i];
+        }
+        __syncthreads();
+        h *= 2;
+    }
+    if (threadIdx.x == 0) atomicOr(flags, ERR_INTERNAL);
 }
 
 __global__ void k_big_heads(const uint32_t *act_g, const uint32_t *bstart, uint32_t nbig, uint32_t *bhead)
@@ -840,6 +933,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
     static bool ss_attr = false;
     if (!ss_attr) {
         check_cuda(cudaFuncSetAttribute(k_seg_sort<Rem>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS_SMEM));
+        check_cuda(cudaFuncSetAttribute(k_seg_rounds<Rem>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS_SMEM));
         ss_attr = true;
     }
     const bool debug = getenv("GBWT_DEBUG") != nullptr;
@@ -869,6 +963,17 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
             if (exact) throw Error{GBWT_INTERNAL_ERROR};
             read_back();
             if (hw[(r + 1) & 1] != 0) throw Error{GBWT_INTERNAL_ERROR};
+            break;
+        }
+        if (exact && A_ub <= (uint32_t)SS_CAP && !debug) {
+            // the rest in one CTA; nobody waits for it: its round count comes
+            // with the call's last read-back
+            probe_begin(st, GBWT_PROBE_SEG_SORT);
+            k_seg_rounds<Rem><<<1, SS_THREADS, SS_SMEM, st->stream>>>(act_x, act_g, A_ub, N, h, rem, isa, sa,
+                                                                      DR_MAXR - r, st->d_flags + st->round_words,
+                                                                      st->d_flags);
+            probe_end(st, GBWT_PROBE_SEG_SORT, 0);
+            after_launch(st);
             break;
         }
         const uint32_t h2 = (uint32_t)(2 * h < 0xFFFFFFFFull ? 2 * h : 0xFFFFFFFFull);
@@ -934,7 +1039,7 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
         }
     }
     // rounds that had work, and the probe's algorithmic bytes per round (the
-    // loop ends on a read-back)
+    // last read-back has the counts of all rounds so far)
     int rounds = 0;
     for (int i = 0; i < r; i++) {
         const uint32_t a = hw[8 + i];
