@@ -228,7 +228,8 @@ typedef struct gbwt_tuning {
     int32_t batch_radix_bits;   /* batch output sort digit width: 8, 9, or 0 = fewest passes         */
     int32_t unbwt_rate_log2;    /* inverse BWT: one row in 2^k is a ruler (2..12; default 5)           */
     int32_t dict_key_bits;      /* dictionary sort, first key: at most this many bits of recoded
-                                   symbols (8..64; default 64: as many symbols as fit)             */
+                                   symbols (8..64; default 40, or 64 = as many as fit where phrases
+                                   average 64 bytes and more)                                       */
     int32_t parse_key_phrases;  /* parse suffix array, first round: 1 or 2 phrase ranks sorted by
                                    radix; 0 (default): a large repetitive text's parse is parsed
                                    again and sorted at that level; else the first round comes

@@ -173,7 +173,6 @@ inline int tune_hash_log2(const Storage *st) { return st->tuning.hash_log2_max ?
 inline int tune_seg_tiles(const Storage *st) { return st->tuning.batch_seg_tiles ? st->tuning.batch_seg_tiles : 8; }
 inline int tune_pad_eighths(const Storage *st) { return st->tuning.batch_pad_eighths ? st->tuning.batch_pad_eighths : 1; }
 inline int tune_unbwt_rate_log2(const Storage *st) { return st->tuning.unbwt_rate_log2 ? st->tuning.unbwt_rate_log2 : 5; }
-inline int tune_dict_key_bits(const Storage *st) { return st->tuning.dict_key_bits ? st->tuning.dict_key_bits : 64; }
 // 0 (default): single-text parses are parsed again when large and repetitive,
 // else round 0 comes from the phrase buckets, no sort (the batch parse then
 // sorts two phrase ranks); 1 or 2: a radix sort of the first one or two phrase

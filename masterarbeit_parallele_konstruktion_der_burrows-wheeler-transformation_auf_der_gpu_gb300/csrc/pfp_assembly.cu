@@ -520,7 +520,7 @@ void run_assembly(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph
                                  (uint32_t *)st->d_scalars);
     // a mixed block has at least two bytes
     uint32_t *delta = slot<uint32_t>(st, S_DELTA, (size_t)(N < n_out / 2 ? N : n_out / 2) + 1);
-    device_scan<Sum4, OpAdd>(st, nw, LoadMixWord{stat, heads, mixed}, StoreMixWord{stat, mixed, delta}, false,
+    device_scan<Sum4, OpAdd, 1>(st, nw, LoadMixWord{stat, heads, mixed}, StoreMixWord{stat, mixed, delta}, false,
                              (Sum4 *)(st->d_scalars + 1));
     fetch_scalars(st, 3);
     const uint32_t total = (uint32_t)st->h_scalars[0], M = (uint32_t)st->h_scalars[1];

@@ -345,12 +345,13 @@ struct StoreArr {
 // items per thread, so that they spread over the SMs instead of running as
 // one long chain of dependent loads; larger ones take as many as fit about 32
 // KB of shared memory: fewer tiles for a prefix to travel over (130 M 32-bit
-// items in 314 us with 32 per thread, 367 us with 16).
-template <typename T, typename Op, typename Load, typename Store>
+// items in 314 us with 32 per thread, 367 us with 16).  SMALL = 1 is for loads that
+// loop themselves.
+template <typename T, typename Op, int SMALL = 4, typename Load, typename Store>
 void device_scan(Storage *st, size_t n, Load load, Store store, bool inclusive, T *total_dev)
 {
     if (n == 0) return;
-    constexpr int BIG = sizeof(T) == 4 ? 32 : sizeof(T) == 8 ? 16 : 8, SMALL = 4;
+    constexpr int BIG = sizeof(T) == 4 ? 32 : sizeof(T) == 8 ? 16 : 8;
     const bool small = n <= (size_t)st->num_sms * 8 * SC_THREADS * SMALL;
     const size_t per = (size_t)SC_THREADS * (small ? SMALL : BIG);
     const size_t tiles = (n + per - 1) / per;
@@ -477,15 +478,13 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *__restrict__
     }
 }
 
-// Digit counts of all `np` passes: hist[(p * nseg + segment) * D + digit].  A
-// CTA counts RH_TILES consecutive tiles at a time in shared memory (several
-// copies: the digits of a small alphabet repeat) and adds to the global counts
-// when the segment changes and at its end.
-constexpr int RH_TILES = 8;
+// Digit counts of all passes of a sort of few tiles, one CTA per tile (eight
+// tiles a CTA took 24 us for the 168 tiles of an 8 MiB text's dictionary, one 12
+// us): hist[(p * nseg + segment) * D + digit], added up from shared memory
+// (several copies: the digits of a small alphabet repeat).
 template <typename K, int BITS>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K *__restrict__ keys, uint32_t n, int begin_bit,
-                                                        int end_bit, RsSegs sg, uint32_t num_tiles,
-                                                        uint32_t *__restrict__ hist)
+                                                        int end_bit, RsSegs sg, uint32_t *__restrict__ hist)
 {
     constexpr int D = 1 << BITS;
     constexpr int PMAX = ((int)sizeof(K) * 8 + BITS - 1) / BITS;
@@ -493,64 +492,30 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K *__restrict__ ke
     constexpr int COPIES = FIT >= 4 ? 4 : FIT >= 2 ? 2 : 1;
     __shared__ uint32_t h[COPIES * PMAX * D];
     const int np = (end_bit - begin_bit + BITS - 1) / BITS;
-    for (int i = threadIdx.x; i < COPIES * PMAX * D; i += RS_THREADS) h[i] = 0;
+    for (int c = 0; c < COPIES; c++)
+        for (int i = threadIdx.x; i < np * D; i += RS_THREADS) h[c * (PMAX * D) + i] = 0;
     __syncthreads();
     uint32_t *mine = h + ((threadIdx.x >> 5) % COPIES) * (PMAX * D);
-    const uint32_t chunks = (num_tiles + RH_TILES - 1) / RH_TILES;
-    uint32_t cur = 0xFFFFFFFFu;               // segment whose counts are in shared memory
-    auto flush = [&]() {
-        __syncthreads();
-        for (int i = threadIdx.x; i < np * D; i += RS_THREADS) {
-            uint32_t c = 0;
+    const uint32_t base = blockIdx.x * (uint32_t)RS_TILE;
 #pragma unroll
-            for (int k = 0; k < COPIES; k++) {
-                c += h[k * (PMAX * D) + i];
-                h[k * (PMAX * D) + i] = 0;
-            }
-            const uint32_t pass = (uint32_t)i / D, d = (uint32_t)i % D;
-            if (c) atomicAdd(hist + ((size_t)pass * sg.nseg + cur) * D + d, c);
-        }
-        __syncthreads();
-    };
-    auto count = [&](K k) {
+    for (int j = 0; j < RS_ITEMS; j++) {
+        const uint32_t i = base + (uint32_t)j * RS_THREADS + threadIdx.x;
+        if (i >= n) break;
+        const K k = keys[i];
         for (int p = 0; p < np; p++) {
             const int shift = begin_bit + p * BITS;
             const int bits = end_bit - shift < BITS ? end_bit - shift : BITS;
             atomicAdd(&mine[p * D + rs_digit(k, shift, (1u << bits) - 1u)], 1u);
         }
-    };
-    constexpr int KPV = 16 / (int)sizeof(K);          // keys per 16-byte load
-    constexpr int NV = RS_ITEMS / KPV;
-    const bool aligned = (((uintptr_t)keys) & 15u) == 0;
-    for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-        for (uint32_t b = c * RH_TILES; b < num_tiles && b < (c + 1) * RH_TILES; b++) {
-            const uint32_t s = sg.sid ? sg.sid[b] : 0u;
-            if (s != cur) {
-                if (cur != 0xFFFFFFFFu) flush();
-                cur = s;
-            }
-            const size_t base = (size_t)b * RS_TILE;
-            if (aligned && base + RS_TILE <= n) {
-                uint4 v[NV];
-#pragma unroll
-                for (int j = 0; j < NV; j++)
-                    v[j] = __ldg((const uint4 *)(keys + base) + (size_t)j * RS_THREADS + threadIdx.x);
-#pragma unroll
-                for (int j = 0; j < NV; j++) {
-                    K kk[KPV];
-                    memcpy(kk, &v[j], 16);
-#pragma unroll
-                    for (int q = 0; q < KPV; q++) count(kk[q]);
-                }
-            } else {
-                for (int j = 0; j < RS_ITEMS; j++) {
-                    const size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
-                    if (i < n) count(keys[i]);
-                }
-            }
-        }
     }
-    if (cur != 0xFFFFFFFFu) flush();
+    __syncthreads();
+    const uint32_t seg = sg.sid ? sg.sid[blockIdx.x] : 0u;
+    for (int i = threadIdx.x; i < np * D; i += RS_THREADS) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < COPIES; k++) c += h[k * (PMAX * D) + i];
+        if (c) atomicAdd(hist + ((size_t)(i / D) * sg.nseg + seg) * D + i % D, c);
+    }
 }
 
 template <typename K, bool HAS_VAL, int BITS>
@@ -853,9 +818,7 @@ void radix_sort(Storage *st, K *&keys, K *&keys_alt, uint32_t *&vals, uint32_t *
         const size_t words = (size_t)np * sg.nseg * D;
         hist = slot<uint32_t>(st, S_RSHIST, words);
         check_cuda(cudaMemsetAsync(hist, 0, words * sizeof(uint32_t), st->stream));
-        unsigned grid = grid_for(num_tiles, RH_TILES);
-        if (grid > (unsigned)st->num_sms * 6) grid = (unsigned)st->num_sms * 6;
-        k_rs_hist<K, BITS><<<grid, RS_THREADS, 0, st->stream>>>(keys, n, begin_bit, end_bit, sg, num_tiles, hist);
+        k_rs_hist<K, BITS><<<num_tiles, RS_THREADS, 0, st->stream>>>(keys, n, begin_bit, end_bit, sg, hist);
         after_launch(st);
     }
     for (int p = 0; p < np; p++) {
