@@ -168,6 +168,12 @@ __device__ __forceinline__ uint64_t lb_load(const uint64_t *p)
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t lb_load32(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 template <typename T>
 __device__ __forceinline__ void lb_publish(const LookBack &lb, uint32_t tile, T v, uint32_t state)
 {
@@ -525,13 +531,21 @@ constexpr size_t rs_smem_bytes()
            (size_t)(1 << BITS) * 4 * 2 + 32 * 8;
 }
 
-// Scatter of one pass, places from the scanned tile histograms.
+// Scatter of one pass, places from the scanned tile histograms.  The time of a
+// tile is a chain of latencies (three or two CTAs an SM, DRAM and issue slots
+// half idle), so the chain is kept short: the tile's offsets (num_tiles words
+// apart) and all keys are in flight before the first barrier, every warp
+// clears its own counters, a digit's start in the tile is folded into the
+// counters and into its offset (one shared read per key less in both places).
+// Passes of 512 MiB DNA: 243 M 32-bit keys 740 -> 542 us (offsets loaded after
+// ranking and one barrier more: 667; offsets early: 604), 34 M 32-bit keys with
+// values 204 -> 178 us, 26 M 64-bit keys with values 136 -> 111 us.  Three CTAs
+// of 32-bit keys fit in 80 registers, more or wider keys would spill.
 template <typename K, bool HAS_VAL, int BITS, int BALLOT>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict__ kin, K *__restrict__ kout,
-                                                             const uint32_t *__restrict__ vin,
-                                                             uint32_t *__restrict__ vout, uint32_t n, int shift,
-                                                             uint32_t mask, const uint32_t *__restrict__ tile_off,
-                                                             uint32_t num_tiles, RsSegs sg)
+__global__ void __launch_bounds__(RS_THREADS, sizeof(K) == 4 && !HAS_VAL ? 3 : 2)
+k_rs_downsweep(const K *__restrict__ kin, K *__restrict__ kout, const uint32_t *__restrict__ vin,
+               uint32_t *__restrict__ vout, uint32_t n, int shift, uint32_t mask,
+               const uint32_t *__restrict__ tile_off, uint32_t num_tiles, RsSegs sg)
 {
     constexpr int D = 1 << BITS;
     constexpr int DPT = D / RS_THREADS;       // digits per thread in the per-digit phase
@@ -539,14 +553,14 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
     K *s_k = (K *)rs_smem;
     uint32_t *s_v = (uint32_t *)(s_k + RS_TILE);
     uint32_t *s_wh = HAS_VAL ? s_v + RS_TILE : s_v;
-    uint32_t *s_dstart = s_wh + RS_WARPS * D;
-    uint32_t *s_goff = s_dstart + D;
+    uint32_t *s_goff = s_wh + RS_WARPS * D;
     uint32_t *s_scan = s_goff + D;
 
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < RS_WARPS * D; i += RS_THREADS) s_wh[i] = 0;
-    __syncthreads();
-
+    uint32_t off[DPT];                        // loaded early: num_tiles words apart
+#pragma unroll
+    for (int e = 0; e < DPT; e++)
+        off[e] = tile_off[rs_hist_index(sg, blockIdx.x, threadIdx.x * DPT + e, num_tiles, D)];
     const size_t tile_base = (size_t)blockIdx.x * RS_TILE;
     const size_t wbase = tile_base + (size_t)warp * (RS_ITEMS * 32);
     K k[RS_ITEMS];
@@ -562,22 +576,21 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
         dg[i] = valid ? rs_digit(k[i], shift, mask) : 0xFFFFFFFFu;
     }
     uint32_t *wh = s_wh + warp * D;
+    for (int i = lane; i < D; i += 32) wh[i] = 0;
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < RS_ITEMS; i++) {
-        // the lowest lane of each digit class reads and advances the warp's
-        // counter; the others take the old value from it
+        // every lane reads its digit's counter (one bank access per digit, as
+        // for one lane), then the lowest lane of the class advances it
         const uint32_t d = dg[i];
         const unsigned peers = (BALLOT > 0 && i % (BALLOT > 0 ? BALLOT : 1) == (BALLOT > 0 ? BALLOT - 1 : 0))
                                    ? rs_peers_ballot<BITS>(d)
                                    : __match_any_sync(0xFFFFFFFFu, d);
-        const unsigned leader = (unsigned)(__ffs(peers) - 1);
-        uint32_t prior = 0;
-        if (lane == leader && d != 0xFFFFFFFFu) {
-            prior = wh[d];
-            wh[d] = prior + (uint32_t)__popc(peers);
-        }
-        prior = __shfl_sync(0xFFFFFFFFu, prior, leader);
-        rk[i] = prior + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        const uint32_t below = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        const uint32_t prior = d != 0xFFFFFFFFu ? wh[d] : 0u;
+        __syncwarp();
+        if (below == 0 && d != 0xFFFFFFFFu) wh[d] = prior + (uint32_t)__popc(peers);
+        rk[i] = prior + below;
         __syncwarp();
     }
     __syncthreads();
@@ -590,11 +603,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
             const uint32_t d = threadIdx.x * DPT + e;
             uint32_t run = 0;
 #pragma unroll
-            for (int w = 0; w < RS_WARPS; w++) {
-                uint32_t c = s_wh[w * D + d];
-                s_wh[w * D + d] = run;
-                run += c;
-            }
+            for (int w = 0; w < RS_WARPS; w++) run += s_wh[w * D + d];
             cnt[e] = run;
             sum += run;
         }
@@ -603,16 +612,22 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
 #pragma unroll
         for (int e = 0; e < DPT; e++) {
             const uint32_t d = threadIdx.x * DPT + e;
-            s_dstart[d] = ex;
+            s_goff[d] = off[e] - ex;
+            uint32_t run = ex;
+#pragma unroll
+            for (int w = 0; w < RS_WARPS; w++) {
+                const uint32_t c = s_wh[w * D + d];
+                s_wh[w * D + d] = run;
+                run += c;
+            }
             ex += cnt[e];
-            s_goff[d] = tile_off[rs_hist_index(sg, blockIdx.x, d, num_tiles, D)];
         }
     }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RS_ITEMS; i++) {
         if (dg[i] != 0xFFFFFFFFu) {
-            uint32_t lp = s_dstart[dg[i]] + s_wh[warp * D + dg[i]] + rk[i];
+            uint32_t lp = wh[dg[i]] + rk[i];
             s_k[lp] = k[i];
             if (HAS_VAL) s_v[lp] = v[i];
         }
@@ -622,7 +637,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
     for (uint32_t j = threadIdx.x; j < tile_n; j += RS_THREADS) {
         K kk = s_k[j];
         uint32_t d = rs_digit(kk, shift, mask);
-        size_t g = (size_t)s_goff[d] + (j - s_dstart[d]);
+        size_t g = (size_t)(uint32_t)(s_goff[d] + j);
         kout[g] = kk;
         if (HAS_VAL) vout[g] = s_v[j];
     }
@@ -634,11 +649,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const K *__restrict
 // memory, so most predecessors have theirs in place when the look-back
 // starts.  A single tile needs neither counts nor look-back.
 template <typename K, bool HAS_VAL, int BITS, int BALLOT>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ kin, K *__restrict__ kout,
-                                                        const uint32_t *__restrict__ vin,
-                                                        uint32_t *__restrict__ vout, uint32_t n, int shift,
-                                                        uint32_t mask, const uint32_t *__restrict__ hist, RsSegs sg,
-                                                        LookBack lb)
+__global__ void __launch_bounds__(RS_THREADS, 2)
+k_rs_pass(const K *__restrict__ kin, K *__restrict__ kout, const uint32_t *__restrict__ vin,
+          uint32_t *__restrict__ vout, uint32_t n, int shift, uint32_t mask, const uint32_t *hist, RsSegs sg,
+          LookBack lb)
 {
     constexpr int D = 1 << BITS;
     constexpr int DPT = D / RS_THREADS;       // digits per thread in the per-digit phases
@@ -657,9 +671,20 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ ki
         if (tile == gridDim.x - 1) *lb.ticket = 0;
         s_dstart[0] = tile;
     }
-    for (int i = threadIdx.x; i < RS_WARPS * D; i += RS_THREADS) s_wh[i] = 0;
+    uint32_t *wh = s_wh + warp * D;
+    for (int i = lane; i < D; i += 32) wh[i] = 0;
     __syncthreads();
     if (gridDim.x > 1) tile = s_dstart[0];
+    // Tiles of the segment (first, count) and its digit counts, loaded early.
+    // The counts are read in program order on purpose: through a `const
+    // __restrict__` pointer the compiled kernel summed other digits' counts in
+    // some instances (9-bit digits, two tiles), and with plain loads in none.
+    uint2 q = make_uint2(0u, gridDim.x);
+    uint32_t seg = 0;
+    if (sg.tseg) { q = sg.tseg[tile]; seg = sg.sid[tile]; }
+    uint32_t hd[DPT];
+#pragma unroll
+    for (int e = 0; e < DPT; e++) hd[e] = q.y > 1 ? lb_load32(hist + (size_t)seg * D + threadIdx.x * DPT + e) : 0u;
 
     const size_t tile_base = (size_t)tile * RS_TILE;
     const size_t wbase = tile_base + (size_t)warp * (RS_ITEMS * 32);
@@ -675,31 +700,22 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ ki
         if (HAS_VAL) v[i] = !vin ? (uint32_t)idx : valid ? vin[idx] : 0u;
         dg[i] = valid ? rs_digit(k[i], shift, mask) : 0xFFFFFFFFu;
     }
-    uint32_t *wh = s_wh + warp * D;
 #pragma unroll
     for (int i = 0; i < RS_ITEMS; i++) {
-        // the lowest lane of each digit class reads and advances the warp's
-        // counter; the others take the old value from it
-        const uint32_t d = dg[i];
+        const uint32_t d = dg[i];           // ranked as in k_rs_downsweep
         const unsigned peers = (BALLOT > 0 && i % (BALLOT > 0 ? BALLOT : 1) == (BALLOT > 0 ? BALLOT - 1 : 0))
                                    ? rs_peers_ballot<BITS>(d)
                                    : __match_any_sync(0xFFFFFFFFu, d);
-        const unsigned leader = (unsigned)(__ffs(peers) - 1);
-        uint32_t prior = 0;
-        if (lane == leader && d != 0xFFFFFFFFu) {
-            prior = wh[d];
-            wh[d] = prior + (uint32_t)__popc(peers);
-        }
-        prior = __shfl_sync(0xFFFFFFFFu, prior, leader);
-        rk[i] = prior + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        const uint32_t below = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        const uint32_t prior = d != 0xFFFFFFFFu ? wh[d] : 0u;
+        __syncwarp();
+        if (below == 0 && d != 0xFFFFFFFFu) wh[d] = prior + (uint32_t)__popc(peers);
+        rk[i] = prior + below;
         __syncwarp();
     }
     __syncthreads();
     // thread t owns digits [t*DPT, t*DPT + DPT): the tile's counts (low words)
     // and the segment's (high words) scanned together
-    uint2 q = make_uint2(0u, gridDim.x);
-    uint32_t seg = 0;
-    if (sg.tseg) { q = sg.tseg[tile]; seg = sg.sid[tile]; }
     uint32_t cnt[DPT], gbase[DPT];
     {
         uint64_t both[DPT], sum = 0;
@@ -717,7 +733,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ ki
             if (q.y > 1) {
                 lb_store(lb.status + (size_t)tile * D + d,
                          ((uint64_t)((lb.seq << 2) | (tile == q.x ? LB_PREFIX : LB_TOTAL)) << 32) | run);
-                both[e] = ((uint64_t)hist[(size_t)seg * D + d] << 32) | run;
+                both[e] = ((uint64_t)hd[e] << 32) | run;
             } else {
                 both[e] = ((uint64_t)run << 32) | run;       // alone in its segment
             }
@@ -736,7 +752,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ ki
 #pragma unroll
     for (int i = 0; i < RS_ITEMS; i++) {
         if (dg[i] != 0xFFFFFFFFu) {
-            uint32_t lp = s_dstart[dg[i]] + s_wh[warp * D + dg[i]] + rk[i];
+            uint32_t lp = s_dstart[dg[i]] + wh[dg[i]] + rk[i];
             s_k[lp] = k[i];
             if (HAS_VAL) s_v[lp] = v[i];
         }
@@ -746,18 +762,31 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const K *__restrict__ ki
         const uint32_t d = threadIdx.x * DPT + e;
         uint32_t pre = 0;
         if (tile != q.x) {
+            // four predecessors a step: all tiles run at once, and the last ones
+            // walk far before a prefix meets them (168 tiles, 64-bit keys with
+            // values: 15.0 -> 14.4 us a pass with the early loads)
             uint32_t p = tile, polls = 0;
-            for (;;) {
-                const uint64_t w = lb_load(lb.status + (size_t)(p - 1u) * D + d);
-                const uint32_t tag = (uint32_t)(w >> 32);
-                if ((tag >> 2) != lb.seq) {
-                    // never runs out (tickets, see above); places only shrink, the host refuses the result
-                    if (++polls >= LB_MAX_POLLS) { *(volatile uint32_t *)lb.err = 1u; break; }
-                    continue;
+            bool found = false;
+            while (!found) {
+                uint64_t w[4];
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++)
+                    w[j] = j < p - q.x ? lb_load(lb.status + (size_t)(p - 1u - j) * D + d) : 0u;
+                const uint32_t from = p;
+                bool go = true;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++) {
+                    const uint32_t tag = (uint32_t)(w[j] >> 32);
+                    go = go && (tag >> 2) == lb.seq;
+                    if (go) {
+                        pre += (uint32_t)w[j];
+                        p--;
+                        found = (tag & 3u) == LB_PREFIX;
+                        go = !found;
+                    }
                 }
-                pre += (uint32_t)w;
-                p--;
-                if ((tag & 3u) == LB_PREFIX) break;
+                // never runs out (tickets, see above); places only shrink, the host refuses the result
+                if (p == from && ++polls >= LB_MAX_POLLS) { *(volatile uint32_t *)lb.err = 1u; break; }
             }
             lb_store(lb.status + (size_t)tile * D + d,
                      ((uint64_t)((lb.seq << 2) | LB_PREFIX) << 32) | (pre + cnt[e]));
