@@ -21,7 +21,13 @@ namespace gbwt {
 constexpr int PH_THREADS = 256;
 constexpr int PH_SPAN = 24576;
 constexpr uint64_t M61 = (1ull << 61) - 1ull;
-constexpr uint32_t PH_PROBES = 2048;      // a longer run means a table too full to go on
+// A longer run means a table too full to go on.  Linear probing of a table at 0.7
+// of its slots (the limit is 0.75) has runs of about 250 slots; the full-size
+// table is at most half full and gets room to spare, since nothing larger
+// follows it.  When a small table overflows, every thread in flight runs into
+// the dense rest of it before the first CTA reports its count: 102 MB of
+// versions, first attempt 703 -> 329 us with 2048 -> 256.
+constexpr uint32_t PH_PROBES = 2048, PH_PROBES_SMALL = 256;
 
 // Phrase k spans [start, end]: end = D[k]; start = D[k-1]-W+1 (consecutive
 // phrases overlap by W, K:578-592).  In a batch of texts (xsep = the padded
@@ -83,6 +89,7 @@ struct HashArgs {
     uint32_t *slot_of;
     uint32_t *flags;
     const uint8_t *xsep;    // batch: padded text buffer, else null
+    uint32_t probes;        // longest run
     uint32_t *full;         // set with ERR_TABLE_FULL: away from the counters that every insert updates
     unsigned long long *bytes;      // PART: sum of the distinct phrases' lengths
 };
@@ -135,7 +142,7 @@ __device__ __forceinline__ void phrase_insert(const HashArgs &a, uint32_t k, con
         }
         if (cur == key) { ok = true; break; }
         pos = (pos + 1u) & a.cmask;
-        if (probe >= PH_PROBES || ((probe & 7u) == 7u && *(volatile uint32_t *)a.full)) break;
+        if (probe >= a.probes || ((probe & 7u) == 7u && *(volatile uint32_t *)a.full)) break;
     }
     if (!ok) {
         atomicOr(a.flags, ERR_TABLE_FULL);
@@ -425,6 +432,7 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         while ((1u << logc) < c) logc++;
         a.logc = logc;
         a.limit = (uint32_t)(((uint64_t)c * 3) / 4);
+        a.probes = c < full_c ? PH_PROBES_SMALL : PH_PROBES;
         a.slot_of = slot_of; a.flags = st->d_flags; a.xsep = xsep;
         a.bytes = may_part ? &part->bytes : nullptr;
         probe_begin(st, GBWT_PROBE_PHRASE_HASH);
