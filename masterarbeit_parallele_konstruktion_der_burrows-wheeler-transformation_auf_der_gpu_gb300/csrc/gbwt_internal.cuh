@@ -261,7 +261,7 @@ struct ParseOrder {
 };
 // Pieces of the two sorts that the second-level parse uses on its own strings.
 int sort_phrase_suffixes(Storage *st, uint32_t N, int key_bits, uint32_t h0, const uint32_t *dphr, const uint32_t *doff,
-                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa);
+                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa, uint32_t texts = 1);
 void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, const uint32_t *doff, uint32_t *lexrank);
 int parse_sa_buckets(Storage *st, uint32_t z, uint32_t d, const uint32_t *pid, const uint32_t *lexrank,
                      const uint32_t *occ, int stride, uint32_t *isa, uint32_t *sa);   // occ[q * stride]

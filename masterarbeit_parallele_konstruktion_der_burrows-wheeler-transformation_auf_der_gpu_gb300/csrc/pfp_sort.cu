@@ -158,6 +158,15 @@ struct LoadHeadActive {
         return ((uint64_t)top << 32) | (uint32_t)__popc(active[w]);
     }
 };
+// Ranks of round 0 go to random positions of the text they belong to.  While
+// these fit the L2 (129 MB) it collects the writes of a sector; above that each
+// costs a sector read and written back, and the ranks are written a window of
+// 64 MB at a time instead, the sorted positions read once per window.  Both
+// kernels, before / after: N = 130 M (512 MiB DNA, W=35) 4.91 / 2.46 ms, 57 M
+// (102 MB of versions) 1.32 / 0.78 ms, 26 M (512 MiB DNA) 0.49 / 0.40 ms; 4096
+// texts kept apart (N = 46 M in small ranges): the call 0.1 ms longer, so not there.
+// Windows of 16, 32, 64, 128 MB at 130 M: 5.83, 3.51, 2.46, 3.27 ms.
+constexpr uint32_t R0_WINDOW = 1u << 24;
 __global__ void k_round0_ranks(const uint32_t *vals, uint32_t n, const uint32_t *heads, const uint32_t *active,
                                const uint64_t *pre, uint32_t *isa, uint32_t *sa, uint32_t *act_x, uint32_t *act_g)
 {
@@ -167,7 +176,7 @@ __global__ void k_round0_ranks(const uint32_t *vals, uint32_t n, const uint32_t 
     const uint64_t p = pre[w];
     const uint32_t upto = heads[w] & (0xFFFFFFFFu >> (31u - lane));
     const uint32_t h = upto ? w * 32u + 31u - (uint32_t)__clz(upto) : (uint32_t)(p >> 32);
-    isa[x] = h;
+    if (isa) isa[x] = h;
     const uint32_t am = active[w];
     if ((am >> lane) & 1u) {
         const uint32_t pos = (uint32_t)p + (uint32_t)__popc(am & ((1u << lane) - 1u));
@@ -175,6 +184,33 @@ __global__ void k_round0_ranks(const uint32_t *vals, uint32_t n, const uint32_t 
         act_g[pos] = h;
     } else {
         sa[t] = x;
+    }
+}
+// The ranks of the positions [lo, lo + R0_WINDOW) only, four elements a thread.
+__global__ void k_round0_window(const uint32_t *vals, uint32_t n, const uint32_t *heads, const uint64_t *pre,
+                                uint32_t lo, uint32_t *isa)
+{
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
+    if (t >= n) return;
+    uint32_t x[4];
+    if (t + 4u <= n) {
+        const uint4 v = __ldg((const uint4 *)(vals + t));
+        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) x[j] = t + j < n ? vals[t + j] : 0xFFFFFFFFu;
+    }
+    bool in = false;
+#pragma unroll
+    for (int j = 0; j < 4; j++) in |= x[j] >= lo && x[j] - lo < R0_WINDOW && x[j] < n;
+    if (!in) return;
+    const uint32_t w = t >> 5;
+    const uint32_t hw = heads[w], top = (uint32_t)(pre[w] >> 32);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        if (x[j] < lo || x[j] - lo >= R0_WINDOW || x[j] >= n) continue;
+        const uint32_t upto = hw & (0xFFFFFFFFu >> (31u - ((t + j) & 31u)));
+        isa[x[j]] = upto ? w * 32u + 31u - (uint32_t)__clz(upto) : top;
     }
 }
 
@@ -1055,10 +1091,10 @@ static int doubling_rounds(Storage *st, uint32_t N, uint64_t h, uint32_t A, Rem 
 // Sorts N positions; key0 (in slot S_KEY0) holds the initial keys covering
 // h0 symbols; with key0_cont, bit 0 of every initial key tells whether the
 // suffix is longer than h0 (rem > h0).  Fills isa[N] and sa[N]; returns the
-// number of rounds.
+// number of rounds.  `texts`: the keys are led by the text, in position order.
 template <typename Rem>
 static int prefix_doubling(Storage *st, uint32_t N, int key0_bits, uint32_t h0, Rem rem, uint32_t *isa,
-                           uint32_t *sa, bool key0_cont = false)
+                           uint32_t *sa, bool key0_cont = false, uint32_t texts = 1)
 {
     uint64_t *keys = slot<uint64_t>(st, S_KEY0, N);
     uint64_t *keys_alt = slot<uint64_t>(st, S_KEY1, N);
@@ -1080,8 +1116,15 @@ static int prefix_doubling(Storage *st, uint32_t N, int key0_bits, uint32_t h0, 
     after_launch(st);
     device_scan<uint64_t, OpMaxAdd>(st, nw, LoadHeadActive{heads, active}, StoreArr<uint64_t>{pre}, false,
                                     (uint64_t *)st->d_scalars);
-    k_round0_ranks<<<grid_for(N, 256), 256, 0, st->stream>>>(vals, N, heads, active, pre, isa, sa, act_x, act_g);
+    const bool windows = N / texts > R0_WINDOW + R0_WINDOW / 2u;     // a text's ranks stay among themselves
+    k_round0_ranks<<<grid_for(N, 256), 256, 0, st->stream>>>(vals, N, heads, active, pre, windows ? nullptr : isa, sa,
+                                                             act_x, act_g);
     after_launch(st);
+    for (uint64_t lo = 0; windows && lo < N; lo += R0_WINDOW) {
+        k_round0_window<<<grid_for(((size_t)N + 3) / 4, 256), 256, 0, st->stream>>>(vals, N, heads, pre, (uint32_t)lo,
+                                                                                    isa);
+        after_launch(st);
+    }
     fetch_scalars(st, 1);
     const uint32_t A = (uint32_t)st->h_scalars[0];      // low word of the total: active elements
     return 1 + doubling_rounds(st, N, h0, A, rem, isa, sa, act_x, act_g, act_x2, act_g2, true);
@@ -1217,9 +1260,9 @@ void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, cons
 }
 
 int sort_phrase_suffixes(Storage *st, uint32_t N, int key_bits, uint32_t h0, const uint32_t *dphr, const uint32_t *doff,
-                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa)
+                         const uint32_t *dlen, const uint8_t *rem8, uint32_t *isa, uint32_t *sa, uint32_t texts)
 {
-    return prefix_doubling(st, N, key_bits, h0, DictRem{dphr, doff, dlen, rem8}, isa, sa, true);
+    return prefix_doubling(st, N, key_bits, h0, DictRem{dphr, doff, dlen, rem8}, isa, sa, true, texts);
 }
 
 void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
@@ -1267,7 +1310,7 @@ void run_dict_sort(Storage *st, Phrases &ph, int W, bool small, DictOrder &dord)
     dord.isa = slot<uint32_t>(st, S_ISA, N);
     dord.sa = slot<uint32_t>(st, S_SA, N);
     dord.rounds = sort_phrase_suffixes(st, N, tb + h0 * bps + 1, (uint32_t)h0, ph.dphr, ph.doff, ph.dlen, rem8, dord.isa,
-                                       dord.sa);
+                                       dord.sa, tb ? ph.texts : 1u);
     dord.lexrank = slot<uint32_t>(st, S_LEXRANK, ph.d);
     phrase_ranks(st, N, ph.d, dord.isa, ph.doff, dord.lexrank);
 }
