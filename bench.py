@@ -8,7 +8,7 @@ One step = one BWT (W=5, P=16) of the whole 512 MiB text.
   e2e       the same through the public C ABI with pinned HOST buffers: the
             host->device copy of the text and the device->host copy of the
             BWT are inside every timed step;
-  roofline  the dominant kernel's algorithmic bytes per launch / its average
+  roofline  the segmented round's algorithmic bytes per launch / its average
             launch time (events around each of its launches in the timed
             region) against the measured HBM copy bandwidth;
   roofline_pipeline  the whole pipeline's algorithmic bytes
@@ -62,7 +62,7 @@ WORKLOAD = ("512 MiB repetitive DNA: 4 MiB uniform ACGT base (seed 2), 128 copie
 
 # Kernels whose launches are timed for the roofline (gbwt_set_kernel_probe in
 # include/gbwt.h), with the library's algorithmic bytes per launch:
-#   k_seg_sort (the dominant kernel, prefix-doubling rounds sorted inside CTAs):
+#   k_seg_sort (prefix-doubling rounds sorted inside CTAs):
 #     24 B per active element (read x, group, key; write rank and next entry)
 #   k_rs_downsweep (radix scatter): every key and value read and written once
 PROBE_SEG_SORT = 6
