@@ -815,8 +815,13 @@ static __global__ void k_iota(uint32_t *v, uint32_t n)
 // garbage).  With `iota` the values are the positions 0..n-1 (vals need not be
 // filled).  With segments (n a multiple of RS_TILE) every segment is sorted on
 // its own.
+//
+// Internal linkage: every source file has kernels of its own, and attr_set has
+// to speak for those.  With one attr_set for the library, the first file to
+// sort 64-bit keys with values (59 KB of shared memory) left the other's
+// kernels at 48 KB and their launches failed.
 template <typename K, bool HAS_VAL, int BITS = 8, int BALLOT = 0>
-void radix_sort(Storage *st, K *&keys, K *&keys_alt, uint32_t *&vals, uint32_t *&vals_alt, uint32_t n,
+static void radix_sort(Storage *st, K *&keys, K *&keys_alt, uint32_t *&vals, uint32_t *&vals_alt, uint32_t n,
                 int begin_bit, int end_bit, RsSegs sg = RsSegs(), bool iota = false)
 {
     static_assert((1 << BITS) % RS_THREADS == 0, "digit count must be a multiple of the CTA size");
