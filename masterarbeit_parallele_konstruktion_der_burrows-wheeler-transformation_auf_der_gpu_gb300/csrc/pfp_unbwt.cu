@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__r
 // LF of every row (entries as UbHash::entry).  Row 0 precedes all rows of its
 // symbol c0 in the sort: with PFP input its element is left out of the counts
 // and every other position at or above c0's bucket moves up by one.
-__global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t *__restrict__ tile_off,
-                                                        uint32_t num_tiles, UbHash hash, uint32_t *__restrict__ LF)
+__global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t *tile_off, uint32_t num_tiles,
+                                                        UbHash hash, uint32_t *__restrict__ LF, uint32_t *flags)
 {
     constexpr int D = 256;
     __shared__ uint32_t s_wh[RS_WARPS * D];
@@ -184,10 +184,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t 
             s_wh[w * D + d] = run;
             run += c;
         }
-        const uint32_t off = tile_off[(size_t)d * num_tiles + blockIdx.x];
-        s_goff[d] = 1u + off + (c0 <= d ? 1u : 0u);
+        const uint32_t off = lb_load32(tile_off + (size_t)d * num_tiles + blockIdx.x);
+        s_goff[d] = rs_checked(1u + off + (c0 <= d ? 1u : 0u), run, hash.rows, flags);     // the walks stay in the table
         // row 0 (PFP) and the '$' row, by the first tile
-        if (blockIdx.x == 0 && d == c0) LF[0] = hash.entry(1u + off);
+        if (blockIdx.x == 0 && d == c0) LF[0] = hash.entry(rs_checked(1u + off, 1u, hash.rows, flags));
         if (blockIdx.x == 0 && d == 0) LF[in.dollar] = UB_RULER;      // row 0 is ruler 0
     }
     __syncthreads();
@@ -355,7 +355,7 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
                                  (uint32_t *)nullptr);
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
-    k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF);
+    k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF, st->d_flags);
     after_launch(st);
     uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
     k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);
