@@ -29,8 +29,12 @@
 // The hash is a permutation of [0, 2^kb), 2^kb the power of two at or above the
 // number of blocks, so a block's number is its hash over the rate and its place
 // the inverse hash of that: no list of rulers, no search in it.  The chain is
-// ranked through one ruler in 16: sequential hops between those, pointer
-// jumping over them, and the hops again.
+// ranked through one ruler in 16 (the carriers): sequential hops between those,
+// pointer jumping over them, and the hops again.  Which of 16 is hashed too:
+// between the copies of an exactly repeated text a walk keeps its row modulo the
+// number of copies, and with the first of every 16 rulers as carrier one thread
+// hopped over the chain of whole copies (16 copies: 8 MiB took 149 ms, now 16 MiB
+// take 0.56 ms).
 //
 // 128 MiB of DNA copies, before / after on GB300, one row in 64 a ruler: LF 1.37 / 0.31
 // ms, first walk 2.22 / 1.25, list ranking 1.11 / 0.18, second walk 3.46 / 1.75, in
@@ -45,7 +49,7 @@ namespace gbwt {
 
 constexpr uint32_t UB_RULER = 0x80000000u;
 constexpr uint32_t UB_NIL = 0xFFFFFFFFu;
-constexpr int UB_SUPER_LOG2 = 4;          // one ruler in 16 carries the list ranking
+constexpr int UB_SUPER_LOG2 = 4;          // log2 of the rulers to a carrier of the list ranking
 constexpr int UB_LUT_LOG2 = 12;
 
 // Permutation of [0, 2^kb): xor-shifts by at least half the bits undo
@@ -91,6 +95,15 @@ struct UbHash {
         return (unmix((ruler >> 5) << rate_log2) << 5) | (ruler & 31u);
     }
 };
+
+// The ruler of [16 s, 16 s + 16) that carries the list ranking; ruler 0 for s = 0.
+__host__ __device__ __forceinline__ uint32_t ub_carrier(uint32_t s)
+{
+    uint32_t x = s * UB_MUL1;
+    x ^= x >> 15;
+    x *= UB_MUL2;
+    return (s << UB_SUPER_LOG2) | (x >> (32 - UB_SUPER_LOG2));
+}
 
 // Where the input's elements belong.  PFP: element e is row e + 1, except
 // element p, whose symbol is row 0's (its place is the '$' row).  libcubwt:
@@ -219,14 +232,14 @@ __global__ void k_walk_count(const uint32_t *__restrict__ LF, UbHash hash, uint3
     }
 }
 
-// Hops between super-rulers (numbers that are multiples of 2^UB_SUPER_LOG2):
-// the next one and the distance.  The one whose next is ruler 0 ends the chain.
+// Hops between carriers: the next one and the distance.  The one whose next is
+// ruler 0 ends the chain.
 __global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
                              uint32_t *ssucc, uint32_t *swt)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= supers) return;
-    uint32_t j = s << UB_SUPER_LOG2, acc = 0, hops = 0;
+    uint32_t j = ub_carrier(s), acc = 0, hops = 0;
     if (hash.row_of(j) >= hash.rows) {
         ssucc[s] = UB_NIL;
         swt[s] = 0;
@@ -235,13 +248,13 @@ __global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbHash ha
     do {
         acc += wt[j];
         j = succ[j];
-    } while (j < slots && (j & ((1u << UB_SUPER_LOG2) - 1u)) && ++hops < slots);
+    } while (j < slots && j != ub_carrier(j >> UB_SUPER_LOG2) && ++hops < slots);
     ssucc[s] = j == 0 || j >= slots ? UB_NIL : j >> UB_SUPER_LOG2;
     swt[s] = acc;
 }
 
 // Pointer jumping: after r rounds wt[s] is the distance over the next 2^r
-// super-rulers (or to the chain's end).  Double-buffered.
+// carriers (or to the chain's end).  Double-buffered.
 __global__ void k_jump(const uint32_t *succ, const uint32_t *wt, uint32_t m, uint32_t *succ2, uint32_t *wt2)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,20 +265,20 @@ __global__ void k_jump(const uint32_t *succ, const uint32_t *wt, uint32_t m, uin
 }
 
 // Distances from row 0 for every ruler: the hops again, from rows - (distance
-// of the super-ruler to the end).
+// of the carrier to the end).
 __global__ void k_ruler_off(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
                             const uint32_t *sdist, uint32_t *off)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= supers) return;
-    uint32_t j = s << UB_SUPER_LOG2, hops = 0;
+    uint32_t j = ub_carrier(s), hops = 0;
     if (hash.row_of(j) >= hash.rows) return;
     uint32_t o = hash.rows - sdist[s];
     do {
         off[j] = o;
         o += wt[j];
         j = succ[j];
-    } while (j < slots && (j & ((1u << UB_SUPER_LOG2) - 1u)) && ++hops < slots);
+    } while (j < slots && j != ub_carrier(j >> UB_SUPER_LOG2) && ++hops < slots);
 }
 
 // Second walk: every ruler writes the text bytes of its stretch, from high to
