@@ -29,8 +29,8 @@
 // The hash is a permutation of [0, 2^kb), 2^kb the power of two at or above the
 // number of blocks, so a block's number is its hash over the rate and its place
 // the inverse hash of that: no list of rulers, no search in it.  The chain is
-// ranked through one ruler in 16 (the carriers): sequential hops between those,
-// pointer jumping over them, and the hops again.  Which of 16 is hashed too:
+// ranked through one ruler in 8 or 16 (the carriers): sequential hops between
+// those, pointer jumping over them, and the hops again.  Which one is hashed too:
 // between the copies of an exactly repeated text a walk keeps its row modulo the
 // number of copies, and with the first of every 16 rulers as carrier one thread
 // hopped over the chain of whole copies (16 copies: 8 MiB took 149 ms, now 16 MiB
@@ -41,6 +41,17 @@
 // all 9.1 / 3.6 ms; one in 16, 32, 64, 128: 3.0, 3.0, 3.5, 4.3 ms (512 MiB: 12.2,
 // 10.6, 10.7, 12.5; 64 MiB of random DNA: 3.0, 3.3, 3.7, 4.9, before 4.7 at best).
 //
+// In a long run of one symbol, and where the text repeats a short period, LF
+// leads from row to row of one block: 31 of its 32 rulers end at the next row and
+// the last one walks alone through all blocks up to the next ruler block.
+// Tiles that hold one symbol therefore mark one target row in 32 to 256 as a ruler
+// of its own (numbers from `slots` on, rows in a list).  16 MiB of one symbol 2.36 ->
+// 0.53 ms, of period 7 2.26 -> 0.63, half of it zeros 2.02 -> 0.64 (with rulers row
+// by row 1.10, 1.17, 1.27); 128 MiB of one symbol 13.1 -> 2.6 ms (5.6).  Fewer
+// listed rows (an eighth of the rulers' density) than fit such texts best: a text
+// of thousands of copies has such tiles too and its blocks walk well (Fibonacci word
+// of 128 MiB 2.6 -> 3.2 ms, with four times as many 3.5).  DNA has no such tile.
+//
 // LF is a permutation, so a walk ends at the latest at its own ruler; the input
 // is a BWT exactly when the cycle of row 0 has all n + 1 rows.
 #include "prims.cuh"
@@ -49,7 +60,7 @@ namespace gbwt {
 
 constexpr uint32_t UB_RULER = 0x80000000u;
 constexpr uint32_t UB_NIL = 0xFFFFFFFFu;
-constexpr int UB_SUPER_LOG2 = 4;          // log2 of the rulers to a carrier of the list ranking
+constexpr int UB_EXTRA_LOG2 = 3;          // one listed ruler in 2^(rate_log2 + UB_EXTRA_LOG2) rows of such a tile
 constexpr int UB_LUT_LOG2 = 12;
 
 // Permutation of [0, 2^kb): xor-shifts by at least half the bits undo
@@ -96,14 +107,25 @@ struct UbHash {
     }
 };
 
-// The ruler of [16 s, 16 s + 16) that carries the list ranking; ruler 0 for s = 0.
-__host__ __device__ __forceinline__ uint32_t ub_carrier(uint32_t s)
-{
-    uint32_t x = s * UB_MUL1;
-    x ^= x >> 15;
-    x *= UB_MUL2;
-    return (s << UB_SUPER_LOG2) | (x >> (32 - UB_SUPER_LOG2));
-}
+// All rulers: `slots` numbers of blocks, then the listed rows.
+struct UbRulers {
+    UbHash hash;
+    uint32_t slots;
+    uint32_t *extra;             // rows of the listed rulers
+    uint32_t *extra_n;           // their number, at most extra_cap
+    uint32_t extra_cap, extra_mask;
+    int super_log2;              // one ruler in 2^super_log2 carries the list ranking
+    __device__ __forceinline__ uint32_t count() const { return slots + min(*extra_n, extra_cap); }
+    __device__ __forceinline__ uint32_t row_of(uint32_t j) const { return j < slots ? hash.row_of(j) : extra[j - slots]; }
+    // The ruler of the s-th group that carries the list ranking; ruler 0 for s = 0.
+    // The groups of a block pick alike: walks that keep their row modulo the
+    // group's size move and stop together.
+    __device__ __forceinline__ uint32_t carrier(uint32_t s) const
+    {
+        return (s << super_log2) | (((s >> (5 - super_log2)) * 0x9E3779B1u) >> (32 - super_log2));
+    }
+    __device__ __forceinline__ bool carries(uint32_t j) const { return j == carrier(j >> super_log2); }
+};
 
 // Where the input's elements belong.  PFP: element e is row e + 1, except
 // element p, whose symbol is row 0's (its place is the '$' row).  libcubwt:
@@ -116,8 +138,10 @@ struct UbIn {
     __device__ __forceinline__ uint32_t row(uint32_t e) const { return p != UB_NIL ? e + 1u : (e < dollar ? e : e + 1u); }
 };
 
-// Symbol counts of every tile (element p left out), digit-major over the tiles.
-__global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__restrict__ tile_hist, uint32_t num_tiles)
+// Symbol counts of every tile (element p left out), digit-major over the tiles;
+// and whether it holds one symbol.
+__global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__restrict__ tile_hist, uint32_t num_tiles,
+                                                          uint8_t *__restrict__ one_symbol)
 {
     constexpr int D = 256;
     __shared__ uint32_t h[RS_WARPS * D];       // one histogram per warp
@@ -138,6 +162,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__r
             if (i < in.n) atomicAdd(&wh[in.L[i]], 1u);
         }
     }
+    if (threadIdx.x == 0) one_symbol[blockIdx.x] = 0;
     __syncthreads();
     for (int d = threadIdx.x; d < D; d += RS_THREADS) {
         uint32_t sum = 0;
@@ -145,6 +170,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__r
         for (int w = 0; w < RS_WARPS; w++) sum += h[w * D + d];
         if (in.p != UB_NIL && in.p >= base && in.p < base + RS_TILE && in.L[in.p] == d) sum--;
         tile_hist[(size_t)d * num_tiles + blockIdx.x] = sum;
+        if (sum + 1u >= (uint32_t)RS_TILE) one_symbol[blockIdx.x] = 1;      // element p may be left out
     }
 }
 
@@ -212,19 +238,53 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t 
     }
 }
 
+// Listed rulers: in tiles of one symbol every target row that is a multiple of
+// 2^extra_log2, numbered with one atomic per tile.  A CTA looks at UB_XTILES
+// tiles.
+constexpr int UB_XTILES = 8;
+__global__ void __launch_bounds__(RS_THREADS) k_lf_extra(UbIn in, const uint8_t *__restrict__ one_symbol,
+                                                         uint32_t num_tiles, UbRulers ru, uint32_t *LF)
+{
+    __shared__ uint32_t s_warp[32], s_first;
+    const uint32_t b0 = blockIdx.x * UB_XTILES, b1 = min(b0 + UB_XTILES, num_tiles);
+    const bool set = threadIdx.x < b1 - b0 && one_symbol[b0 + threadIdx.x];
+    if (!__syncthreads_or(set)) return;
+    for (uint32_t b = b0; b < b1; b++) {
+        if (!one_symbol[b]) continue;
+        uint32_t mine = 0, total;
+#pragma unroll
+        for (int q = 0; q < RS_ITEMS; q++) {
+            const uint32_t e = b * RS_TILE + q * RS_THREADS + threadIdx.x;
+            if (e >= in.n || e == in.p) continue;
+            const uint32_t v = LF[in.row(e)];
+            if (!(v & (UB_RULER | ru.extra_mask))) mine |= 1u << q;
+        }
+        uint32_t j = block_excl_scan<uint32_t, OpAdd>((uint32_t)__popc(mine), total, OpAdd(), s_warp);
+        if (threadIdx.x == 0) s_first = atomicAdd(ru.extra_n, total);
+        __syncthreads();
+        j += s_first;
+        for (uint32_t m = mine; m && j < ru.extra_cap; m &= m - 1u, j++) {
+            const uint32_t r = in.row(b * RS_TILE + (uint32_t)(__ffs(m) - 1) * RS_THREADS + threadIdx.x);
+            ru.extra[j] = LF[r];
+            LF[r] = UB_RULER | (ru.slots + j);
+        }
+        __syncthreads();
+    }
+}
+
 // First walk: the next ruler and the distance to it.  A warp takes block after
 // block of 32 ruler rows.
-__global__ void k_walk_count(const uint32_t *__restrict__ LF, UbHash hash, uint32_t slots, uint32_t *succ, uint32_t *wt)
+__global__ void k_walk_count(const uint32_t *__restrict__ LF, UbRulers ru, uint32_t *succ, uint32_t *wt)
 {
-    const uint32_t step = gridDim.x * blockDim.x;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < slots; j += step) {
-        uint32_t r = hash.row_of(j), steps = 0, v = UB_NIL;
-        if (r < hash.rows) {               // else a hash value past the rows: no ruler
+    const uint32_t step = gridDim.x * blockDim.x, count = ru.count(), rows = ru.hash.rows;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += step) {
+        uint32_t r = ru.row_of(j), steps = 0, v = UB_NIL;
+        if (r < rows) {               // else a hash value past the rows: no ruler
             do {
                 v = __ldg(LF + r);
                 r = v;
                 steps++;
-            } while (!(v & UB_RULER) && steps <= hash.rows);
+            } while (!(v & UB_RULER) && steps <= rows);
             v &= ~UB_RULER;
         }
         succ[j] = v;
@@ -234,13 +294,13 @@ __global__ void k_walk_count(const uint32_t *__restrict__ LF, UbHash hash, uint3
 
 // Hops between carriers: the next one and the distance.  The one whose next is
 // ruler 0 ends the chain.
-__global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
-                             uint32_t *ssucc, uint32_t *swt)
+__global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbRulers ru, uint32_t supers, uint32_t *ssucc,
+                             uint32_t *swt)
 {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= supers) return;
-    uint32_t j = ub_carrier(s), acc = 0, hops = 0;
-    if (hash.row_of(j) >= hash.rows) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x, slots = ru.count();
+    if (s >= supers) return;           // from an upper bound of the rulers: the last ones may not be there
+    uint32_t j = ru.carrier(s), acc = 0, hops = 0;
+    if (j >= slots || ru.row_of(j) >= ru.hash.rows) {
         ssucc[s] = UB_NIL;
         swt[s] = 0;
         return;
@@ -248,8 +308,8 @@ __global__ void k_super_hops(const uint32_t *succ, const uint32_t *wt, UbHash ha
     do {
         acc += wt[j];
         j = succ[j];
-    } while (j < slots && j != ub_carrier(j >> UB_SUPER_LOG2) && ++hops < slots);
-    ssucc[s] = j == 0 || j >= slots ? UB_NIL : j >> UB_SUPER_LOG2;
+    } while (j < slots && !ru.carries(j) && ++hops < slots);
+    ssucc[s] = j == 0 || j >= slots ? UB_NIL : j >> ru.super_log2;
     swt[s] = acc;
 }
 
@@ -266,53 +326,39 @@ __global__ void k_jump(const uint32_t *succ, const uint32_t *wt, uint32_t m, uin
 
 // Distances from row 0 for every ruler: the hops again, from rows - (distance
 // of the carrier to the end).
-__global__ void k_ruler_off(const uint32_t *succ, const uint32_t *wt, UbHash hash, uint32_t supers, uint32_t slots,
-                            const uint32_t *sdist, uint32_t *off)
+__global__ void k_ruler_off(const uint32_t *succ, const uint32_t *wt, UbRulers ru, const uint32_t *sdist, uint32_t *off)
 {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= supers) return;
-    uint32_t j = ub_carrier(s), hops = 0;
-    if (hash.row_of(j) >= hash.rows) return;
-    uint32_t o = hash.rows - sdist[s];
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x, slots = ru.count();
+    uint32_t j = ru.carrier(s), hops = 0;
+    if (j >= slots || ru.row_of(j) >= ru.hash.rows) return;
+    uint32_t o = ru.hash.rows - sdist[s];
     do {
         off[j] = o;
         o += wt[j];
         j = succ[j];
-    } while (j < slots && j != ub_carrier(j >> UB_SUPER_LOG2) && ++hops < slots);
+    } while (j < slots && !ru.carries(j) && ++hops < slots);
 }
 
 // Second walk: every ruler writes the text bytes of its stretch, from high to
 // low addresses, gathered into 8-byte words.  sym(row) is the bucket of
 // LF(row) - 1 among the cumulative counts cum[0..256]: a table over the value's
-// high bits gives the first candidate.
-__global__ void __launch_bounds__(256) k_walk_emit(const uint32_t *__restrict__ LF, UbHash hash, uint32_t slots,
-                                                   const uint32_t *off, const uint32_t *cum, int lut_shift, uint32_t n,
-                                                   uint8_t *T)
+// high bits gives the first candidate.  LISTED: there are listed rulers (a look at
+// the list in the loop takes 2 % of texts that have none).
+template <bool LISTED>
+__device__ __forceinline__ void emit_stretches(const uint32_t *__restrict__ LF, const UbRulers &ru, const uint32_t *off,
+                                               const uint32_t *s_cum, const uint8_t *s_lut, int lut_shift, uint32_t n,
+                                               uint8_t *T)
 {
-    __shared__ uint32_t s_cum[257];
-    __shared__ uint8_t s_lut[1 << UB_LUT_LOG2];
-    for (int c = threadIdx.x; c < 257; c += blockDim.x) s_cum[c] = cum[c];
-    __syncthreads();
-    for (uint32_t q = threadIdx.x; q < (1u << UB_LUT_LOG2); q += blockDim.x) {
-        const uint64_t first = (uint64_t)q << lut_shift;
-        uint32_t lo = 0, hi = 255;           // last c with cum[c] <= first
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1u) >> 1;
-            if (s_cum[mid] <= first) lo = mid; else hi = mid - 1u;
-        }
-        s_lut[q] = (uint8_t)lo;
-    }
-    __syncthreads();
-    const uint32_t step = gridDim.x * blockDim.x;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < slots; j += step) {
-        uint32_t r = hash.row_of(j);
-        if (r >= hash.rows) continue;
+    const uint32_t step = gridDim.x * blockDim.x, count = LISTED ? ru.count() : ru.slots;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += step) {
+        uint32_t r = LISTED ? ru.row_of(j) : ru.hash.row_of(j);
+        if (r >= ru.hash.rows) continue;
         uint32_t k = off[j], in_word = 0;    // bytes gathered in `word`
         uint64_t word = 0;
         for (bool last = false; !last; k++) {
             const uint32_t v = __ldg(LF + r);
             last = (v & UB_RULER) != 0;
-            r = last ? hash.row_of(v & ~UB_RULER) : v;
+            r = !last ? v : LISTED ? ru.row_of(v & ~UB_RULER) : ru.hash.row_of(v & ~UB_RULER);
             if (k >= n || r == 0) break;     // the '$' row: the stretch ends here
             uint32_t c = s_lut[(r - 1u) >> lut_shift];
             while (s_cum[c + 1] <= r - 1u) c++;
@@ -329,6 +375,26 @@ __global__ void __launch_bounds__(256) k_walk_emit(const uint32_t *__restrict__ 
         // bytes before the '$' row: the lowest is T[0]
         for (uint32_t q = 0; q < in_word; q++) T[q] = (uint8_t)(word >> (8u * q));
     }
+}
+__global__ void __launch_bounds__(256) k_walk_emit(const uint32_t *__restrict__ LF, UbRulers ru, const uint32_t *off,
+                                                   const uint32_t *cum, int lut_shift, uint32_t n, uint8_t *T)
+{
+    __shared__ uint32_t s_cum[257];
+    __shared__ uint8_t s_lut[1 << UB_LUT_LOG2];
+    for (int c = threadIdx.x; c < 257; c += blockDim.x) s_cum[c] = cum[c];
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < (1u << UB_LUT_LOG2); q += blockDim.x) {
+        const uint64_t first = (uint64_t)q << lut_shift;
+        uint32_t lo = 0, hi = 255;           // last c with cum[c] <= first
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1u) >> 1;
+            if (s_cum[mid] <= first) lo = mid; else hi = mid - 1u;
+        }
+        s_lut[q] = (uint8_t)lo;
+    }
+    __syncthreads();
+    if (*ru.extra_n) emit_stretches<true>(LF, ru, off, s_cum, s_lut, lut_shift, n, T);
+    else emit_stretches<false>(LF, ru, off, s_cum, s_lut, lut_shift, n, T);
 }
 
 // Cumulative symbol counts of all non-'$' rows from the scanned tile
@@ -359,30 +425,40 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     while ((1u << hash.rate_log2) < rate && hash.rate_log2 < kb) hash.rate_log2++;
     hash.rows = rows;
     const uint32_t slots = (uint32_t)((1ull << kb) >> hash.rate_log2) << 5;
-    const uint32_t supers = (slots + (1u << UB_SUPER_LOG2) - 1u) >> UB_SUPER_LOG2;
+    const int extra_log2 = hash.rate_log2 + UB_EXTRA_LOG2;
+    const uint32_t extra_cap = (rows >> extra_log2) + 1u, rulers = slots + extra_cap;       // upper bounds
+    // 1 MiB of mutated copies 281 us with one in 16, 259 with one in 8 (shorter
+    // hops); 128 MiB 3.26 and 3.28 ms (one round of pointer jumping more)
+    const int super_log2 = rows < (1u << 25) ? 3 : 4;
+    const uint32_t supers = (rulers + (1u << super_log2) - 1u) >> super_log2;
+    UbRulers ru{hash, slots, slot<uint32_t>(st, S_ACTX, extra_cap), st->d_flags + 56, extra_cap, (1u << extra_log2) - 1u,
+                super_log2};
     // LF
     const uint32_t num_tiles = (uint32_t)(((size_t)n + RS_TILE - 1) / RS_TILE);
     uint32_t *hist = slot<uint32_t>(st, S_RSHIST, (size_t)256 * num_tiles);
-    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles);
+    uint8_t *one_symbol = slot<uint8_t>(st, S_ACTG, num_tiles);
+    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, one_symbol);
     after_launch(st);
     device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
                                  (uint32_t *)nullptr);
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
     k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF, st->d_flags);
     after_launch(st);
+    k_lf_extra<<<grid_for(num_tiles, UB_XTILES), RS_THREADS, 0, st->stream>>>(in, one_symbol, num_tiles, ru, LF);
+    after_launch(st);
     uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
     k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);
     after_launch(st);
     // walk 1 and list ranking of the ruler chain
-    uint32_t *succ = slot<uint32_t>(st, S_TMP0, slots), *wt = slot<uint32_t>(st, S_TMP1, slots);
-    unsigned grid = grid_for(slots, 256);
+    uint32_t *succ = slot<uint32_t>(st, S_TMP0, rulers), *wt = slot<uint32_t>(st, S_TMP1, rulers);
+    unsigned grid = grid_for(rulers, 256);
     const unsigned full = (unsigned)st->num_sms * 8u;          // 2048 threads per SM
     if (grid > full) grid = full;
-    k_walk_count<<<grid, 256, 0, st->stream>>>(LF, hash, slots, succ, wt);
+    k_walk_count<<<grid, 256, 0, st->stream>>>(LF, ru, succ, wt);
     after_launch(st);
     uint32_t *ssucc = slot<uint32_t>(st, S_VAL0, supers), *ssucc2 = slot<uint32_t>(st, S_VAL1, supers);
     uint32_t *swt = slot<uint32_t>(st, S_KEY0, supers), *swt2 = slot<uint32_t>(st, S_KEY1, supers);
-    k_super_hops<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, hash, supers, slots, ssucc, swt);
+    k_super_hops<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, ru, supers, ssucc, swt);
     after_launch(st);
     const int rounds = bits_for(supers);
     for (int r = 0; r < rounds; r++) {
@@ -396,11 +472,11 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     check_cuda(cudaMemcpyAsync(st->h_scalars + 2, swt, 4, cudaMemcpyDeviceToHost, st->stream));
     sync_stream(st);
     if ((uint32_t)st->h_scalars[1] != UB_NIL || (uint32_t)st->h_scalars[2] != rows) throw Error{GBWT_BAD_PARAMETER};
-    uint32_t *off = slot<uint32_t>(st, S_SA, slots);
-    k_ruler_off<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, hash, supers, slots, swt, off);
+    uint32_t *off = slot<uint32_t>(st, S_SA, rulers);
+    k_ruler_off<<<grid_for(supers, 128), 128, 0, st->stream>>>(succ, wt, ru, swt, off);
     after_launch(st);
     const int lut_shift = kb + 5 > UB_LUT_LOG2 ? kb + 5 - UB_LUT_LOG2 : 0;
-    k_walk_emit<<<grid, 256, 0, st->stream>>>(LF, hash, slots, off, cum, lut_shift, n, dT);
+    k_walk_emit<<<grid, 256, 0, st->stream>>>(LF, ru, off, cum, lut_shift, n, dT);
     after_launch(st);
 }
 

@@ -40,3 +40,37 @@ def mutated(storage):
 def test_exact_copies(storage, mutated, copies):
     base = np.random.default_rng(copies).integers(2, 6, size=N // copies).astype(np.uint8)
     assert _inverse(storage, np.tile(base, copies)) < 12 * mutated
+
+
+@pytest.mark.parametrize("kind", ["constant", "period 2", "period 7", "half zeros", "zeros between"])
+def test_long_runs(storage, mutated, kind):
+    # LF leads from row to row: rulers of their own inside the runs, or one lane walks for its block
+    rng = np.random.default_rng(2)
+    if kind == "constant":
+        t = np.full(N, 5, np.uint8)
+    elif kind.startswith("period"):
+        t = np.resize(rng.integers(2, 250, size=int(kind[7:])).astype(np.uint8), N)
+    elif kind == "half zeros":
+        t = np.concatenate([rng.integers(2, 6, size=N // 2), np.full(N // 2, 9)]).astype(np.uint8)
+    else:
+        t = np.full(N, 9, np.uint8)
+        for a in range(0, N, N // 8):
+            t[a:a + 5000] = rng.integers(10, 200, size=5000)
+    assert _inverse(storage, t) < 3 * mutated
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 8191, 8193, 12_289, 70_000])
+@pytest.mark.parametrize("runs", [1, 3])
+def test_tiles_of_one_symbol(storage, pkg, orc, n, runs):
+    # tiles of one symbol at every place, the row of the whole text among them; both conventions
+    t = np.repeat(np.arange(runs).astype(np.uint8) * 7 + 3, -(-n // runs))[:n]
+    for u in (t, t[::-1].copy(), np.concatenate([t, t])):
+        L = orc.sa_bwt(u)
+        assert np.array_equal(storage.unbwt(L, orc.primary_index(u)), u)
+        C, i = storage.libcubwt_bwt(u)
+        assert np.array_equal(storage.libcubwt_unbwt(C, i), u)
+    for p in (0, n // 2, n - 1):                     # rows that no text of these symbols has
+        try:
+            assert len(storage.unbwt(t, p)) == n
+        except pkg.GbwtError as e:
+            assert e.code == pkg.BAD_PARAMETER
