@@ -28,6 +28,7 @@ constexpr uint64_t M61 = (1ull << 61) - 1ull;
 // the dense rest of it before the first CTA reports its count: 102 MB of
 // versions, first attempt 703 -> 329 us with 2048 -> 256.
 constexpr uint32_t PH_PROBES = 2048, PH_PROBES_SMALL = 256;
+constexpr uint32_t PH_FEW = 4096;       // occurrences of a phrase on average: few phrases (DNA copies 10 to 100)
 
 // Phrase k spans [start, end]: end = D[k]; start = D[k-1]-W+1 (consecutive
 // phrases overlap by W, K:578-592).  In a batch of texts (xsep = the padded
@@ -329,23 +330,39 @@ struct StoreDense {
 // every distinct phrase.
 __global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, int W,
                                   const uint32_t *slot_of, const uint32_t *tdense, uint32_t *pid, uint32_t *pidpc,
-                                  uint2 *occpc, const uint8_t *xsep,
+                                  uint2 *occpc, bool few, const uint8_t *xsep,
                                   const uint32_t *ptid, const uint8_t *lastb)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= z) return;
-    const uint32_t id = tdense[slot_of[k]];
-    pid[k] = id;
-    uint32_t s, e, c;
-    phrase_span(D, k, W, xsep, s, e);
-    // the first phrase of a text is preceded by the text's last byte
-    if (xsep && (k == 0 || xsep[D[k - 1]] == 1)) c = lastb[ptid[k]];
-    else c = preceding_byte(T, n, s);
-    if (pidpc) pidpc[k] = (id << 8) | c;     // only when ids fit 24 bits
-    // one atomic each per occurrence: neighbouring occurrences rarely share a
-    // phrase, so warp aggregation (a match per warp) costs more than it saves
-    atomicAdd(&occpc[id].x, 1u);
-    atomicOr(&occpc[id].y, c | ((c ^ 0xFFu) << 16));
+    uint32_t id = 0xFFFFFFFFu, seen = 0;
+    if (k < z) {
+        id = tdense[slot_of[k]];
+        pid[k] = id;
+        uint32_t s, e, c;
+        phrase_span(D, k, W, xsep, s, e);
+        // the first phrase of a text is preceded by the text's last byte
+        if (xsep && (k == 0 || xsep[D[k - 1]] == 1)) c = lastb[ptid[k]];
+        else c = preceding_byte(T, n, s);
+        if (pidpc) pidpc[k] = (id << 8) | c;     // only when ids fit 24 bits
+        seen = c | ((c ^ 0xFFu) << 16);
+    }
+    // Two reductions per occurrence: neighbouring occurrences rarely share a
+    // phrase, and a match per warp costs more than it saves.  But a run of one
+    // phrase sends them all to one address (0.6 ns each: 16 MiB of one byte
+    // took 20.8 ms, now 0.7), so a warp whose 32 occurrences are of one phrase
+    // adds once.  `few` distinct phrases that alternate share addresses as well: there
+    // a look at the bytes seen saves most of the second reductions (Fibonacci word
+    // of 16 MiB 10.9 -> 8.7 ms; with DNA the look itself costs 1 % of the call).
+    if (__all_sync(0xFFFFFFFFu, id == __shfl_sync(0xFFFFFFFFu, id, 0))) {
+        seen = __reduce_or_sync(0xFFFFFFFFu, seen);
+        if ((threadIdx.x & 31u) == 0 && k < z) {
+            atomicAdd(&occpc[id].x, 32u);
+            atomicOr(&occpc[id].y, seen);
+        }
+    } else if (k < z) {
+        if (!few || (seen & ~__ldcg(&occpc[id].y))) atomicOr(&occpc[id].y, seen);
+        atomicAdd(&occpc[id].x, 1u);
+    }
 }
 
 struct LoadLen64 {
@@ -476,7 +493,7 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
     check_cuda(cudaMemsetAsync(occpc, 0, (size_t)d * sizeof(uint2), st->stream));
     uint32_t *pidpc = d < (1u << 24) ? slot<uint32_t>(st, S_PIDPC, z) : nullptr;
     k_phrase_finalize<<<grid_for(z, 256), 256, 0, st->stream>>>(dT, n, ph.D, z, W, slot_of, tdense, pid, pidpc,
-                                                                occpc, xsep,
+                                                                occpc, z / d >= PH_FEW, xsep,
                                                                 bt ? bt->ptid : nullptr,
                                                                 bt ? bt->lastb : nullptr);
     ph.pidpc = pidpc;

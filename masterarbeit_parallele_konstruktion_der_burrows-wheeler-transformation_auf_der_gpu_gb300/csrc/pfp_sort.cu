@@ -939,7 +939,7 @@ static void big_groups(Storage *st, uint32_t N, uint32_t nbig, const uint32_t *d
     device_scan<uint64_t, OpMax2>(st, total, LoadRoundHead{k, lb}, StoreBigRound<Rem>{t, lb, bhead, isa, head, sa},
                                   true, (uint64_t *)nullptr);
     check_cuda(cudaMemsetAsync(big_total, 0, 4, st->stream));
-    device_scan<uint32_t, OpAdd>(st, total, LoadActive<Rem>{t},
+    device_scan<uint32_t, OpAdd, 4, 8>(st, total, LoadActive<Rem>{t},
                                  StoreBigActive<Rem>{t, head, counter, out_x, out_g}, false, big_total);
 }
 
