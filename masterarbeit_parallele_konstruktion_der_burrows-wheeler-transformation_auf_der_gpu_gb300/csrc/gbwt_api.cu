@@ -127,7 +127,9 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
             h2.resize(z);
             check_cuda(cudaMemcpyAsync(h2.data(), pord.sa, (size_t)z * 4, cudaMemcpyDeviceToHost, st->stream));
         }
-        sync_stream(st);
+        const uint32_t *hflags = read_flags(st);         // waits for the copies as well
+        if (hflags[0] & ERR_TIMEOUT) return GBWT_TIMEOUT;
+        if (hflags[0] & ERR_INTERNAL) return GBWT_INTERNAL_ERROR;
         for (uint32_t i = 0; i < z; i++) so->ranks[i] = (int32_t)h[i];
         if (so->parse_sa)
             for (uint32_t i = 0; i < z; i++) so->parse_sa[i] = (int32_t)h2[i];
