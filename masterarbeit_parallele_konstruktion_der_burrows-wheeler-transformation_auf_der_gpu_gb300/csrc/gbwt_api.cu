@@ -202,7 +202,9 @@ extern "C" int64_t gbwt_allocate_device_storage(void **storage, int64_t max_leng
         check_cuda(cudaHostAlloc(&st->h_scalars, 256 * sizeof(uint64_t), cudaHostAllocDefault));
         st->h_err = (uint32_t *)(st->h_scalars + 255);
         *st->h_err = 0;
-        check_cuda(cudaMemsetAsync(st->d_scalars, 0, 64 * sizeof(uint64_t), st->stream));   // look-back ticket
+        // look-back ticket; in place before the first call, which may use another stream
+        check_cuda(cudaMemsetAsync(st->d_scalars, 0, 64 * sizeof(uint64_t), st->stream));
+        check_cuda(cudaStreamSynchronize(st->stream));
         for (int i = 0; i < 10; i++) check_cuda(cudaEventCreate(&st->ev[i]));
         st->max_length = max_length;
         if (max_length > 0) {
