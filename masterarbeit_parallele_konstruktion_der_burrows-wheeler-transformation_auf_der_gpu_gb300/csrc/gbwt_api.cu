@@ -160,13 +160,15 @@ static int64_t pipeline(Storage *st, const uint8_t *T, uint8_t *L, int64_t n, in
 }
 
 // Runs f and turns what it throws into a return code.  A call that failed
-// half-way leaves no work queued: the next one may use another stream.
+// half-way leaves no work queued, since the next one may use another stream, and
+// takes along a wait of its own that gave up.
 template <typename F>
 static int64_t guarded(Storage *st, F f)
 {
     int64_t rc;
     try {
-        return f();
+        rc = f();
+        if (rc >= 0) return rc;
     } catch (const Error &e) {
         rc = e.code;
     } catch (const std::bad_alloc &) {
@@ -175,6 +177,7 @@ static int64_t guarded(Storage *st, F f)
         rc = GBWT_INTERNAL_ERROR;
     }
     if (st->stream) cudaStreamSynchronize(st->stream);
+    if (st->h_err) *(volatile uint32_t *)st->h_err = 0;
     return rc;
 }
 
