@@ -179,6 +179,17 @@ inline int tune_unbwt_rate_log2(const Storage *st) { return st->tuning.unbwt_rat
 // ranks.
 inline int tune_parse_key_phrases(const Storage *st) { return st->tuning.parse_key_phrases; }
 
+// Windows in which the first ranks of N sorted positions are written (64 MB of
+// ranks each, see k_round0_ranks), 0: one pass.  Below 1.5 windows the ranks stay in
+// the L2, and so do those of a text's own range where a dictionary keeps `texts`
+// apart; above 20 the reads of all windows cost more than the single pass.
+constexpr uint32_t R0_WINDOW = 1u << 24, R0_MAX_WINDOWS = 20;
+inline uint32_t round0_windows(uint32_t N, uint32_t texts)
+{
+    const uint32_t w = (uint32_t)(((uint64_t)N + R0_WINDOW - 1) / R0_WINDOW);
+    return N / texts > R0_WINDOW + R0_WINDOW / 2u && w <= R0_MAX_WINDOWS ? w : 0u;
+}
+
 inline int bits_for(uint64_t v)   // bits needed to represent values in [0, v]
 {
     int b = 0;

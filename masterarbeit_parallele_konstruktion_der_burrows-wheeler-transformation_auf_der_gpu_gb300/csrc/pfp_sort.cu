@@ -165,8 +165,10 @@ struct LoadHeadActive {
 // kernels, before / after: N = 130 M (512 MiB DNA, W=35) 4.91 / 2.46 ms, 57 M
 // (102 MB of versions) 1.32 / 0.78 ms, 26 M (512 MiB DNA) 0.49 / 0.40 ms; 4096
 // texts kept apart (N = 46 M in small ranges): the call 0.1 ms longer, so not there.
-// Windows of 16, 32, 64, 128 MB at 130 M: 5.83, 3.51, 2.46, 3.27 ms.
-constexpr uint32_t R0_WINDOW = 1u << 24;
+// Windows of 16, 32, 64, 128 MB at 130 M: 5.83, 3.51, 2.46, 3.27 ms.  Every window
+// reads all sorted positions, so the windows' time grows with N^2: random ranks of
+// N = 2^26 .. 2^31 2.2, 5.0, 10.6, 21.8, 44.1, 88.7 ms in one pass and 1.0, 2.7, 8.5, 27.3,
+// 92.2, 328 ms in windows.  They are level at 384 M: see round0_windows.
 __global__ void k_round0_ranks(const uint32_t *vals, uint32_t n, const uint32_t *heads, const uint32_t *active,
                                const uint64_t *pre, uint32_t *isa, uint32_t *sa, uint32_t *act_x, uint32_t *act_g)
 {
@@ -1116,13 +1118,13 @@ static int prefix_doubling(Storage *st, uint32_t N, int key0_bits, uint32_t h0, 
     after_launch(st);
     device_scan<uint64_t, OpMaxAdd>(st, nw, LoadHeadActive{heads, active}, StoreArr<uint64_t>{pre}, false,
                                     (uint64_t *)st->d_scalars);
-    const bool windows = N / texts > R0_WINDOW + R0_WINDOW / 2u;     // a text's ranks stay among themselves
+    const uint32_t windows = round0_windows(N, texts);
     k_round0_ranks<<<grid_for(N, 256), 256, 0, st->stream>>>(vals, N, heads, active, pre, windows ? nullptr : isa, sa,
                                                              act_x, act_g);
     after_launch(st);
-    for (uint64_t lo = 0; windows && lo < N; lo += R0_WINDOW) {
-        k_round0_window<<<grid_for(((size_t)N + 3) / 4, 256), 256, 0, st->stream>>>(vals, N, heads, pre, (uint32_t)lo,
-                                                                                    isa);
+    for (uint32_t i = 0; i < windows; i++) {
+        k_round0_window<<<grid_for(((size_t)N + 3) / 4, 256), 256, 0, st->stream>>>(vals, N, heads, pre,
+                                                                                    i * R0_WINDOW, isa);
         after_launch(st);
     }
     fetch_scalars(st, 1);
