@@ -42,9 +42,10 @@ struct Job {
 };
 
 // Device-memory estimates (bytes) of one pipeline call.  Measured scratch
-// (gbwt_stats.device_bytes) after 512 MiB of repetitive DNA: 14.8 bytes per
-// text byte for one text, 22.5 for a batch of 4096 texts (plus the batch's
-// staged input and output, 2 bytes per byte).
+// (gbwt_stats.device_bytes) after 512 MiB of repetitive DNA: 12.2 bytes per
+// text byte for one text, 14.8 for a batch of 4096 texts (plus the batch's
+// staged input and output, 2 bytes per byte); 22.6 with W=35.  They are no bounds: a
+// text without repetition, whose dictionary is longer than the text, takes 115.
 int64_t est_single(int64_t n) { return 20 * n + ((int64_t)64 << 20); }
 int64_t est_batch(int64_t total, int64_t jobs) { return 28 * total + 64 * jobs + ((int64_t)64 << 20); }
 

@@ -21,12 +21,12 @@ namespace gbwt {
 constexpr int PH_THREADS = 256;
 constexpr int PH_SPAN = 24576;
 constexpr uint64_t M61 = (1ull << 61) - 1ull;
-// A longer run means a table too full to go on.  Linear probing of a table at 0.7
-// of its slots (the limit is 0.75) has runs of about 250 slots; the full-size
-// table is at most half full and gets room to spare, since nothing larger
-// follows it.  When a small table overflows, every thread in flight runs into
-// the dense rest of it before the first CTA reports its count: 102 MB of
-// versions, first attempt 703 -> 329 us with 2048 -> 256.
+// More probes mean a table too full to go on.  Linear probing up to the limit of
+// 0.75 of the slots takes at most 160 to 240 for tables of 2^20 to 2^24 slots (random
+// keys, four runs each); the full-size table is at most half full and gets room
+// to spare, since nothing larger follows it.  When a small table overflows, every
+// thread in flight runs into the dense rest of it before the first CTA reports its
+// count: 102 MB of versions, first attempt 703 -> 329 us with 2048 -> 256.
 constexpr uint32_t PH_PROBES = 2048, PH_PROBES_SMALL = 256;
 constexpr uint32_t PH_FEW = 4096;       // occurrences of a phrase on average: few phrases (DNA copies 10 to 100)
 
