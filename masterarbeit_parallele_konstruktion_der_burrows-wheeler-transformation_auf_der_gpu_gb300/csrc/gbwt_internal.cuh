@@ -200,9 +200,6 @@ inline int bits_for(uint64_t v)   // bits needed to represent values in [0, v]
 // ---------------------------------------------------------------------
 // Device helpers
 // ---------------------------------------------------------------------
-__device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
-__device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
-
 // Text byte with the reference's implicit sentinel: positions n..n+W-1
 // read byte 1 (K:146-149).
 __device__ __forceinline__ uint8_t text_at(const uint8_t *T, uint32_t n, uint32_t i)

@@ -11,9 +11,9 @@
 // Here S comes out of the dictionary suffix order directly: equal suffixes
 // are one group of the prefix-doubling result, named by the sorted position
 // of its first member.  For every group we add the occurrence counts of its
-// phrases (block length) and check whether all preceding bytes agree (run).  Runs are written one group per thread with
-// 16-byte stores (long blocks one CTA each).  For mixed groups, every phrase
-// occurrence -- visited in parse
+// phrases (block length) and check whether all preceding bytes agree (run).
+// Runs are written one group per thread with 16-byte stores (long blocks one CTA
+// each).  For mixed groups, every phrase occurrence -- visited in parse
 // suffix-array order, which is exactly the "rank of the next parse suffix"
 // order the reference sorts by -- emits one (group, byte) element per mixed
 // suffix of its phrase; one stable radix sort by group then places every
@@ -184,10 +184,6 @@ __global__ void k_mix_flags(uint32_t N, PosInfo pi, uint32_t W, const uint32_t *
     const unsigned m = __ballot_sync(0xFFFFFFFFu, set);
     if ((threadIdx.x & 31u) == 0 && x < N) words[x >> 5] = m;
 }
-struct LoadPopc {
-    const uint32_t *w;
-    __device__ __forceinline__ uint32_t operator()(size_t i) const { return (uint32_t)__popc(w[i]); }
-};
 __device__ __forceinline__ uint32_t bits_before(const uint32_t *words, const uint32_t *pre, uint32_t x)
 {
     return pre[x >> 5] + (uint32_t)__popc(words[x >> 5] & ((1u << (x & 31u)) - 1u));

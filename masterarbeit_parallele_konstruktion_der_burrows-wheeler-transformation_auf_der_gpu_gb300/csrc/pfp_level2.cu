@@ -47,7 +47,6 @@ constexpr uint32_t L2_MAXLEN = 4096;
 constexpr uint32_t L2_MIN_Z = 1u << 22;
 constexpr uint32_t L2_DISTINCT = 10;
 constexpr int L2_TABLE_LOG2 = 22;
-constexpr uint64_t L2_M61 = (1ull << 61) - 1ull;
 
 __device__ __forceinline__ bool l2_trigger(uint32_t v)
 {
@@ -77,10 +76,6 @@ __global__ void k_l2_symbols(const uint32_t *pid, const uint32_t *lexrank, const
         if (tstart) tstart[i >> 5] = tm;
     }
 }
-struct LoadTrigWord {
-    const uint32_t *w;
-    __device__ __forceinline__ uint32_t operator()(size_t i) const { return (uint32_t)__popc(w[i]); }
-};
 // s[1 + j] = position of trigger j (s[0] = 0 and s[z2] = z are set apart).
 struct StoreStarts {
     const uint32_t *w;
@@ -111,14 +106,6 @@ struct L2Text {
     }
 };
 
-__device__ __forceinline__ uint64_t l2_mulmod(uint64_t a, uint64_t b)
-{
-    const uint64_t lo = a * b, hi = __umul64hi(a, b);
-    uint64_t r = (lo & L2_M61) + (lo >> 61) + (hi << 3);
-    r = (r & L2_M61) + (r >> 61);
-    return r >= L2_M61 ? r - L2_M61 : r;
-}
-
 // Fingerprint (polynomial mod 2^61 - 1) and table slot of every phrase.
 // give_up: [0] phrase too long or table full, [1] distinct phrases so far,
 // [2] two phrases share a fingerprint.
@@ -136,8 +123,8 @@ __global__ void k_l2_hash(L2Text V, const uint32_t *s, uint32_t z2, uint64_t bas
     }
     uint64_t h = len;
     for (uint32_t i = a; i <= e; i++) {
-        h = l2_mulmod(h, base) + (i < e ? V.inside(i) : V.end(e)) + 1u;
-        if (h >= L2_M61) h -= L2_M61;
+        h = mulmod61(h, base) + (i < e ? V.inside(i) : V.end(e)) + 1u;
+        if (h >= M61) h -= M61;
     }
     const unsigned long long key = h + 1u;                       // 0 marks an empty slot
     const uint32_t cmask = (1u << logc) - 1u;
@@ -382,7 +369,7 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     // positions, more means symbols that hash alike (or tiny texts) and no gain
     const uint32_t cap = z / 3u;
     uint32_t *s = slot<uint32_t>(st, S_2START, (size_t)cap + 2);
-    device_scan<uint32_t, OpAdd>(st, zw, LoadTrigWord{trig}, StoreStarts{trig, s, cap}, false, (uint32_t *)st->d_scalars);
+    device_scan<uint32_t, OpAdd>(st, zw, LoadPopc{trig}, StoreStarts{trig, s, cap}, false, (uint32_t *)st->d_scalars);
     fetch_scalars(st, 1);
     const uint32_t z2 = (uint32_t)st->h_scalars[0] + 1u;
     if (z2 > cap) return false;
@@ -453,7 +440,7 @@ bool run_parse_sa_level2(Storage *st, Phrases &ph, DictOrder &dord, ParseOrder &
     check_cuda(cudaMemsetAsync(bits, 0, nw * 4, st->stream));
     k_l2_heads<<<grid_for(N, 256), 256, 0, st->stream>>>(N, rem8, isa, bits);
     after_launch(st);
-    device_scan<uint32_t, OpAdd>(st, nw, LoadTrigWord{bits}, StoreArr<uint32_t>{pre}, false, (uint32_t *)st->d_scalars);
+    device_scan<uint32_t, OpAdd>(st, nw, LoadPopc{bits}, StoreArr<uint32_t>{pre}, false, (uint32_t *)st->d_scalars);
     k_l2_groups<<<grid_for(N, 256), 256, 0, st->stream>>>(N, rem8, isa, bits, pre, grp);
     after_launch(st);
     // emission and the sort by group

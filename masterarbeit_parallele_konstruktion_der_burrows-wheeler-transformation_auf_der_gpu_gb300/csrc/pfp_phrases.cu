@@ -20,7 +20,6 @@ namespace gbwt {
 
 constexpr int PH_THREADS = 256;
 constexpr int PH_SPAN = 24576;
-constexpr uint64_t M61 = (1ull << 61) - 1ull;
 // More probes mean a table too full to go on.  Linear probing up to the limit of
 // 0.75 of the slots takes at most 160 to 240 for tables of 2^20 to 2^24 slots (random
 // keys, four runs each); the full-size table is at most half full and gets room
@@ -41,14 +40,6 @@ __device__ __forceinline__ void phrase_span(const uint32_t *D, uint32_t k, int W
     if (!k) { start = 0; return; }
     const uint32_t p = D[k - 1];
     start = (xsep && xsep[p] == 1) ? p + 1u : p - (uint32_t)W + 1u;
-}
-
-__device__ __forceinline__ uint64_t mulmod61(uint64_t a, uint64_t b)
-{
-    uint64_t lo = a * b, hi = __umul64hi(a, b);
-    uint64_t r = (lo & M61) + (lo >> 61) + (hi << 3);
-    r = (r & M61) + (r >> 61);
-    return r >= M61 ? r - M61 : r;
 }
 
 // What keeping a batch's texts apart would cost: bytes of the distinct phrases
@@ -298,11 +289,6 @@ __global__ void k_phrase_verify(const uint8_t *T, uint32_t n, const uint32_t *D,
     }
 }
 
-struct LoadU32 {
-    const uint32_t *a;
-    __device__ __forceinline__ uint32_t operator()(size_t i) const { return a[i]; }
-};
-
 // Dense ids in first-occurrence order: id of representative k = prefix.
 struct StoreDense {
     const uint32_t *D;
@@ -326,8 +312,8 @@ struct StoreDense {
     }
 };
 
-// pid per occurrence; occurrence counts and the min/max preceding byte of
-// every distinct phrase.
+// pid per occurrence; occurrence counts and the preceding bytes seen (byte c as
+// c | (~c << 16), OR-ed) of every distinct phrase.
 __global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, int W,
                                   const uint32_t *slot_of, const uint32_t *tdense, uint32_t *pid, uint32_t *pidpc,
                                   uint2 *occpc, bool few, const uint8_t *xsep,
@@ -466,7 +452,7 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
         k_phrase_verify<<<grid_for(z, 256), 256, 0, st->stream>>>(dT, n, ph.D, z, W, tvals, slot_of, isrep,
                                                                   st->d_flags, xsep, pvals, pslot, may_part ? part : nullptr);
         after_launch(st);
-        device_scan<uint32_t, OpAdd>(st, z, LoadU32{isrep}, StoreDense{ph.D, slot_of, tdense, dlen, dstart, W, xsep, ptid, dtid},
+        device_scan<uint32_t, OpAdd>(st, z, LoadArr<uint32_t>{isrep}, StoreDense{ph.D, slot_of, tdense, dlen, dstart, W, xsep, ptid, dtid},
                                      false, st->d_flags + 6);
         check_cuda(cudaMemcpyAsync(st->h_scalars, st->d_flags, 32, cudaMemcpyDeviceToHost, st->stream));
         if (may_part)

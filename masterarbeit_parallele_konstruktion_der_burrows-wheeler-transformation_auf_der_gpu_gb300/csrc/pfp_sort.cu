@@ -1230,14 +1230,6 @@ __global__ void k_mark_phrase_heads(const uint32_t *isa, const uint32_t *doff, u
     const uint32_t p = isa[doff[q]];
     atomicOr(&bits[p >> 5], 1u << (p & 31));
 }
-struct LoadPopc {
-    const uint32_t *bits;
-    __device__ __forceinline__ uint32_t operator()(size_t t) const { return (uint32_t)__popc(bits[t]); }
-};
-struct StoreWordPre {
-    uint32_t *pre;
-    __device__ __forceinline__ void operator()(size_t t, uint32_t p, uint32_t) const { pre[t] = p; }
-};
 __global__ void k_phrase_lexrank(const uint32_t *isa, const uint32_t *doff, uint32_t d, const uint32_t *bits,
                                  const uint32_t *pre, uint32_t *lexrank)
 {
@@ -1256,7 +1248,7 @@ void phrase_ranks(Storage *st, uint32_t N, uint32_t d, const uint32_t *isa, cons
     check_cuda(cudaMemsetAsync(bits, 0, words * sizeof(uint32_t), st->stream));
     k_mark_phrase_heads<<<grid_for(d, 256), 256, 0, st->stream>>>(isa, doff, d, bits);
     after_launch(st);
-    device_scan<uint32_t, OpAdd>(st, words, LoadPopc{bits}, StoreWordPre{pre}, false, (uint32_t *)nullptr);
+    device_scan<uint32_t, OpAdd>(st, words, LoadPopc{bits}, StoreArr<uint32_t>{pre}, false, (uint32_t *)nullptr);
     k_phrase_lexrank<<<grid_for(d, 256), 256, 0, st->stream>>>(isa, doff, d, bits, pre, lexrank);
     after_launch(st);
 }

@@ -64,7 +64,8 @@ constexpr int UB_EXTRA_LOG2 = 3;          // one listed ruler in 2^(rate_log2 + 
 constexpr int UB_LUT_LOG2 = 12;
 
 // Permutation of [0, 2^kb): xor-shifts by at least half the bits undo
-// themselves, odd factors have inverses modulo 2^32.
+// themselves, odd factors have inverses modulo 2^32 (these two: any with mixed bits
+// do).
 constexpr uint32_t UB_MUL1 = 0x2C1B3C6Du, UB_MUL2 = 0x297A2D39u;
 constexpr uint32_t ub_inverse(uint32_t a)
 {

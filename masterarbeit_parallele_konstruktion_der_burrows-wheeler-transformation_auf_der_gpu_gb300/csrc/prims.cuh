@@ -17,14 +17,10 @@ constexpr int SC_THREADS = 256;
 
 // Scan operators.  diff(inc, ex) returns a value v with op(ex, v) == inc:
 // the item itself for sums, the inclusive prefix for maxima (the scan hands
-// stores that v, see k_scan_down).
+// stores that v, see k_scan).
 struct OpAdd {
     template <typename T> __device__ __forceinline__ T operator()(T a, T b) const { return a + b; }
     template <typename T> __device__ __forceinline__ T diff(T inc, T ex) const { return inc - ex; }
-};
-struct OpMax {
-    template <typename T> __device__ __forceinline__ T operator()(T a, T b) const { return a > b ? a : b; }
-    template <typename T> __device__ __forceinline__ T diff(T inc, T) const { return inc; }
 };
 // Component-wise max of the two 32-bit halves of a 64-bit word.
 struct OpMax2 {
@@ -337,6 +333,10 @@ struct LoadArr {
     const T *a;
     __device__ __forceinline__ T operator()(size_t i) const { return a[i]; }
 };
+struct LoadPopc {                      // bits set in a word
+    const uint32_t *w;
+    __device__ __forceinline__ uint32_t operator()(size_t i) const { return (uint32_t)__popc(w[i]); }
+};
 template <typename T>
 struct StoreArr {
     T *a;
@@ -367,6 +367,16 @@ void device_scan(Storage *st, size_t n, Load load, Store store, bool inclusive, 
     if (small) k_scan<T, Op, SMALL><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, store, n, lb, inclusive, total_dev);
     else k_scan<T, Op, BIG><<<(unsigned)tiles, SC_THREADS, 0, st->stream>>>(load, store, n, lb, inclusive, total_dev);
     after_launch(st);
+}
+
+// Product modulo 2^61 - 1 of two values below it (phrase fingerprints).
+constexpr uint64_t M61 = (1ull << 61) - 1ull;
+__device__ __forceinline__ uint64_t mulmod61(uint64_t a, uint64_t b)
+{
+    uint64_t lo = a * b, hi = __umul64hi(a, b);
+    uint64_t r = (lo & M61) + (lo >> 61) + (hi << 3);
+    r = (r & M61) + (r >> 61);
+    return r >= M61 ? r - M61 : r;
 }
 
 // ---------------------------------------------------------------------
