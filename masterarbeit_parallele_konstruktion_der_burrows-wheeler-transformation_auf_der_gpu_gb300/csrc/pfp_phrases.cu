@@ -27,7 +27,6 @@ constexpr int PH_SPAN = 24576;
 // thread in flight runs into the dense rest of it before the first CTA reports its
 // count: 102 MB of versions, first attempt 703 -> 329 us with 2048 -> 256.
 constexpr uint32_t PH_PROBES = 2048, PH_PROBES_SMALL = 256;
-constexpr uint32_t PH_FEW = 4096;       // occurrences of a phrase on average: few phrases (DNA copies 10 to 100)
 
 // Phrase k spans [start, end]: end = D[k]; start = D[k-1]-W+1 (consecutive
 // phrases overlap by W, K:578-592).  In a batch of texts (xsep = the padded
@@ -317,40 +316,59 @@ struct StoreDense {
 
 // pid per occurrence; occurrence counts and the preceding bytes seen (byte c as
 // c | (~c << 16), OR-ed) of every distinct phrase.
-__global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, int W,
+//
+// Two reductions per occurrence: neighbouring occurrences rarely share a phrase,
+// and a match per warp costs more than it saves.  Where they do share one, the
+// reductions meet at one address, 0.6 ns each.  A warp whose 32 occurrences are of
+// one phrase adds once (runs of one byte between others, 16 MiB: the call 20.8 ->
+// 15.6 ms).  FEW: at most PH_FEW phrases of hundreds of occurrences each are counted in
+// shared memory, a CTA many rows of occurrences: 16 MiB of one byte, the call 59.5 ->
+// 36.8 ms (20.8 ms of it were this kernel), 200 texts of random DNA with W = 1, P = 1 (20 M
+// occurrences of 20 phrases) 14.0 -> 7.9 ms.
+constexpr uint32_t PH_FEW = 2048, PH_FEW_OCC = 256;
+template <bool FEW>
+__global__ void k_phrase_finalize(const uint8_t *T, uint32_t n, const uint32_t *D, uint32_t z, uint32_t d, int W,
                                   const uint32_t *slot_of, const uint32_t *tdense, uint32_t *pid, uint32_t *pidpc,
-                                  uint2 *occpc, bool few, const uint8_t *xsep,
-                                  const uint32_t *ptid, const uint8_t *lastb)
+                                  uint2 *occpc, const uint8_t *xsep, const uint32_t *ptid, const uint8_t *lastb)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t id = 0xFFFFFFFFu, seen = 0;
-    if (k < z) {
-        id = tdense[slot_of[k]];
-        pid[k] = id;
-        uint32_t s, e, c;
-        phrase_span(D, k, W, xsep, s, e);
-        // the first phrase of a text is preceded by the text's last byte
-        if (xsep && (k == 0 || xsep[D[k - 1]] == 1)) c = lastb[ptid[k]];
-        else c = preceding_byte(T, n, s);
-        if (pidpc) pidpc[k] = (id << 8) | c;     // only when ids fit 24 bits
-        seen = c | ((c ^ 0xFFu) << 16);
+    __shared__ uint32_t s_occ[FEW ? PH_FEW : 1], s_seen[FEW ? PH_FEW : 1];
+    if constexpr (FEW) {
+        for (uint32_t q = threadIdx.x; q < d; q += blockDim.x) s_occ[q] = s_seen[q] = 0;
+        __syncthreads();
     }
-    // Two reductions per occurrence: neighbouring occurrences rarely share a
-    // phrase, and a match per warp costs more than it saves.  But a run of one
-    // phrase sends them all to one address (0.6 ns each: 16 MiB of one byte
-    // took 20.8 ms, now 0.7), so a warp whose 32 occurrences are of one phrase
-    // adds once.  `few` distinct phrases that alternate share addresses as well: there
-    // a look at the bytes seen saves most of the second reductions (Fibonacci word
-    // of 16 MiB 10.9 -> 8.7 ms; with DNA the look itself costs 1 % of the call).
-    if (__all_sync(0xFFFFFFFFu, id == __shfl_sync(0xFFFFFFFFu, id, 0))) {
-        seen = __reduce_or_sync(0xFFFFFFFFu, seen);
-        if ((threadIdx.x & 31u) == 0 && k < z) {
-            atomicAdd(&occpc[id].x, 32u);
+    // one row of occurrences per CTA, or (FEW) as many as there are
+    for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < z; k0 += gridDim.x * blockDim.x) {
+        const uint32_t k = k0 + threadIdx.x;
+        uint32_t id = 0xFFFFFFFFu, seen = 0;
+        if (k < z) {
+            id = tdense[slot_of[k]];
+            pid[k] = id;
+            uint32_t s, e, c;
+            phrase_span(D, k, W, xsep, s, e);
+            // the first phrase of a text is preceded by the text's last byte
+            if (xsep && (k == 0 || xsep[D[k - 1]] == 1)) c = lastb[ptid[k]];
+            else c = preceding_byte(T, n, s);
+            if (pidpc) pidpc[k] = (id << 8) | c;     // only when ids fit 24 bits
+            seen = c | ((c ^ 0xFFu) << 16);
+        }
+        const bool one = __all_sync(0xFFFFFFFFu, id == __shfl_sync(0xFFFFFFFFu, id, 0));
+        if (one) seen = __reduce_or_sync(0xFFFFFFFFu, seen);
+        if (k >= z || (one && (threadIdx.x & 31u))) continue;
+        if constexpr (FEW) {
+            atomicAdd(&s_occ[id], one ? 32u : 1u);
+            if (seen & ~*(volatile uint32_t *)&s_seen[id]) atomicOr(&s_seen[id], seen);
+        } else {
+            atomicAdd(&occpc[id].x, one ? 32u : 1u);
             atomicOr(&occpc[id].y, seen);
         }
-    } else if (k < z) {
-        if (!few || (seen & ~__ldcg(&occpc[id].y))) atomicOr(&occpc[id].y, seen);
-        atomicAdd(&occpc[id].x, 1u);
+    }
+    if constexpr (FEW) {
+        __syncthreads();
+        for (uint32_t q = threadIdx.x; q < d; q += blockDim.x)
+            if (s_occ[q]) {
+                atomicAdd(&occpc[q].x, s_occ[q]);
+                atomicOr(&occpc[q].y, s_seen[q]);
+            }
     }
 }
 
@@ -481,10 +499,17 @@ void run_phrases(Storage *st, const uint8_t *dT, uint32_t n, int W, Phrases &ph,
     uint2 *occpc = slot<uint2>(st, S_OCC, d);
     check_cuda(cudaMemsetAsync(occpc, 0, (size_t)d * sizeof(uint2), st->stream));
     uint32_t *pidpc = d < (1u << 24) ? slot<uint32_t>(st, S_PIDPC, z) : nullptr;
-    k_phrase_finalize<<<grid_for(z, 256), 256, 0, st->stream>>>(dT, n, ph.D, z, W, slot_of, tdense, pid, pidpc,
-                                                                occpc, z / d >= PH_FEW, xsep,
-                                                                bt ? bt->ptid : nullptr,
-                                                                bt ? bt->lastb : nullptr);
+    const bool few = d <= PH_FEW && z / d >= PH_FEW_OCC;
+    unsigned fgrid = grid_for(z, 256);
+    if (few && fgrid > (unsigned)st->num_sms * 8u) fgrid = (unsigned)st->num_sms * 8u;
+    const uint32_t *ptids = bt ? bt->ptid : nullptr;
+    const uint8_t *lastb = bt ? bt->lastb : nullptr;
+    if (few)
+        k_phrase_finalize<true><<<fgrid, 256, 0, st->stream>>>(dT, n, ph.D, z, d, W, slot_of, tdense, pid, pidpc, occpc,
+                                                                xsep, ptids, lastb);
+    else
+        k_phrase_finalize<false><<<fgrid, 256, 0, st->stream>>>(dT, n, ph.D, z, d, W, slot_of, tdense, pid, pidpc, occpc,
+                                                                 xsep, ptids, lastb);
     ph.pidpc = pidpc;
     after_launch(st);
     // dictionary offsets (64-bit scan, checked against 2^32)
