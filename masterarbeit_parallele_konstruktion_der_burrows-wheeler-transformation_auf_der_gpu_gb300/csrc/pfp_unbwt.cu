@@ -44,13 +44,14 @@
 // In a long run of one symbol, and where the text repeats a short period, LF
 // leads from row to row of one block: 31 of its 32 rulers end at the next row and
 // the last one walks alone through all blocks up to the next ruler block.
-// Tiles that hold one symbol therefore mark one target row in 32 to 256 as a ruler
-// of its own (numbers from `slots` on, rows in a list).  16 MiB of one symbol 2.36 ->
-// 0.53 ms, of period 7 2.26 -> 0.63, half of it zeros 2.02 -> 0.64 (with rulers row
-// by row 1.10, 1.17, 1.27); 128 MiB of one symbol 13.1 -> 2.6 ms (5.6).  Fewer
-// listed rows (an eighth of the rulers' density) than fit such texts best: a text
-// of thousands of copies has such tiles too and its blocks walk well (Fibonacci word
-// of 128 MiB 2.6 -> 3.2 ms, with four times as many 3.5).  DNA has no such tile.
+// Stretches of 1024 rows and more of long runs therefore mark one target row in 32
+// to 256 as a ruler of its own (numbers from `slots` on, rows in a list).  16 MiB of
+// one symbol 2.36 -> 0.53 ms, of period 7 2.26 -> 0.56, half of it zeros 2.02 -> 0.65
+// (with rulers row by row 1.10, 1.17, 1.27); 200 KB of each 0.34, 0.26, 0.39 -> 0.18, 0.18,
+// 0.23 (0.22, 0.21, 0.23); 128 MiB of one symbol 13.1 -> 2.7 ms (5.6).  Fewer listed
+// rows (an eighth of the rulers' density) than fit such texts best: a text of
+// thousands of copies has such stretches too and its blocks walk well (Fibonacci
+// word of 128 MiB 2.6 -> 3.2 ms, with four times as many 3.5).  DNA has none.
 //
 // LF is a permutation, so a walk ends at the latest at its own ruler; the input
 // is a BWT exactly when the cycle of row 0 has all n + 1 rows.
@@ -139,10 +140,11 @@ struct UbIn {
     __device__ __forceinline__ uint32_t row(uint32_t e) const { return p != UB_NIL ? e + 1u : (e < dollar ? e : e + 1u); }
 };
 
-// Symbol counts of every tile (element p left out), digit-major over the tiles;
-// and whether it holds one symbol.
+// Symbol counts of every tile (element p left out), digit-major over the tiles; and
+// for each of its eight parts (512 elements, 16 a thread) whether it holds long
+// runs: at most one thread of the part's warp sees a change of symbol.
 __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__restrict__ tile_hist, uint32_t num_tiles,
-                                                          uint8_t *__restrict__ one_symbol)
+                                                          uint8_t *__restrict__ long_runs)
 {
     constexpr int D = 256;
     __shared__ uint32_t h[RS_WARPS * D];       // one histogram per warp
@@ -150,20 +152,28 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__r
     __syncthreads();
     uint32_t *wh = h + (threadIdx.x >> 5) * D;
     const size_t base = (size_t)blockIdx.x * RS_TILE;
+    bool change = false;
     if (base + RS_TILE <= in.n && (((uintptr_t)in.L) & 15u) == 0) {
         const uint4 v = __ldg((const uint4 *)(in.L + base) + threadIdx.x);       // 16 symbols per thread
         uint8_t kk[16];
         memcpy(kk, &v, 16);
 #pragma unroll
         for (int q = 0; q < 16; q++) atomicAdd(&wh[kk[q]], 1u);
+        change = v.x != __byte_perm(v.x, 0u, 0u) || v.x != v.y || v.x != v.z || v.x != v.w;
     } else {
+        const size_t i0 = base + (size_t)threadIdx.x * RS_ITEMS;
+        uint8_t first = i0 < in.n ? in.L[i0] : 0;
 #pragma unroll 4
-        for (int j = 0; j < RS_ITEMS; j++) {
-            const size_t i = base + (size_t)j * RS_THREADS + threadIdx.x;
-            if (i < in.n) atomicAdd(&wh[in.L[i]], 1u);
-        }
+        for (int j = 0; j < RS_ITEMS; j++)
+            if (i0 + j < in.n) {
+                const uint8_t c = in.L[i0 + j];
+                atomicAdd(&wh[c], 1u);
+                change |= c != first;
+            }
     }
-    if (threadIdx.x == 0) one_symbol[blockIdx.x] = 0;
+    static_assert(RS_ITEMS == 16 && RS_WARPS == 8, "a part is a warp's 16 symbols a thread, a tile has eight");
+    const bool runs = __popc(__ballot_sync(0xFFFFFFFFu, change)) <= 1;
+    if ((threadIdx.x & 31u) == 0) long_runs[(size_t)blockIdx.x * RS_WARPS + (threadIdx.x >> 5)] = runs;
     __syncthreads();
     for (int d = threadIdx.x; d < D; d += RS_THREADS) {
         uint32_t sum = 0;
@@ -171,7 +181,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_byte_hist(UbIn in, uint32_t *__r
         for (int w = 0; w < RS_WARPS; w++) sum += h[w * D + d];
         if (in.p != UB_NIL && in.p >= base && in.p < base + RS_TILE && in.L[in.p] == d) sum--;
         tile_hist[(size_t)d * num_tiles + blockIdx.x] = sum;
-        if (sum + 1u >= (uint32_t)RS_TILE) one_symbol[blockIdx.x] = 1;      // element p may be left out
     }
 }
 
@@ -239,24 +248,28 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t 
     }
 }
 
-// Listed rulers: in tiles of one symbol every target row that is a multiple of
+// Listed rulers: in parts of long runs every target row that is a multiple of
 // 2^extra_log2, numbered with one atomic per tile.  A CTA looks at UB_XTILES
 // tiles.
 constexpr int UB_XTILES = 8;
-__global__ void __launch_bounds__(RS_THREADS) k_lf_extra(UbIn in, const uint8_t *__restrict__ one_symbol,
+__global__ void __launch_bounds__(RS_THREADS) k_lf_extra(UbIn in, const uint64_t *__restrict__ long_runs,
                                                          uint32_t num_tiles, UbRulers ru, uint32_t *LF)
 {
     __shared__ uint32_t s_warp[32], s_first;
     const uint32_t b0 = blockIdx.x * UB_XTILES, b1 = min(b0 + UB_XTILES, num_tiles);
-    const bool set = threadIdx.x < b1 - b0 && one_symbol[b0 + threadIdx.x];
+    const bool set = threadIdx.x < b1 - b0 && long_runs[b0 + threadIdx.x];
     if (!__syncthreads_or(set)) return;
     for (uint32_t b = b0; b < b1; b++) {
-        if (!one_symbol[b]) continue;
+        // a byte each; two neighbours at least (a single one comes up by chance: 64
+        // copies that agree on the symbol before eight contexts in a row)
+        uint64_t parts = long_runs[b];
+        parts &= (parts >> 8) | (parts << 8);
+        if (!parts) continue;
         uint32_t mine = 0, total;
 #pragma unroll
         for (int q = 0; q < RS_ITEMS; q++) {
-            const uint32_t e = b * RS_TILE + q * RS_THREADS + threadIdx.x;
-            if (e >= in.n || e == in.p) continue;
+            const uint32_t i = q * RS_THREADS + threadIdx.x, e = b * RS_TILE + i;
+            if (e >= in.n || e == in.p || !((parts >> (8u * (i / (32 * RS_ITEMS)))) & 1u)) continue;
             const uint32_t v = LF[in.row(e)];
             if (!(v & (UB_RULER | ru.extra_mask))) mine |= 1u << q;
         }
@@ -437,15 +450,15 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     // LF
     const uint32_t num_tiles = (uint32_t)(((size_t)n + RS_TILE - 1) / RS_TILE);
     uint32_t *hist = slot<uint32_t>(st, S_RSHIST, (size_t)256 * num_tiles);
-    uint8_t *one_symbol = slot<uint8_t>(st, S_ACTG, num_tiles);
-    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, one_symbol);
+    uint64_t *long_runs = slot<uint64_t>(st, S_ACTG, num_tiles);
+    k_byte_hist<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, (uint8_t *)long_runs);
     after_launch(st);
     device_scan<uint32_t, OpAdd>(st, (size_t)256 * num_tiles, LoadArr<uint32_t>{hist}, StoreArr<uint32_t>{hist}, false,
                                  (uint32_t *)nullptr);
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
     k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF, st->d_flags);
     after_launch(st);
-    k_lf_extra<<<grid_for(num_tiles, UB_XTILES), RS_THREADS, 0, st->stream>>>(in, one_symbol, num_tiles, ru, LF);
+    k_lf_extra<<<grid_for(num_tiles, UB_XTILES), RS_THREADS, 0, st->stream>>>(in, long_runs, num_tiles, ru, LF);
     after_launch(st);
     uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
     k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);

@@ -74,3 +74,15 @@ def test_tiles_of_one_symbol(storage, pkg, orc, n, runs):
             assert len(storage.unbwt(t, p)) == n
         except pkg.GbwtError as e:
             assert e.code == pkg.BAD_PARAMETER
+
+
+@pytest.mark.parametrize("run", [511, 512, 1023, 1024, 1025, 1536, 4096, 9000])
+@pytest.mark.parametrize("at", [0, 1, 512, 4095, 6001])
+def test_parts_of_long_runs(storage, orc, run, at):
+    rng = np.random.default_rng(run + at)
+    t = rng.integers(2, 6, size=20_000).astype(np.uint8)
+    t[at:at + run] = 9
+    L = orc.sa_bwt(t)
+    assert np.array_equal(storage.unbwt(L, orc.primary_index(t)), t)
+    C, i = storage.libcubwt_bwt(t)
+    assert np.array_equal(storage.libcubwt_unbwt(C, i), t)
