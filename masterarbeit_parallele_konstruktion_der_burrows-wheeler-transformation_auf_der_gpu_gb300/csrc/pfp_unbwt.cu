@@ -249,14 +249,16 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t 
 }
 
 // Listed rulers: in parts of long runs every target row that is a multiple of
-// 2^extra_log2, numbered with one atomic per tile.  A CTA looks at UB_XTILES
-// tiles.
-constexpr int UB_XTILES = 8;
+// 2^extra_log2, numbered with one atomic per tile.  A CTA looks at up to UB_XTILES
+// tiles, one where there are few (a tile of long runs takes 4.5 us: 800 KB of one
+// byte 36 us with eight tiles a CTA, 7 with one; 128 MiB of DNA 5 us with eight, 8 with
+// four).
+constexpr uint32_t UB_XTILES = 8;
 __global__ void __launch_bounds__(RS_THREADS) k_lf_extra(UbIn in, const uint64_t *__restrict__ long_runs,
-                                                         uint32_t num_tiles, UbRulers ru, uint32_t *LF)
+                                                         uint32_t num_tiles, uint32_t per_cta, UbRulers ru, uint32_t *LF)
 {
     __shared__ uint32_t s_warp[32], s_first;
-    const uint32_t b0 = blockIdx.x * UB_XTILES, b1 = min(b0 + UB_XTILES, num_tiles);
+    const uint32_t b0 = blockIdx.x * per_cta, b1 = min(b0 + per_cta, num_tiles);
     const bool set = threadIdx.x < b1 - b0 && long_runs[b0 + threadIdx.x];
     if (!__syncthreads_or(set)) return;
     for (uint32_t b = b0; b < b1; b++) {
@@ -458,7 +460,9 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
     k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF, st->d_flags);
     after_launch(st);
-    k_lf_extra<<<grid_for(num_tiles, UB_XTILES), RS_THREADS, 0, st->stream>>>(in, long_runs, num_tiles, ru, LF);
+    uint32_t xtiles = num_tiles / ((uint32_t)st->num_sms * 8u);
+    xtiles = xtiles < 1u ? 1u : xtiles < UB_XTILES ? xtiles : UB_XTILES;
+    k_lf_extra<<<grid_for(num_tiles, xtiles), RS_THREADS, 0, st->stream>>>(in, long_runs, num_tiles, xtiles, ru, LF);
     after_launch(st);
     uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
     k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);
