@@ -254,10 +254,19 @@ __global__ void __launch_bounds__(RS_THREADS) k_lf_rank(UbIn in, const uint32_t 
 // byte 36 us with eight tiles a CTA, 7 with one; 128 MiB of DNA 5 us with eight, 8 with
 // four).
 constexpr uint32_t UB_XTILES = 8;
+//
+// The first CTA also writes the cumulative symbol counts of all non-'$' rows from
+// the scanned tile histograms (row 0's symbol added back for PFP input).
 __global__ void __launch_bounds__(RS_THREADS) k_lf_extra(UbIn in, const uint64_t *__restrict__ long_runs,
-                                                         uint32_t num_tiles, uint32_t per_cta, UbRulers ru, uint32_t *LF)
+                                                         uint32_t num_tiles, uint32_t per_cta, UbRulers ru, uint32_t *LF,
+                                                         const uint32_t *tile_off, uint32_t *cum)
 {
     __shared__ uint32_t s_warp[32], s_first;
+    if (blockIdx.x == 0) {
+        const uint32_t c = threadIdx.x, c0 = in.p != UB_NIL ? in.L[in.p] : 256u;
+        cum[c] = tile_off[(size_t)c * num_tiles] + (c0 < c ? 1u : 0u);
+        if (c == 0) cum[256] = in.n;
+    }
     const uint32_t b0 = blockIdx.x * per_cta, b1 = min(b0 + per_cta, num_tiles);
     const bool set = threadIdx.x < b1 - b0 && long_runs[b0 + threadIdx.x];
     if (!__syncthreads_or(set)) return;
@@ -413,16 +422,6 @@ __global__ void __launch_bounds__(256) k_walk_emit(const uint32_t *__restrict__ 
     else emit_stretches<false>(LF, ru, off, s_cum, s_lut, lut_shift, n, T);
 }
 
-// Cumulative symbol counts of all non-'$' rows from the scanned tile
-// histograms (row 0's symbol added back for PFP input).
-__global__ void k_unbwt_cum(UbIn in, const uint32_t *tile_off, uint32_t num_tiles, uint32_t *cum)
-{
-    const uint32_t c = threadIdx.x;
-    const uint32_t c0 = in.p != UB_NIL ? in.L[in.p] : 256u;
-    cum[c] = tile_off[(size_t)c * num_tiles] + (c0 < c ? 1u : 0u);
-    if (c == 0) cum[256] = in.n;
-}
-
 // Inverse of the PFP output (p: its primary row, i unused) or of libcubwt's L
 // (p = 0xFFFFFFFF, i its primary index in [1, n]).
 void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t p, uint8_t *dT)
@@ -444,8 +443,9 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     const int extra_log2 = hash.rate_log2 + UB_EXTRA_LOG2;
     const uint32_t extra_cap = (rows >> extra_log2) + 1u, rulers = slots + extra_cap;       // upper bounds
     // 1 MiB of mutated copies 281 us with one in 16, 259 with one in 8 (shorter
-    // hops); 128 MiB 3.26 and 3.28 ms (one round of pointer jumping more)
-    const int super_log2 = rows < (1u << 25) ? 3 : 4;
+    // hops), 3 MB 300 and 280; 22 MiB of versions 703 and 727, 128 MiB of DNA 3.26 and 3.28 ms
+    // (one round of pointer jumping more, over twice the carriers)
+    const int super_log2 = rows < (1u << 23) ? 3 : 4;
     const uint32_t supers = (rulers + (1u << super_log2) - 1u) >> super_log2;
     UbRulers ru{hash, slots, slot<uint32_t>(st, S_ACTX, extra_cap), st->d_flags + 56, extra_cap, (1u << extra_log2) - 1u,
                 super_log2};
@@ -460,12 +460,11 @@ void run_unbwt(Storage *st, const uint8_t *dL, uint32_t n, uint32_t i, uint32_t 
     uint32_t *LF = slot<uint32_t>(st, S_ISA, rows);
     k_lf_rank<<<num_tiles, RS_THREADS, 0, st->stream>>>(in, hist, num_tiles, hash, LF, st->d_flags);
     after_launch(st);
+    uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
     uint32_t xtiles = num_tiles / ((uint32_t)st->num_sms * 8u);
     xtiles = xtiles < 1u ? 1u : xtiles < UB_XTILES ? xtiles : UB_XTILES;
-    k_lf_extra<<<grid_for(num_tiles, xtiles), RS_THREADS, 0, st->stream>>>(in, long_runs, num_tiles, xtiles, ru, LF);
-    after_launch(st);
-    uint32_t *cum = slot<uint32_t>(st, S_TMP2, 257);
-    k_unbwt_cum<<<1, 256, 0, st->stream>>>(in, hist, num_tiles, cum);
+    k_lf_extra<<<grid_for(num_tiles, xtiles), RS_THREADS, 0, st->stream>>>(in, long_runs, num_tiles, xtiles, ru, LF,
+                                                                               hist, cum);
     after_launch(st);
     // walk 1 and list ranking of the ruler chain
     uint32_t *succ = slot<uint32_t>(st, S_TMP0, rulers), *wt = slot<uint32_t>(st, S_TMP1, rulers);
